@@ -12,6 +12,7 @@ workloads (thrust_b200/datagen.py), made on the GPU from the seed.
     run(state)          one call, and everything it produced
     work(case)          bytes that any implementation reads and writes: every input and output once
     tolerance(case)     how far two correct results may be apart
+    exact(case, seed)   the floating-point sums as torch gives them without rounding error, for the cases that have any
 
 The in-place algorithms (sort, sort_by_key, stable_sort_zip, partition) overwrite their input, so a
 pass copies the input into the work buffer first, as a program does that still needs the original.
@@ -249,7 +250,40 @@ def work(case):
 def tolerance(case):
     """Whole numbers, copies and orders are exact.  Sums of floats depend on how they are associated:
     the figures are about four times what the library's sums differ by from sums in twice the precision."""
-    summed = case.get("value") if case["op"] == "reduce_by_key" else case["type"] if case["op"] in ("reduce", "inclusive_scan", "exclusive_scan") else None
-    if summed not in ("f32", "f64") or case.get("fold", "plus") != "plus":
+    summed = _summed(case)
+    if summed is None:
         return "exact"
     return {"rel": 2e-6, "max": 1e-5} if summed == "f32" else {"rel": 1e-14, "max": 1e-13}
+
+
+def _summed(case):
+    """The type in which the case adds floats up, or None."""
+    t = case.get("value") if case["op"] == "reduce_by_key" else case["type"] if case["op"] in ("reduce", "inclusive_scan", "exclusive_scan") else None
+    return t if t in ("f32", "f64") and case.get("fold", "plus") == "plus" else None
+
+
+def _prefix_sums(x):
+    """Inclusive prefix sums of x, whose values lie in [0, 1) on torch.rand's grid (multiples of 2^-24, or of 2^-53
+    for doubles): added up in whole numbers, so that the only rounding is that of the result to 64 bits."""
+    if x.dtype == torch.float32:
+        return torch.cumsum((x.double() * 2.0 ** 24).long(), 0).double() * 2.0 ** -24
+    scaled = (x * 2.0 ** 53).long()
+    high, low = torch.cumsum(scaled >> 27, 0), torch.cumsum(scaled & ((1 << 27) - 1), 0)
+    return high.double() * 2.0 ** -26 + low.double() * 2.0 ** -53
+
+
+def exact(case, seed):
+    """What run() returns, its float sums free of rounding errors; None where nothing is added up in floats
+    (those outputs are whole numbers and copies, which are compared exactly)."""
+    if _summed(case) is None:
+        return None
+    s = prepare(case, seed)
+    if case["op"] == "reduce":
+        return float(_prefix_sums(s["x"])[-1])
+    if case["op"] == "inclusive_scan":
+        return _prefix_sums(s["x"])
+    if case["op"] == "exclusive_scan":
+        return torch.cat([torch.zeros(1, dtype=torch.float64, device="cuda"), _prefix_sums(s["x"])[:-1]])
+    _, lengths = torch.unique_consecutive(s["keys"], return_counts=True)
+    ends = _prefix_sums(s["vals"])[torch.cumsum(lengths, 0) - 1]
+    return None, torch.diff(ends, prepend=torch.zeros(1, dtype=torch.float64, device="cuda"))
