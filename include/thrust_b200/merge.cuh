@@ -1,32 +1,30 @@
 // Merge-path merge and merge sort for sm_100a.
 //
 // merge / merge_by_key (replaces PartitionAgent + MergeAgent of
-// thrust/system/cuda/detail/merge.h:152-660): merge_partition_kernel finds, for every output
-// tile boundary, how many items of range A precede it (binary search along the merge-path
-// diagonal); merge_kernel then loads a tile's slice of A and of B into shared memory with
-// coalesced loads, every thread finds its own start with a second merge-path search in shared
-// memory and merges ITEMS outputs serially, and keys (then payloads, gathered by source index)
-// go back through shared memory so that the stores are coalesced.  Ties take from A first, so
-// the merge is stable.
+// thrust/system/cuda/detail/merge.h:152-660): a first kernel finds, for every output tile boundary, how
+// many items of range A precede it (search along the merge-path diagonal); then every thread of a tile
+// finds its own start with a second merge-path search in shared memory and merges its outputs serially.
+// Ties take from A first, so the merge is stable.  Two kernels do that:
+//   merge_slices_kernel   plain arrays of 4- and 8-byte keys and payloads: bulk copies bring the tile's slices,
+//                         the merge records source positions, keys and payloads are gathered by them;
+//   merge_kernel          any iterators and sizes: loads and results pass through shared memory.
 //
 // merge sort (replaces BlockSortAgent + PartitionAgent + MergeAgent of
 // thrust/system/cuda/detail/sort.h:235-1138): block_sort_kernel sorts each tile (per-thread
 // odd-even transposition network, then log2(BLOCK) rounds of pairwise merge-path merges in
-// shared memory, all stable), and the same two merge kernels run in "pairwise" mode over runs of
+// shared memory, all stable), and the same merge kernels run in "pairwise" mode over runs of
 // doubling length, ping-ponging between the data and a scratch copy.
 #pragma once
+#include "bulk_copy.cuh"
 #include "common.cuh"
 
 namespace tb200 {
 
 constexpr int MERGE_BLOCK = 256;
-// Tunables: items per thread and resident CTAs per SM asked of the compiler (a register cap) for
-// items of up to 8 and up to 12 bytes (key + payload).  The merge kernels are bound by the latency
-// of their barrier-separated phases, not by issue slots or memory, so small tiles and many resident
-// CTAs pay: measured on B200, 11 items per thread at 8 CTAs per SM (32 registers) for 8-byte items
-// and 7 items at 7 CTAs (36 registers) for 12-byte items took a merge pass over 2^26 (u32, f32)
-// pairs from 0.545 to 0.32 ms and merge_by_key of 2 x 2^27 (u64, u32) from 2.16 to 1.79 ms against
-// 15 / 11 items at the compiler's own 58 registers (4 CTAs).  The block sort gains little (5 CTAs).
+// Tunables of merge_kernel: items per thread and resident CTAs per SM asked of the compiler (a register cap)
+// for items of up to 8 and up to 12 bytes (key + payload).  It is bound by the latency of its
+// barrier-separated phases and by the shared-memory pipe, so small tiles and many resident CTAs pay:
+// 15 / 11 items at the compiler's own 58 registers (4 CTAs per SM) took 1.2 to 1.7 times as long.
 #ifndef TB200_MERGE_IPT8
 #define TB200_MERGE_IPT8 11
 #endif
@@ -73,20 +71,14 @@ __host__ __device__ __forceinline__ size_t merge_path(KeyItA a, size_t na, KeyIt
 // Which slices a tile merges.  The output is cut into "pairs": in single mode one pair, A = [0, na)
 // of one array and B = [0, nb) of another; in pairwise mode (merge sort) one array of n items in
 // sorted runs of length `run`, pair p merging runs 2p and 2p+1.  Tiles never straddle a pair:
-// each pair is covered by tiles_per_pair tiles of TILE outputs.
+// each pair is covered by tiles_per_pair tiles of TILE outputs (cut() sets it).
 struct merge_geometry {
   size_t na, nb;          // single mode
   size_t n, run;          // pairwise mode (run == 0 selects single mode)
   size_t tiles_per_pair;
-  template <int TILE> __host__ __device__ static merge_geometry single(size_t na, size_t nb) {
-    merge_geometry g; g.na = na; g.nb = nb; g.n = na + nb; g.run = 0;
-    g.tiles_per_pair = (na + nb + TILE - 1) / TILE; if (g.tiles_per_pair == 0) g.tiles_per_pair = 1;
-    return g;
-  }
-  template <int TILE> __host__ __device__ static merge_geometry pairwise(size_t n, size_t run) {
-    merge_geometry g; g.na = g.nb = 0; g.n = n; g.run = run; g.tiles_per_pair = (2 * run + TILE - 1) / TILE;
-    return g;
-  }
+  static merge_geometry single(size_t na, size_t nb) { merge_geometry g; g.na = na; g.nb = nb; g.n = na + nb; g.run = 0; g.tiles_per_pair = 1; return g; }
+  static merge_geometry pairwise(size_t n, size_t run) { merge_geometry g; g.na = g.nb = 0; g.n = n; g.run = run; g.tiles_per_pair = 1; return g; }
+  void cut(size_t tile) { tiles_per_pair = ((run == 0 ? na + nb : 2 * run) + tile - 1) / tile; if (tiles_per_pair == 0) tiles_per_pair = 1; }
   __host__ __device__ size_t num_tiles() const {
     if (run == 0) return tiles_per_pair;
     return (n + 2 * run - 1) / (2 * run) * tiles_per_pair;
@@ -191,12 +183,185 @@ merge_kernel(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutIt ko, ValOutIt v
   }
 }
 
+// ---------------------------------------------------------------- merge of contiguous arrays
+// The kernel for plain arrays of 4- and 8-byte keys and payloads.  merge_kernel above is bound by the
+// shared-memory pipe: staging stores, the keys' way back through shared memory, three accesses per payload.
+// Here the copy engine brings the four slices (keys and payloads of A and B) into shared memory, the merge
+// leaves only each output's source position there (16 bits; a thread's eight in one 16-byte store), and
+// keys and payloads are gathered by it straight into the coalesced stores: two barriers instead of eight and
+// about half the shared-memory wavefronts.  Measured on B200 against merge_kernel: 2 x 2^27 (u64, u32) 1.46 ms
+// (1.73), (u32, u32) 0.97 ms (1.31), 2 x 4 M (u64, u32) 57 us (84), 2 x 50 k 16 us (22).
+template <int KB, int VB> struct merge_slices_tuning {
+  static constexpr int IPT = 8;                          // source positions of a thread: one 16-byte store
+  static constexpr int TILE = MERGE_BLOCK * IPT;
+  // a slice keeps its distance from a 16-byte boundary, so up to 15 bytes are lost in front of A, behind it and in front of B
+  static constexpr int KEY_BYTES = TILE * KB + 48, VAL_BYTES = VB ? TILE * VB + 48 : 0;
+  static constexpr int MIN_CTAS = KB + VB <= 8 ? 8 : KB + VB <= 12 ? 7 : 6;   // as many as shared memory holds
+};
+
+// Items [0, n) at `src` to the same offsets of `dst`, which has src's distance from a 16-byte boundary: the
+// 16-byte pieces inside by one bulk copy (thread `issuer`; returns its bytes to every caller), the ragged ends
+// by the lanes of one warp.
+template <class T> __device__ __forceinline__ unsigned slice_head(const T* src, unsigned n) {
+  const unsigned h = (unsigned)((16 - (reinterpret_cast<uintptr_t>(src) & 15)) & 15) / sizeof(T);
+  return h < n ? h : n;
+}
+template <class T> __device__ __forceinline__ unsigned slice_bulk_bytes(const T* src, unsigned n) {
+  return (unsigned)((n - slice_head(src, n)) * sizeof(T)) & ~15u;
+}
+template <class T> __device__ __forceinline__ void slice_issue(T* dst, const T* src, unsigned n, unsigned long long* bar, unsigned long long policy) {
+  const unsigned bytes = slice_bulk_bytes(src, n), h = slice_head(src, n);
+  if (bytes) bulk_load(dst + h, src + h, bytes, bar, policy);
+}
+template <class T> __device__ __forceinline__ void slice_ends(T* dst, const T* src, unsigned n) {
+  const unsigned h = slice_head(src, n), t = h + slice_bulk_bytes(src, n) / sizeof(T), lane = lane_id();
+  if (lane < h) dst[lane] = src[lane];
+  if (t + lane < n) dst[t + lane] = src[t + lane];   // fewer than 16 / sizeof(T) items
+}
+
+// First item of A in every tile, by a warp per tile: 32 probes of the diagonal per round trip, so that the
+// search over 2^k items takes k / 5 of them instead of k (a chain of cache misses that small inputs waited for).
+template <class K, class Comp, int TILE>
+__global__ void __launch_bounds__(256)
+merge_split_kernel(const K* ka, const K* kb, merge_geometry g, unsigned num_tiles, Comp comp, size_t* a_split) {
+  const unsigned t = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (t >= num_tiles) return;
+  size_t a0, alen, b0, blen, pair_out, local;
+  g.locate<TILE>(t, a0, alen, b0, blen, pair_out, local);
+  const size_t total = alen + blen, diag = local < total ? local : total;
+  const K* a = ka + a0;
+  const K* b = kb + b0;
+  size_t lo = diag > blen ? diag - blen : 0, hi = diag < alen ? diag : alen;
+  while (lo < hi) {
+    const size_t step = (hi - lo + 31) / 32, mid = lo + lane_id() * step;
+    const unsigned below = __popc(__ballot_sync(FULL_MASK, mid < hi && !comp(b[diag - 1 - mid], a[mid])));   // a prefix of the lanes
+    if (below < 32 && lo + below * step < hi) hi = lo + below * step;
+    if (below) lo += (below - 1) * step + 1;
+  }
+  if (lane_id() == 0) a_split[t] = a0 + lo;
+}
+
+template <class K, class V, bool HAS_V, class Comp>
+__global__ void __launch_bounds__(MERGE_BLOCK, (merge_slices_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>::MIN_CTAS))
+merge_slices_kernel(const K* ka, const K* kb, const V* va, const V* vb, K* ko, V* vo, merge_geometry g, Comp comp, const size_t* a_split, unsigned* err) {
+  using Tuning = merge_slices_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>;
+  constexpr int IPT = Tuning::IPT, TILE = Tuning::TILE;
+  __shared__ __align__(16) unsigned char s_keys[Tuning::KEY_BYTES];
+  __shared__ __align__(16) unsigned char s_vals[HAS_V ? Tuning::VAL_BYTES : 16];
+  __shared__ __align__(16) unsigned short s_src[TILE];
+  __shared__ unsigned long long bars[2];               // the keys' slices have arrived, the payloads'
+  const unsigned t = blockIdx.x;
+  size_t a0p, alen, b0p, blen, pair_out, local;
+  g.locate<TILE>(t, a0p, alen, b0p, blen, pair_out, local);
+  const size_t pair_total = alen + blen;
+  if (local >= pair_total) return;                     // a short last pair leaves its later tiles empty
+  const unsigned tile_n = pair_total - local < TILE ? (unsigned)(pair_total - local) : (unsigned)TILE;
+  const size_t a_begin = a_split[t];
+  const size_t a_end = local + TILE < pair_total ? a_split[t + 1] : a0p + alen;
+  const size_t b_begin = b0p + local - (a_begin - a0p);
+  const unsigned na = (unsigned)(a_end - a_begin), nb = tile_n - na;
+  auto phase = [](const void* p) { return (unsigned)(reinterpret_cast<uintptr_t>(p) & 15); };
+
+  // ---- the slices' places: A first, B behind it on the next 16-byte boundary, each shifted by its phase
+  const unsigned ka_at = phase(ka + a_begin), kb_at = ((ka_at + na * (unsigned)sizeof(K) + 15) & ~15u) + phase(kb + b_begin);
+  K* const sk_a = reinterpret_cast<K*>(s_keys + ka_at);
+  K* const sk_b = reinterpret_cast<K*>(s_keys + kb_at);
+  V* sv_a = nullptr;
+  V* sv_b = nullptr;
+  if constexpr (HAS_V) {
+    const unsigned va_at = phase(va + a_begin), vb_at = ((va_at + na * (unsigned)sizeof(V) + 15) & ~15u) + phase(vb + b_begin);
+    sv_a = reinterpret_cast<V*>(s_vals + va_at);
+    sv_b = reinterpret_cast<V*>(s_vals + vb_at);
+  }
+  if (threadIdx.x == 0) {
+    mbar_init(&bars[0], 1);
+    if (HAS_V) mbar_init(&bars[1], 1);
+    mbar_init_fence();
+    const unsigned long long policy = l2_stream_policy();
+    mbar_arrive_expect(&bars[0], slice_bulk_bytes(ka + a_begin, na) + slice_bulk_bytes(kb + b_begin, nb));
+    slice_issue(sk_a, ka + a_begin, na, &bars[0], policy);
+    slice_issue(sk_b, kb + b_begin, nb, &bars[0], policy);
+    if constexpr (HAS_V) {
+      mbar_arrive_expect(&bars[1], slice_bulk_bytes(va + a_begin, na) + slice_bulk_bytes(vb + b_begin, nb));
+      slice_issue(sv_a, va + a_begin, na, &bars[1], policy);
+      slice_issue(sv_b, vb + b_begin, nb, &bars[1], policy);
+    }
+  }
+  const int warp = threadIdx.x >> 5;
+  if (warp == 1) slice_ends(sk_a, ka + a_begin, na);
+  if (warp == 2) slice_ends(sk_b, kb + b_begin, nb);
+  if constexpr (HAS_V) {
+    if (warp == 3) slice_ends(sv_a, va + a_begin, na);
+    if (warp == 4) slice_ends(sv_b, vb + b_begin, nb);
+  }
+  __syncthreads();
+  auto wait = [&](unsigned long long* bar) {
+    for (unsigned iter = 0; !mbar_try_wait(bar, 0); ++iter)
+      if (iter > MBAR_SPIN_LIMIT) { record_error(err, ERR_LOOKBACK_TIMEOUT); break; }
+  };
+  wait(&bars[0]);
+
+  // ---- per-thread merge path, then a serial merge that records where each output comes from
+  unsigned d0 = threadIdx.x * IPT; if (d0 > tile_n) d0 = tile_n;
+  unsigned ai, bi;
+  {
+    unsigned lo = d0 > nb ? d0 - nb : 0, hi = d0 < na ? d0 : na;
+    while (lo < hi) {
+      const unsigned mid = (lo + hi) >> 1;
+      if (!comp(sk_b[d0 - 1 - mid], sk_a[mid])) lo = mid + 1; else hi = mid;
+    }
+    ai = lo; bi = d0 - lo;
+  }
+  unsigned packed[IPT / 2];
+  // the candidates stay in registers; only the side that was taken is read again (never past its slice's end)
+  K key_a = K(), key_b = K();
+  if (ai < na) key_a = sk_a[ai];
+  if (bi < nb) key_b = sk_b[bi];
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) {
+    const bool take_b = bi < nb && (ai >= na || comp(key_b, key_a));
+    const unsigned src = take_b ? na + bi : ai;
+    if (i & 1) packed[i / 2] |= src << 16; else packed[i / 2] = src;
+    if (take_b) { ++bi; if (bi < nb) key_b = sk_b[bi]; }
+    else { ++ai; if (ai < na) key_a = sk_a[ai]; }
+  }
+  *reinterpret_cast<uint4*>(s_src + threadIdx.x * IPT) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+  if constexpr (HAS_V) wait(&bars[1]);
+  __syncthreads();
+
+  // ---- consecutive threads on consecutive outputs
+  const size_t out0 = pair_out + local;
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) {
+    const unsigned c = threadIdx.x + i * MERGE_BLOCK;
+    if (c < tile_n) {
+      const unsigned src = s_src[c];
+      const bool from_b = src >= na;
+      ko[out0 + c] = from_b ? sk_b[src - na] : sk_a[src];
+      if constexpr (HAS_V) vo[out0 + c] = from_b ? sv_b[src - na] : sv_a[src];
+    }
+  }
+}
+
+// Whether merge_slices_kernel may serve a call: plain arrays of the key and payload types.
+template <class T> struct merge_slice_type { static constexpr bool value = std::is_trivially_copyable<T>::value && (sizeof(T) == 4 || sizeof(T) == 8) && alignof(T) == sizeof(T); };
+template <class It, class T> struct is_array_of : std::false_type {};
+template <class T> struct is_array_of<T*, T> : std::true_type {};
+template <class T> struct is_array_of<const T*, T> : std::true_type {};
+template <class K, class V, bool HAS_V, class KeyItA, class KeyItB, class ValItA, class ValItB, class KeyOutIt, class ValOutIt> struct merge_slices_ok {
+  static constexpr bool keys = merge_slice_type<K>::value && is_array_of<KeyItA, K>::value && is_array_of<KeyItB, K>::value && is_array_of<KeyOutIt, K>::value;
+  static constexpr bool vals = !HAS_V || (merge_slice_type<V>::value && is_array_of<ValItA, V>::value && is_array_of<ValItB, V>::value && is_array_of<ValOutIt, V>::value);
+  static constexpr bool value = keys && vals;
+};
+
 template <class K, class V, bool HAS_V> constexpr int merge_tile_items() { return MERGE_BLOCK * merge_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>::IPT; }
 
 template <class K, class V, bool HAS_V> size_t merge_workspace_bytes(size_t total) {
   // pairwise passes round every pair up to whole tiles: at most one extra tile per pair, and a pair
   // is never smaller than a block-sort tile, so 2x the single-mode tile count is a safe bound
-  size_t tiles = (total + merge_tile_items<K, V, HAS_V>() - 1) / merge_tile_items<K, V, HAS_V>();
+  constexpr size_t slices = merge_slices_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>::TILE, items = merge_tile_items<K, V, HAS_V>();
+  constexpr size_t tile = slices < items ? slices : items;   // either kernel may run
+  size_t tiles = (total + tile - 1) / tile;
   return sizeof(ws_header) + align_up((4 * tiles + 8) * sizeof(size_t), 256);
 }
 
@@ -207,13 +372,24 @@ cudaError_t merge_pass_async(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutI
   constexpr int IPT = merge_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>::IPT;
   constexpr int TILE = MERGE_BLOCK * IPT;
   if (g.n == 0) return cudaSuccess;
-  const size_t tiles = g.num_tiles();
   size_t* a_split = reinterpret_cast<size_t*>(static_cast<char*>(ws) + sizeof(ws_header));
+  if constexpr (merge_slices_ok<K, V, HAS_V, KeyItA, KeyItB, ValItA, ValItB, KeyOutIt, ValOutIt>::value) {
+    using Tuning = merge_slices_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>;
+    g.cut(Tuning::TILE);
+    const unsigned tiles = (unsigned)g.num_tiles();
+    merge_split_kernel<K, Comp, Tuning::TILE><<<(tiles + 7) / 8, 256, 0, stream>>>(ka, kb, g, tiles, comp, a_split);
+    timed_launch tl(KID_MERGE, stream);
+    merge_slices_kernel<K, V, HAS_V, Comp><<<tiles, MERGE_BLOCK, 0, stream>>>(ka, kb, va, vb, ko, vo, g, comp, a_split, &static_cast<ws_header*>(ws)->error);
+    return cudaGetLastError();
+  } else {
+  g.cut(TILE);
+  const size_t tiles = g.num_tiles();
   merge_partition_kernel<KeyItA, KeyItB, Comp, TILE><<<(unsigned)((tiles + 255) / 256), 256, 0, stream>>>(ka, kb, g, tiles, comp, a_split);
   timed_launch tl(KID_MERGE, stream);
   merge_kernel<KeyItA, KeyItB, ValItA, ValItB, KeyOutIt, ValOutIt, K, V, HAS_V, Comp, IPT>
       <<<(unsigned)tiles, MERGE_BLOCK, 0, stream>>>(ka, kb, va, vb, ko, vo, g, comp, a_split);
   return cudaGetLastError();
+  }
 }
 
 // thrust::merge / merge_by_key: A[0,na) and B[0,nb) sorted by comp -> out[0, na+nb).
@@ -222,8 +398,7 @@ cudaError_t merge_async(KeyItA ka, size_t na, KeyItB kb, size_t nb, ValItA va, V
                         cudaStream_t stream) {
   cudaError_t e = cudaMemsetAsync(ws, 0, sizeof(ws_header), stream);
   if (e != cudaSuccess) return e;
-  constexpr int TILE = merge_tile_items<K, V, HAS_V>();
-  return merge_pass_async<K, V, HAS_V>(ka, kb, va, vb, ko, vo, merge_geometry::single<TILE>(na, nb), comp, ws, stream);
+  return merge_pass_async<K, V, HAS_V>(ka, kb, va, vb, ko, vo, merge_geometry::single(na, nb), comp, ws, stream);
 }
 
 // ---------------------------------------------------------------- merge sort
@@ -353,9 +528,8 @@ cudaError_t merge_sort_async(K* keys, K* keys_alt, V* vals, V* vals_alt, size_t 
   block_sort_kernel<const K*, const V*, K*, V*, K, V, HAS_V, Comp, BS_IPT><<<(unsigned)tiles, MERGE_BLOCK, 0, stream>>>(keys, vals, cur_k, cur_v, n, comp); }
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   for (size_t run = BS_TILE; run < n; run <<= 1) {
-    constexpr int TILE = merge_tile_items<K, V, HAS_V>();
     e = merge_pass_async<K, V, HAS_V>((const K*)cur_k, (const K*)cur_k, (const V*)cur_v, (const V*)cur_v, oth_k, oth_v,
-                                      merge_geometry::pairwise<TILE>(n, run), comp, ws, stream);
+                                      merge_geometry::pairwise(n, run), comp, ws, stream);
     if (e != cudaSuccess) return e;
     K* tk = cur_k; cur_k = oth_k; oth_k = tk;
     V* tv = cur_v; cur_v = oth_v; oth_v = tv;

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from thrust_b200 import datagen as dg
-from gpu_util import dev, host, rand_of
+from gpu_util import dev, host, misaligned, rand_of
 
 pytestmark = pytest.mark.gpu
 KEY_TYPES = [np.int32, np.uint32, np.float32, np.int64, np.uint64, np.float64]
@@ -91,3 +91,18 @@ def test_merge_runs_tree(tb, port, num_runs):
     ws = api._call_with_ws("merge", "tb200_merge_runs", kp, vp, cn, num_runs, api._ptr(ko), api._ptr(vo), api._ptr(kt), api._ptr(vt), 5, 4, 0)
     api._sync_and_check(ws, "merge_runs")
     assert np.array_equal(host(ko), wk) and np.array_equal(host(vo), wv)
+
+
+@pytest.mark.parametrize("shift", [(0, 1), (1, 0), (3, 2), (1, 3)])
+@pytest.mark.parametrize("n", [1, 5, 1023, 2047, 2048, 2049, 6151])
+def test_merge_of_slices_at_any_alignment(tb, port, shift, n):
+    """Inputs that start anywhere between two 16-byte boundaries, tiles of 2048 outputs and their remainders."""
+    for dt, vt in [(np.uint32, np.uint32), (np.uint64, np.uint32), (np.uint32, np.uint64), (np.float64, np.uint64)]:
+        a, _ = port.sort_by_key(rand_of(dt, n, 91, small=True), None, False)
+        b, _ = port.sort_by_key(rand_of(dt, n // 2 + 1, 92), None, False)
+        va, vb = np.arange(a.size, dtype=vt), np.arange(b.size, dtype=vt) + vt(1 << 30)
+        args = [misaligned(x, (s * (q + 1)) % 4) for q, (x, s) in enumerate([(a, shift[0]), (b, shift[1]), (va, shift[1]), (vb, shift[0])])]
+        ko, vo = tb.merge_by_key(*args)
+        rk, rv = port.merge_by_key(a, b, va, vb)
+        assert np.array_equal(host(ko), rk) and np.array_equal(host(vo), rv), (dt, vt)
+        assert np.array_equal(host(tb.merge(args[0], args[1])), rk), dt

@@ -76,7 +76,6 @@ int merge_runs_typed(const void* const* run_keys, const void* const* run_vals, c
     }
     return 0;
   }
-  constexpr int TILE = tb200::merge_tile_items<K, V, HAS_V>();
   for (int level = 1; level <= levels; ++level) {
     K* dk = static_cast<K*>(((levels - level) % 2 == 0) ? out_k : tmp_k);
     V* dv = static_cast<V*>(((levels - level) % 2 == 0) ? out_v : tmp_v);
@@ -87,10 +86,10 @@ int merge_runs_typed(const void* const* run_keys, const void* const* run_vals, c
         const size_t na = cn[i], nb = cn[i + 1];
         if (na + nb) {
           if (descending)
-            e = tb200::merge_pass_async<K, V, HAS_V>(ck[i], ck[i + 1], cv[i], cv[i + 1], dk + off, dv + (HAS_V ? off : 0), tb200::merge_geometry::single<TILE>(na, nb),
+            e = tb200::merge_pass_async<K, V, HAS_V>(ck[i], ck[i + 1], cv[i], cv[i + 1], dk + off, dv + (HAS_V ? off : 0), tb200::merge_geometry::single(na, nb),
                                                    tb200::greater_op(), d_ws, stream);
           else
-            e = tb200::merge_pass_async<K, V, HAS_V>(ck[i], ck[i + 1], cv[i], cv[i + 1], dk + off, dv + (HAS_V ? off : 0), tb200::merge_geometry::single<TILE>(na, nb),
+            e = tb200::merge_pass_async<K, V, HAS_V>(ck[i], ck[i + 1], cv[i], cv[i + 1], dk + off, dv + (HAS_V ? off : 0), tb200::merge_geometry::single(na, nb),
                                                    tb200::less_op(), d_ws, stream);
           if (e != cudaSuccess) return (int)e;
         }
