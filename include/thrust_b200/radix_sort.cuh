@@ -22,17 +22,14 @@
 //   4. radix_copy_back_kernel only if an odd number of places ran: moves the result from the
 //                             alternate buffer to the caller's.
 // A pass therefore reads and writes each key (and value) exactly once.  The sort is stable.
-// Key order is defined on an unsigned code of the key: unsigned keys unchanged, signed keys
-// with the sign bit flipped, IEEE floats with all bits flipped when negative and the sign bit
-// flipped otherwise (the encoders of thrust/system/detail/sequential/stable_radix_sort.inl:54-138);
-// descending order complements the code.
+// Inputs of up to 128 k items take one launch of one thread-block cluster instead (cluster_sort.cuh).
 #pragma once
+#include "cluster_sort.cuh"
 #include "common.cuh"
+#include "radix_keys.cuh"
 
 namespace tb200 {
 
-constexpr int RADIX_BITS = 8;
-constexpr int RADIX_BINS = 256;
 constexpr int RADIX_MAX_PASSES = 8;
 #ifndef TB200_SWEEP_BLOCK
 #define TB200_SWEEP_BLOCK 512
@@ -40,30 +37,6 @@ constexpr int RADIX_MAX_PASSES = 8;
 constexpr int ONESWEEP_BLOCK = TB200_SWEEP_BLOCK;
 constexpr int ONESWEEP_CTAS_PER_SM = 1024 / ONESWEEP_BLOCK;
 constexpr int HIST_BLOCK = 1024;
-
-enum key_kind : int { KEY_UNSIGNED = 0, KEY_SIGNED = 1, KEY_FLOAT = 2 };
-
-struct key_coding {
-  int kind; int descending;
-};
-
-// Digit `shift / 8` of the key's order-preserving unsigned code.  For integer keys the code
-// differs from the raw bits by a constant, so the digit is the raw byte XOR `dmask` (the matching
-// byte of that constant); float keys first flip all bits of negative values.
-template <class UK> __host__ __device__ __forceinline__ unsigned digit_mask(key_coding c, int shift) {
-  constexpr int B = 8 * sizeof(UK);
-  UK m = c.descending ? (UK)~(UK)0 : (UK)0;
-  if (c.kind != KEY_UNSIGNED) m ^= (UK)1 << (B - 1);
-  return (unsigned)(m >> shift) & 0xffu;
-}
-template <bool IS_FLOAT, class UK> __device__ __forceinline__ unsigned key_digit(UK k, int shift, unsigned dmask) {
-  constexpr int B = 8 * sizeof(UK);
-  if (IS_FLOAT) {
-    using SK = typename std::make_signed<UK>::type;
-    k ^= (UK)((SK)k >> (B - 1)) & (UK)~((UK)1 << (B - 1));   // negative: flip the non-sign bits too
-  }
-  return ((unsigned)(k >> shift) & 0xffu) ^ dmask;
-}
 
 // Control block in the workspace, after ws_header.
 struct radix_ctrl {
@@ -790,6 +763,12 @@ cudaError_t radix_sort_async(UK* keys_a, UK* keys_b, UV* vals_a, UV* vals_b, siz
   const size_t lb_bytes = align_up(sweep_tiles_of<KB, VB>(n) * RADIX_BINS * (lb32 ? 4 : 8), 256);
   char* base = static_cast<char*>(ws);
   ws_header* hdr = reinterpret_cast<ws_header*>(base);
+  // small inputs: one launch of one cluster
+  {
+    bool launched = false;
+    const cudaError_t ce = cluster_sort_async<UK, UV, HAS_V>(keys_a, vals_a, n, coding, first_pass, num_passes, hdr, stream, launched);
+    if (launched || ce != cudaSuccess) return ce;
+  }
   radix_ctrl* ctrl = reinterpret_cast<radix_ctrl*>(base + sizeof(ws_header));
   char* lb0 = base + sizeof(ws_header) + sizeof(radix_ctrl);
   cudaError_t e = cudaMemsetAsync(base, 0, (size_t)(lb0 - base) + lb_bytes * num_passes, stream);

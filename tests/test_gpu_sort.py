@@ -50,6 +50,26 @@ def test_sort_all_key_types_orders_and_payloads(tb, port):
                 assert np.array_equal(host(kd), ok) and np.array_equal(host(vd), ov), (dt, vt, desc)
 
 
+@pytest.mark.parametrize("n", [2, 31, 2047, 2048, 2049, 8191, 16385, 32767, 32769, 65535, 65537, 100003, 131071, 131072, 131073])
+def test_small_sorts_at_the_edges_of_the_cluster(tb, port, n):
+    """Inputs that one thread-block cluster sorts: where its CTA count, rows per warp and last row change, with
+    keys alone, 4- and 8-byte pairs, few distinct keys, one key, and a window of the bits."""
+    for dt, vt in [(np.float32, None), (np.uint32, np.uint32), (np.int64, np.uint32), (np.float64, np.uint64), (np.uint8, np.uint64)]:
+        for small in (False, True):
+            k = rand_of(dt, n, 57, small=small)
+            v = None if vt is None else np.arange(n, dtype=vt)
+            for desc in (False, True):
+                kd, vd = dev(k), None if v is None else dev(v)
+                tb.sort(kd, desc) if v is None else tb.sort_by_key(kd, vd, desc)
+                ok, ov = port.sort_by_key(k, v, desc)
+                assert np.array_equal(host(kd), ok) and (v is None or np.array_equal(host(vd), ov)), (dt, vt, small, desc)
+    k, v = dg.sort_keys_u32(n), np.arange(n, dtype=np.uint32)
+    kd, vd = dev(k), dev(v)
+    tb.sort_by_key(kd, vd, begin_bit=8, end_bit=24)
+    order = np.argsort((k >> 8) & 0xFFFF, kind="stable")
+    assert np.array_equal(host(vd), v[order]) and np.array_equal(host(kd), k[order])
+
+
 def test_sort_special_values(tb, port):
     k = np.array([3.5, -0.0, 0.0, -1e30, np.inf, -np.inf, 1e-40, -1e-40, 2.0, -2.0], np.float32)
     k = np.concatenate([k, rand_of(np.float32, 5000, 53)])
