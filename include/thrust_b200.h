@@ -49,6 +49,12 @@ int tb200_sm_arch(void);
  * cuda_cub::throw_on_error (thrust/system/cuda/detail/util.h:180-243). */
 int tb200_workspace_status(const void* d_ws, tb200_stream_t stream, unsigned* h_status);
 
+/* Synchronises `stream` and copies the first `bytes` (at most 256) of a workspace's header to h_dst, in one
+ * transfer through pinned memory: bytes 0-3 the status word above, bytes 8-15 the count that the selecting and
+ * counting entry points leave there.  Bytes 32-255 are free for a caller's own small results once a call has been
+ * enqueued: tb200_reduce may be given d_ws + 32 as its d_out. */
+int tb200_workspace_read(const void* d_ws, size_t bytes, void* h_dst, tb200_stream_t stream);
+
 /* thrust::reduce(first, last, init, op) -- thrust/system/cuda/detail/reduce.h:1015-1067
  * (cuda_cub::reduce_n).  Accumulates in acc_t, the type of *h_init; each input element is
  * converted to acc_t first.  Result: one acc_t at d_out.  n == 0 stores init.

@@ -8,6 +8,7 @@ used only to own device memory and to name the stream.  Every call goes through
 libthrust_b200.so; there is no fallback path.
 """
 import ctypes as C
+import struct
 
 import numpy as np
 import torch
@@ -38,11 +39,15 @@ def _check(rc, what):
 
 
 def _ptr(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
+
+
+# the raw handle of a device's current stream, without building a torch.cuda.Stream around it where torch offers that
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda dev: torch.cuda.current_stream(dev).cuda_stream)
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _require_cuda(*tensors):
@@ -58,8 +63,17 @@ class _Workspaces:
     def __init__(self):
         self._bufs = {}
 
+    @staticmethod
+    def _key(tag):
+        dev = torch.cuda.current_device()
+        return dev, _raw_stream(dev), tag
+
+    def kept(self, tag):
+        """The buffer kept for this call site on the current stream, whatever its size, or None."""
+        return self._bufs.get(self._key(tag))
+
     def get(self, tag, nbytes):
-        key = (torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream, tag)
+        key = self._key(tag)
         buf = self._bufs.get(key)
         if buf is None or buf.numel() < nbytes:
             buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device="cuda")
@@ -73,22 +87,50 @@ class _Workspaces:
 workspaces = _Workspaces()
 
 
+_TOO_SMALL = 1      # cudaErrorInvalidValue: the workspace is too small (or another argument is wrong)
+
+
 def _call_with_ws(tag, fn, *args):
-    """fn(*args, d_ws, &ws_bytes, stream): size query, then the real call.  Returns the workspace."""
+    """fn(*args, d_ws, &ws_bytes, stream) in the workspace kept for the call site; the size is asked for only if
+    there is none yet or it is refused as too small.  Returns the workspace."""
     lib_fn = getattr(_lib.load(), fn)
+    stream = _stream()
+    ws = workspaces.kept(tag)
+    if ws is not None:
+        rc = lib_fn(*args, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream)
+        if rc != _TOO_SMALL:
+            _check(rc, fn)
+            return ws
     need = C.c_size_t(0)
-    _check(lib_fn(*args, None, C.byref(need), _stream()), fn + " (size query)")
+    _check(lib_fn(*args, None, C.byref(need), stream), fn + " (size query)")
     ws = workspaces.get(tag, need.value)
-    have = C.c_size_t(ws.numel())
-    _check(lib_fn(*args, _ptr(ws), C.byref(have), _stream()), fn)
+    _check(lib_fn(*args, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream), fn)
     return ws
 
 
+# the workspace header (ws_header in common.cuh): status, ticket, count, ..., and room that a result may use
+_HEADER = struct.Struct("<IIQ")
+_HEADER_RESULT = 32
+
+
+def _read_header(ws, what, nbytes=_HEADER.size):
+    """Waits for the stream, then the first `nbytes` of the workspace's header in one copy; raises if the
+    kernels reported a wait that ran out."""
+    head = C.create_string_buffer(nbytes)
+    _check(_lib.load().tb200_workspace_read(ws.data_ptr(), nbytes, head, _stream()), what + " (result)")
+    status = _HEADER.unpack_from(head)[0]
+    if status != 0:
+        raise Tb200Error("%s: device reported status %d (an inter-CTA wait ran out)" % (what, status))
+    return head
+
+
 def _sync_and_check(ws, what):
-    status = C.c_uint(0)
-    _check(_lib.load().tb200_workspace_status(_ptr(ws), _stream(), C.byref(status)), what + " (status)")
-    if status.value != 0:
-        raise Tb200Error("%s: device reported status %d (an inter-CTA wait ran out)" % (what, status.value))
+    _read_header(ws, what)
+
+
+def _sync_and_count(ws, what):
+    """The same for calls that select or count: the number that the kernels left in the header."""
+    return _HEADER.unpack_from(_read_header(ws, what))[2]
 
 
 # ------------------------------------------------------------------------------------- reduce
@@ -99,11 +141,22 @@ def reduce(x, init=None, op="plus", acc_dtype=None):
     if acc_dtype is None:
         acc_dtype = x.dtype if init is None or not isinstance(init, np.generic) else TORCH_OF[np.dtype(init.dtype)]
     h_init = np.asarray(0 if init is None else init, dtype=NP_OF[acc_dtype])
-    out = torch.empty(1, dtype=acc_dtype, device=x.device)
-    ws = _call_with_ws("reduce", "tb200_reduce", _ptr(x), x.numel(), DTYPE_CODE[x.dtype], DTYPE_CODE[acc_dtype],
-                       OPS[op], C.c_void_p(h_init.ctypes.data), _ptr(out))
-    _sync_and_check(ws, "reduce")
-    return out.cpu().numpy().view(NP_OF[acc_dtype])[0]
+    # the result lands in the workspace's header and comes back together with the status
+    lib_fn = _lib.load().tb200_reduce
+    stream = _stream()
+    args = (_ptr(x), x.numel(), DTYPE_CODE[x.dtype], DTYPE_CODE[acc_dtype], OPS[op], h_init.ctypes.data)
+    ws = workspaces.kept("reduce")
+    rc = _TOO_SMALL
+    if ws is not None:
+        rc = lib_fn(*args, ws.data_ptr() + _HEADER_RESULT, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream)
+    if rc == _TOO_SMALL:
+        need = C.c_size_t(0)
+        _check(lib_fn(*args, None, None, C.byref(need), stream), "tb200_reduce (size query)")
+        ws = workspaces.get("reduce", need.value)
+        rc = lib_fn(*args, ws.data_ptr() + _HEADER_RESULT, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream)
+    _check(rc, "tb200_reduce")
+    head = _read_header(ws, "reduce", _HEADER_RESULT + 8)
+    return np.frombuffer(head.raw, dtype=NP_OF[acc_dtype], count=1, offset=_HEADER_RESULT)[0]
 
 
 def reduce_to_device(x, init, op="plus", acc_dtype=None, out=None):
@@ -114,7 +167,7 @@ def reduce_to_device(x, init, op="plus", acc_dtype=None, out=None):
     h_init = np.asarray(init, dtype=NP_OF[acc_dtype])
     out = torch.empty(1, dtype=acc_dtype, device=x.device) if out is None else out
     _call_with_ws("reduce", "tb200_reduce", _ptr(x), x.numel(), DTYPE_CODE[x.dtype], DTYPE_CODE[acc_dtype], OPS[op],
-                  C.c_void_p(h_init.ctypes.data), _ptr(out))
+                  h_init.ctypes.data, _ptr(out))
     return out
 
 
@@ -130,7 +183,7 @@ def inclusive_scan(x, out=None, op="plus", init=None, sync=True):
     else:
         h_init = None if init is None else np.asarray(init, dtype=NP_OF[x.dtype])
         ws = _call_with_ws("scan", "tb200_inclusive_scan", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], OPS[op],
-                           None if h_init is None else C.c_void_p(h_init.ctypes.data))
+                           None if h_init is None else h_init.ctypes.data)
     if sync:
         _sync_and_check(ws, "inclusive_scan")
     return out
@@ -145,7 +198,7 @@ def exclusive_scan(x, init=0, out=None, op="plus", sync=True):
     else:
         h_init = np.asarray(init, dtype=NP_OF[x.dtype])
         ws = _call_with_ws("scan", "tb200_exclusive_scan", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], OPS[op],
-                           C.c_void_p(h_init.ctypes.data))
+                           h_init.ctypes.data)
     if sync:
         _sync_and_check(ws, "exclusive_scan")
     return out
@@ -237,34 +290,22 @@ def sort_by_key_host(h_keys, h_vals, h_keys_out=None, h_vals_out=None, descendin
 
 
 # ------------------------------------------------------------------------------------- compaction
-def _count_word():
-    return torch.zeros(1, dtype=torch.int64, device="cuda")
-
-
-def _read_count(cnt):
-    return int(cnt.cpu().item())
-
-
 def copy_if(x, pred, a=0, b=0, stencil=None, out=None):
     """thrust::copy_if(first, last, [stencil,] result, pred): returns out[:count] (stable)."""
     _require_cuda(x, stencil, out)
     out = torch.empty_like(x) if out is None else out
-    cnt = _count_word()
     ws = _call_with_ws("select", "tb200_copy_if", _ptr(x), _ptr(stencil), _ptr(out), x.numel(), DTYPE_CODE[x.dtype],
-                       0 if stencil is None else DTYPE_CODE[stencil.dtype], PREDS[pred], a, b, _ptr(cnt))
-    _sync_and_check(ws, "copy_if")
-    return out[:_read_count(cnt)]
+                       0 if stencil is None else DTYPE_CODE[stencil.dtype], PREDS[pred], a, b, None)
+    return out[:_sync_and_count(ws, "copy_if")]
 
 
 def partition_copy(x, pred, a=0, b=0, stencil=None):
     """thrust::stable_partition_copy: returns (selected, rejected), both in input order."""
     _require_cuda(x, stencil)
     out_t, out_f = torch.empty_like(x), torch.empty_like(x)
-    cnt = _count_word()
     ws = _call_with_ws("select", "tb200_partition_copy", _ptr(x), _ptr(stencil), _ptr(out_t), _ptr(out_f), x.numel(),
-                       DTYPE_CODE[x.dtype], 0 if stencil is None else DTYPE_CODE[stencil.dtype], PREDS[pred], a, b, _ptr(cnt))
-    _sync_and_check(ws, "partition_copy")
-    k = _read_count(cnt)
+                       DTYPE_CODE[x.dtype], 0 if stencil is None else DTYPE_CODE[stencil.dtype], PREDS[pred], a, b, None)
+    k = _sync_and_count(ws, "partition_copy")
     return out_t[:k], out_f[:x.numel() - k]
 
 
@@ -274,10 +315,8 @@ stable_partition_copy = partition_copy
 def partition(x, pred, a=0, b=0):
     """thrust::partition / thrust::stable_partition in place; returns the split point."""
     _require_cuda(x)
-    cnt = _count_word()
-    ws = _call_with_ws("partition", "tb200_partition", _ptr(x), x.numel(), DTYPE_CODE[x.dtype], PREDS[pred], a, b, _ptr(cnt))
-    _sync_and_check(ws, "partition")
-    return _read_count(cnt)
+    ws = _call_with_ws("partition", "tb200_partition", _ptr(x), x.numel(), DTYPE_CODE[x.dtype], PREDS[pred], a, b, None)
+    return _sync_and_count(ws, "partition")
 
 
 stable_partition = partition
@@ -287,10 +326,8 @@ def unique_copy(x, out=None):
     """thrust::unique_copy(first, last, result): returns out[:count]."""
     _require_cuda(x, out)
     out = torch.empty_like(x) if out is None else out
-    cnt = _count_word()
-    ws = _call_with_ws("select", "tb200_unique_copy", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], _ptr(cnt))
-    _sync_and_check(ws, "unique_copy")
-    return out[:_read_count(cnt)]
+    ws = _call_with_ws("select", "tb200_unique_copy", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], None)
+    return out[:_sync_and_count(ws, "unique_copy")]
 
 
 def unique(x):
@@ -303,11 +340,9 @@ def reduce_by_key(keys, vals, op="plus"):
     returns (keys_out[:runs], values_out[:runs])."""
     _require_cuda(keys, vals)
     ko, vo = torch.empty_like(keys), torch.empty_like(vals)
-    cnt = _count_word()
     ws = _call_with_ws("rbk", "tb200_reduce_by_key", _ptr(keys), _ptr(vals), _ptr(ko), _ptr(vo), keys.numel(),
-                       DTYPE_CODE[keys.dtype], DTYPE_CODE[vals.dtype], OPS[op], _ptr(cnt))
-    _sync_and_check(ws, "reduce_by_key")
-    k = _read_count(cnt)
+                       DTYPE_CODE[keys.dtype], DTYPE_CODE[vals.dtype], OPS[op], None)
+    k = _sync_and_count(ws, "reduce_by_key")
     return ko[:k], vo[:k]
 
 
@@ -327,7 +362,7 @@ def exclusive_scan_by_key(keys, vals, init=0, out=None, op="plus"):
     out = torch.empty_like(vals) if out is None else out
     h_init = np.asarray(init, dtype=NP_OF[vals.dtype])
     ws = _call_with_ws("rbk", "tb200_scan_by_key", _ptr(keys), _ptr(vals), _ptr(out), keys.numel(), DTYPE_CODE[keys.dtype],
-                       DTYPE_CODE[vals.dtype], OPS[op], 1, C.c_void_p(h_init.ctypes.data))
+                       DTYPE_CODE[vals.dtype], OPS[op], 1, h_init.ctypes.data)
     _sync_and_check(ws, "exclusive_scan_by_key")
     return out
 
@@ -337,11 +372,9 @@ def unique_by_key_copy(keys, vals, keys_out=None, vals_out=None):
     _require_cuda(keys, vals, keys_out, vals_out)
     ko = torch.empty_like(keys) if keys_out is None else keys_out
     vo = torch.empty_like(vals) if vals_out is None else vals_out
-    cnt = _count_word()
     ws = _call_with_ws("rbk", "tb200_unique_by_key_copy", _ptr(keys), _ptr(vals), _ptr(ko), _ptr(vo), keys.numel(),
-                       DTYPE_CODE[keys.dtype], vals.element_size(), _ptr(cnt))
-    _sync_and_check(ws, "unique_by_key_copy")
-    k = _read_count(cnt)
+                       DTYPE_CODE[keys.dtype], vals.element_size(), None)
+    k = _sync_and_count(ws, "unique_by_key_copy")
     return ko[:k], vo[:k]
 
 
@@ -415,11 +448,9 @@ def set_operation(op, keys_a, keys_b, vals_a=None, vals_b=None, descending=False
     ko = torch.empty(cap, dtype=keys_a.dtype, device=keys_a.device)
     vo = None if vals_a is None else torch.empty(cap, dtype=vals_a.dtype, device=keys_a.device)
     vb = 0 if vals_a is None else vals_a.element_size()
-    cnt = _count_word()
     ws = _call_with_ws("setop", "tb200_set_operation", code, _ptr(keys_a), na, _ptr(keys_b), nb, _ptr(vals_a), _ptr(vals_b), _ptr(ko), _ptr(vo),
-                       DTYPE_CODE[keys_a.dtype], vb, int(descending), _ptr(cnt))
-    _sync_and_check(ws, "set_" + op)
-    m = _read_count(cnt)
+                       DTYPE_CODE[keys_a.dtype], vb, int(descending), None)
+    m = _sync_and_count(ws, "set_" + op)
     return ko[:m], (None if vo is None else vo[:m])
 
 

@@ -1,4 +1,4 @@
-// C ABI: tb200_reduce, tb200_version, tb200_sm_arch, tb200_workspace_status.
+// C ABI: tb200_reduce, tb200_version, tb200_sm_arch, tb200_workspace_status, tb200_workspace_read.
 #include "abi_common.cuh"
 #include "thrust_b200/reduce.cuh"
 
@@ -12,6 +12,27 @@ TB200_API int tb200_workspace_status(const void* d_ws, tb200_stream_t stream, un
   cudaError_t e = cudaMemcpyAsync(h_status, d_ws, sizeof(unsigned), cudaMemcpyDeviceToHost, stream);
   if (e != cudaSuccess) return (int)e;
   return (int)cudaStreamSynchronize(stream);
+}
+
+namespace {
+
+// One pinned header's worth per host thread: a read-back into pageable memory is staged by the driver first.
+struct pinned_header {
+  void* p = nullptr;
+  void* get() { if (!p && cudaHostAlloc(&p, sizeof(tb200::ws_header), cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); p = nullptr; } return p; }
+  ~pinned_header() { if (p) cudaFreeHost(p); }
+};
+
+}  // namespace
+
+TB200_API int tb200_workspace_read(const void* d_ws, size_t bytes, void* h_dst, tb200_stream_t stream) {
+  if (!d_ws || !h_dst || bytes > sizeof(tb200::ws_header)) return ERR_INVALID;
+  static thread_local pinned_header pinned;
+  void* const via = pinned.get();
+  cudaError_t e = cudaMemcpyAsync(via ? via : h_dst, d_ws, bytes, cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  if (e == cudaSuccess && via) memcpy(h_dst, via, bytes);
+  return (int)e;
 }
 
 namespace {
