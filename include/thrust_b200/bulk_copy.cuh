@@ -23,6 +23,12 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned 
                : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity), "r"(1000u) : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ bool mbar_test(unsigned long long* bar, unsigned parity) {   // never suspends
+  unsigned ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
+  return ok != 0;
+}
 // global -> shared, evict-first in L2; both addresses and the size are multiples of 16 bytes
 __device__ __forceinline__ unsigned long long l2_stream_policy() {
   unsigned long long pol;

@@ -73,6 +73,41 @@ def test_scan_chunked_route_bit_exact(tb, oracles, dt):
         assert np.array_equal(mx, o.inclusive_scan(x, "max"))
 
 
+@pytest.mark.parametrize("items", [1 << 20, (1 << 20) + 1, 148 * 8192 - 1, 148 * 8192, 148 * 8192 + 1, 2 * 148 * 8192 + 8191, 7 * 148 * 8192 + 4097])
+def test_scan_pipeline_edges(tb, port, items):
+    """Around the size where the pipeline starts, at whole and ragged rounds of 148 tiles of 32 KB; fp32 sums are
+    within 25 roundings (the additions on the way of one element) of the exact ones."""
+    for dt in (np.int32, np.uint32, np.int64, np.float32, np.float64):
+        n = items * 4 // np.dtype(dt).itemsize
+        x = dg.scan_input_f32(n) if dt == np.float32 else dg.scan_input_i32(n).astype(dt)
+        for op, init in (("plus", 3), ("max", 0), ("min", 0)):
+            incl, excl = host(tb.inclusive_scan(dev(x), op=op)), host(tb.exclusive_scan(dev(x), init, op=op))
+            if dt == np.float32 and op == "plus":
+                want = np.cumsum(x.astype(np.float64))
+                assert np.all(np.abs(incl - want) <= 25 * 2.0 ** -24 * want) and excl[0] == init
+                assert np.all(np.abs(excl[1:] - (want[:-1] + init)) <= 26 * 2.0 ** -24 * (want[:-1] + init))
+            else:
+                assert np.array_equal(incl, port.inclusive_scan(x, op)), (dt, op)
+                assert np.array_equal(excl, port.exclusive_scan(x, np.asarray(init, dt)[()], op)), (dt, op)
+
+
+def test_scan_pipeline_float_extremes(tb):
+    """Infinities pass through the sums, signed zeros through their identity, and the smallest float is no absent value."""
+    n = (1 << 21) + 5
+    z = torch.full((n,), -0.0, device="cuda")
+    assert bool(torch.signbit(tb.inclusive_scan(z)).all())
+    for dt in (torch.float32, torch.float64):
+        x = torch.ones(n, device="cuda", dtype=dt)
+        x[n // 2] = float("inf")
+        s = tb.inclusive_scan(x)
+        assert bool(torch.isinf(s[n // 2:]).all()) and float(s[n // 2 - 1]) == n // 2
+        x[n // 2 + 1] = float("-inf")
+        s = tb.inclusive_scan(x)
+        assert bool(torch.isnan(s[n // 2 + 1:]).all()) and float(s[n // 2 - 1]) == n // 2
+    low = torch.full((1 << 23,), torch.finfo(torch.float32).min, device="cuda")
+    assert torch.equal(tb.inclusive_scan(low, op="max"), low) and torch.equal(tb.inclusive_scan(-low, op="min"), -low)
+
+
 def test_scan_in_place_and_misaligned(tb, port):
     x = dg.scan_input_i32(100001)
     d = dev(x)
