@@ -1,5 +1,5 @@
 // Two-pass reduce_by_key for large contiguous inputs on sm_100a (keys and values of the same size,
-// 4 or 8 bytes), in the manner of select_stream.cuh: no thread waits for another warp.
+// 4 or 8 bytes): no thread waits for another warp.
 //
 // The input is cut into batches of RBK_STREAM_ROWS rows of 32 lanes x 16 bytes; consecutive warps of
 // the grid take consecutive batches.  A batch is summarised by the pair
@@ -19,9 +19,58 @@
 #pragma once
 #include "common.cuh"
 #include "scan.cuh"
-#include "select_stream.cuh"
 
 namespace tb200 {
+
+// This lane's VEC items of row `row` (32 lanes x VEC items); items past the end read as T().
+// FULL: the caller knows that the row lies wholly inside the input (no bounds checks at all).
+template <class T, int VEC, bool FULL = false>
+__device__ __forceinline__ void select_row_load(const T* in, size_t n, size_t row, int lane, T (&x)[VEC]) {
+  const size_t i0 = (row * 32 + lane) * VEC;
+  if (FULL || (row + 1) * 32 * VEC <= n) {
+    vec16 r = load_stream16(reinterpret_cast<const char*>(in) + i0 * sizeof(T));
+    const T* e = reinterpret_cast<const T*>(&r);
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) x[k] = e[k];
+  } else {
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) x[k] = i0 + k < n ? in[i0 + k] : T();
+  }
+}
+
+// Shared by both passes: this lane's keep bits for the items x of row `row`.  `prev_tail` carries
+// the last item of the previous row for SEL_UNIQUE-style predicates.
+template <bool UNIQUE, class T, class Pred, int VEC, bool FULL = false>
+__device__ __forceinline__ unsigned select_row_flags(size_t n, size_t row, int lane, Pred pred, const T (&x)[VEC], T& prev_tail, bool& have_prev) {
+  const size_t i0 = (row * 32 + lane) * VEC;
+  const bool row_full = FULL || (row + 1) * 32 * VEC <= n;
+  unsigned bits = 0;
+  if constexpr (UNIQUE) {
+    // predecessor of this lane's first item: the previous lane's last item, or the previous row's
+    T prev = shfl_up(x[VEC - 1], 1);
+    bool has = true;
+    if (lane == 0) { prev = prev_tail; has = have_prev; }
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) {
+      const bool head = (k == 0 && !has) ? true : !pred(k == 0 ? prev : x[k - 1], x[k]);
+      if ((row_full || i0 + k < n) && head) bits |= 1u << k;
+    }
+    prev_tail = shfl_idx(x[VEC - 1], 31);
+    have_prev = true;
+  } else {
+#pragma unroll
+    for (int k = 0; k < VEC; ++k)
+      if ((row_full || i0 + k < n) && pred(x[k])) bits |= 1u << k;
+  }
+  return bits;
+}
+
+// predecessor of a batch's first item, for SEL_UNIQUE-style predicates
+template <class T> __device__ __forceinline__ void select_batch_start(const T* in, size_t first_row, int vec, T& prev_tail, bool& have_prev) {
+  have_prev = first_row > 0;
+  prev_tail = have_prev ? in[first_row * 32 * vec - 1] : T();
+}
+
 
 constexpr int RBK_STREAM_BLOCK = 256;
 // Measured on B200, 2^28 int32 keys + fp32 values, runs of mean length 4: 1.24 ms with two rows per batch

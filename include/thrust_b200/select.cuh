@@ -1,7 +1,7 @@
 // Stream compaction for sm_100a: copy_if (with or without a stencil), partition, partition_copy and
 // unique / unique_copy.  This file holds the single-pass kernel that serves every case (any iterator,
 // stencils, in-place forms, small and medium inputs) and the dispatch; large contiguous inputs whose
-// outputs do not overlap them go to the two-pass streaming kernels of select_stream.cuh.
+// outputs do not overlap them, and the large in-place partition, go to the tile pipeline (select_pipe.cuh).
 //
 // Single pass:
 // One CTA per tile (dynamic ticket).  A tile loads its items with the same lane-interleaved
@@ -19,7 +19,7 @@
 // restores input order; so partition here is always the stable one.
 #pragma once
 #include "common.cuh"
-#include "select_stream.cuh"
+#include "select_pipe.cuh"
 
 namespace tb200 {
 
@@ -165,38 +165,57 @@ partition_finish_kernel(OutIt data, const T* scratch, size_t n, const ws_header*
 template <class T> constexpr size_t select_tile_items() { return (size_t)SELECT_BLOCK * select_tuning<T>::IPT; }
 template <class T> size_t select_workspace_bytes(size_t n) {
   size_t tiles = (n + select_tile_items<T>() - 1) / select_tile_items<T>();
-  const size_t single = sizeof(ws_header) + tile_state<unsigned long long>::bytes(tiles + 1);   // large enough for either offset width
-  const size_t stream = select_stream_workspace_bytes<T>(n);
-  return single > stream ? single : stream;
+  // large enough for either offset width; the pipeline's tiles of 4- and 8-byte items are the same size and so are its descriptors
+  return sizeof(ws_header) + tile_state<unsigned long long>::bytes(tiles + 1);
+}
+
+// Where the pipeline starts.  2^20 int32 selected 13.3 us against 14.3 single-pass, 2^18 12.0 against 11.4; with the
+// dropped items written too 2^20 14.9 against 17.6, 2^18 12.3 against 15.1.
+constexpr size_t SELECT_PIPE_MIN_BYTES = (size_t)1 << 22;
+constexpr size_t SELECT_PIPE_MIN_BYTES_REJECTS = (size_t)1 << 20;
+
+// Whether the pipeline may serve a call: a large, 16-byte aligned input and outputs that do not overlap it
+// (out_rej: null if
+// there is no second one).  rejects: dropped items are written too.
+inline bool select_pipe_eligible(const void* in, const void* out_sel, const void* out_rej, size_t n, size_t item_bytes, bool rejects) {
+  const char* ib = static_cast<const char*>(in);
+  const char* ob = static_cast<const char*>(out_sel);
+  const char* rb = static_cast<const char*>(out_rej);
+  const size_t bytes = n * item_bytes;
+  if (bytes < (rejects ? SELECT_PIPE_MIN_BYTES_REJECTS : SELECT_PIPE_MIN_BYTES) || (reinterpret_cast<uintptr_t>(in) & 15) != 0) return false;
+  if (ob < ib + bytes && ib < ob + bytes) return false;
+  return !rb || rb >= ib + bytes || ib >= rb + bytes;
 }
 
 // Launches the compaction; no sync.  The number of kept items goes to the workspace header and,
 // if d_count != nullptr, to *d_count.
-// ALLOW_STREAM = false keeps a caller that has already tried select_stream_async itself from
-// instantiating those kernels a second time.
-template <int MODE, bool KEEP_REJECTS, bool ALLOW_STREAM = true, class InIt, class StIt, class SelIt, class RejIt, class T, class Pred>
+// ALLOW_PIPE = false keeps a caller that has already tried select_pipe_launch itself from
+// instantiating its kernel a second time.
+template <int MODE, bool KEEP_REJECTS, bool ALLOW_PIPE = true, class InIt, class StIt, class SelIt, class RejIt, class T, class Pred>
 cudaError_t select_async(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, size_t n, T /*type tag*/, Pred pred, bool mirrored,
                          unsigned long long* d_count, void* ws, cudaStream_t stream) {
   char* base = static_cast<char*>(ws);
   ws_header* hdr = reinterpret_cast<ws_header*>(base);
   constexpr int IPT = select_tuning<T>::IPT;
   const size_t tiles = (n + select_tile_items<T>() - 1) / select_tile_items<T>();
-  // large contiguous inputs whose outputs are plain arrays that do not overlap the input: the
-  // two-pass streaming kernels (select_stream.cuh)
-  if constexpr (ALLOW_STREAM && MODE != SEL_STENCIL && std::is_pointer<InIt>::value && std::is_pointer<SelIt>::value && std::is_arithmetic<T>::value &&
+  // large contiguous inputs whose outputs are plain arrays that do not overlap the input: the pipeline
+  if constexpr (ALLOW_PIPE && MODE != SEL_STENCIL && std::is_pointer<InIt>::value && std::is_pointer<SelIt>::value && std::is_arithmetic<T>::value &&
                 (sizeof(T) == 4 || sizeof(T) == 8) && (!KEEP_REJECTS || std::is_pointer<RejIt>::value)) {
     using In = typename std::remove_cv<typename std::remove_pointer<InIt>::type>::type;
     using Sel = typename std::remove_pointer<SelIt>::type;
     if constexpr (std::is_same<In, T>::value && std::is_same<Sel, T>::value) {
-      bool ok = true;
+      bool ok = !mirrored;
       T* rej = nullptr;
       if constexpr (KEEP_REJECTS) {
         using Rej = typename std::remove_pointer<RejIt>::type;
         if constexpr (std::is_same<Rej, T>::value) rej = out_rej; else ok = false;
+        ok = ok && rej != nullptr;
       }
-      if (ok && select_stream_eligible(in, out_sel, rej, KEEP_REJECTS && !mirrored, n, sizeof(T)))
-        return select_stream_async<MODE == SEL_UNIQUE, KEEP_REJECTS, T, Pred>(in, out_sel, rej, n, pred, mirrored ? SELECT_REJ_MIRRORED : SELECT_REJ_SECOND_ARRAY, d_count, ws,
-                                                                              stream);
+      if (ok && select_pipe_eligible(in, out_sel, rej, n, sizeof(T), KEEP_REJECTS)) {
+        bool launched = false;
+        const cudaError_t pe = select_pipe_launch<MODE == SEL_UNIQUE, KEEP_REJECTS ? SELECT_SECOND_ARRAY : SELECT_DROP, T, Pred>(in, out_sel, rej, n, pred, d_count, ws, stream, launched);
+        if (launched || pe != cudaSuccess) return pe;
+      }
     }
   }
   cudaError_t e = cudaMemsetAsync(base, 0, sizeof(ws_header) + tile_state<unsigned long long>::bytes(tiles + 1), stream);
@@ -235,21 +254,27 @@ cudaError_t partition_finish_async(T* data, const T* scratch, size_t n, const vo
   return cudaGetLastError();
 }
 
-// The in-place partition through the streaming kernels only (the caller has checked
-// select_stream_eligible()): they know the number of kept items before they scatter, so the dropped
-// items land behind the kept ones in input order and the way back is a plain copy.
+// The in-place partition on the pipeline (select_pipe.cuh): kept items straight to their places in `data`, dropped
+// ones through `scratch`.
 template <class T, class Pred>
-cudaError_t partition_inplace_stream_async(T* data, T* scratch, size_t n, Pred pred, unsigned long long* d_count, void* ws, cudaStream_t stream) {
-cudaError_t e = select_stream_async<false, true, T, Pred>((const T*)data, scratch, (T*)nullptr, n, pred, SELECT_REJ_BEHIND_SELECTED, d_count, ws, stream);
-  if (e != cudaSuccess) return e;
-  return cudaMemcpyAsync(data, scratch, n * sizeof(T), cudaMemcpyDeviceToDevice, stream);
+cudaError_t partition_inplace_pipe_async(T* data, T* scratch, size_t n, Pred pred, unsigned long long* d_count, void* ws, cudaStream_t stream, bool& launched) {
+  cudaError_t e = select_pipe_launch<false, SELECT_SECOND_ARRAY, T, Pred>((const T*)data, data, scratch, n, pred, d_count, ws, stream, launched);
+  if (e != cudaSuccess || !launched) return e;
+  size_t grid = (n + 256 * 16 - 1) / (256 * 16);
+  if (grid > (size_t)current_device_info().sm_count * 8) grid = (size_t)current_device_info().sm_count * 8;
+  partition_rejects_kernel<T><<<(unsigned)grid, 256, 0, stream>>>(data, scratch, n, reinterpret_cast<const ws_header*>(ws));
+  return cudaGetLastError();
 }
 
 // In-place stable partition of data[0, n): `scratch` holds n items.
-template <bool ALLOW_STREAM = true, class T, class Pred>
+template <bool ALLOW_PIPE = true, class T, class Pred>
 cudaError_t partition_inplace_async(T* data, T* scratch, size_t n, Pred pred, unsigned long long* d_count, void* ws, cudaStream_t stream) {
-  if constexpr (ALLOW_STREAM && std::is_arithmetic<T>::value && (sizeof(T) == 4 || sizeof(T) == 8)) {
-    if (select_stream_eligible(data, scratch, nullptr, false, n, sizeof(T))) return partition_inplace_stream_async(data, scratch, n, pred, d_count, ws, stream);
+  if constexpr (ALLOW_PIPE && std::is_arithmetic<T>::value && (sizeof(T) == 4 || sizeof(T) == 8)) {
+    if (select_pipe_eligible(data, scratch, nullptr, n, sizeof(T), true)) {
+      bool launched = false;
+      const cudaError_t pe = partition_inplace_pipe_async(data, scratch, n, pred, d_count, ws, stream, launched);
+      if (launched || pe != cudaSuccess) return pe;
+    }
   }
   cudaError_t e = select_async<SEL_PRED, true, false>((const T*)data, (const T*)nullptr, scratch, (T*)nullptr, n, T(), pred, true, d_count, ws, stream);
   if (e != cudaSuccess || n == 0) return e;

@@ -209,3 +209,24 @@ def test_full_size_reduce_by_key_fp32(tb):
         yard.index_add_(0, keys[lo:lo + step].long(), vals[lo:lo + step].double())
     err = (gv.double() - yard).abs() / yard.clamp(min=1e-30)
     assert float(err.max()) < 1e-6, float(err.max())
+
+
+@pytest.mark.parametrize("items", [1 << 18, (1 << 20) - 1, (1 << 20) + 1, 148 * 8192, 148 * 8192 + 1, 3 * 148 * 8192 + 4099])
+def test_compaction_pipeline_edges(tb, port, items):
+    """Around the sizes where the pipeline starts, whole and ragged rounds of 148 tiles, nothing / few / half / all kept, and
+    outputs that start off a 16-byte boundary."""
+    for dt in (np.int32, np.int64, np.float32):
+        n = items * 4 // np.dtype(dt).itemsize
+        x = (dg.rand64(61, n) % np.uint64(1 << 20)).astype(dt)
+        for bound in (0, 1 << 10, 1 << 19, 1 << 20):
+            want = port.copy_if(x, "lt", bound, 0)
+            out = misaligned(np.zeros(n, dt), 1)
+            assert np.array_equal(host(tb.copy_if(dev(x), "lt", bound, 0, out=out)), want), (dt, bound)
+            sel, rej = tb.partition_copy(dev(x), "lt", bound, 0)
+            assert np.array_equal(host(sel), want) and np.array_equal(host(rej), x[x >= bound]), (dt, bound)
+            d = dev(x)
+            assert tb.partition(d, "lt", bound, 0) == want.size
+            assert np.array_equal(host(d), np.concatenate([want, x[x >= bound]])), (dt, bound)
+        for run in (1, 3, 1000, n + 1):
+            r = (np.arange(n) // run).astype(dt)
+            assert np.array_equal(host(tb.unique_copy(dev(r))), port.unique_copy(r)), (dt, run)

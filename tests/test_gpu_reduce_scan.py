@@ -1,6 +1,7 @@
 """Parity of the CUDA reduce and scan (through the C ABI) with the CPU oracle."""
 import numpy as np
 import pytest
+import torch
 
 from thrust_b200 import datagen as dg
 from gpu_util import EDGE_SIZES, WIDE, dev, host, misaligned, rand_of

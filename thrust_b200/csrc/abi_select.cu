@@ -14,12 +14,16 @@ int select_pred(const void* in, const void* stencil, int stencil_t, void* out_se
   T* os = static_cast<T*>(out_sel);
   T* orj = static_cast<T*>(out_rej);
   if (!stencil) {
-    // large inputs: the streaming kernels, compiled per predicate kind
+    // large inputs: the pipeline, compiled per predicate kind
     if constexpr (sizeof(T) == 4 || sizeof(T) == 8) {
-      if (tb200::select_stream_eligible(in, out_sel, out_rej, REJ, n, sizeof(T)))
-        return pred.visit([&](auto typed) {
-          return (int)tb200::select_stream_async<false, REJ, T, decltype(typed)>(i, os, orj, n, typed, false, d_count, d_ws, stream);
+      if (tb200::select_pipe_eligible(in, out_sel, REJ ? out_rej : nullptr, n, sizeof(T), REJ)) {
+        bool launched = false;
+        const int rc = pred.visit([&](auto typed) {
+          return (int)tb200::select_pipe_launch<false, REJ ? tb200::SELECT_SECOND_ARRAY : tb200::SELECT_DROP, T, decltype(typed)>(i, os, orj, n, typed, d_count, d_ws,
+                                                                                                                                stream, launched);
         });
+        if (launched || rc != 0) return rc;
+      }
     }
     return (int)tb200::select_async<tb200::SEL_PRED, REJ, false>(i, (const T*)nullptr, os, orj, n, T(), pred, false, d_count, d_ws, stream);
   }
