@@ -230,3 +230,17 @@ def test_compaction_pipeline_edges(tb, port, items):
         for run in (1, 3, 1000, n + 1):
             r = (np.arange(n) // run).astype(dt)
             assert np.array_equal(host(tb.unique_copy(dev(r))), port.unique_copy(r)), (dt, run)
+
+
+@pytest.mark.parametrize("items", [131071, 131073, 148 * 4096, 148 * 4096 + 1, 3 * 148 * 4096 + 2050])
+def test_reduce_by_key_pipeline_edges(tb, port, items):
+    """Around the size where the pipeline starts, whole and ragged rounds of 148 tiles, one run, runs that end with a tile
+    and runs of one item; mixed sizes of keys and values.  Doubles hold whole numbers, so their sums are exact."""
+    for kt, vt in [(np.int32, np.int32), (np.uint32, np.float64), (np.int64, np.int32), (np.uint64, np.float64), (np.float32, np.int64)]:
+        v = dg.scan_input_i32(items, 7).astype(vt)
+        for run in (1, 2, 37, 4096, items + 1):
+            k = (np.arange(items) // run).astype(kt)
+            for op in ("plus", "max"):
+                gk, gv = tb.reduce_by_key(dev(k), dev(v), op=op)
+                wk, wv = port.reduce_by_key(k, v, op)
+                assert np.array_equal(host(gk), wk) and np.array_equal(host(gv), wv), (kt, vt, run, op)
