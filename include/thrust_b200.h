@@ -44,8 +44,8 @@ int tb200_version(void);
 int tb200_sm_arch(void);
 
 /* Reads the status word of a workspace after the work that used it has completed: synchronises
- * `stream`, copies 4 bytes back.  *h_status: 0 = ok, 1 = a look-back wait ran out (results of
- * that call are invalid).  Stands in for the reference's post-launch error check,
+ * `stream`, copies 4 bytes back.  *h_status: 0 = ok, 1 = a look-back wait ran out, 2 = two looks
+ * at a tile disagree (results of that call are invalid).  Stands in for the reference's post-launch error check,
  * cuda_cub::throw_on_error (thrust/system/cuda/detail/util.h:180-243). */
 int tb200_workspace_status(const void* d_ws, tb200_stream_t stream, unsigned* h_status);
 

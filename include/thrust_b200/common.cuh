@@ -39,7 +39,7 @@ template <class T> __device__ __forceinline__ void stash(T* slot, const T& v) {
 }
 
 // Error codes a kernel may leave in the workspace status word (see ws_header).
-enum : unsigned { ERR_NONE = 0, ERR_LOOKBACK_TIMEOUT = 1 };
+enum : unsigned { ERR_NONE = 0, ERR_LOOKBACK_TIMEOUT = 1, ERR_INCONSISTENT = 2 };   // 2: two evaluations of a tile disagree
 
 // Number of polls of a predecessor's status word before a look-back gives up, records
 // ERR_LOOKBACK_TIMEOUT and carries on with whatever it has.  Polls past the first few sleep

@@ -231,6 +231,13 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
         const unsigned incl = warp_inclusive_scan(packed, plus_op());
         const unsigned totals = __shfl_sync(FULL_MASK, incl, 31);
         const unsigned excl = incl - packed;
+        // what is stored now is what was counted then, and lies inside the outputs (an equality that does not answer the
+        // same twice is reported and nothing is stored)
+        const unsigned part_heads = __reduce_add_sync(FULL_MASK, (unsigned)__popc(bits));
+        if (part_heads != st.part[s][mine].heads || run0 > (size_t)tile * ITEMS + (size_t)mine * PART) {
+          if (lane == 0) record_error(&hdr->error, ERR_INCONSISTENT);
+          return;
+        }
         const unsigned kshift = run_shift(keys_out + run0);
         const unsigned vshift = run_shift(vals_out + run0 - 1);   // a value belongs to the run before its head
         unsigned row_off = 0;

@@ -137,9 +137,18 @@ select_pipe_kernel(const T* in, T* out_sel, T* out_rej, size_t n, unsigned tiles
         const C kept0 = st.carry[s] + before;      // kept items in front of this warp's part
         const size_t first = (size_t)tile * ITEMS + (size_t)mine * CHUNK;
         const unsigned part_n = first >= n ? 0u : n - first < (size_t)CHUNK ? (unsigned)(n - first) : (unsigned)CHUNK;
+        unsigned row_off = 0;
+#pragma unroll
+        for (int q = 0; q < PIPE_ROWS / 4; ++q) row_off += (totals[q] & 255) + ((totals[q] >> 8) & 255) + ((totals[q] >> 16) & 255) + (totals[q] >> 24);
+        // what is stored now is what was counted then, and lies inside the output: a predicate that does not answer the same
+        // twice (or a broken carry) is reported and nothing is stored
+        if (row_off != st.part[s][mine] || kept0 > first || row_off > part_n) {
+          if (lane == 0) record_error(&hdr->error, ERR_INCONSISTENT);
+          return;
+        }
         T* const dst = out_sel + kept0;
         const unsigned shift = run_shift(dst);
-        unsigned row_off = 0;
+        row_off = 0;
 #pragma unroll
         for (int v = 0; v < PIPE_ROWS; ++v) {
           unsigned r = shift + row_off + ((excl[v / 4] >> (8 * (v % 4))) & 255);
@@ -185,6 +194,7 @@ __global__ void __launch_bounds__(256)
 partition_rejects_kernel(T* data, const T* rejects, size_t n, const ws_header* hdr) {
   constexpr int VEC = 16 / sizeof(T);
   const size_t kept = (size_t)hdr->count;
+  if (kept > n) return;
   const size_t count = n - kept;
   T* const dst = data + kept;
   const size_t head = ((16 - (reinterpret_cast<uintptr_t>(dst) & 15)) & 15) / sizeof(T);   // items in front of dst's first 16-byte boundary

@@ -120,7 +120,7 @@ def _read_header(ws, what, nbytes=_HEADER.size):
     _check(_lib.load().tb200_workspace_read(ws.data_ptr(), nbytes, head, _stream()), what + " (result)")
     status = _HEADER.unpack_from(head)[0]
     if status != 0:
-        raise Tb200Error("%s: device reported status %d (an inter-CTA wait ran out)" % (what, status))
+        raise Tb200Error("%s: device reported status %d (%s)" % (what, status, "an inter-CTA wait ran out" if status == 1 else "two looks at a tile disagree"))
     return head
 
 
