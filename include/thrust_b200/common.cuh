@@ -141,6 +141,30 @@ inline void log_launch(const char* kernel, size_t grid, int block, size_t smem, 
   fprintf(stderr, "thrust_b200: %s<<<%zu, %d, %zu>>> items=%zu status=%s\n", kernel, grid, block, smem, items, cudaGetErrorName(e));
 }
 
+// ---------------------------------------------------------------- chains of dependent launches
+// A kernel launched with launch_after may be scheduled while its predecessor on the stream is still running; it calls
+// grid_dependency_wait() before it touches memory, which returns once the predecessor has completed and its writes
+// are visible.  What is saved is the launch latency between the kernels of a sort on a small input (a chain of eight
+// kernels: several microseconds each).  grid_dependents_launch() lets the successor be scheduled from then on.  Both do
+// nothing in a kernel that was launched the ordinary way.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... Params, class... Args>
+cudaError_t launch_after(void (*kernel)(Params...), size_t grid, int block, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // ---------------------------------------------------------------- functors
 struct plus_op { template <class T> __host__ __device__ T operator()(const T& a, const T& b) const { return a + b; } };
 struct min_op { template <class T> __host__ __device__ T operator()(const T& a, const T& b) const { return b < a ? b : a; } };

@@ -59,6 +59,7 @@ radix_hist_kernel(const UK* keys, size_t n, key_coding coding, int first_pass, i
   constexpr int COPIES = hist_tuning<UK>::COPIES;
   constexpr int VEC = 16 / sizeof(UK);
   extern __shared__ __align__(16) unsigned hist_bins[];   // [NP][256][COPIES]
+  grid_dependents_launch();
   for (int i = threadIdx.x; i < NP * RADIX_BINS * COPIES; i += HIST_BLOCK) hist_bins[i] = 0;
   __syncthreads();
   const int col = lane_id() & (COPIES - 1);
@@ -116,6 +117,8 @@ radix_hist_kernel(const UK* keys, size_t n, key_coding coding, int first_pass, i
 template <int UNUSED = 0>   // a template only so that the header can be included in several translation units
 __global__ void __launch_bounds__(RADIX_BINS)
 radix_scan_hist_kernel(radix_ctrl* ctrl, size_t n, int first_pass) {
+  grid_dependents_launch();
+  grid_dependency_wait();
   const int p = first_pass + blockIdx.x;
   __shared__ unsigned long long warp_tot[RADIX_BINS / 32];
   __shared__ unsigned degenerate;
@@ -447,6 +450,8 @@ template <class UK, class UV, bool HAS_V, bool IS_FLOAT, class LB, int IPT>
 __global__ void __launch_bounds__(ONESWEEP_BLOCK, ONESWEEP_CTAS_PER_SM)
 onesweep_kernel(UK* buf_a, UK* buf_b, UV* val_a, UV* val_b, unsigned n, key_coding coding, int pass, int first_pass,
                 radix_ctrl* ctrl, LB* lookback, ws_header* hdr) {
+  grid_dependents_launch();
+  grid_dependency_wait();
   if (ctrl->skip[pass]) return;
   int flips = 0;
   for (int q = first_pass; q < pass; ++q) flips += ctrl->skip[q] ? 0 : 1;
@@ -699,6 +704,7 @@ template <class UK, class UV, bool HAS_V>
 __global__ void __launch_bounds__(256)
 radix_copy_back_kernel(UK* buf_a, const UK* buf_b, UV* val_a, const UV* val_b, size_t n, int first_pass, int num_passes,
                        const radix_ctrl* ctrl) {
+  grid_dependency_wait();
   int active = 0;
   for (int q = first_pass; q < first_pass + num_passes; ++q) active += ctrl->skip[q] ? 0 : 1;
   if (!(active & 1)) return;
@@ -761,7 +767,9 @@ cudaError_t radix_sort_async(UK* keys_a, UK* keys_b, UV* vals_a, UV* vals_b, siz
   { timed_launch tl(KID_RADIX_HIST, stream);
   hk<<<(unsigned)hist_grid, HIST_BLOCK, hist_smem, stream>>>(keys_a, n, coding, first_pass, num_passes, ctrl); }
   log_launch("radix_hist_kernel", hist_grid, HIST_BLOCK, hist_smem, n, stream);
-  radix_scan_hist_kernel<><<<num_passes, RADIX_BINS, 0, stream>>>(ctrl, n, first_pass);
+  // the rest of the chain overlaps its launches with the kernels before (131 k u32 + u32 pairs 55 us against 69, 4 M 122
+  // against 133, 2^28 5.34 ms against 5.35)
+  if ((e = launch_after(radix_scan_hist_kernel<>, num_passes, RADIX_BINS, 0, stream, ctrl, n, first_pass)) != cudaSuccess) return e;
 
   const size_t smem = onesweep_smem_bytes<KB, VB>();
   const bool isf = coding.kind == KEY_FLOAT;
@@ -776,17 +784,17 @@ cudaError_t radix_sort_async(UK* keys_a, UK* keys_b, UV* vals_a, UV* vals_b, siz
     char* lb = lb0 + lb_bytes * p;
     timed_launch tl(KID_ONESWEEP, stream);
     if (lb32)
-      k32<<<grid, ONESWEEP_BLOCK, smem, stream>>>(keys_a, keys_b, vals_a, vals_b, (unsigned)n, coding, first_pass + p, first_pass, ctrl,
-                                                  reinterpret_cast<uint32_t*>(lb), hdr);
+      e = launch_after(k32, grid, ONESWEEP_BLOCK, smem, stream, keys_a, keys_b, vals_a, vals_b, (unsigned)n, coding, first_pass + p, first_pass, ctrl,
+                       reinterpret_cast<uint32_t*>(lb), hdr);
     else
-      k64<<<grid, ONESWEEP_BLOCK, smem, stream>>>(keys_a, keys_b, vals_a, vals_b, (unsigned)n, coding, first_pass + p, first_pass, ctrl,
-                                                  reinterpret_cast<unsigned long long*>(lb), hdr);
+      e = launch_after(k64, grid, ONESWEEP_BLOCK, smem, stream, keys_a, keys_b, vals_a, vals_b, (unsigned)n, coding, first_pass + p, first_pass, ctrl,
+                       reinterpret_cast<unsigned long long*>(lb), hdr);
+    if (e != cudaSuccess) return e;
     log_launch("onesweep_kernel", grid, ONESWEEP_BLOCK, smem, n, stream);
   }
   size_t cb_grid = (n + 256 * 8 - 1) / (256 * 8);
   if (cb_grid > (size_t)di.sm_count * 8) cb_grid = (size_t)di.sm_count * 8;
-  radix_copy_back_kernel<UK, UV, HAS_V><<<(unsigned)cb_grid, 256, 0, stream>>>(keys_a, keys_b, vals_a, vals_b, n, first_pass, num_passes, ctrl);
-  return cudaGetLastError();
+  return launch_after(radix_copy_back_kernel<UK, UV, HAS_V>, cb_grid, 256, 0, stream, keys_a, keys_b, vals_a, vals_b, n, first_pass, num_passes, ctrl);
 }
 
 // counts[0..buckets) += histogram of bucket ids (the caller zeroes counts); no sync
