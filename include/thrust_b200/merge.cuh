@@ -423,7 +423,11 @@ template <int KB, int VB> struct block_sort_tuning {
   // power-of-two friendly tile of 256 * IPT items whose keys (+ a 2-byte index each) fit 44 KB of shared memory
   static constexpr int FIT = MERGE_SMEM_BUDGET / (MERGE_BLOCK * (KB + 2));
   static constexpr int IPT = (KB + VB) <= 8 ? TB200_BSORT_IPT8 : (FIT >= 8 ? 8 : FIT >= 4 ? 4 : FIT >= 2 ? 2 : 1);
-  static_assert(MERGE_BLOCK * IPT * (KB + 2) + KB + 2 <= 48 * 1024, "key too large for the block sort tile (more than 170 bytes)");
+  // one slot of padding per thread, where static shared memory has room for it (20-byte keys at 8 items: it has not)
+  static constexpr int TILE = MERGE_BLOCK * IPT, SMEM = 48 * 1024;
+  static constexpr bool PADDED = IPT >= 8 && (TILE + MERGE_BLOCK + 1) * (KB + 2) + 16 <= SMEM;
+  static constexpr int SLOTS = TILE + (PADDED ? MERGE_BLOCK : 0) + 1;
+  static_assert(SLOTS * (KB + 2) <= SMEM, "key too large for the block sort tile (more than 170 bytes)");
 };
 
 // What bounds it is shared memory: a thread's IPT consecutive items are written and read back in every round,
@@ -435,8 +439,10 @@ template <class KeyIt, class ValIt, class KeyOutIt, class ValOutIt, class K, cla
 __global__ void __launch_bounds__(MERGE_BLOCK, sizeof(K) <= 4 ? TB200_BSORT_CTAS8 : 1)
 block_sort_kernel(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOutIt vals_out, size_t n, Comp comp) {
   constexpr int TILE = MERGE_BLOCK * IPT;
-  constexpr bool PADDED = IPT >= 8;
-  constexpr int SLOTS = (PADDED ? TILE + TILE / IPT : TILE) + 1;
+  using Tuning = block_sort_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>;
+  constexpr bool PADDED = Tuning::PADDED;
+  constexpr int SLOTS = Tuning::SLOTS;
+  static_assert(IPT == Tuning::IPT, "the tile is the tuning's");
   TB200_SHARED_ARRAY(K, s_key, SLOTS);
   __shared__ unsigned short s_idx[SLOTS];
   auto slot = [](unsigned j) { return PADDED ? j + j / IPT : j; };
