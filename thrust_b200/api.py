@@ -9,6 +9,7 @@ libthrust_b200.so; there is no fallback path.
 """
 import ctypes as C
 import struct
+import threading
 
 import numpy as np
 import torch
@@ -58,22 +59,31 @@ def _require_cuda(*tensors):
 
 class _Workspaces:
     """Scratch buffers cached per (device, stream, call site) and grown on demand, standing in for
-    the reference's per-call temporary_array (thrust/system/cuda/detail/reduce.h:959)."""
+    the reference's per-call temporary_array (thrust/system/cuda/detail/reduce.h:959).
+
+    Threads that share a stream share its buffers too, and a call's status, count or result lies in one until it
+    is read back; a call therefore holds the buffer's lock from its first launch to that read-back."""
 
     def __init__(self):
         self._bufs = {}
+        self._locks = {}
 
     @staticmethod
-    def _key(tag):
+    def key(tag):
+        """What the buffer of this call site on the current stream is kept under: (device, stream handle, tag)."""
         dev = torch.cuda.current_device()
         return dev, _raw_stream(dev), tag
 
-    def kept(self, tag):
-        """The buffer kept for this call site on the current stream, whatever its size, or None."""
-        return self._bufs.get(self._key(tag))
+    def lock(self, key):
+        """The lock of a buffer (re-entrant)."""
+        return self._locks.get(key) or self._locks.setdefault(key, threading.RLock())
 
-    def get(self, tag, nbytes):
-        key = self._key(tag)
+    def kept(self, key):
+        """The buffer kept under `key`, whatever its size, or None."""
+        return self._bufs.get(key)
+
+    def get(self, tag, nbytes, key=None):
+        key = key or self.key(tag)
         buf = self._bufs.get(key)
         if buf is None or buf.numel() < nbytes:
             buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device="cuda")
@@ -90,12 +100,12 @@ workspaces = _Workspaces()
 _TOO_SMALL = 1      # cudaErrorInvalidValue: the workspace is too small (or another argument is wrong)
 
 
-def _call_with_ws(tag, fn, *args):
-    """fn(*args, d_ws, &ws_bytes, stream) in the workspace kept for the call site; the size is asked for only if
-    there is none yet or it is refused as too small.  Returns the workspace."""
+def _enqueue(key, fn, args):
+    """fn(*args, d_ws, &ws_bytes, stream) in the workspace kept under `key`, whose lock the caller holds; the size is
+    asked for only if there is none yet or it is refused as too small.  Returns the workspace."""
     lib_fn = getattr(_lib.load(), fn)
-    stream = _stream()
-    ws = workspaces.kept(tag)
+    stream = key[1]
+    ws = workspaces.kept(key)
     if ws is not None:
         rc = lib_fn(*args, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream)
         if rc != _TOO_SMALL:
@@ -103,9 +113,25 @@ def _call_with_ws(tag, fn, *args):
             return ws
     need = C.c_size_t(0)
     _check(lib_fn(*args, None, C.byref(need), stream), fn + " (size query)")
-    ws = workspaces.get(tag, need.value)
+    ws = workspaces.get(key[2], need.value, key)
     _check(lib_fn(*args, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream), fn)
     return ws
+
+
+def _call_with_ws(tag, fn, *args):
+    """Enqueues fn in the workspace of the call site; returns the workspace."""
+    key = workspaces.key(tag)
+    with workspaces.lock(key):
+        return _enqueue(key, fn, args)
+
+
+def _call_and_wait(tag, what, fn, *args, sync=True):
+    """The same, then (sync) waits for the stream and checks the status.  Returns the number that the kernels of
+    a selecting or counting call left in the header."""
+    key = workspaces.key(tag)
+    with workspaces.lock(key):
+        ws = _enqueue(key, fn, args)
+        return _HEADER.unpack_from(_read_header(ws, what, stream=key[1]))[2] if sync else None
 
 
 # the workspace header (ws_header in common.cuh): status, ticket, count, ..., and room that a result may use
@@ -113,11 +139,11 @@ _HEADER = struct.Struct("<IIQ")
 _HEADER_RESULT = 32
 
 
-def _read_header(ws, what, nbytes=_HEADER.size):
+def _read_header(ws, what, nbytes=_HEADER.size, stream=None):
     """Waits for the stream, then the first `nbytes` of the workspace's header in one copy; raises if the
     kernels reported a wait that ran out."""
     head = C.create_string_buffer(nbytes)
-    _check(_lib.load().tb200_workspace_read(ws.data_ptr(), nbytes, head, _stream()), what + " (result)")
+    _check(_lib.load().tb200_workspace_read(ws.data_ptr(), nbytes, head, _stream() if stream is None else stream), what + " (result)")
     status = _HEADER.unpack_from(head)[0]
     if status != 0:
         raise Tb200Error("%s: device reported status %d (%s)" % (what, status, "an inter-CTA wait ran out" if status == 1 else "two looks at a tile disagree"))
@@ -126,11 +152,6 @@ def _read_header(ws, what, nbytes=_HEADER.size):
 
 def _sync_and_check(ws, what):
     _read_header(ws, what)
-
-
-def _sync_and_count(ws, what):
-    """The same for calls that select or count: the number that the kernels left in the header."""
-    return _HEADER.unpack_from(_read_header(ws, what))[2]
 
 
 # ------------------------------------------------------------------------------------- reduce
@@ -143,19 +164,21 @@ def reduce(x, init=None, op="plus", acc_dtype=None):
     h_init = np.asarray(0 if init is None else init, dtype=NP_OF[acc_dtype])
     # the result lands in the workspace's header and comes back together with the status
     lib_fn = _lib.load().tb200_reduce
-    stream = _stream()
+    key = workspaces.key("reduce")
+    stream = key[1]
     args = (_ptr(x), x.numel(), DTYPE_CODE[x.dtype], DTYPE_CODE[acc_dtype], OPS[op], h_init.ctypes.data)
-    ws = workspaces.kept("reduce")
-    rc = _TOO_SMALL
-    if ws is not None:
-        rc = lib_fn(*args, ws.data_ptr() + _HEADER_RESULT, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream)
-    if rc == _TOO_SMALL:
-        need = C.c_size_t(0)
-        _check(lib_fn(*args, None, None, C.byref(need), stream), "tb200_reduce (size query)")
-        ws = workspaces.get("reduce", need.value)
-        rc = lib_fn(*args, ws.data_ptr() + _HEADER_RESULT, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream)
-    _check(rc, "tb200_reduce")
-    head = _read_header(ws, "reduce", _HEADER_RESULT + 8)
+    with workspaces.lock(key):
+        ws = workspaces.kept(key)
+        rc = _TOO_SMALL
+        if ws is not None:
+            rc = lib_fn(*args, ws.data_ptr() + _HEADER_RESULT, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream)
+        if rc == _TOO_SMALL:
+            need = C.c_size_t(0)
+            _check(lib_fn(*args, None, None, C.byref(need), stream), "tb200_reduce (size query)")
+            ws = workspaces.get("reduce", need.value, key)
+            rc = lib_fn(*args, ws.data_ptr() + _HEADER_RESULT, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream)
+        _check(rc, "tb200_reduce")
+        head = _read_header(ws, "reduce", _HEADER_RESULT + 8, stream)
     return np.frombuffer(head.raw, dtype=NP_OF[acc_dtype], count=1, offset=_HEADER_RESULT)[0]
 
 
@@ -179,13 +202,12 @@ def inclusive_scan(x, out=None, op="plus", init=None, sync=True):
     _require_cuda(x, out)
     out = torch.empty_like(x) if out is None else out
     if isinstance(init, torch.Tensor):
-        ws = _call_with_ws("scan", "tb200_inclusive_scan_dinit", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], OPS[op], _ptr(init))
+        _call_and_wait("scan", "inclusive_scan", "tb200_inclusive_scan_dinit", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], OPS[op],
+                       _ptr(init), sync=sync)
     else:
         h_init = None if init is None else np.asarray(init, dtype=NP_OF[x.dtype])
-        ws = _call_with_ws("scan", "tb200_inclusive_scan", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], OPS[op],
-                           None if h_init is None else h_init.ctypes.data)
-    if sync:
-        _sync_and_check(ws, "inclusive_scan")
+        _call_and_wait("scan", "inclusive_scan", "tb200_inclusive_scan", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], OPS[op],
+                       None if h_init is None else h_init.ctypes.data, sync=sync)
     return out
 
 
@@ -194,13 +216,12 @@ def exclusive_scan(x, init=0, out=None, op="plus", sync=True):
     _require_cuda(x, out)
     out = torch.empty_like(x) if out is None else out
     if isinstance(init, torch.Tensor):
-        ws = _call_with_ws("scan", "tb200_exclusive_scan_dinit", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], OPS[op], _ptr(init))
+        _call_and_wait("scan", "exclusive_scan", "tb200_exclusive_scan_dinit", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], OPS[op],
+                       _ptr(init), sync=sync)
     else:
         h_init = np.asarray(init, dtype=NP_OF[x.dtype])
-        ws = _call_with_ws("scan", "tb200_exclusive_scan", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], OPS[op],
-                           h_init.ctypes.data)
-    if sync:
-        _sync_and_check(ws, "exclusive_scan")
+        _call_and_wait("scan", "exclusive_scan", "tb200_exclusive_scan", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], OPS[op],
+                       h_init.ctypes.data, sync=sync)
     return out
 
 
@@ -211,13 +232,12 @@ def _sort_impl(keys, vals, descending, begin_bit, end_bit, sync=True):
         raise ValueError("keys and values differ in length")
     n = keys.numel()
     vb = 0 if vals is None else vals.element_size()
-    kalt = workspaces.get("sort_keys_alt", n * keys.element_size())
-    valt = None if vals is None else workspaces.get("sort_vals_alt", n * vb)
     end_bit = 8 * keys.element_size() if end_bit is None else end_bit
-    ws = _call_with_ws("sort", "tb200_sort_by_key", _ptr(keys), _ptr(kalt), _ptr(vals), _ptr(valt), n,
-                       DTYPE_CODE[keys.dtype], vb, int(descending), begin_bit, end_bit)
-    if sync:
-        _sync_and_check(ws, "sort")
+    with workspaces.lock(workspaces.key("sort_keys_alt")):
+        kalt = workspaces.get("sort_keys_alt", n * keys.element_size())
+        valt = None if vals is None else workspaces.get("sort_vals_alt", n * vb)
+        _call_and_wait("sort", "sort", "tb200_sort_by_key", _ptr(keys), _ptr(kalt), _ptr(vals), _ptr(valt), n,
+                       DTYPE_CODE[keys.dtype], vb, int(descending), begin_bit, end_bit, sync=sync)
 
 
 def sort(keys, descending=False, sync=True):
@@ -294,18 +314,17 @@ def copy_if(x, pred, a=0, b=0, stencil=None, out=None):
     """thrust::copy_if(first, last, [stencil,] result, pred): returns out[:count] (stable)."""
     _require_cuda(x, stencil, out)
     out = torch.empty_like(x) if out is None else out
-    ws = _call_with_ws("select", "tb200_copy_if", _ptr(x), _ptr(stencil), _ptr(out), x.numel(), DTYPE_CODE[x.dtype],
-                       0 if stencil is None else DTYPE_CODE[stencil.dtype], PREDS[pred], a, b, None)
-    return out[:_sync_and_count(ws, "copy_if")]
+    count = _call_and_wait("select", "copy_if", "tb200_copy_if", _ptr(x), _ptr(stencil), _ptr(out), x.numel(), DTYPE_CODE[x.dtype],
+                           0 if stencil is None else DTYPE_CODE[stencil.dtype], PREDS[pred], a, b, None)
+    return out[:count]
 
 
 def partition_copy(x, pred, a=0, b=0, stencil=None):
     """thrust::stable_partition_copy: returns (selected, rejected), both in input order."""
     _require_cuda(x, stencil)
     out_t, out_f = torch.empty_like(x), torch.empty_like(x)
-    ws = _call_with_ws("select", "tb200_partition_copy", _ptr(x), _ptr(stencil), _ptr(out_t), _ptr(out_f), x.numel(),
+    k = _call_and_wait("select", "partition_copy", "tb200_partition_copy", _ptr(x), _ptr(stencil), _ptr(out_t), _ptr(out_f), x.numel(),
                        DTYPE_CODE[x.dtype], 0 if stencil is None else DTYPE_CODE[stencil.dtype], PREDS[pred], a, b, None)
-    k = _sync_and_count(ws, "partition_copy")
     return out_t[:k], out_f[:x.numel() - k]
 
 
@@ -315,8 +334,7 @@ stable_partition_copy = partition_copy
 def partition(x, pred, a=0, b=0):
     """thrust::partition / thrust::stable_partition in place; returns the split point."""
     _require_cuda(x)
-    ws = _call_with_ws("partition", "tb200_partition", _ptr(x), x.numel(), DTYPE_CODE[x.dtype], PREDS[pred], a, b, None)
-    return _sync_and_count(ws, "partition")
+    return _call_and_wait("partition", "partition", "tb200_partition", _ptr(x), x.numel(), DTYPE_CODE[x.dtype], PREDS[pred], a, b, None)
 
 
 stable_partition = partition
@@ -326,8 +344,8 @@ def unique_copy(x, out=None):
     """thrust::unique_copy(first, last, result): returns out[:count]."""
     _require_cuda(x, out)
     out = torch.empty_like(x) if out is None else out
-    ws = _call_with_ws("select", "tb200_unique_copy", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], None)
-    return out[:_sync_and_count(ws, "unique_copy")]
+    count = _call_and_wait("select", "unique_copy", "tb200_unique_copy", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], None)
+    return out[:count]
 
 
 def unique(x):
@@ -340,9 +358,8 @@ def reduce_by_key(keys, vals, op="plus"):
     returns (keys_out[:runs], values_out[:runs])."""
     _require_cuda(keys, vals)
     ko, vo = torch.empty_like(keys), torch.empty_like(vals)
-    ws = _call_with_ws("rbk", "tb200_reduce_by_key", _ptr(keys), _ptr(vals), _ptr(ko), _ptr(vo), keys.numel(),
+    k = _call_and_wait("rbk", "reduce_by_key", "tb200_reduce_by_key", _ptr(keys), _ptr(vals), _ptr(ko), _ptr(vo), keys.numel(),
                        DTYPE_CODE[keys.dtype], DTYPE_CODE[vals.dtype], OPS[op], None)
-    k = _sync_and_count(ws, "reduce_by_key")
     return ko[:k], vo[:k]
 
 
@@ -350,9 +367,8 @@ def inclusive_scan_by_key(keys, vals, out=None, op="plus"):
     """thrust::inclusive_scan_by_key(keys_first, keys_last, values_first, result, equal_to, op)."""
     _require_cuda(keys, vals, out)
     out = torch.empty_like(vals) if out is None else out
-    ws = _call_with_ws("rbk", "tb200_scan_by_key", _ptr(keys), _ptr(vals), _ptr(out), keys.numel(), DTYPE_CODE[keys.dtype],
-                       DTYPE_CODE[vals.dtype], OPS[op], 0, None)
-    _sync_and_check(ws, "inclusive_scan_by_key")
+    _call_and_wait("rbk", "inclusive_scan_by_key", "tb200_scan_by_key", _ptr(keys), _ptr(vals), _ptr(out), keys.numel(), DTYPE_CODE[keys.dtype],
+                   DTYPE_CODE[vals.dtype], OPS[op], 0, None)
     return out
 
 
@@ -361,9 +377,8 @@ def exclusive_scan_by_key(keys, vals, init=0, out=None, op="plus"):
     _require_cuda(keys, vals, out)
     out = torch.empty_like(vals) if out is None else out
     h_init = np.asarray(init, dtype=NP_OF[vals.dtype])
-    ws = _call_with_ws("rbk", "tb200_scan_by_key", _ptr(keys), _ptr(vals), _ptr(out), keys.numel(), DTYPE_CODE[keys.dtype],
-                       DTYPE_CODE[vals.dtype], OPS[op], 1, h_init.ctypes.data)
-    _sync_and_check(ws, "exclusive_scan_by_key")
+    _call_and_wait("rbk", "exclusive_scan_by_key", "tb200_scan_by_key", _ptr(keys), _ptr(vals), _ptr(out), keys.numel(), DTYPE_CODE[keys.dtype],
+                   DTYPE_CODE[vals.dtype], OPS[op], 1, h_init.ctypes.data)
     return out
 
 
@@ -372,9 +387,8 @@ def unique_by_key_copy(keys, vals, keys_out=None, vals_out=None):
     _require_cuda(keys, vals, keys_out, vals_out)
     ko = torch.empty_like(keys) if keys_out is None else keys_out
     vo = torch.empty_like(vals) if vals_out is None else vals_out
-    ws = _call_with_ws("rbk", "tb200_unique_by_key_copy", _ptr(keys), _ptr(vals), _ptr(ko), _ptr(vo), keys.numel(),
+    k = _call_and_wait("rbk", "unique_by_key_copy", "tb200_unique_by_key_copy", _ptr(keys), _ptr(vals), _ptr(ko), _ptr(vo), keys.numel(),
                        DTYPE_CODE[keys.dtype], vals.element_size(), None)
-    k = _sync_and_count(ws, "unique_by_key_copy")
     return ko[:k], vo[:k]
 
 
@@ -387,8 +401,7 @@ def unique_by_key(keys, vals):
 def _extrema(fn, x, words):
     _require_cuda(x)
     idx = torch.zeros(words, dtype=torch.int64, device="cuda")
-    ws = _call_with_ws("reduce", fn, _ptr(x), x.numel(), DTYPE_CODE[x.dtype], _ptr(idx))
-    _sync_and_check(ws, fn)
+    _call_and_wait("reduce", fn, fn, _ptr(x), x.numel(), DTYPE_CODE[x.dtype], _ptr(idx))
     return [int(v) for v in idx.cpu().tolist()]
 
 
@@ -419,10 +432,8 @@ def merge_by_key(keys_a, keys_b, vals_a=None, vals_b=None, descending=False, syn
     ko = torch.empty(na + nb, dtype=keys_a.dtype, device=keys_a.device)
     vo = None if vals_a is None else torch.empty(na + nb, dtype=vals_a.dtype, device=keys_a.device)
     vb = 0 if vals_a is None else vals_a.element_size()
-    ws = _call_with_ws("merge", "tb200_merge_by_key", _ptr(keys_a), _ptr(vals_a), na, _ptr(keys_b), _ptr(vals_b), nb, _ptr(ko),
-                       _ptr(vo), DTYPE_CODE[keys_a.dtype], vb, int(descending))
-    if sync:
-        _sync_and_check(ws, "merge_by_key")
+    _call_and_wait("merge", "merge_by_key", "tb200_merge_by_key", _ptr(keys_a), _ptr(vals_a), na, _ptr(keys_b), _ptr(vals_b), nb, _ptr(ko),
+                   _ptr(vo), DTYPE_CODE[keys_a.dtype], vb, int(descending), sync=sync)
     return ko, vo
 
 
@@ -448,9 +459,8 @@ def set_operation(op, keys_a, keys_b, vals_a=None, vals_b=None, descending=False
     ko = torch.empty(cap, dtype=keys_a.dtype, device=keys_a.device)
     vo = None if vals_a is None else torch.empty(cap, dtype=vals_a.dtype, device=keys_a.device)
     vb = 0 if vals_a is None else vals_a.element_size()
-    ws = _call_with_ws("setop", "tb200_set_operation", code, _ptr(keys_a), na, _ptr(keys_b), nb, _ptr(vals_a), _ptr(vals_b), _ptr(ko), _ptr(vo),
-                       DTYPE_CODE[keys_a.dtype], vb, int(descending), None)
-    m = _sync_and_count(ws, "set_" + op)
+    m = _call_and_wait("setop", "set_" + op, "tb200_set_operation", code, _ptr(keys_a), na, _ptr(keys_b), nb, _ptr(vals_a), _ptr(vals_b),
+                       _ptr(ko), _ptr(vo), DTYPE_CODE[keys_a.dtype], vb, int(descending), None)
     return ko[:m], (None if vo is None else vo[:m])
 
 
@@ -459,11 +469,11 @@ def merge_sort_by_key(keys, vals=None, descending=False):
     _require_cuda(keys, vals)
     n = keys.numel()
     vb = 0 if vals is None else vals.element_size()
-    kalt = workspaces.get("sort_keys_alt", n * keys.element_size())
-    valt = None if vals is None else workspaces.get("sort_vals_alt", n * vb)
-    ws = _call_with_ws("merge_sort", "tb200_merge_sort_by_key", _ptr(keys), _ptr(kalt), _ptr(vals), _ptr(valt), n,
+    with workspaces.lock(workspaces.key("sort_keys_alt")):
+        kalt = workspaces.get("sort_keys_alt", n * keys.element_size())
+        valt = None if vals is None else workspaces.get("sort_vals_alt", n * vb)
+        _call_and_wait("merge_sort", "merge_sort_by_key", "tb200_merge_sort_by_key", _ptr(keys), _ptr(kalt), _ptr(vals), _ptr(valt), n,
                        DTYPE_CODE[keys.dtype], vb, int(descending))
-    _sync_and_check(ws, "merge_sort_by_key")
     return keys, vals
 
 
