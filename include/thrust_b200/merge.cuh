@@ -98,6 +98,18 @@ struct merge_geometry {
   }
 };
 
+// A tile's slices of A and B, from the splits of its two diagonals.  Each split lies inside its own diagonal's bounds
+// whatever the comparator answers; under one that is no strict weak order on the data (keys that are NaN) two
+// neighbouring splits need not agree, and then the slices are no ranges: `consistent` is false and the tile must not be merged.
+struct merge_slices {
+  size_t a_begin, b_begin;
+  unsigned na, nb;
+  bool consistent;
+  __host__ __device__ merge_slices(size_t split_begin, size_t split_end, size_t a0, size_t b0, size_t local, unsigned tile_n)
+      : a_begin(split_begin), b_begin(b0 + local - (split_begin - a0)), na((unsigned)(split_end - split_begin)), nb(tile_n - na),
+        consistent(split_end >= split_begin && split_end - split_begin <= tile_n) {}
+};
+
 // One thread per tile: where in A the tile's outputs start and end.
 template <class KeyItA, class KeyItB, class Comp, int TILE>
 __global__ void __launch_bounds__(256)
@@ -115,7 +127,7 @@ merge_partition_kernel(KeyItA ka, KeyItB kb, merge_geometry g, size_t num_tiles,
 
 template <class KeyItA, class KeyItB, class ValItA, class ValItB, class KeyOutIt, class ValOutIt, class K, class V, bool HAS_V, class Comp, int IPT>
 __global__ void __launch_bounds__(MERGE_BLOCK, merge_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>::MIN_CTAS)
-merge_kernel(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutIt ko, ValOutIt vo, merge_geometry g, Comp comp, const size_t* a_split) {
+merge_kernel(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutIt ko, ValOutIt vo, merge_geometry g, Comp comp, const size_t* a_split, unsigned* err) {
   constexpr int TILE = MERGE_BLOCK * IPT;
   TB200_SHARED_ARRAY(K, s_key, TILE + 1);
   TB200_SHARED_ARRAY(V, s_val, HAS_V ? TILE : 1);
@@ -126,9 +138,10 @@ merge_kernel(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutIt ko, ValOutIt v
   if (local >= pair_total) return;                       // a short last pair leaves its later tiles empty
   const size_t out0 = pair_out + local;
   const unsigned tile_n = pair_total - local < TILE ? (unsigned)(pair_total - local) : (unsigned)TILE;
-  const size_t a_begin = a_split[2 * t], a_end = a_split[2 * t + 1];
-  const size_t b_begin = b0p + local - (a_begin - a0p);
-  const unsigned na = (unsigned)(a_end - a_begin), nb = tile_n - na;
+  const merge_slices slices(a_split[2 * t], a_split[2 * t + 1], a0p, b0p, local, tile_n);
+  if (!slices.consistent) { if (threadIdx.x == 0) record_error(err, ERR_INCONSISTENT); return; }
+  const size_t a_begin = slices.a_begin, b_begin = slices.b_begin;
+  const unsigned na = slices.na, nb = slices.nb;
 
   // ---- stage both key slices: A at [0, na), B at [na, na + nb)
 #pragma unroll
@@ -261,10 +274,10 @@ merge_slices_kernel(const K* ka, const K* kb, const V* va, const V* vb, K* ko, V
   const size_t pair_total = alen + blen;
   if (local >= pair_total) return;                     // a short last pair leaves its later tiles empty
   const unsigned tile_n = pair_total - local < TILE ? (unsigned)(pair_total - local) : (unsigned)TILE;
-  const size_t a_begin = a_split[t];
-  const size_t a_end = local + TILE < pair_total ? a_split[t + 1] : a0p + alen;
-  const size_t b_begin = b0p + local - (a_begin - a0p);
-  const unsigned na = (unsigned)(a_end - a_begin), nb = tile_n - na;
+  const merge_slices slices(a_split[t], local + TILE < pair_total ? a_split[t + 1] : a0p + alen, a0p, b0p, local, tile_n);
+  if (!slices.consistent) { if (threadIdx.x == 0) record_error(err, ERR_INCONSISTENT); return; }   // before any copy is sized by them
+  const size_t a_begin = slices.a_begin, b_begin = slices.b_begin;
+  const unsigned na = slices.na, nb = slices.nb;
   auto phase = [](const void* p) { return (unsigned)(reinterpret_cast<uintptr_t>(p) & 15); };
 
   // ---- the slices' places: A first, B behind it on the next 16-byte boundary, each shifted by its phase
@@ -404,7 +417,7 @@ cudaError_t merge_pass_async(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutI
   merge_partition_kernel<KeyItA, KeyItB, Comp, TILE><<<(unsigned)((tiles + 255) / 256), 256, 0, stream>>>(ka, kb, g, tiles, comp, a_split);
   timed_launch tl(KID_MERGE, stream);
   merge_kernel<KeyItA, KeyItB, ValItA, ValItB, KeyOutIt, ValOutIt, K, V, HAS_V, Comp, IPT>
-      <<<(unsigned)tiles, MERGE_BLOCK, 0, stream>>>(ka, kb, va, vb, ko, vo, g, comp, a_split);
+      <<<(unsigned)tiles, MERGE_BLOCK, 0, stream>>>(ka, kb, va, vb, ko, vo, g, comp, a_split, &static_cast<ws_header*>(ws)->error);
   return cudaGetLastError();
   }
 }

@@ -106,3 +106,24 @@ def test_merge_of_slices_at_any_alignment(tb, port, shift, n):
         rk, rv = port.merge_by_key(a, b, va, vb)
         assert np.array_equal(host(ko), rk) and np.array_equal(host(vo), rv), (dt, vt)
         assert np.array_equal(host(tb.merge(args[0], args[1])), rk), dt
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_merge_of_keys_with_nans_ends(tb, port, dt):
+    """Keys that are NaN have no order: the call gives some order or reports that its tiles disagree, and the next call
+    on the same workspace is right."""
+    n = 200003
+    a, b = np.sort(rand_of(dt, n, 93)), np.sort(rand_of(dt, n // 2, 94))
+    va, vb = np.arange(n, dtype=np.uint32), np.arange(n // 2, dtype=np.uint32) + np.uint32(1 << 30)
+    for share in (0.002, 0.02, 0.1):
+        an, bn = a.copy(), b.copy()
+        an[dg.rand64(95, n) % np.uint64(1000) < int(1000 * share)] = np.nan
+        bn[dg.rand64(96, n // 2) % np.uint64(1000) < int(1000 * share)] = np.nan
+        for call in (lambda: tb.merge_by_key(dev(an), dev(bn), dev(va), dev(vb)), lambda: tb.stable_sort_zip_by_first(dev(an[dg.rand64(97, n) % np.uint64(n)]), dev(va))):
+            try:
+                assert call()[0].numel() >= n
+            except tb.api.Tb200Error as e:
+                assert "status 2" in str(e)
+        ko, vo = tb.merge_by_key(dev(a), dev(b), dev(va), dev(vb))
+        rk, rv = port.merge_by_key(a, b, va, vb)
+        assert np.array_equal(host(ko), rk) and np.array_equal(host(vo), rv)

@@ -35,3 +35,17 @@ def test_comparator_sort_of_any_key_size_compiles(tmp_path, words):
     r = subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I" + os.path.join(ROOT, "include"), "-c", str(src),
                         "-o", str(tmp_path / "sort_sizes.o")], capture_output=True, text=True, timeout=900)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_merge_tiles_stay_inside_their_inputs(tmp_path):
+    """Sorted keys with NaNs strewn in are no ordered ranges: tiles whose two splits disagree are refused, all others have
+    slices inside A and B (tests/cpp/merge_slices_host.cu, host code only)."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.isfile(nvcc):
+        pytest.skip("nvcc is not available on this machine")
+    exe = str(tmp_path / "merge_slices_host")
+    r = subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I" + os.path.join(ROOT, "include"),
+                        os.path.join(ROOT, "tests", "cpp", "merge_slices_host.cu"), "-o", exe], capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stdout + r.stderr
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
