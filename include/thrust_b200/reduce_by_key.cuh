@@ -185,19 +185,16 @@ cudaError_t reduce_by_key_async(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOu
   const size_t tiles = (n + rbk_tile_items<K, V>() - 1) / rbk_tile_items<K, V>();
   // large contiguous inputs and outputs elsewhere: the tile pipeline (reduce_by_key_pipe.cuh) where the operator
   // has an identity, the two-pass streaming kernels (reduce_by_key_stream.cuh) otherwise, for keys and values of
-  // one size
+  // one size.  Floating min and max have none (min_op(infinity, NaN) is infinity).
   if constexpr (std::is_pointer<KeyIt>::value && std::is_pointer<ValIt>::value && std::is_pointer<KeyOutIt>::value && std::is_pointer<ValOutIt>::value &&
                 std::is_arithmetic<K>::value && std::is_arithmetic<V>::value && (sizeof(K) == 4 || sizeof(K) == 8) && (sizeof(V) == 4 || sizeof(V) == 8) &&
-                is_commutative_op<Op>::value) {
+                is_commutative_op<Op>::value && (std::is_integral<V>::value || std::is_same<Op, plus_op>::value)) {
     using KIn = typename std::remove_cv<typename std::remove_pointer<KeyIt>::type>::type;
     using VIn = typename std::remove_cv<typename std::remove_pointer<ValIt>::type>::type;
     using KOut = typename std::remove_pointer<KeyOutIt>::type;
     using VOut = typename std::remove_pointer<ValOutIt>::type;
     if constexpr (std::is_same<KIn, K>::value && std::is_same<VIn, V>::value && std::is_same<KOut, K>::value && std::is_same<VOut, V>::value) {
-      // NaNs make floating min and max depend on the grouping: those leave the single-pass kernel only where they always did
-      constexpr bool regrouping_shows = std::is_floating_point<V>::value && !std::is_same<Op, plus_op>::value;
-      const bool large = regrouping_shows ? n >= RBK_STREAM_MIN_ITEMS && sizeof(K) == sizeof(V) : n * (sizeof(K) + sizeof(V)) >= RBK_PIPE_MIN_BYTES;
-      if (large && (ALLOW_BIG || n < (1ull << 31)) && rbk_pipe_eligible<K, V>(keys, vals, keys_out, vals_out, n)) {
+      if (n * (sizeof(K) + sizeof(V)) >= RBK_PIPE_MIN_BYTES && (ALLOW_BIG || n < (1ull << 31)) && rbk_pipe_eligible<K, V>(keys, vals, keys_out, vals_out, n)) {
         bool launched = false;
         const cudaError_t pe = rbk_pipe_launch<K, V, Eq, Op>(keys, vals, keys_out, vals_out, n, eq, d_count, ws, stream, launched);
         if (launched || pe != cudaSuccess) return pe;

@@ -244,3 +244,20 @@ def test_reduce_by_key_pipeline_edges(tb, port, items):
                 gk, gv = tb.reduce_by_key(dev(k), dev(v), op=op)
                 wk, wv = port.reduce_by_key(k, v, op)
                 assert np.array_equal(host(gk), wk) and np.array_equal(host(gv), wv), (kt, vt, run, op)
+
+
+@pytest.mark.parametrize("kt,vt", [(np.int32, np.float32), (np.int64, np.float64)])
+def test_reduce_by_key_float_min_max_of_nans(tb, kt, vt):
+    """Runs of nothing but NaNs reduce to NaN wherever they lie -- at the ends of rows, warps' parts and tiles, over
+    several of them -- and never to an infinity that is not in the input; runs without NaNs are exact."""
+    n = (1 << 24) + 4099
+    for run in (1, 2, 7, 512, 4096, 10000):
+        k = (np.arange(n) // run).astype(kt)
+        v = (dg.rand64(53, n) % np.uint64(1 << 20)).astype(vt)
+        nan_run = dg.rand64(54, int(k[-1]) + 1) % np.uint64(3) == 0
+        v[nan_run[k]] = np.nan
+        starts = np.arange(0, n, run)
+        for op, fold in (("min", np.minimum), ("max", np.maximum)):
+            gk, gv = tb.reduce_by_key(dev(k), dev(v), op=op)
+            assert np.array_equal(host(gk), np.arange(starts.size).astype(kt)), (run, op)
+            assert np.array_equal(host(gv), fold.reduceat(v, starts), equal_nan=True), (run, op)
