@@ -165,6 +165,7 @@ scan_window_kernel(InIt in, T* out, size_t n, size_t tiles, unsigned tiles_per_c
   const T ID = op_identity<Op, T>::value();
   __shared__ T s_part[2][NWARPS];          // each warp's total of its part of the chunk, by window parity
   __shared__ T s_fold[2][NWARPS];          // per warp: fold of the chunks before this CTA's, of all chunks
+  __shared__ T s_first;                    // what a loop would start from (first_value_rules)
   const int lane = lane_id(), warp = threadIdx.x >> 5;
   const size_t G = gridDim.x, c = blockIdx.x;
   const size_t wtiles = (n + WT - 1) / WT;
@@ -224,6 +225,11 @@ scan_window_kernel(InIt in, T* out, size_t n, size_t tiles, unsigned tiles_per_c
   };
 
   T running = has_init ? init : ID;   // init (+) everything before the current window
+  if constexpr (first_value_rules<Op>::value) {
+    // read before this CTA publishes, so before anybody stores: the iterator may read from where the output goes
+    if (threadIdx.x == 0) s_first = has_init ? init : (T)in[0];
+    __syncthreads();
+  }
   phase_a(0);
   for (size_t w = 0; w < windows; ++w) {
     if (w + 1 < windows) phase_a(w + 1);
@@ -312,6 +318,11 @@ scan_window_kernel(InIt in, T* out, size_t n, size_t tiles, unsigned tiles_per_c
 #pragma unroll
           for (int k = 1; k < VEC; ++k) y[k] = op(E, x[v][k - 1]);
         }
+        if constexpr (first_value_rules<Op>::value) {
+          const T first = s_first;
+#pragma unroll
+          for (int k = 0; k < VEC; ++k) if (first != first) y[k] = first;
+        }
         const size_t i0 = base + (size_t)(v * 32 + lane) * VEC;
         if (full) {
           vec16 o;
@@ -338,7 +349,11 @@ template <class Kernel> int resident_ctas(Kernel kernel, int block, size_t smem)
 
 // Where the pipeline starts: 2^20 int32 12.4 us against 15.4 single-pass, 2^18 12.0 against 12.4.
 constexpr size_t SCAN_PIPE_MIN_BYTES = (size_t)1 << 22;
-constexpr size_t SCAN_PIPE_MIN_BYTES_MINMAX = (size_t)1 << 24;   // floating min / max, see scan_async
+// inputs of two tiles and more for every CTA of the windowed kernel: where that one starts
+template <class T> bool scan_fills_windows(size_t n) {
+  const size_t tile = (size_t)SCAN_BLOCK * scanw_tuning<T>::IPT, ctas = (size_t)current_device_info().sm_count * SCANW_CTAS_PER_SM;
+  return (n + tile - 1) / tile >= SCANW_MIN_TILES_PER_CTA * ctas;
+}
 
 template <class T> size_t scan_tile_items() { return (size_t)SCAN_BLOCK * scan_tuning<T>::IPT; }
 // descriptors of the windowed route: one per chunk, the last window padded to a whole grid
@@ -354,13 +369,14 @@ template <class T> size_t scan_workspace_bytes(size_t n) {
 }
 
 // The windowed route: launches it if the input is large enough for windows to pay (launched = true).
-template <bool INCLUSIVE, class InIt, class T, class Op>
-cudaError_t scan_window_launch(InIt in, T* out, size_t n, T init, bool has_init, const T* d_init, Op op, char* base, ws_header* hdr,
+template <bool INCLUSIVE, class InIt, class T, class CallerOp>
+cudaError_t scan_window_launch(InIt in, T* out, size_t n, T init, bool has_init, const T* d_init, CallerOp, char* base, ws_header* hdr,
                                cudaStream_t stream, bool& launched) {
   launched = false;
   constexpr int VEC = 16 / sizeof(T);
   constexpr int IPT2 = scanw_tuning<T>::IPT;
   const size_t tiles2 = (n + (size_t)SCAN_BLOCK * IPT2 - 1) / ((size_t)SCAN_BLOCK * IPT2);
+  using Op = typename route_op<CallerOp, T>::type;
   auto kern = scan_window_kernel<InIt, T, Op, INCLUSIVE, VEC, IPT2>;
   static thread_local int resident[64] = {0};
   int dev = 0;
@@ -377,7 +393,7 @@ cudaError_t scan_window_launch(InIt in, T* out, size_t n, T init, bool has_init,
   if (e3 != cudaSuccess) return e3;
   launched = true;
   timed_launch tl(KID_SCAN, stream);
-  kern<<<(unsigned)grid, SCAN_BLOCK, 0, stream>>>(in, out, n, tiles2, tpc, init, has_init, d_init, op, tsw, hdr);
+  kern<<<(unsigned)grid, SCAN_BLOCK, 0, stream>>>(in, out, n, tiles2, tpc, init, has_init, d_init, Op(), tsw, hdr);
   log_launch("scan_window_kernel", grid, SCAN_BLOCK, 0, n, stream);
   return cudaGetLastError();
 }
@@ -401,10 +417,10 @@ cudaError_t scan_async(InIt in, OutIt out, size_t n, T init, bool has_init, Op o
     if constexpr (vec_ok) {
       vectors = is_aligned16(in) && is_aligned16(out);
       if constexpr (is_commutative_op<Op>::value) {
-        // NaNs make floating min and max depend on the grouping: those keep the single-pass kernel's up to the size at which they always left it
-        constexpr bool regrouping_shows = std::is_floating_point<T>::value && !std::is_same<Op, plus_op>::value;
-        const size_t floor_bytes = regrouping_shows ? SCAN_PIPE_MIN_BYTES_MINMAX : SCAN_PIPE_MIN_BYTES;
-        if (vectors && n * sizeof(T) >= floor_bytes) {
+        // With NaNs among the values the single-pass kernel's floating min and max depend on its grouping; the pipeline's
+        // do not (skip_nan).  So that no size's results change with it, they leave the single-pass kernel where they always did.
+        constexpr bool grouping_shows = first_value_rules<typename route_op<Op, T>::type>::value;
+        if (vectors && (grouping_shows ? scan_fills_windows<T>(n) : n * sizeof(T) >= SCAN_PIPE_MIN_BYTES)) {
           bool launched = false;
           cudaError_t e2 = scan_pipe_launch<INCLUSIVE, T, Op>(in, out, n, init, has_init, d_init, ws, stream, launched);
           if (launched || e2 != cudaSuccess) return e2;
@@ -417,9 +433,7 @@ cudaError_t scan_async(InIt in, OutIt out, size_t n, T init, bool has_init, Op o
   if constexpr (!std::is_pointer<InIt>::value && std::is_pointer<OutIt>::value && is_commutative_op<Op>::value) {
     using Out = typename std::remove_pointer<OutIt>::type;
     if constexpr (std::is_same<Out, T>::value && std::is_arithmetic<T>::value && (sizeof(T) == 4 || sizeof(T) == 8)) {
-      const size_t ctas = (size_t)current_device_info().sm_count * SCANW_CTAS_PER_SM;
-      const size_t tiles2 = (n + (size_t)SCAN_BLOCK * scanw_tuning<T>::IPT - 1) / ((size_t)SCAN_BLOCK * scanw_tuning<T>::IPT);
-      if (is_aligned16(out) && tiles2 >= SCANW_MIN_TILES_PER_CTA * ctas) {
+      if (is_aligned16(out) && scan_fills_windows<T>(n)) {
         bool launched = false;
         cudaError_t e3 = scan_window_launch<INCLUSIVE>(in, out, n, init, has_init, d_init, op, base, hdr, stream, launched);
         if (launched || e3 != cudaSuccess) return e3;

@@ -1,5 +1,5 @@
 // Inclusive / exclusive scan of large contiguous inputs on sm_100a on the tile pipeline (tile_pipe.cuh), for
-// operators with an identity on 4- and 8-byte arithmetic types.  A tile is read from HBM once into shared
+// operators with an identity on 4- and 8-byte arithmetic types (floating min and max as skip_nan).  A tile is read from HBM once into shared
 // memory; the compute warps reduce it there ahead of time, and once its carry is known scan it from the
 // same shared memory and stream the result out: 2 * sizeof(T) bytes of HBM traffic per element and no
 // second trip of the input through L2.  Bound by HBM: 2^28 int32 or fp32 0.33 ms (6470 GB/s; 0.43 with the input
@@ -48,6 +48,10 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
     pipe_folder(st, chain, tiles, first, &hdr->error, [](const C&) {});
   } else {
     const int mine = warp % PIPE_WARPS;
+    // what a loop would start from: if that is a NaN, so is every result (in place in[0] is stored unchanged)
+    T first = T();
+    if constexpr (first_value_rules<Op>::value) first = init_ptr ? *init_ptr : has_init ? init : in[0];
+    const bool stuck = first != first;
     auto rows_of = [&](unsigned s) { return reinterpret_cast<const vec16*>(stages + (size_t)s * PIPE_TILE_BYTES) + mine * (PIPE_ROWS * 32) + lane; };
     pipe_compute<false>(st, tiles, &hdr->error,
       [&](unsigned s, unsigned) {
@@ -115,6 +119,10 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
 #pragma unroll
             for (int k = 0; k < VEC; ++k) y[k] = op(carry, y[k]);
           }
+          if constexpr (first_value_rules<Op>::value) {
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) if (stuck) y[k] = first;
+          }
           const size_t i0 = base + (size_t)(v * 32 + lane) * VEC;
           if (full) {
             vec16 o;
@@ -135,9 +143,10 @@ template <class T> constexpr size_t scan_pipe_tile_items() { return PIPE_TILE_BY
 
 // Launches the pipeline scan if the device can hold it (launched = true).  `in` and `out` are 16-byte aligned;
 // they may be the same array.  The workspace holds the header and one descriptor per tile.
-template <bool INCLUSIVE, class T, class Op>
+template <bool INCLUSIVE, class T, class CallerOp>
 cudaError_t scan_pipe_launch(const T* in, T* out, size_t n, T init, bool has_init, const T* d_init, void* ws, cudaStream_t stream, bool& launched) {
   launched = false;
+  using Op = typename route_op<CallerOp, T>::type;
   const size_t tiles = (n + scan_pipe_tile_items<T>() - 1) / scan_pipe_tile_items<T>();
   if (tiles >= 0xffffff00ull) return cudaSuccess;
   static thread_local bool ready[64] = {false};

@@ -185,3 +185,36 @@ def test_full_size_reduce_and_scan(tb, oracles):
     assert int(out[-1]) == int(tb.reduce(s, np.int64(0)))
     ex = tb.exclusive_scan(s, 0)
     assert torch.equal(ex[1:], out[:-1]) and int(ex[0]) == 0
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("items", [2 * 592 * 4096, 2 * 592 * 4096 + 4099, (1 << 24) + 5])
+def test_float_min_max_scan_of_nans(tb, port, dt, items):
+    """From the size on at which floating min and max take the pipeline: leading NaNs, whole tiles of them and single ones
+    come out as the oracle's loop gives them, and no value appears that is not in the input."""
+    n = items * 4 // np.dtype(dt).itemsize
+    base = (dg.rand64(51, n) % np.uint64(1 << 20)).astype(dt) - dt(1 << 19)
+    strewn, lead, tiles = base.copy(), base.copy(), base.copy()
+    strewn[dg.rand64(52, n) % np.uint64(5) == 0] = np.nan
+    strewn[0] = 7.0
+    lead[:3] = np.nan
+    tiles[1:8192 * 150] = np.nan
+    for x in (strewn, lead, tiles, np.full(n, np.nan, dt), np.full(n, np.inf, dt)):
+        for op in ("min", "max"):
+            d, want = dev(x), port.inclusive_scan(x, op)
+            assert np.array_equal(host(tb.inclusive_scan(d, op=op)), want, equal_nan=True), op
+            for init in (3.0, float("nan")):
+                excl = port.exclusive_scan(x, dt(init), op)
+                assert np.array_equal(host(tb.exclusive_scan(d, init, op=op)), excl, equal_nan=True), (op, init)
+                assert np.array_equal(host(tb.inclusive_scan(d, op=op, init=init))[:-1], excl[1:], equal_nan=True), (op, init)
+            tb.inclusive_scan(d, out=d, op=op)
+            assert np.array_equal(host(d), want, equal_nan=True), op
+
+
+@pytest.mark.parametrize("op", ["min", "max"])
+def test_float_min_max_scan_keeps_its_first_value(tb, op):
+    """At every size an inclusive scan's first output is its first input."""
+    for n in (1, 100, 8193, 1 << 20, (1 << 22) + 3):
+        x = torch.zeros(n, device="cuda")
+        x[0] = float("nan")
+        assert bool(torch.isnan(tb.inclusive_scan(x, op=op)[0])), n
