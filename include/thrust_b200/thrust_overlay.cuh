@@ -444,8 +444,9 @@ thrust::pair<SelectedOutIt, RejectedOutIt> partition_copy(Policy& policy, InputI
                                                            RejectedOutIt rejected, Pred pred) {
   return cuda_cub::stable_partition_copy(policy, first, last, stencil, selected, rejected, pred);
 }
-// in place: kept items first and dropped items mirrored into a scratch copy, then written back in
-// order -- always the stable result, which also satisfies thrust::partition
+// in place, always the stable result, which also satisfies thrust::partition.  Plain arrays: partition_inplace_async, which
+// takes the pipeline where it may; any other iterator: kept items first and dropped items mirrored into a scratch copy, then
+// written back in order
 template <class Policy, class It, class Pred, tb200_overlay::enable_for<Policy> = 0>
 It stable_partition(Policy& policy, It first, It last, Pred pred) {
   namespace ov = tb200_overlay;
@@ -456,13 +457,18 @@ It stable_partition(Policy& policy, It first, It last, Pred pred) {
   ov::scratch<Policy> tmp(policy, wsb + n * sizeof(T));
   T* copy = reinterpret_cast<T*>(tmp.at(wsb));
   auto in = ov::unwrap(first);
-  cudaError_t e = ::tb200::select_async<::tb200::SEL_PRED, true>(in, in, copy, copy, n, T(), pred, true, nullptr, tmp.at(), cuda_cub::stream(policy));
-  cuda_cub::throw_on_error(e, "partition failed");
-  const ::tb200::device_info& di = ::tb200::current_device_info();
-  std::size_t grid = (n + 2047) / 2048;
-  if (grid > (std::size_t)di.sm_count * 8) grid = (std::size_t)di.sm_count * 8;
-  ::tb200::partition_finish_kernel<<<(unsigned)grid, 256, 0, cuda_cub::stream(policy)>>>(in, (const T*)copy, n, reinterpret_cast<const ::tb200::ws_header*>(tmp.at()));
-  return first + ov::finish(policy, cudaGetLastError(), tmp.at(), "partition failed");
+  if constexpr (std::is_same<decltype(in), T*>::value) {
+    const cudaError_t pe = ::tb200::partition_inplace_async(in, copy, n, pred, nullptr, tmp.at(), cuda_cub::stream(policy));
+    return first + ov::finish(policy, pe, tmp.at(), "partition failed");
+  } else {
+    cudaError_t e = ::tb200::select_async<::tb200::SEL_PRED, true>(in, in, copy, copy, n, T(), pred, true, nullptr, tmp.at(), cuda_cub::stream(policy));
+    cuda_cub::throw_on_error(e, "partition failed");
+    const ::tb200::device_info& di = ::tb200::current_device_info();
+    std::size_t grid = (n + 2047) / 2048;
+    if (grid > (std::size_t)di.sm_count * 8) grid = (std::size_t)di.sm_count * 8;
+    ::tb200::partition_finish_kernel<<<(unsigned)grid, 256, 0, cuda_cub::stream(policy)>>>(in, (const T*)copy, n, reinterpret_cast<const ::tb200::ws_header*>(tmp.at()));
+    return first + ov::finish(policy, cudaGetLastError(), tmp.at(), "partition failed");
+  }
 }
 template <class Policy, class It, class StencilIt, class Pred, tb200_overlay::enable_for<Policy> = 0>
 It stable_partition(Policy& policy, It first, It last, StencilIt stencil, Pred pred) {
