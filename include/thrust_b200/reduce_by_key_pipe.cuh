@@ -147,6 +147,11 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
     });
   } else {
     const int mine = warp % PIPE_WARPS;
+    // the key in front of the stage's tile, for its first warp; the input's first key is compared with itself (and opens a
+    // run whatever comes out), because `eq` may only ever see keys of the input
+    auto tile_front = [&](unsigned s, unsigned tile) {
+      return tile > 0 ? reinterpret_cast<const K*>(&s_edge[s])[16 / sizeof(K) - 1] : Shape::Keys::part(stages + s * Shape::STAGE_BYTES, 0)[0];
+    };
     // this lane's items and their head flags, bit v * VEC + k; items past the end are no heads and hold the identity;
     // `edge`: the key in front of the warp's part
     auto load_heads = [&](unsigned s, unsigned tile, const K& edge, K (&k)[ROWS][VEC], V (&x)[ROWS][VEC]) {
@@ -191,7 +196,7 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
         K k[ROWS][VEC]; V x[ROWS][VEC];
         // nobody compacts its part of this tile before every warp has been here
         unsigned char* const kstage = stages + s * Shape::STAGE_BYTES;
-        const K edge = mine > 0 ? Shape::Keys::part(kstage, mine > 0 ? mine - 1 : 0)[PART - 1] : reinterpret_cast<const K*>(&s_edge[s])[16 / sizeof(K) - 1];
+        const K edge = mine > 0 ? Shape::Keys::part(kstage, mine > 0 ? mine - 1 : 0)[PART - 1] : tile_front(s, tile);
         if (lane == 0) s_last[s][mine] = Shape::Keys::part(kstage, mine)[PART - 1];
         const unsigned bits = load_heads(s, tile, edge, k, x);
         // only what lies behind the part's last head counts: later rows entirely, the head's row from the head's lane on
@@ -214,7 +219,7 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
       },
       [&](unsigned s, unsigned tile) {
         K k[ROWS][VEC]; V x[ROWS][VEC];
-        const K edge = mine > 0 ? s_last[s][mine > 0 ? mine - 1 : 0] : reinterpret_cast<const K*>(&s_edge[s])[16 / sizeof(K) - 1];
+        const K edge = mine > 0 ? s_last[s][mine > 0 ? mine - 1 : 0] : tile_front(s, tile);
         const unsigned bits = load_heads(s, tile, edge, k, x);
         K* const kbuf = Shape::Keys::part(stages + s * Shape::STAGE_BYTES, mine);
         V* const vbuf = Shape::Vals::part(stages + s * Shape::STAGE_BYTES + Shape::Keys::BYTES, mine);

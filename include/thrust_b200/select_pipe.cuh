@@ -63,6 +63,11 @@ select_pipe_kernel(const T* in, T* out_sel, T* out_rej, size_t n, unsigned tiles
     pipe_folder(st, chain, tiles, (C)0, &hdr->error, [&](C total) { hdr->count = total; if (d_count) *d_count = total; });
   } else {
     const int mine = warp % PIPE_WARPS;
+    // UNIQUE: the item in front of the stage's tile, for its first warp.  Nothing lies in front of the input: its first item is
+    // then compared with itself (and kept whatever comes out), because `pred` may only ever see items of the input
+    auto tile_front = [&](unsigned s, unsigned tile) {
+      return tile > 0 ? reinterpret_cast<const T*>(&s_edge[UNIQUE ? s : 0])[VEC - 1] : Parts::part(stages + (size_t)s * Parts::BYTES, 0)[0];
+    };
     // this lane's items of the warp's part and their keep flags, bit v * VEC + k
     static_assert(PIPE_ROWS * VEC <= 32, "a lane's flags fit a word");
     auto load_flags = [&](unsigned s, unsigned tile, const T& edge, T (&x)[PIPE_ROWS][VEC]) {
@@ -108,7 +113,7 @@ select_pipe_kernel(const T* in, T* out_sel, T* out_rej, size_t n, unsigned tiles
         T edge = T();
         if constexpr (UNIQUE) {
           // nobody compacts its part of this tile before every warp has been here
-          edge = mine > 0 ? Parts::part(stages + (size_t)s * Parts::BYTES, mine > 0 ? mine - 1 : 0)[CHUNK - 1] : reinterpret_cast<const T*>(&s_edge[s])[VEC - 1];
+          edge = mine > 0 ? Parts::part(stages + (size_t)s * Parts::BYTES, mine > 0 ? mine - 1 : 0)[CHUNK - 1] : tile_front(s, tile);
           if (lane == 0) s_last[s][mine] = Parts::part(stages + (size_t)s * Parts::BYTES, mine)[CHUNK - 1];
         }
         return __reduce_add_sync(FULL_MASK, (unsigned)__popc(load_flags(s, tile, edge, x)));
@@ -116,7 +121,7 @@ select_pipe_kernel(const T* in, T* out_sel, T* out_rej, size_t n, unsigned tiles
       [&](unsigned s, unsigned tile) {
         T x[PIPE_ROWS][VEC];
         T edge = T();
-        if constexpr (UNIQUE) edge = mine > 0 ? s_last[s][mine > 0 ? mine - 1 : 0] : reinterpret_cast<const T*>(&s_edge[s])[VEC - 1];
+        if constexpr (UNIQUE) edge = mine > 0 ? s_last[s][mine > 0 ? mine - 1 : 0] : tile_front(s, tile);
         const unsigned bits = load_flags(s, tile, edge, x);
         T* const buf = Parts::part(stages + (size_t)s * Parts::BYTES, mine);
         __syncwarp();   // every lane has its items: the part may be overwritten

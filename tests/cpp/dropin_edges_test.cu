@@ -1,5 +1,5 @@
 // Corners of the drop-in, compiled like dropin_test.cu: in-place partition of plain arrays and of other iterators at ragged
-// sizes, comparator sorts of keys around the size at which the
+// sizes, functors that must only ever see the caller's own elements, comparator sorts of keys around the size at which the
 // sort's tile changes.  With THRUST_B200_LOG=1 in the environment the launches name the kernels that served the calls.
 #include <thrust/device_vector.h>
 #include <thrust/execution_policy.h>
@@ -7,9 +7,11 @@
 #include <thrust/host_vector.h>
 #include <thrust/iterator/zip_iterator.h>
 #include <thrust/partition.h>
+#include <thrust/reduce.h>
 #include <thrust/sequence.h>
 #include <thrust/sort.h>
 #include <thrust/tuple.h>
+#include <thrust/unique.h>
 
 #include <algorithm>
 #include <cstdio>
@@ -47,6 +49,27 @@ template <class T> static void check_partition(int n) {
 }
 struct first_below { int bound; template <class Z> __host__ __device__ bool operator()(const Z& z) const { return thrust::get<0>(z) < bound; } };
 
+// ---- functors that report an argument which is not one of the caller's elements
+struct same_in_range {
+  int lo, hi; int* strange;
+  __device__ bool operator()(int a, int b) const { if (a < lo || a > hi || b < lo || b > hi) atomicExch(strange, 1); return a == b; }
+};
+static void check_functors(int n) {
+  std::vector<int> h(n);
+  for (int i = 0; i < n; ++i) h[i] = 1000000 + i / 3;
+  const int runs = (n + 2) / 3;
+  thrust::device_vector<int> d(h.begin(), h.end()), out(n), ones(n, 1), sums(n), strange(1, 0);
+  const same_in_range eq{1000000, h.back(), thrust::raw_pointer_cast(strange.data())};
+  // leave other numbers in shared memory first: a reduction over small values
+  thrust::device_vector<int> noise(1 << 22, 7);
+  thrust::sort(thrust::device, noise.begin(), noise.end());
+  CHECK(thrust::unique_copy(thrust::device, d.begin(), d.end(), out.begin(), eq) - out.begin() == runs);
+  CHECK(strange[0] == 0);
+  const auto e = thrust::reduce_by_key(thrust::device, d.begin(), d.end(), ones.begin(), out.begin(), sums.begin(), eq);
+  CHECK(e.first - out.begin() == runs && thrust::reduce(thrust::device, sums.begin(), e.second, 0) == n);
+  CHECK(strange[0] == 0);
+}
+
 // ---- comparator sorts of struct keys
 template <int WORDS> struct key { int w[WORDS]; };
 struct by_first_word { template <class K> __host__ __device__ bool operator()(const K& a, const K& b) const { return a.w[0] < b.w[0]; } };
@@ -69,6 +92,8 @@ int main() {
   { const int n = 300007; thrust::device_vector<int> a(n), b(n); thrust::sequence(a.begin(), a.end()); thrust::sequence(b.begin(), b.end());
     const auto z = thrust::make_zip_iterator(thrust::make_tuple(a.begin(), b.begin()));
     CHECK(thrust::stable_partition(thrust::device, z, z + n, first_below{1000}) - z == 1000); }
+  check_functors(1 << 18);
+  check_functors(3000001);
   check_sort<4>(50021); check_sort<5>(50021); check_sort<5>(100); check_sort<6>(50021);
   if (cudaDeviceSynchronize() != cudaSuccess) { std::printf("FAILED: sticky CUDA error\n"); ++failures; }
   std::printf(failures ? "dropin_edges_test: %d FAILURES\n" : "dropin_edges_test: all checks passed\n", failures);

@@ -28,8 +28,8 @@ def test_thrust_program_runs_on_overlay(tb, tmp_path):
 
 
 def test_corners_of_the_drop_in(tb, tmp_path):
-    """tests/cpp/dropin_edges_test.cu: in-place partition of plain arrays takes the pipeline from 1 MB on; struct keys
-    around a change of the sort's tile."""
+    """tests/cpp/dropin_edges_test.cu: in-place partition of plain arrays takes the pipeline from 1 MB on; functors see only the
+    caller's elements; struct keys around a change of the sort's tile."""
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.isfile(nvcc):
         pytest.skip("nvcc is not available on this machine")
