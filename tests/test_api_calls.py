@@ -93,3 +93,22 @@ def test_threads_on_one_stream_get_their_own_answers(fake, name):
     for t in threads:
         t.join()
     assert got == ([45, 190] if name == "reduce" else [9, 19])
+
+
+@pytest.mark.parametrize("name", ["reduce", "copy_if"])
+def test_a_refused_call_is_made_again_only_for_its_size(fake, name):
+    """Error 1 from behind the size check is an error of the call, which may have launched something: raised, not retried.
+    A workspace that is too small is replaced and the call made once more."""
+    x = torch.arange(10, dtype=torch.int64)
+    call = (lambda: api.reduce(x)) if name == "reduce" else (lambda: api.copy_if(x, "ne", 3))
+    call()
+    assert fake.launches == [name]
+    fake.result = 1
+    with pytest.raises(api.Tb200Error, match="cudaError 1"):
+        call()
+    assert fake.launches == [name] * 2
+    fake.result = 0
+    key = api.workspaces.key("reduce" if name == "reduce" else "select")
+    api.workspaces._bufs[key] = torch.empty(NEED - 1, dtype=torch.uint8)
+    call()
+    assert fake.launches == [name] * 3 and api.workspaces.kept(key).numel() == NEED

@@ -97,24 +97,36 @@ class _Workspaces:
 workspaces = _Workspaces()
 
 
-_TOO_SMALL = 1      # cudaErrorInvalidValue: the workspace is too small (or another argument is wrong)
+_TOO_SMALL = 1      # cudaErrorInvalidValue: the workspace is too small, or something else about the call is wrong
 
 
-def _enqueue(key, fn, args):
-    """fn(*args, d_ws, &ws_bytes, stream) in the workspace kept under `key`, whose lock the caller holds; the size is
-    asked for only if there is none yet or it is refused as too small.  Returns the workspace."""
+def _enqueue(key, fn, args, result=None):
+    """fn(*args, d_ws, &ws_bytes, stream) in the workspace kept under `key`, whose lock the caller holds; with `result`, an
+    offset into the workspace, its address goes in front of d_ws.  The size is asked for only if there is no workspace yet
+    or the call is refused, and the call made again only if the workspace was indeed too small (then nothing was
+    launched: every entry point checks the size first).  Returns the workspace."""
     lib_fn = getattr(_lib.load(), fn)
     stream = key[1]
+
+    def call(ws):
+        at = ws.data_ptr()
+        out = () if result is None else (at + result,)
+        return lib_fn(*args, *out, at, C.byref(C.c_size_t(ws.numel())), stream)
+
     ws = workspaces.kept(key)
+    rc = None
     if ws is not None:
-        rc = lib_fn(*args, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream)
+        rc = call(ws)
         if rc != _TOO_SMALL:
             _check(rc, fn)
             return ws
     need = C.c_size_t(0)
-    _check(lib_fn(*args, None, C.byref(need), stream), fn + " (size query)")
+    none = () if result is None else (None,)
+    _check(lib_fn(*args, *none, None, C.byref(need), stream), fn + " (size query)")
+    if ws is not None and ws.numel() >= need.value:
+        _check(rc, fn)
     ws = workspaces.get(key[2], need.value, key)
-    _check(lib_fn(*args, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream), fn)
+    _check(call(ws), fn)
     return ws
 
 
@@ -163,22 +175,11 @@ def reduce(x, init=None, op="plus", acc_dtype=None):
         acc_dtype = x.dtype if init is None or not isinstance(init, np.generic) else TORCH_OF[np.dtype(init.dtype)]
     h_init = np.asarray(0 if init is None else init, dtype=NP_OF[acc_dtype])
     # the result lands in the workspace's header and comes back together with the status
-    lib_fn = _lib.load().tb200_reduce
     key = workspaces.key("reduce")
-    stream = key[1]
     args = (_ptr(x), x.numel(), DTYPE_CODE[x.dtype], DTYPE_CODE[acc_dtype], OPS[op], h_init.ctypes.data)
     with workspaces.lock(key):
-        ws = workspaces.kept(key)
-        rc = _TOO_SMALL
-        if ws is not None:
-            rc = lib_fn(*args, ws.data_ptr() + _HEADER_RESULT, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream)
-        if rc == _TOO_SMALL:
-            need = C.c_size_t(0)
-            _check(lib_fn(*args, None, None, C.byref(need), stream), "tb200_reduce (size query)")
-            ws = workspaces.get("reduce", need.value, key)
-            rc = lib_fn(*args, ws.data_ptr() + _HEADER_RESULT, ws.data_ptr(), C.byref(C.c_size_t(ws.numel())), stream)
-        _check(rc, "tb200_reduce")
-        head = _read_header(ws, "reduce", _HEADER_RESULT + 8, stream)
+        ws = _enqueue(key, "tb200_reduce", args, _HEADER_RESULT)
+        head = _read_header(ws, "reduce", _HEADER_RESULT + 8, key[1])
     return np.frombuffer(head.raw, dtype=NP_OF[acc_dtype], count=1, offset=_HEADER_RESULT)[0]
 
 
