@@ -392,6 +392,12 @@ __device__ __forceinline__ void st_relaxed_b128(void* p, unsigned long long lo, 
 __device__ __forceinline__ void ld_relaxed_b128(const void* p, unsigned long long& lo, unsigned long long& hi) {
   asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
 }
+__device__ __forceinline__ void st_release_b128(void* p, unsigned long long lo, unsigned long long hi) {
+  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.release.gpu.global.b128 [%0], t;\n\t}" ::"l"(p), "l"(lo), "l"(hi) : "memory");
+}
+__device__ __forceinline__ void ld_acquire_b128(const void* p, unsigned long long& lo, unsigned long long& hi) {
+  asm volatile("{\n\t.reg .b128 t;\n\tld.acquire.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+}
 
 template <class T> struct tile_state_mode {
   static constexpr int value = (sizeof(T) == 4 && std::is_trivially_copyable<T>::value) ? 1
@@ -428,6 +434,18 @@ template <class T> struct tile_state<T, 2> {
   __device__ __forceinline__ unsigned poll(size_t tile, T& v) const {
     unsigned long long u, st;
     ld_relaxed_b128(words + 2 * tile, u, st);
+    memcpy(&v, &u, 8);
+    return (unsigned)st;
+  }
+  // the same, where the descriptor also orders what the two sides do to other memory
+  __device__ __forceinline__ void publish_release(size_t tile, unsigned status, const T& v) const {
+    unsigned long long u;
+    memcpy(&u, &v, 8);
+    st_release_b128(words + 2 * tile, u, (unsigned long long)status);
+  }
+  __device__ __forceinline__ unsigned poll_acquire(size_t tile, T& v) const {
+    unsigned long long u, st;
+    ld_acquire_b128(words + 2 * tile, u, st);
     memcpy(&v, &u, 8);
     return (unsigned)st;
   }

@@ -138,9 +138,9 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
       else if (lane < 2 * PIPE_WARPS) Shape::Vals::copy(vstage, vals + base, left, lane - PIPE_WARPS, &st.full[s], policy);
     });
   } else if (warp == PIPE_PUBLISHER) {
-    pipe_publisher(st, chain, tiles, &hdr->error, [&](const rbk_part<V>& part) { return fold_parts(lane < PIPE_WARPS ? Chain::lift(part) : Chain::identity()); });
+    pipe_publisher<false>(st, chain, tiles, &hdr->error, [&](const rbk_part<V>& part) { return fold_parts(lane < PIPE_WARPS ? Chain::lift(part) : Chain::identity()); });
   } else if (warp == PIPE_FOLDER) {
-    pipe_folder(st, chain, tiles, Chain::identity(), &hdr->error, [&](const C& all) {
+    pipe_folder<false>(st, chain, tiles, Chain::identity(), &hdr->error, [&](const C& all) {
       vals_out[all.heads - 1] = (V)all.value;   // the last run ends with the input
       hdr->count = all.heads;
       if (d_count) *d_count = all.heads;

@@ -36,7 +36,7 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
       }
     });
   } else if (warp == PIPE_PUBLISHER) {
-    pipe_publisher(st, chain, tiles, &hdr->error, [&](const T& part) {
+    pipe_publisher<false>(st, chain, tiles, &hdr->error, [&](const T& part) {
       C t = lane < PIPE_WARPS ? Chain::lift(part) : Chain::identity();
 #pragma unroll
       for (int d = 1; d < PIPE_WARPS; d <<= 1) t = Chain::join(t, shfl_down(t, d));   // lane 0: all parts, in order
@@ -45,7 +45,7 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
   } else if (warp == PIPE_FOLDER) {
     C first = Chain::identity();
     if (init_ptr) first = Chain::lift(*init_ptr); else if (has_init) first = Chain::lift(init);
-    pipe_folder(st, chain, tiles, first, &hdr->error, [](const C&) {});
+    pipe_folder<false>(st, chain, tiles, first, &hdr->error, [](const C&) {});
   } else {
     const int mine = warp % PIPE_WARPS;
     // what a loop would start from: if that is a NaN, so is every result (in place in[0] is stored unchanged)

@@ -213,7 +213,7 @@ cudaError_t select_async(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, si
       }
       if (ok && select_pipe_eligible(in, out_sel, rej, n, sizeof(T), KEEP_REJECTS)) {
         bool launched = false;
-        const cudaError_t pe = select_pipe_launch<MODE == SEL_UNIQUE, KEEP_REJECTS ? SELECT_SECOND_ARRAY : SELECT_DROP, T, Pred>(in, out_sel, rej, n, pred, d_count, ws, stream, launched);
+        const cudaError_t pe = select_pipe_launch<MODE == SEL_UNIQUE, KEEP_REJECTS ? SELECT_SECOND_ARRAY : SELECT_DROP, false, T, Pred>(in, out_sel, rej, n, pred, d_count, ws, stream, launched);
         if (launched || pe != cudaSuccess) return pe;
       }
     }
@@ -258,7 +258,7 @@ cudaError_t partition_finish_async(T* data, const T* scratch, size_t n, const vo
 // ones through `scratch`.
 template <class T, class Pred>
 cudaError_t partition_inplace_pipe_async(T* data, T* scratch, size_t n, Pred pred, unsigned long long* d_count, void* ws, cudaStream_t stream, bool& launched) {
-  cudaError_t e = select_pipe_launch<false, SELECT_SECOND_ARRAY, T, Pred>((const T*)data, data, scratch, n, pred, d_count, ws, stream, launched);
+  cudaError_t e = select_pipe_launch<false, SELECT_SECOND_ARRAY, true, T, Pred>((const T*)data, data, scratch, n, pred, d_count, ws, stream, launched);
   if (e != cudaSuccess || !launched) return e;
   size_t grid = (n + 256 * 16 - 1) / (256 * 16);
   if (grid > (size_t)current_device_info().sm_count * 8) grid = (size_t)current_device_info().sm_count * 8;

@@ -8,7 +8,9 @@
 //
 // In-place partition: a tile's carry is known only after every earlier tile has been summarised, so after
 // all of them lie in shared memory; the kept items' places (never behind the tile's own end) can then be
-// overwritten.  Only the dropped items take a trip through scratch memory (partition_rejects_kernel).
+// overwritten.  A carry must order those stores behind the other CTAs' copies of what lay there (the pipeline's ORDERED
+// form): with released and acquired descriptors the two kernels take 376 us at 2^27 int32, with relaxed ones 357, with
+// fences around relaxed ones 396.  Only the dropped items take a trip through scratch memory (partition_rejects_kernel).
 //
 // Measured on B200, 2^28 int32, half of the items kept (unique: a quarter), against two streaming passes that read
 // the input twice / one pass with look-back: copy_if 0.343 ms against 0.460 / 0.613, partition_copy 0.478 against
@@ -25,7 +27,8 @@ enum : int { SELECT_DROP = 0, SELECT_SECOND_ARRAY = 1 };
 
 template <class T> using select_parts = pipe_parts<T, PIPE_ROWS * 512 / (int)sizeof(T)>;
 
-template <bool UNIQUE, int REJ, class T, class Pred>
+// IN_PLACE: out_sel is the input
+template <bool UNIQUE, int REJ, bool IN_PLACE, class T, class Pred>
 __global__ void __launch_bounds__(PIPE_BLOCK, 1)
 select_pipe_kernel(const T* in, T* out_sel, T* out_rej, size_t n, unsigned tiles, Pred pred, tile_chain<unsigned long long, plus_op> chain, ws_header* hdr,
                    unsigned long long* d_count) {
@@ -58,9 +61,9 @@ select_pipe_kernel(const T* in, T* out_sel, T* out_rej, size_t n, unsigned tiles
       if (lane < PIPE_WARPS) Parts::copy(stage, in + base, n - base, lane, &st.full[s], policy);
     });
   } else if (warp == PIPE_PUBLISHER) {
-    pipe_publisher(st, chain, tiles, &hdr->error, [&](unsigned part) { return (C)__reduce_add_sync(FULL_MASK, lane < PIPE_WARPS ? part : 0u); });
+    pipe_publisher<IN_PLACE>(st, chain, tiles, &hdr->error, [&](unsigned part) { return (C)__reduce_add_sync(FULL_MASK, lane < PIPE_WARPS ? part : 0u); });
   } else if (warp == PIPE_FOLDER) {
-    pipe_folder(st, chain, tiles, (C)0, &hdr->error, [&](C total) { hdr->count = total; if (d_count) *d_count = total; });
+    pipe_folder<IN_PLACE>(st, chain, tiles, (C)0, &hdr->error, [&](C total) { hdr->count = total; if (d_count) *d_count = total; });
   } else {
     const int mine = warp % PIPE_WARPS;
     // UNIQUE: the item in front of the stage's tile, for its first warp.  Nothing lies in front of the input: its first item is
@@ -232,13 +235,13 @@ template <class T> size_t select_pipe_workspace_bytes(size_t n) {
 }
 
 // Launches the pipeline compaction if the device can hold it (launched = true).  `in` is 16-byte aligned.
-template <bool UNIQUE, int REJ, class T, class Pred>
+template <bool UNIQUE, int REJ, bool IN_PLACE, class T, class Pred>
 cudaError_t select_pipe_launch(const T* in, T* out_sel, T* out_rej, size_t n, Pred pred, unsigned long long* d_count, void* ws, cudaStream_t stream, bool& launched) {
   launched = false;
   const size_t tiles = (n + select_pipe_tile_items<T>() - 1) / select_pipe_tile_items<T>();
   if (tiles >= 0xffffff00ull || n == 0) return cudaSuccess;
   static thread_local bool ready[64] = {false};
-  auto kern = select_pipe_kernel<UNIQUE, REJ, T, Pred>;
+  auto kern = select_pipe_kernel<UNIQUE, REJ, IN_PLACE, T, Pred>;
   const size_t smem = pipe_smem_bytes(select_parts<T>::BYTES, 0);
   const size_t grid = pipe_grid(kern, smem, tiles, ready);
   if (grid == 0) return cudaSuccess;

@@ -138,6 +138,8 @@ template <class T, class Op> struct tile_chain {
   __device__ static C fold_round(const C (&v)[PIPE_SLOTS], int count) { return pipe_fold_round<tile_chain>(v, count); }
   __device__ void publish(size_t tile, unsigned status, const C& v) const { ts.publish(tile, status, v); }
   __device__ unsigned poll(size_t tile, C& v) const { return ts.poll(tile, v); }
+  __device__ void publish_release(size_t tile, unsigned status, const C& v) const { ts.publish_release(tile, status, v); }
+  __device__ unsigned poll_acquire(size_t tile, C& v) const { return ts.poll_acquire(tile, v); }
 };
 template <> struct tile_chain<float, plus_op> {
   using C = double;
@@ -262,14 +264,20 @@ __device__ __forceinline__ void pipe_loader(S& st, unsigned tiles, unsigned* err
     for (unsigned iter = 0; !mbar_try_wait(&st.full[i % PIPE_STAGES], (i / PIPE_STAGES) & 1) && iter < MBAR_SPIN_LIMIT; ++iter) {}
 }
 
+// Order between CTAs.  A descriptor is one word, stored and polled relaxed: its value is all that a CTA takes from another
+// one.  Where the output goes over the input (ORDERED: the in-place partition) it must also order this CTA's stores behind
+// the other CTAs' copies of what lay there: the publisher releases what its CTA has seen arrive, the folder acquires it.
+//
 // The publisher warp.  fold(part) turns the warps' summaries (lane w < PIPE_WARPS holds warp w's) into the tile's total, valid in lane 0.
-template <class S, class Chain, class Fold>
+template <bool ORDERED, class S, class Chain, class Fold>
 __device__ __forceinline__ void pipe_publisher(S& st, const Chain& chain, unsigned tiles, unsigned* err, Fold fold) {
   for (pipe_cursor cur; cur.tile < tiles; cur.next()) {
     pipe_wait(&st.summed[cur.stage], cur.parity, &st.dead, err);
     if (pipe_dead(st)) return;
     const auto total = fold(st.part[cur.stage][lane_id() & (PIPE_WARPS - 1)]);
-    if (lane_id() == 0) chain.publish(cur.tile, TILE_AGGREGATE, total);
+    if (lane_id() == 0) {
+      if constexpr (ORDERED) chain.publish_release(cur.tile, TILE_AGGREGATE, total); else chain.publish(cur.tile, TILE_AGGREGATE, total);
+    }
   }
 }
 
@@ -286,10 +294,11 @@ template <class Chain> __device__ __forceinline__ typename Chain::C pipe_fold_ro
 }
 
 // The folder warp.  last(total) is called by lane 0 of the last tile's CTA with everything up to the input's end.
-template <class S, class Chain, class Last>
+template <bool ORDERED, class S, class Chain, class Last>
 __device__ __forceinline__ void pipe_folder(S& st, const Chain& chain, unsigned tiles, const typename Chain::C& init, unsigned* err, Last last) {
   using C = typename Chain::C;
   const int lane = lane_id();
+  auto poll = [&](size_t tile, C& value) { if constexpr (ORDERED) return chain.poll_acquire(tile, value); else return chain.poll(tile, value); };
   typename Chain::R running = Chain::start(init);   // everything before the current round
   for (pipe_cursor cur; cur.tile < tiles; cur.next()) {
     const unsigned base = cur.tile - blockIdx.x, round = tiles - base < gridDim.x ? tiles - base : gridDim.x;
@@ -298,7 +307,7 @@ __device__ __forceinline__ void pipe_folder(S& st, const Chain& chain, unsigned 
 #pragma unroll
     for (int j = 0; j < PIPE_SLOTS; ++j) {
       status[j] = TILE_AGGREGATE; v[j] = Chain::identity();
-      if (j * 32 + lane < round) status[j] = chain.poll(base + j * 32 + lane, v[j]);
+      if (j * 32 + lane < round) status[j] = poll(base + j * 32 + lane, v[j]);
     }
     bool handed = false;
     for (unsigned iter = 0;; ++iter) {
@@ -311,6 +320,11 @@ __device__ __forceinline__ void pipe_folder(S& st, const Chain& chain, unsigned 
       }
       if (!handed && !__any_sync(FULL_MASK, before_missing)) {
         // the carry needs the CTAs before this one only (and this one's tile in its stage: what the stage held before is finished then)
+        // That this CTA's own descriptor was there implies that its warps have summarised the tile, but by way of a relaxed word
+        // in global memory.  Waiting for `summed` itself (it never has to) orders the warps' reads of each other's summaries,
+        // and their stores over items that their neighbours looked at, behind the summaries.
+        pipe_wait(&st.summed[cur.stage], cur.parity, &st.dead, err);
+        __syncwarp();
         const C carry = Chain::value(Chain::extend(running, Chain::fold_round(v, (int)blockIdx.x)));
         if (lane == 0) { st.carry[cur.stage] = carry; mbar_arrive(&st.carried[cur.stage]); }
         handed = true;
@@ -320,7 +334,7 @@ __device__ __forceinline__ void pipe_folder(S& st, const Chain& chain, unsigned 
       if (pipe_dead(st)) return;
       __nanosleep(PIPE_POLL_NS);
 #pragma unroll
-      for (int j = 0; j < PIPE_SLOTS; ++j) if (status[j] == TILE_INVALID) status[j] = chain.poll(base + j * 32 + lane, v[j]);
+      for (int j = 0; j < PIPE_SLOTS; ++j) if (status[j] == TILE_INVALID) status[j] = poll(base + j * 32 + lane, v[j]);
     }
     running = Chain::extend(running, Chain::fold_round(v, PIPE_MAX_GRID));
     if (cur.tile == tiles - 1 && lane == 0) last(Chain::value(running));
@@ -339,7 +353,7 @@ __device__ __forceinline__ void pipe_compute(S& st, unsigned tiles, unsigned* er
   unsigned idle = 0;
   while (cur.tile < tiles) {
     // whichever can be done now: a tile that has arrived is summarised (the other CTAs wait for its total), else the
-    // oldest one finished if its carry is known; a warp never sits on a ready carry because a load is late
+    // oldest one finished if its carry is known; a warp never sits on a ready carry because a load is late.
     if (ahead.tile < tiles && open <= PIPE_LOOKAHEAD && __all_sync(FULL_MASK, mbar_test(&st.full[ahead.stage], ahead.parity))) {
       __syncwarp();
       const auto part = summarise(ahead.stage, ahead.tile);

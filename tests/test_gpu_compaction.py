@@ -261,3 +261,20 @@ def test_reduce_by_key_float_min_max_of_nans(tb, kt, vt):
             gk, gv = tb.reduce_by_key(dev(k), dev(v), op=op)
             assert np.array_equal(host(gk), np.arange(starts.size).astype(kt)), (run, op)
             assert np.array_equal(host(gv), fold.reduceat(v, starts), equal_nan=True), (run, op)
+
+
+@pytest.mark.parametrize("keep", [0.5, 0.97, 1.0])
+def test_in_place_partition_over_its_own_input(tb, keep):
+    """Kept items land on what other CTAs read just before; with nearly all kept, on their neighbours' tiles.  Many passes, a
+    copy running beside them on another stream."""
+    n = (1 << 24) + 4099
+    x = dev((dg.rand64(62, n) % np.uint64(1 << 20)).astype(np.int32))
+    bound = int(keep * (1 << 20))
+    want = torch.cat([x[x < bound], x[x >= bound]])
+    d, other, side = torch.empty_like(x), torch.empty_like(x), torch.cuda.Stream()
+    for _ in range(50):
+        d.copy_(x)
+        with torch.cuda.stream(side):
+            other.copy_(x)
+        assert tb.partition(d, "lt", bound, 0) == int((x < bound).sum())
+        assert torch.equal(d, want)

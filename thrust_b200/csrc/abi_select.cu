@@ -19,7 +19,7 @@ int select_pred(const void* in, const void* stencil, int stencil_t, void* out_se
       if (tb200::select_pipe_eligible(in, out_sel, REJ ? out_rej : nullptr, n, sizeof(T), REJ)) {
         bool launched = false;
         const int rc = pred.visit([&](auto typed) {
-          return (int)tb200::select_pipe_launch<false, REJ ? tb200::SELECT_SECOND_ARRAY : tb200::SELECT_DROP, T, decltype(typed)>(i, os, orj, n, typed, d_count, d_ws,
+          return (int)tb200::select_pipe_launch<false, REJ ? tb200::SELECT_SECOND_ARRAY : tb200::SELECT_DROP, false, T, decltype(typed)>(i, os, orj, n, typed, d_count, d_ws,
                                                                                                                                 stream, launched);
         });
         if (launched || rc != 0) return rc;
