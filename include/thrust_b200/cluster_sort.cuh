@@ -260,9 +260,11 @@ cudaError_t cluster_sort_launch(UK* keys, UV* vals, size_t n, key_coding coding,
     largest[dev] = most;
   }
   if (ctas > largest[dev]) return cudaSuccess;
-  launched = true;
   timed_launch tl(KID_ONESWEEP, stream);
-  return cudaLaunchKernelEx(&cfg, kern, keys, vals, (unsigned)n, rows, coding, first_pass, num_passes, hdr);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, keys, vals, (unsigned)n, rows, coding, first_pass, num_passes, hdr);
+  if (launch_refused(e)) return cudaSuccess;
+  launched = true;
+  return e;
 }
 
 template <class UK, class UV, bool HAS_V>

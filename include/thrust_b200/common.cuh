@@ -141,6 +141,14 @@ inline void log_launch(const char* kernel, size_t grid, int block, size_t smem, 
   fprintf(stderr, "thrust_b200: %s<<<%zu, %d, %zu>>> items=%zu status=%s\n", kernel, grid, block, smem, items, cudaGetErrorName(e));
 }
 
+// A cooperative or cluster launch that the device cannot place -- a context that was given fewer SMs than the chip
+// has, say -- is refused before anything runs.  True for such an error, which is then cleared: another kernel serves the call.
+inline bool launch_refused(cudaError_t e) {
+  if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorLaunchOutOfResources && e != cudaErrorInvalidClusterSize) return false;
+  cudaGetLastError();
+  return true;
+}
+
 // ---------------------------------------------------------------- chains of dependent launches
 // A kernel launched with launch_after may be scheduled while its predecessor on the stream is still running; it calls
 // grid_dependency_wait() before it touches memory, which returns once the predecessor has completed and its writes

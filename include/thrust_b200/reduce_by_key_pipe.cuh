@@ -292,7 +292,7 @@ bool rbk_pipe_eligible(const K* keys, const V* vals, const K* keys_out, const V*
          apart(vals, sizeof(V), vals_out, sizeof(V));
 }
 
-// Launches the pipeline if the device can hold it (launched = true); n > 0.
+// Launches the pipeline if the device can hold it and takes the launch (launched = true); n > 0.
 template <class K, class V, class Eq, class Op>
 cudaError_t rbk_pipe_launch(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n, Eq eq, unsigned long long* d_count, void* ws, cudaStream_t stream,
                             bool& launched) {
@@ -311,9 +311,10 @@ cudaError_t rbk_pipe_launch(const K* keys, const V* vals, K* keys_out, V* vals_o
   chain.bind(base + sizeof(ws_header), tiles);
   cudaError_t e = cudaMemsetAsync(base, 0, sizeof(ws_header) + rbk_chain<V, Op>::bytes(tiles), stream);
   if (e != cudaSuccess) return e;
-  launched = true;
   timed_launch tl(KID_REDUCE_BY_KEY, stream);
   e = pipe_launch(kern, grid, smem, stream, keys, vals, keys_out, vals_out, n, (unsigned)tiles, eq, chain, hdr, d_count);
+  if (launch_refused(e)) return cudaSuccess;
+  launched = true;
   log_launch("rbk_pipe_kernel", grid, PIPE_BLOCK, smem, n, stream);
   return e;
 }

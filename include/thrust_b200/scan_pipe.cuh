@@ -141,7 +141,7 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
 
 template <class T> constexpr size_t scan_pipe_tile_items() { return PIPE_TILE_BYTES / sizeof(T); }
 
-// Launches the pipeline scan if the device can hold it (launched = true).  `in` and `out` are 16-byte aligned;
+// Launches the pipeline scan if the device can hold it and takes the launch (launched = true).  `in` and `out` are 16-byte aligned;
 // they may be the same array.  The workspace holds the header and one descriptor per tile.
 template <bool INCLUSIVE, class T, class CallerOp>
 cudaError_t scan_pipe_launch(const T* in, T* out, size_t n, T init, bool has_init, const T* d_init, void* ws, cudaStream_t stream, bool& launched) {
@@ -160,9 +160,10 @@ cudaError_t scan_pipe_launch(const T* in, T* out, size_t n, T init, bool has_ini
   chain.bind(base + sizeof(ws_header), tiles);
   cudaError_t e = cudaMemsetAsync(base, 0, sizeof(ws_header) + tile_chain<T, Op>::bytes(tiles), stream);
   if (e != cudaSuccess) return e;
-  launched = true;
   timed_launch tl(KID_SCAN, stream);
   e = pipe_launch(kern, grid, smem, stream, in, out, n, (unsigned)tiles, init, has_init, d_init, chain, hdr);
+  if (launch_refused(e)) return cudaSuccess;
+  launched = true;
   log_launch("scan_pipe_kernel", grid, PIPE_BLOCK, smem, n, stream);
   return e;
 }

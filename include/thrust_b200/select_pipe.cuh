@@ -234,7 +234,7 @@ template <class T> size_t select_pipe_workspace_bytes(size_t n) {
   return sizeof(ws_header) + tile_chain<unsigned long long, plus_op>::bytes((n + select_pipe_tile_items<T>() - 1) / select_pipe_tile_items<T>());
 }
 
-// Launches the pipeline compaction if the device can hold it (launched = true).  `in` is 16-byte aligned.
+// Launches the pipeline compaction if the device can hold it and takes the launch (launched = true).  `in` is 16-byte aligned.
 template <bool UNIQUE, int REJ, bool IN_PLACE, class T, class Pred>
 cudaError_t select_pipe_launch(const T* in, T* out_sel, T* out_rej, size_t n, Pred pred, unsigned long long* d_count, void* ws, cudaStream_t stream, bool& launched) {
   launched = false;
@@ -251,9 +251,10 @@ cudaError_t select_pipe_launch(const T* in, T* out_sel, T* out_rej, size_t n, Pr
   chain.bind(base + sizeof(ws_header), tiles);
   cudaError_t e = cudaMemsetAsync(base, 0, sizeof(ws_header) + tile_chain<unsigned long long, plus_op>::bytes(tiles), stream);
   if (e != cudaSuccess) return e;
-  launched = true;
   timed_launch tl(KID_SELECT, stream);
   e = pipe_launch(kern, grid, smem, stream, in, out_sel, out_rej, n, (unsigned)tiles, pred, chain, hdr, d_count);
+  if (launch_refused(e)) return cudaSuccess;
+  launched = true;
   log_launch("select_pipe_kernel", grid, PIPE_BLOCK, smem, n, stream);
   return e;
 }
