@@ -40,6 +40,11 @@ template <class T> __device__ __forceinline__ void stash(T* slot, const T& v) {
 
 // Error codes a kernel may leave in the workspace status word (see ws_header).
 enum : unsigned { ERR_NONE = 0, ERR_LOOKBACK_TIMEOUT = 1, ERR_INCONSISTENT = 2 };   // 2: two evaluations of a tile disagree
+inline const char* error_text(unsigned code) {
+  return code == ERR_LOOKBACK_TIMEOUT ? "thrust_b200: an inter-CTA wait ran out"
+       : code == ERR_INCONSISTENT ? "thrust_b200: two looks at a tile disagree (a functor that does not answer the same twice, or is no order on the data)"
+       : "thrust_b200: a kernel reported an unknown error";
+}
 
 // Number of polls of a predecessor's status word before a look-back gives up, records
 // ERR_LOOKBACK_TIMEOUT and carries on with whatever it has.  Polls past the first few sleep

@@ -208,7 +208,8 @@ unsigned long long finish(Policy& policy, cudaError_t launch_status, const void*
   ::tb200::ws_header h;
   cuda_cub::throw_on_error(cudaMemcpyAsync(&h, ws, 16, cudaMemcpyDeviceToHost, cuda_cub::stream(policy)), what);
   cuda_cub::throw_on_error(cudaStreamSynchronize(cuda_cub::stream(policy)), what);
-  if (h.error != ::tb200::ERR_NONE) cuda_cub::throw_on_error(cudaErrorLaunchTimeout, "thrust_b200: an inter-CTA wait ran out");
+  if (h.error != ::tb200::ERR_NONE)
+    cuda_cub::throw_on_error(h.error == ::tb200::ERR_LOOKBACK_TIMEOUT ? cudaErrorLaunchTimeout : cudaErrorUnknown, ::tb200::error_text(h.error));
   return h.count;
 }
 

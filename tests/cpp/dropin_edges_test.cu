@@ -6,15 +6,19 @@
 #include <thrust/functional.h>
 #include <thrust/host_vector.h>
 #include <thrust/iterator/zip_iterator.h>
+#include <thrust/merge.h>
 #include <thrust/partition.h>
 #include <thrust/reduce.h>
 #include <thrust/sequence.h>
 #include <thrust/sort.h>
+#include <thrust/system_error.h>
 #include <thrust/tuple.h>
 #include <thrust/unique.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <vector>
 
 #ifndef THRUST_B200_OVERLAY_EXPECTED
@@ -70,6 +74,16 @@ static void check_functors(int n) {
   CHECK(strange[0] == 0);
 }
 
+// ---- what the kernels report comes out as the exception's text
+static void check_report(int n) {
+  std::vector<float> a(n), b(n);
+  for (int i = 0; i < n; ++i) { a[i] = (float)i; b[i] = (float)i; if (mix(i) % 10 == 0) a[i] = NAN; if (mix(i + n) % 10 == 0) b[i] = NAN; }
+  thrust::device_vector<float> da(a.begin(), a.end()), db(b.begin(), b.end()), dm(2 * n);
+  try { thrust::merge(thrust::device, da.begin(), da.end(), db.begin(), db.end(), dm.begin()); }
+  catch (const thrust::system_error& e) { CHECK(std::strstr(e.what(), "two looks at a tile disagree") != nullptr); return; }
+  CHECK(!"a merge of ranges that are not sorted went unnoticed");
+}
+
 // ---- comparator sorts of struct keys
 template <int WORDS> struct key { int w[WORDS]; };
 struct by_first_word { template <class K> __host__ __device__ bool operator()(const K& a, const K& b) const { return a.w[0] < b.w[0]; } };
@@ -94,6 +108,7 @@ int main() {
     CHECK(thrust::stable_partition(thrust::device, z, z + n, first_below{1000}) - z == 1000); }
   check_functors(1 << 18);
   check_functors(3000001);
+  check_report(200003);
   check_sort<4>(50021); check_sort<5>(50021); check_sort<5>(100); check_sort<6>(50021);
   if (cudaDeviceSynchronize() != cudaSuccess) { std::printf("FAILED: sticky CUDA error\n"); ++failures; }
   std::printf(failures ? "dropin_edges_test: %d FAILURES\n" : "dropin_edges_test: all checks passed\n", failures);
