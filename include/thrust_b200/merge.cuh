@@ -404,12 +404,15 @@ cudaError_t merge_pass_async(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutI
       cudaError_t e = launch_after(merge_split_kernel<K, Comp, Tuning::TILE>, (tiles + 7) / 8, 256, 0, stream, ka, kb, g, tiles, comp, a_split);
       if (e != cudaSuccess) return e;
       timed_launch tl(KID_MERGE, stream);
-      return launch_after(merge_slices_kernel<K, V, HAS_V, Comp>, tiles, MERGE_BLOCK, 0, stream, ka, kb, va, vb, ko, vo, g, comp, (const size_t*)a_split,
-                          &static_cast<ws_header*>(ws)->error);
+      e = launch_after(merge_slices_kernel<K, V, HAS_V, Comp>, tiles, MERGE_BLOCK, 0, stream, ka, kb, va, vb, ko, vo, g, comp, (const size_t*)a_split,
+                       &static_cast<ws_header*>(ws)->error);
+      log_launch("merge_slices_kernel", tiles, MERGE_BLOCK, 0, g.n, stream);
+      return e;
     }
     merge_split_kernel<K, Comp, Tuning::TILE><<<(tiles + 7) / 8, 256, 0, stream>>>(ka, kb, g, tiles, comp, a_split);
     timed_launch tl(KID_MERGE, stream);
     merge_slices_kernel<K, V, HAS_V, Comp><<<tiles, MERGE_BLOCK, 0, stream>>>(ka, kb, va, vb, ko, vo, g, comp, a_split, &static_cast<ws_header*>(ws)->error);
+    log_launch("merge_slices_kernel", tiles, MERGE_BLOCK, 0, g.n, stream);
     return cudaGetLastError();
   } else {
   g.cut(TILE);
@@ -418,6 +421,7 @@ cudaError_t merge_pass_async(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutI
   timed_launch tl(KID_MERGE, stream);
   merge_kernel<KeyItA, KeyItB, ValItA, ValItB, KeyOutIt, ValOutIt, K, V, HAS_V, Comp, IPT>
       <<<(unsigned)tiles, MERGE_BLOCK, 0, stream>>>(ka, kb, va, vb, ko, vo, g, comp, a_split, &static_cast<ws_header*>(ws)->error);
+  log_launch("merge_kernel", tiles, MERGE_BLOCK, 0, g.n, stream);
   return cudaGetLastError();
   }
 }
@@ -578,6 +582,7 @@ cudaError_t merge_sort_async(K* keys, K* keys_alt, V* vals, V* vals_alt, size_t 
   V* oth_v = (passes & 1) ? vals : vals_alt;
   { timed_launch tl(KID_BLOCK_SORT, stream);
   block_sort_kernel<const K*, const V*, K*, V*, K, V, HAS_V, Comp, BS_IPT><<<(unsigned)tiles, MERGE_BLOCK, 0, stream>>>(keys, vals, cur_k, cur_v, n, comp); }
+  log_launch("block_sort_kernel", tiles, MERGE_BLOCK, 0, n, stream);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   for (size_t run = BS_TILE; run < n; run <<= 1) {
     e = merge_pass_async<K, V, HAS_V>((const K*)cur_k, (const K*)cur_k, (const V*)cur_v, (const V*)cur_v, oth_k, oth_v,

@@ -263,6 +263,7 @@ cudaError_t partition_inplace_pipe_async(T* data, T* scratch, size_t n, Pred pre
   size_t grid = (n + 256 * 16 - 1) / (256 * 16);
   if (grid > (size_t)current_device_info().sm_count * 8) grid = (size_t)current_device_info().sm_count * 8;
   partition_rejects_kernel<T><<<(unsigned)grid, 256, 0, stream>>>(data, scratch, n, reinterpret_cast<const ws_header*>(ws));
+  log_launch("partition_rejects_kernel", grid, 256, 0, n, stream);
   return cudaGetLastError();
 }
 
