@@ -67,8 +67,9 @@ struct ws_header {
 static_assert(sizeof(ws_header) == 256, "workspace header is 256 bytes");
 
 #ifdef TB200_TEST_HOOKS
-// Test build of the library only: a process-wide switch that the single-pass scan copies into the
-// workspace header's flags (bit 0: tile 0 does not publish).
+// Test builds only: a process-wide switch.  Bits 0 and 1 are copied into the workspace header's flags (0: tile 0 of the
+// single-pass scan and of the pipelines does not publish; 1: a merge tile waits for bytes that nobody sends), bit 2 asks for
+// more CTAs than the pipelines' cooperative launch can place.
 inline unsigned& test_hook_flags() { static unsigned f = 0; return f; }
 #endif
 

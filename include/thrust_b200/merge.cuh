@@ -296,7 +296,11 @@ merge_slices_kernel(const K* ka, const K* kb, const V* va, const V* vb, K* ko, V
     if (HAS_V) mbar_init(&bars[1], 1);
     mbar_init_fence();
     const unsigned long long policy = l2_stream_policy();
-    mbar_arrive_expect(&bars[0], slice_bulk_bytes(ka + a_begin, na) + slice_bulk_bytes(kb + b_begin, nb));
+    unsigned awaited = slice_bulk_bytes(ka + a_begin, na) + slice_bulk_bytes(kb + b_begin, nb);
+#ifdef TB200_TEST_HOOKS
+    if (reinterpret_cast<const ws_header*>(err)->flags & 2u) awaited += 16;   // err points at the header's first word
+#endif
+    mbar_arrive_expect(&bars[0], awaited);
     slice_issue(sk_a, ka + a_begin, na, &bars[0], policy);
     slice_issue(sk_b, kb + b_begin, nb, &bars[0], policy);
     if constexpr (HAS_V) {
@@ -313,9 +317,10 @@ merge_slices_kernel(const K* ka, const K* kb, const V* va, const V* vb, K* ko, V
     if (warp == 4) slice_ends(sv_b, vb + b_begin, nb);
   }
   __syncthreads();
+  // bounded: reported after the limit, given up after twice that (the CTA should not end while its copies are in flight)
   auto wait = [&](unsigned long long* bar) {
-    for (unsigned iter = 0; !mbar_try_wait(bar, 0); ++iter)
-      if (iter > MBAR_SPIN_LIMIT) { record_error(err, ERR_LOOKBACK_TIMEOUT); break; }
+    for (unsigned iter = 0; !mbar_try_wait(bar, 0) && iter < 2 * MBAR_SPIN_LIMIT; ++iter)
+      if (iter == MBAR_SPIN_LIMIT) record_error(err, ERR_LOOKBACK_TIMEOUT);
   };
   wait(&bars[0]);
 
@@ -431,6 +436,9 @@ template <class K, class V, bool HAS_V, class KeyItA, class KeyItB, class ValItA
 cudaError_t merge_async(KeyItA ka, size_t na, KeyItB kb, size_t nb, ValItA va, ValItB vb, KeyOutIt ko, ValOutIt vo, Comp comp, void* ws,
                         cudaStream_t stream) {
   cudaError_t e = cudaMemsetAsync(ws, 0, sizeof(ws_header), stream);
+#ifdef TB200_TEST_HOOKS
+  if (e == cudaSuccess) e = cudaMemsetAsync(&static_cast<ws_header*>(ws)->flags, (int)(test_hook_flags() & 2u), 1, stream);
+#endif
   if (e != cudaSuccess) return e;
   return merge_pass_async<K, V, HAS_V>(ka, kb, va, vb, ko, vo, merge_geometry::single(na, nb), comp, ws, stream);
 }

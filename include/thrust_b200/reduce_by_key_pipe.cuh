@@ -309,7 +309,7 @@ cudaError_t rbk_pipe_launch(const K* keys, const V* vals, K* keys_out, V* vals_o
   ws_header* hdr = reinterpret_cast<ws_header*>(base);
   rbk_chain<V, Op> chain;
   chain.bind(base + sizeof(ws_header), tiles);
-  cudaError_t e = cudaMemsetAsync(base, 0, sizeof(ws_header) + rbk_chain<V, Op>::bytes(tiles), stream);
+  cudaError_t e = pipe_clear(base, sizeof(ws_header) + rbk_chain<V, Op>::bytes(tiles), stream);
   if (e != cudaSuccess) return e;
   timed_launch tl(KID_REDUCE_BY_KEY, stream);
   e = pipe_launch(kern, grid, smem, stream, keys, vals, keys_out, vals_out, n, (unsigned)tiles, eq, chain, hdr, d_count);

@@ -158,7 +158,7 @@ cudaError_t scan_pipe_launch(const T* in, T* out, size_t n, T init, bool has_ini
   ws_header* hdr = reinterpret_cast<ws_header*>(base);
   tile_chain<T, Op> chain;
   chain.bind(base + sizeof(ws_header), tiles);
-  cudaError_t e = cudaMemsetAsync(base, 0, sizeof(ws_header) + tile_chain<T, Op>::bytes(tiles), stream);
+  cudaError_t e = pipe_clear(base, sizeof(ws_header) + tile_chain<T, Op>::bytes(tiles), stream);
   if (e != cudaSuccess) return e;
   timed_launch tl(KID_SCAN, stream);
   e = pipe_launch(kern, grid, smem, stream, in, out, n, (unsigned)tiles, init, has_init, d_init, chain, hdr);

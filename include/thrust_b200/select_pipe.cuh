@@ -249,7 +249,7 @@ cudaError_t select_pipe_launch(const T* in, T* out_sel, T* out_rej, size_t n, Pr
   ws_header* hdr = reinterpret_cast<ws_header*>(base);
   tile_chain<unsigned long long, plus_op> chain;
   chain.bind(base + sizeof(ws_header), tiles);
-  cudaError_t e = cudaMemsetAsync(base, 0, sizeof(ws_header) + tile_chain<unsigned long long, plus_op>::bytes(tiles), stream);
+  cudaError_t e = pipe_clear(base, sizeof(ws_header) + tile_chain<unsigned long long, plus_op>::bytes(tiles), stream);
   if (e != cudaSuccess) return e;
   timed_launch tl(KID_SELECT, stream);
   e = pipe_launch(kern, grid, smem, stream, in, out_sel, out_rej, n, (unsigned)tiles, pred, chain, hdr, d_count);

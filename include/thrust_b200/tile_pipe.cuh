@@ -275,6 +275,9 @@ __device__ __forceinline__ void pipe_publisher(S& st, const Chain& chain, unsign
     pipe_wait(&st.summed[cur.stage], cur.parity, &st.dead, err);
     if (pipe_dead(st)) return;
     const auto total = fold(st.part[cur.stage][lane_id() & (PIPE_WARPS - 1)]);
+#ifdef TB200_TEST_HOOKS
+    if (cur.tile == 0 && (reinterpret_cast<const ws_header*>(err)->flags & 1u)) continue;   // err points at the header's first word
+#endif
     if (lane_id() == 0) {
       if constexpr (ORDERED) chain.publish_release(cur.tile, TILE_AGGREGATE, total); else chain.publish(cur.tile, TILE_AGGREGATE, total);
     }
@@ -414,8 +417,21 @@ template <class Kernel> size_t pipe_grid(Kernel kernel, size_t smem, size_t tile
     ready[dev] = true;
   }
   size_t grid = (size_t)di.sm_count;
+#ifdef TB200_TEST_HOOKS
+  if (test_hook_flags() & 4u) grid = 2 * PIPE_MAX_GRID;
+  else
+#endif
   if (grid > (size_t)PIPE_MAX_GRID) grid = PIPE_MAX_GRID;
   return grid < tiles ? grid : tiles;
+}
+
+// Clears the header and the descriptors.
+inline cudaError_t pipe_clear(void* ws, size_t bytes, cudaStream_t stream) {
+  cudaError_t e = cudaMemsetAsync(ws, 0, bytes, stream);
+#ifdef TB200_TEST_HOOKS
+  if (e == cudaSuccess) e = cudaMemsetAsync(&static_cast<ws_header*>(ws)->flags, (int)(test_hook_flags() & 1u), 1, stream);
+#endif
+  return e;
 }
 
 // Cooperative, so that the CTAs of a round are all resident whatever else runs on the device.

@@ -53,3 +53,22 @@ def test_lookback_timeout_is_reported_and_recoverable(tb, port, monkeypatch):
     assert short.tb200_inclusive_scan(p(x), p(out), n, 4, 0, None, p(ws), C.byref(need), None) == 0
     assert short.tb200_workspace_status(p(ws), None, C.byref(status)) == 0 and status.value == 0
     assert np.array_equal(out.cpu().numpy(), port.inclusive_scan(x_h))
+
+
+def test_waits_of_the_pipelines_and_the_merge_run_out(tb, tmp_path):
+    """tests/cpp/bounded_waits_test.cu, built here with the test hooks and short waits: a withheld tile descriptor in the
+    scan, compaction, partition and reduce_by_key pipelines and a merge copy that stays incomplete are reported as status 1,
+    and a refused cooperative launch is served by the single-pass kernel."""
+    import shutil
+    import subprocess
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.isfile(nvcc):
+        pytest.skip("nvcc is not available on this machine")
+    exe = str(tmp_path / "bounded_waits_test")
+    r = subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O2", "-DTB200_TEST_HOOKS", "-DTB200_SPIN_LIMIT=65536",
+                        "-I" + os.path.join(root, "include"), os.path.join(root, "tests", "cpp", "bounded_waits_test.cu"), "-o", exe],
+                       capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stdout + r.stderr
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "all checks passed" in r.stdout, r.stdout + r.stderr
