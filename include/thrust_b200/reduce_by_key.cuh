@@ -166,12 +166,16 @@ constexpr size_t RBK_PIPE_MIN_BYTES = (size_t)1 << 20;
 template <class K, class V> constexpr size_t rbk_tile_items() { return (size_t)RBK_BLOCK * rbk_tuning<K, V>::IPT; }
 template <class K, class V> size_t rbk_workspace_bytes(size_t n) {
   size_t tiles = (n + rbk_tile_items<K, V>() - 1) / rbk_tile_items<K, V>();
-  const size_t single = sizeof(ws_header) + tile_state<rbk_pair<unsigned long long, V>>::bytes(tiles + 1);
+  size_t need = sizeof(ws_header) + tile_state<rbk_pair<unsigned long long, V>>::bytes(tiles + 1);
   if constexpr (sizeof(K) == sizeof(V) && (sizeof(K) == 4 || sizeof(K) == 8)) {
     const size_t stream = rbk_stream_workspace_bytes<K, V>(n);
-    return single > stream ? single : stream;
+    if (stream > need) need = stream;
   }
-  return single;
+  if constexpr (std::is_arithmetic<K>::value && std::is_arithmetic<V>::value && (sizeof(K) == 4 || sizeof(K) == 8) && (sizeof(V) == 4 || sizeof(V) == 8)) {
+    const size_t pipe = rbk_pipe_workspace_bytes<K, V>(n);
+    if (pipe > need) need = pipe;
+  }
+  return need;
 }
 
 // Launches reduce_by_key; no sync.  The number of runs goes to the workspace header and, if

@@ -292,6 +292,10 @@ bool rbk_pipe_eligible(const K* keys, const V* vals, const K* keys_out, const V*
          apart(vals, sizeof(V), vals_out, sizeof(V));
 }
 
+template <class K, class V> size_t rbk_pipe_workspace_bytes(size_t n) {
+  return sizeof(ws_header) + rbk_chain<V, plus_op>::bytes((n + rbk_pipe_shape<K, V>::ITEMS - 1) / rbk_pipe_shape<K, V>::ITEMS);
+}
+
 // Launches the pipeline if the device can hold it and takes the launch (launched = true); n > 0.
 template <class K, class V, class Eq, class Op>
 cudaError_t rbk_pipe_launch(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n, Eq eq, unsigned long long* d_count, void* ws, cudaStream_t stream,

@@ -361,11 +361,15 @@ template <class T> size_t scanw_descriptor_bound(size_t n) {
   const size_t tile = (size_t)SCAN_BLOCK * scanw_tuning<T>::IPT;
   return ((n + tile - 1) / tile + TB200_SCANW_TPC - 1) / TB200_SCANW_TPC + SCANW_MAX_GRID;
 }
-template <class T> size_t scan_workspace_bytes(size_t n) {
+template <class T> size_t scan_workspace_bytes(size_t n) {   // every route fits
   size_t tiles = (n + scan_tile_items<T>() - 1) / scan_tile_items<T>();
-  size_t need = tile_state<T>::bytes(tiles + 1);   // single pass; the pipeline's tiles are the same size and so are its descriptors
+  size_t need = tile_state<T>::bytes(tiles + 1);   // single pass
   if (tile_state_mode<T>::value != 0 && tile_state<T>::bytes(scanw_descriptor_bound<T>(n)) > need) need = tile_state<T>::bytes(scanw_descriptor_bound<T>(n));
-  return sizeof(ws_header) + need;   // every route fits
+  if constexpr (std::is_arithmetic<T>::value && (sizeof(T) == 4 || sizeof(T) == 8)) {
+    const size_t pipe = scan_pipe_descriptor_bytes<T>(n);
+    if (pipe > need) need = pipe;
+  }
+  return sizeof(ws_header) + need;
 }
 
 // The windowed route: launches it if the input is large enough for windows to pay (launched = true).

@@ -140,6 +140,11 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
 }
 
 template <class T> constexpr size_t scan_pipe_tile_items() { return PIPE_TILE_BYTES / sizeof(T); }
+template <class T> size_t scan_pipe_descriptor_bytes(size_t n) {   // of the operator that needs most
+  const size_t tiles = (n + scan_pipe_tile_items<T>() - 1) / scan_pipe_tile_items<T>();
+  const size_t sum = tile_chain<T, plus_op>::bytes(tiles), other = tile_chain<T, typename route_op<min_op, T>::type>::bytes(tiles);
+  return sum > other ? sum : other;
+}
 
 // Launches the pipeline scan if the device can hold it and takes the launch (launched = true).  `in` and `out` are 16-byte aligned;
 // they may be the same array.  The workspace holds the header and one descriptor per tile.

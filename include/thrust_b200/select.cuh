@@ -165,8 +165,12 @@ partition_finish_kernel(OutIt data, const T* scratch, size_t n, const ws_header*
 template <class T> constexpr size_t select_tile_items() { return (size_t)SELECT_BLOCK * select_tuning<T>::IPT; }
 template <class T> size_t select_workspace_bytes(size_t n) {
   size_t tiles = (n + select_tile_items<T>() - 1) / select_tile_items<T>();
-  // large enough for either offset width; the pipeline's tiles of 4- and 8-byte items are the same size and so are its descriptors
-  return sizeof(ws_header) + tile_state<unsigned long long>::bytes(tiles + 1);
+  const size_t single = sizeof(ws_header) + tile_state<unsigned long long>::bytes(tiles + 1);   // large enough for either offset width
+  if constexpr (std::is_arithmetic<T>::value && (sizeof(T) == 4 || sizeof(T) == 8)) {
+    const size_t pipe = select_pipe_workspace_bytes<T>(n);
+    return single > pipe ? single : pipe;
+  }
+  return single;
 }
 
 // Where the pipeline starts.  2^20 int32 selected 13.3 us against 14.3 single-pass, 2^18 12.0 against 11.4; with the

@@ -49,3 +49,18 @@ def test_merge_tiles_stay_inside_their_inputs(tmp_path):
     assert r.returncode == 0, r.stdout + r.stderr
     r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("tunables", [[], ["-DTB200_RBK_IPT4=255"]])
+def test_workspaces_hold_every_route(tmp_path, tunables):
+    """Also where the single-pass kernel's tiles are tuned larger than the pipeline's (tests/cpp/workspace_bounds_host.cu, host
+    code only)."""
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.isfile(nvcc):
+        pytest.skip("nvcc is not available on this machine")
+    exe = str(tmp_path / "workspace_bounds_host")
+    r = subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I" + os.path.join(ROOT, "include"), *tunables,
+                        os.path.join(ROOT, "tests", "cpp", "workspace_bounds_host.cu"), "-o", exe], capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stdout + r.stderr
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
