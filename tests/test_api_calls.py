@@ -109,6 +109,6 @@ def test_a_refused_call_is_made_again_only_for_its_size(fake, name):
     assert fake.launches == [name] * 2
     fake.result = 0
     key = api.workspaces.key("reduce" if name == "reduce" else "select")
-    api.workspaces._bufs[key] = torch.empty(NEED - 1, dtype=torch.uint8)
+    api.workspaces.at(key).keep(torch.empty(NEED - 1, dtype=torch.uint8))
     call()
-    assert fake.launches == [name] * 3 and api.workspaces.kept(key).numel() == NEED
+    assert fake.launches == [name] * 3 and api.workspaces.at(key).buf.numel() == NEED

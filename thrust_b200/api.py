@@ -57,6 +57,20 @@ def _require_cuda(*tensors):
             raise ValueError("thrust_b200 operates on contiguous CUDA tensors")
 
 
+class _Kept:
+    """One kept buffer: the tensor, its address and size as the C ABI takes them, and its lock (re-entrant)."""
+    __slots__ = ("lock", "buf", "ptr", "size")
+
+    def __init__(self):
+        self.lock = threading.RLock()
+        self.keep(None)
+
+    def keep(self, buf):
+        self.buf = buf
+        self.ptr = None if buf is None else buf.data_ptr()
+        self.size = C.c_size_t(0 if buf is None else buf.numel())
+
+
 class _Workspaces:
     """Scratch buffers cached per (device, stream, call site) and grown on demand, standing in for
     the reference's per-call temporary_array (thrust/system/cuda/detail/reduce.h:959).
@@ -65,8 +79,7 @@ class _Workspaces:
     is read back; a call therefore holds the buffer's lock from its first launch to that read-back."""
 
     def __init__(self):
-        self._bufs = {}
-        self._locks = {}
+        self._kept = {}
 
     @staticmethod
     def key(tag):
@@ -74,24 +87,19 @@ class _Workspaces:
         dev = torch.cuda.current_device()
         return dev, _raw_stream(dev), tag
 
-    def lock(self, key):
-        """The lock of a buffer (re-entrant)."""
-        return self._locks.get(key) or self._locks.setdefault(key, threading.RLock())
-
-    def kept(self, key):
-        """The buffer kept under `key`, whatever its size, or None."""
-        return self._bufs.get(key)
+    def at(self, key):
+        return self._kept.get(key) or self._kept.setdefault(key, _Kept())
 
     def get(self, tag, nbytes, key=None):
-        key = key or self.key(tag)
-        buf = self._bufs.get(key)
-        if buf is None or buf.numel() < nbytes:
-            buf = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device="cuda")
-            self._bufs[key] = buf
-        return buf
+        kept = self.at(key or self.key(tag))
+        if kept.buf is None or kept.size.value < nbytes:
+            kept.keep(torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device="cuda"))
+        return kept.buf
 
     def clear(self):
-        self._bufs.clear()
+        for kept in list(self._kept.values()):
+            with kept.lock:
+                kept.keep(None)
 
 
 workspaces = _Workspaces()
@@ -100,50 +108,46 @@ workspaces = _Workspaces()
 _TOO_SMALL = 1      # cudaErrorInvalidValue: the workspace is too small, or something else about the call is wrong
 
 
-def _enqueue(key, fn, args, result=None):
+def _enqueue(key, kept, fn, args, result=None):
     """fn(*args, d_ws, &ws_bytes, stream) in the workspace kept under `key`, whose lock the caller holds; with `result`, an
     offset into the workspace, its address goes in front of d_ws.  The size is asked for only if there is no workspace yet
     or the call is refused, and the call made again only if the workspace was indeed too small (then nothing was
-    launched: every entry point checks the size first).  Returns the workspace."""
+    launched: every entry point checks the size first)."""
     lib_fn = getattr(_lib.load(), fn)
     stream = key[1]
-
-    def call(ws):
-        at = ws.data_ptr()
-        out = () if result is None else (at + result,)
-        return lib_fn(*args, *out, at, C.byref(C.c_size_t(ws.numel())), stream)
-
-    ws = workspaces.kept(key)
     rc = None
-    if ws is not None:
-        rc = call(ws)
+    if kept.ptr is not None:
+        out = () if result is None else (kept.ptr + result,)
+        rc = lib_fn(*args, *out, kept.ptr, C.byref(kept.size), stream)
         if rc != _TOO_SMALL:
-            _check(rc, fn)
-            return ws
+            return _check(rc, fn)
     need = C.c_size_t(0)
     none = () if result is None else (None,)
     _check(lib_fn(*args, *none, None, C.byref(need), stream), fn + " (size query)")
-    if ws is not None and ws.numel() >= need.value:
+    if rc is not None and kept.size.value >= need.value:
         _check(rc, fn)
-    ws = workspaces.get(key[2], need.value, key)
-    _check(call(ws), fn)
-    return ws
+    workspaces.get(key[2], need.value, key)
+    out = () if result is None else (kept.ptr + result,)
+    _check(lib_fn(*args, *out, kept.ptr, C.byref(kept.size), stream), fn)
 
 
 def _call_with_ws(tag, fn, *args):
     """Enqueues fn in the workspace of the call site; returns the workspace."""
     key = workspaces.key(tag)
-    with workspaces.lock(key):
-        return _enqueue(key, fn, args)
+    kept = workspaces.at(key)
+    with kept.lock:
+        _enqueue(key, kept, fn, args)
+        return kept.buf
 
 
-def _call_and_wait(tag, what, fn, *args, sync=True):
+def _call_and_wait(tag, what, fn, *args, sync=True, key=None):
     """The same, then (sync) waits for the stream and checks the status.  Returns the number that the kernels of
-    a selecting or counting call left in the header."""
-    key = workspaces.key(tag)
-    with workspaces.lock(key):
-        ws = _enqueue(key, fn, args)
-        return _HEADER.unpack_from(_read_header(ws, what, stream=key[1]))[2] if sync else None
+    a selecting or counting call left in the header.  key: the workspace's, if the caller has it."""
+    key = key or workspaces.key(tag)
+    kept = workspaces.at(key)
+    with kept.lock:
+        _enqueue(key, kept, fn, args)
+        return _HEADER.unpack_from(_read_header(kept.ptr, what, key[1]))[2] if sync else None
 
 
 # the workspace header (ws_header in common.cuh): status, ticket, count, ..., and room that a result may use
@@ -151,11 +155,11 @@ _HEADER = struct.Struct("<IIQ")
 _HEADER_RESULT = 32
 
 
-def _read_header(ws, what, nbytes=_HEADER.size, stream=None):
+def _read_header(ptr, what, stream, nbytes=_HEADER.size):
     """Waits for the stream, then the first `nbytes` of the workspace's header in one copy; raises if the
-    kernels reported a wait that ran out."""
+    kernels reported a wait that ran out or looks at a tile that disagree."""
     head = C.create_string_buffer(nbytes)
-    _check(_lib.load().tb200_workspace_read(ws.data_ptr(), nbytes, head, _stream() if stream is None else stream), what + " (result)")
+    _check(_lib.load().tb200_workspace_read(ptr, nbytes, head, stream), what + " (result)")
     status = _HEADER.unpack_from(head)[0]
     if status != 0:
         raise Tb200Error("%s: device reported status %d (%s)" % (what, status, "an inter-CTA wait ran out" if status == 1 else "two looks at a tile disagree"))
@@ -163,7 +167,7 @@ def _read_header(ws, what, nbytes=_HEADER.size, stream=None):
 
 
 def _sync_and_check(ws, what):
-    _read_header(ws, what)
+    _read_header(ws.data_ptr(), what, _stream())
 
 
 # ------------------------------------------------------------------------------------- reduce
@@ -177,9 +181,10 @@ def reduce(x, init=None, op="plus", acc_dtype=None):
     # the result lands in the workspace's header and comes back together with the status
     key = workspaces.key("reduce")
     args = (_ptr(x), x.numel(), DTYPE_CODE[x.dtype], DTYPE_CODE[acc_dtype], OPS[op], h_init.ctypes.data)
-    with workspaces.lock(key):
-        ws = _enqueue(key, "tb200_reduce", args, _HEADER_RESULT)
-        head = _read_header(ws, "reduce", _HEADER_RESULT + 8, key[1])
+    kept = workspaces.at(key)
+    with kept.lock:
+        _enqueue(key, kept, "tb200_reduce", args, _HEADER_RESULT)
+        head = _read_header(kept.ptr, "reduce", key[1], _HEADER_RESULT + 8)
     return np.frombuffer(head.raw, dtype=NP_OF[acc_dtype], count=1, offset=_HEADER_RESULT)[0]
 
 
@@ -234,11 +239,12 @@ def _sort_impl(keys, vals, descending, begin_bit, end_bit, sync=True):
     n = keys.numel()
     vb = 0 if vals is None else vals.element_size()
     end_bit = 8 * keys.element_size() if end_bit is None else end_bit
-    with workspaces.lock(workspaces.key("sort_keys_alt")):
-        kalt = workspaces.get("sort_keys_alt", n * keys.element_size())
-        valt = None if vals is None else workspaces.get("sort_vals_alt", n * vb)
+    key = workspaces.key("sort_keys_alt")
+    with workspaces.at(key).lock:
+        kalt = workspaces.get("sort_keys_alt", n * keys.element_size(), key)
+        valt = None if vals is None else workspaces.get("sort_vals_alt", n * vb, key[:2] + ("sort_vals_alt",))
         _call_and_wait("sort", "sort", "tb200_sort_by_key", _ptr(keys), _ptr(kalt), _ptr(vals), _ptr(valt), n,
-                       DTYPE_CODE[keys.dtype], vb, int(descending), begin_bit, end_bit, sync=sync)
+                       DTYPE_CODE[keys.dtype], vb, int(descending), begin_bit, end_bit, sync=sync, key=key[:2] + ("sort",))
 
 
 def sort(keys, descending=False, sync=True):
@@ -470,11 +476,12 @@ def merge_sort_by_key(keys, vals=None, descending=False):
     _require_cuda(keys, vals)
     n = keys.numel()
     vb = 0 if vals is None else vals.element_size()
-    with workspaces.lock(workspaces.key("sort_keys_alt")):
-        kalt = workspaces.get("sort_keys_alt", n * keys.element_size())
-        valt = None if vals is None else workspaces.get("sort_vals_alt", n * vb)
+    key = workspaces.key("sort_keys_alt")
+    with workspaces.at(key).lock:
+        kalt = workspaces.get("sort_keys_alt", n * keys.element_size(), key)
+        valt = None if vals is None else workspaces.get("sort_vals_alt", n * vb, key[:2] + ("sort_vals_alt",))
         _call_and_wait("merge_sort", "merge_sort_by_key", "tb200_merge_sort_by_key", _ptr(keys), _ptr(kalt), _ptr(vals), _ptr(valt), n,
-                       DTYPE_CODE[keys.dtype], vb, int(descending))
+                       DTYPE_CODE[keys.dtype], vb, int(descending), key=key[:2] + ("merge_sort",))
     return keys, vals
 
 
