@@ -165,7 +165,7 @@ scan_window_kernel(InIt in, T* out, size_t n, size_t tiles, unsigned tiles_per_c
   const T ID = op_identity<Op, T>::value();
   __shared__ T s_part[2][NWARPS];          // each warp's total of its part of the chunk, by window parity
   __shared__ T s_fold[2][NWARPS];          // per warp: fold of the chunks before this CTA's, of all chunks
-  __shared__ T s_first;                    // what a loop would start from (first_value_rules)
+  __shared__ T s_first;                    // what a loop would start from (drops_nans)
   const int lane = lane_id(), warp = threadIdx.x >> 5;
   const size_t G = gridDim.x, c = blockIdx.x;
   const size_t wtiles = (n + WT - 1) / WT;
@@ -182,7 +182,7 @@ scan_window_kernel(InIt in, T* out, size_t n, size_t tiles, unsigned tiles_per_c
       for (int v = 0; v < VPT; ++v) {
         T* e = reinterpret_cast<T*>(&r[v]);
 #pragma unroll
-        for (int k = 0; k < VEC; ++k) e[k] = (T)in[base + (size_t)(v * 32 + lane) * VEC + k];
+        for (int k = 0; k < VEC; ++k) e[k] = no_nan<Op>((T)in[base + (size_t)(v * 32 + lane) * VEC + k]);
       }
     } else {
 #pragma unroll
@@ -191,7 +191,7 @@ scan_window_kernel(InIt in, T* out, size_t n, size_t tiles, unsigned tiles_per_c
 #pragma unroll
         for (int k = 0; k < VEC; ++k) {
           const size_t i = base + (size_t)(v * 32 + lane) * VEC + k;
-          e[k] = i < n ? (T)in[i] : ID;
+          e[k] = i < n ? no_nan<Op>((T)in[i]) : ID;
         }
       }
     }
@@ -224,8 +224,8 @@ scan_window_kernel(InIt in, T* out, size_t n, size_t tiles, unsigned tiles_per_c
     }
   };
 
-  T running = has_init ? init : ID;   // init (+) everything before the current window
-  if constexpr (first_value_rules<Op>::value) {
+  T running = has_init ? no_nan<Op>(init) : ID;   // init (+) everything before the current window
+  if constexpr (drops_nans<Op, T>::value) {
     // read before this CTA publishes, so before anybody stores: the iterator may read from where the output goes
     if (threadIdx.x == 0) s_first = has_init ? init : (T)in[0];
     __syncthreads();
@@ -318,7 +318,7 @@ scan_window_kernel(InIt in, T* out, size_t n, size_t tiles, unsigned tiles_per_c
 #pragma unroll
           for (int k = 1; k < VEC; ++k) y[k] = op(E, x[v][k - 1]);
         }
-        if constexpr (first_value_rules<Op>::value) {
+        if constexpr (drops_nans<Op, T>::value) {
           const T first = s_first;
 #pragma unroll
           for (int k = 0; k < VEC; ++k) if (first != first) y[k] = first;
@@ -373,14 +373,13 @@ template <class T> size_t scan_workspace_bytes(size_t n) {   // every route fits
 }
 
 // The windowed route: launches it if the input is large enough for windows to pay (launched = true).
-template <bool INCLUSIVE, class InIt, class T, class CallerOp>
-cudaError_t scan_window_launch(InIt in, T* out, size_t n, T init, bool has_init, const T* d_init, CallerOp, char* base, ws_header* hdr,
+template <bool INCLUSIVE, class InIt, class T, class Op>
+cudaError_t scan_window_launch(InIt in, T* out, size_t n, T init, bool has_init, const T* d_init, Op op, char* base, ws_header* hdr,
                                cudaStream_t stream, bool& launched) {
   launched = false;
   constexpr int VEC = 16 / sizeof(T);
   constexpr int IPT2 = scanw_tuning<T>::IPT;
   const size_t tiles2 = (n + (size_t)SCAN_BLOCK * IPT2 - 1) / ((size_t)SCAN_BLOCK * IPT2);
-  using Op = typename route_op<CallerOp, T>::type;
   auto kern = scan_window_kernel<InIt, T, Op, INCLUSIVE, VEC, IPT2>;
   static thread_local int resident[64] = {0};
   int dev = 0;
@@ -397,7 +396,7 @@ cudaError_t scan_window_launch(InIt in, T* out, size_t n, T init, bool has_init,
   if (e3 != cudaSuccess) return e3;
   launched = true;
   timed_launch tl(KID_SCAN, stream);
-  kern<<<(unsigned)grid, SCAN_BLOCK, 0, stream>>>(in, out, n, tiles2, tpc, init, has_init, d_init, Op(), tsw, hdr);
+  kern<<<(unsigned)grid, SCAN_BLOCK, 0, stream>>>(in, out, n, tiles2, tpc, init, has_init, d_init, op, tsw, hdr);
   log_launch("scan_window_kernel", grid, SCAN_BLOCK, 0, n, stream);
   return cudaGetLastError();
 }
@@ -422,8 +421,8 @@ cudaError_t scan_async(InIt in, OutIt out, size_t n, T init, bool has_init, Op o
       vectors = is_aligned16(in) && is_aligned16(out);
       if constexpr (is_commutative_op<Op>::value) {
         // With NaNs among the values the single-pass kernel's floating min and max depend on its grouping; the pipeline's
-        // do not (skip_nan).  So that no size's results change with it, they leave the single-pass kernel where they always did.
-        constexpr bool grouping_shows = first_value_rules<typename route_op<Op, T>::type>::value;
+        // do not (drops_nans).  So that no size's results change with it, they leave the single-pass kernel where they always did.
+        constexpr bool grouping_shows = drops_nans<Op, T>::value;
         if (vectors && (grouping_shows ? scan_fills_windows<T>(n) : n * sizeof(T) >= SCAN_PIPE_MIN_BYTES)) {
           bool launched = false;
           cudaError_t e2 = scan_pipe_launch<INCLUSIVE, T, Op>(in, out, n, init, has_init, d_init, ws, stream, launched);

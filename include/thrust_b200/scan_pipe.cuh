@@ -1,5 +1,5 @@
 // Inclusive / exclusive scan of large contiguous inputs on sm_100a on the tile pipeline (tile_pipe.cuh), for
-// operators with an identity on 4- and 8-byte arithmetic types (floating min and max as skip_nan).  A tile is read from HBM once into shared
+// operators with an identity on 4- and 8-byte arithmetic types (floating min and max without their NaNs, drops_nans).  A tile is read from HBM once into shared
 // memory; the compute warps reduce it there ahead of time, and once its carry is known scan it from the
 // same shared memory and stream the result out: 2 * sizeof(T) bytes of HBM traffic per element and no
 // second trip of the input through L2.  Bound by HBM: 2^28 int32 or fp32 0.33 ms (6470 GB/s; 0.43 with the input
@@ -44,13 +44,13 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
     });
   } else if (warp == PIPE_FOLDER) {
     C first = Chain::identity();
-    if (init_ptr) first = Chain::lift(*init_ptr); else if (has_init) first = Chain::lift(init);
+    if (init_ptr) first = Chain::lift(no_nan<Op>(*init_ptr)); else if (has_init) first = Chain::lift(no_nan<Op>(init));
     pipe_folder<false>(st, chain, tiles, first, &hdr->error, [](const C&) {});
   } else {
     const int mine = warp % PIPE_WARPS;
     // what a loop would start from: if that is a NaN, so is every result (in place in[0] is stored unchanged)
     T first = T();
-    if constexpr (first_value_rules<Op>::value) first = init_ptr ? *init_ptr : has_init ? init : in[0];
+    if constexpr (drops_nans<Op, T>::value) first = init_ptr ? *init_ptr : has_init ? init : in[0];
     const bool stuck = first != first;
     auto rows_of = [&](unsigned s) { return reinterpret_cast<const vec16*>(stages + (size_t)s * PIPE_TILE_BYTES) + mine * (PIPE_ROWS * 32) + lane; };
     pipe_compute<false>(st, tiles, &hdr->error,
@@ -61,9 +61,9 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
         for (int v = 0; v < PIPE_ROWS; ++v) {
           const vec16 r = src[v * 32];
           const T* e = reinterpret_cast<const T*>(&r);
-          acc[v] = e[0];
+          acc[v] = no_nan<Op>(e[0]);
 #pragma unroll
-          for (int k = 1; k < VEC; ++k) acc[v] = op(acc[v], e[k]);
+          for (int k = 1; k < VEC; ++k) acc[v] = op(acc[v], no_nan<Op>(e[k]));
         }
 #pragma unroll
         for (int v = 1; v < PIPE_ROWS; ++v) acc[0] = op(acc[0], acc[v]);
@@ -80,7 +80,7 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
           const vec16 r = src[v * 32];
           const T* e = reinterpret_cast<const T*>(&r);
 #pragma unroll
-          for (int k = 0; k < VEC; ++k) x[v][k] = e[k];
+          for (int k = 0; k < VEC; ++k) x[v][k] = no_nan<Op>(e[k]);
         }
         // what precedes this warp's part: the tile's carry and the warps before this one
         T before = lane < mine ? st.part[s][lane & (PIPE_WARPS - 1)] : ID;
@@ -119,7 +119,7 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
 #pragma unroll
             for (int k = 0; k < VEC; ++k) y[k] = op(carry, y[k]);
           }
-          if constexpr (first_value_rules<Op>::value) {
+          if constexpr (drops_nans<Op, T>::value) {
 #pragma unroll
             for (int k = 0; k < VEC; ++k) if (stuck) y[k] = first;
           }
@@ -142,16 +142,15 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
 template <class T> constexpr size_t scan_pipe_tile_items() { return PIPE_TILE_BYTES / sizeof(T); }
 template <class T> size_t scan_pipe_descriptor_bytes(size_t n) {   // of the operator that needs most
   const size_t tiles = (n + scan_pipe_tile_items<T>() - 1) / scan_pipe_tile_items<T>();
-  const size_t sum = tile_chain<T, plus_op>::bytes(tiles), other = tile_chain<T, typename route_op<min_op, T>::type>::bytes(tiles);
+  const size_t sum = tile_chain<T, plus_op>::bytes(tiles), other = tile_chain<T, min_op>::bytes(tiles);
   return sum > other ? sum : other;
 }
 
 // Launches the pipeline scan if the device can hold it and takes the launch (launched = true).  `in` and `out` are 16-byte aligned;
 // they may be the same array.  The workspace holds the header and one descriptor per tile.
-template <bool INCLUSIVE, class T, class CallerOp>
+template <bool INCLUSIVE, class T, class Op>
 cudaError_t scan_pipe_launch(const T* in, T* out, size_t n, T init, bool has_init, const T* d_init, void* ws, cudaStream_t stream, bool& launched) {
   launched = false;
-  using Op = typename route_op<CallerOp, T>::type;
   const size_t tiles = (n + scan_pipe_tile_items<T>() - 1) / scan_pipe_tile_items<T>();
   if (tiles >= 0xffffff00ull) return cudaSuccess;
   static thread_local bool ready[64] = {false};

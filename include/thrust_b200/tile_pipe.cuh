@@ -59,43 +59,38 @@ __device__ __forceinline__ void pipe_wait(unsigned long long* bar, unsigned pari
 // ---------------------------------------------------------------- operators with an identity
 // The operators of this route have an identity, so nothing here needs the "value may be absent"
 // bookkeeping of the generic kernels: plus starts from -0.0 for floating point (x + -0.0 == x for
-// every x, signed zeros included) and 0 otherwise, min from the largest and max from the smallest whole number.
-// Floating min and max have none: min_op(infinity, NaN) is infinity.  They run as skip_nan, see there.
+// every x, signed zeros included) and 0 otherwise, min from the largest and max from the smallest value.
+// Floating min and max take NaNs out first, see drops_nans.
 template <class Op, class T> struct op_identity;
 template <class T> struct op_identity<plus_op, T> {
   __host__ __device__ static T value() { return std::is_floating_point<T>::value ? (T)-0.0 : (T)0; }
 };
 template <class T> struct op_identity<min_op, T> {
-  static_assert(std::is_integral<T>::value, "floating min runs as skip_nan<min_op>");
   __host__ __device__ static T value() {
-    if constexpr (std::is_signed<T>::value) return (T)(((unsigned long long)1 << (8 * sizeof(T) - 1)) - 1);
+    if constexpr (std::is_floating_point<T>::value) return (T)INFINITY;
+    else if constexpr (std::is_signed<T>::value) return (T)(((unsigned long long)1 << (8 * sizeof(T) - 1)) - 1);
     else return (T)~(T)0;
   }
 };
 template <class T> struct op_identity<max_op, T> {
-  static_assert(std::is_integral<T>::value, "floating max runs as skip_nan<max_op>");
   __host__ __device__ static T value() {
-    if constexpr (std::is_signed<T>::value) return (T)((unsigned long long)1 << (8 * sizeof(T) - 1));
+    if constexpr (std::is_floating_point<T>::value) return (T)-INFINITY;
+    else if constexpr (std::is_signed<T>::value) return (T)((unsigned long long)1 << (8 * sizeof(T) - 1));
     else return (T)0;
   }
 };
 
 // Floating min and max one after the other, as a loop applies them: min_op(a, b) keeps a NaN that stands on its left
 // and drops one on its right, so the result is the first value of all if that is a NaN, else the extreme of
-// the values that are none.  skip_nan drops NaNs on either side, which commutes, may be regrouped and has an identity, NaN;
-// the rule for the first value is the kernel's (first_value_rules).
-template <class Op> struct skip_nan {
-  template <class T> __host__ __device__ T operator()(const T& a, const T& b) const { return a == a ? Op()(a, b) : b; }
+// the values that are none.  With NaNs about the infinities are no identities and the grouping shows; so a scan replaces
+// every NaN by the identity as it loads it (no_nan) and looks at the first value by itself.  Without NaNs nothing changes.
+template <class Op, class T> struct drops_nans {
+  static constexpr bool value = std::is_floating_point<T>::value && (std::is_same<Op, min_op>::value || std::is_same<Op, max_op>::value);
 };
-template <class Op, class T> struct op_identity<skip_nan<Op>, T> { __host__ __device__ static T value() { return (T)NAN; } };
-template <class Op> struct first_value_rules : std::false_type {};
-template <class Op> struct first_value_rules<skip_nan<Op>> : std::true_type {};
-// the operator that a kernel of this route runs for Op
-template <class Op, class T> struct route_op { using type = Op; };
-template <> struct route_op<min_op, float> { using type = skip_nan<min_op>; };
-template <> struct route_op<min_op, double> { using type = skip_nan<min_op>; };
-template <> struct route_op<max_op, float> { using type = skip_nan<max_op>; };
-template <> struct route_op<max_op, double> { using type = skip_nan<max_op>; };
+template <class Op, class T> __device__ __forceinline__ T no_nan(const T& x) {
+  if constexpr (drops_nans<Op, T>::value) return x == x ? x : op_identity<Op, T>::value();
+  else return x;
+}
 
 template <class Op> struct is_commutative_op : std::false_type {};
 template <> struct is_commutative_op<plus_op> : std::true_type {};

@@ -16,7 +16,7 @@ static size_t tiles_of(size_t n, size_t items) { return (n + items - 1) / items;
 template <class T> static void one_type(size_t n) {
   const size_t tiles = tiles_of(n, PIPE_TILE_BYTES / sizeof(T));
   check("scan plus", n, scan_workspace_bytes<T>(n), tile_chain<T, plus_op>::bytes(tiles));
-  check("scan min", n, scan_workspace_bytes<T>(n), tile_chain<T, typename route_op<min_op, T>::type>::bytes(tiles));
+  check("scan min", n, scan_workspace_bytes<T>(n), tile_chain<T, min_op>::bytes(tiles));
   check("select", n, select_workspace_bytes<T>(n), tile_chain<unsigned long long, plus_op>::bytes(tiles));
 }
 template <class K, class V> static void pair(size_t n) {
