@@ -69,3 +69,29 @@ def test_emulated_ranks_exchange_then_local_sort_equals_the_oracle(tb, port, G):
         assert np.array_equal(gk.view(np.uint8), wk.view(np.uint8)) and np.array_equal(gv, wv), (G, kind)
         if kind == "u32":
             assert totals.max() <= 1.1 * totals.mean() + 4096, totals        # balanced to about one bin
+
+
+@pytest.mark.parametrize("buckets", [1, 2, 3, 8, 15, 16])
+def test_buckets_by_splitters(tb, buckets):
+    """tb200_bucket_count and tb200_bucket_scatter agree on which splitters precede a key, ties and equal splitters
+    included; pairs stay in input order inside their bucket."""
+    ops = DeviceOps()
+    for dt, n in ((np.uint32, 50021), (np.int64, 8193), (np.float32, 131072 + 5)):
+        keys = (dg.rand64(71, n) % np.uint64(1000)).astype(dt) - (dt(500) if dt != np.uint32 else dt(0))
+        for desc in (False, True):
+            splits = np.sort(keys[: 4 * buckets: 4][: buckets - 1])
+            if buckets > 3:
+                splits[2] = splits[1]
+            if desc:
+                splits = splits[::-1].copy()
+            bucket = (splits[None, :] >= keys[:, None] if desc else splits[None, :] <= keys[:, None]).sum(axis=1) if buckets > 1 else np.zeros(n, np.int64)
+            vals = np.arange(n, dtype=np.uint32)
+            k, v, sp = dev(keys), dev(vals), dev(splits if buckets > 1 else keys[:1])
+            counts = host(ops.bucket_count(k, sp, buckets, desc))
+            assert np.array_equal(counts, np.bincount(bucket, minlength=buckets)), (dt, desc)
+            ko = [torch.zeros(max(int(c), 1) + 3, dtype=k.dtype, device="cuda") for c in counts]
+            vo = [torch.zeros(max(int(c), 1) + 3, dtype=v.dtype, device="cuda") for c in counts]
+            ops.bucket_scatter(k, v, sp, [t.data_ptr() for t in ko], [t.data_ptr() for t in vo], [3] * buckets, desc)
+            torch.cuda.synchronize()
+            for b in range(buckets):
+                assert np.array_equal(host(ko[b])[3:3 + counts[b]], keys[bucket == b]) and np.array_equal(host(vo[b])[3:3 + counts[b]], vals[bucket == b])
