@@ -16,9 +16,8 @@
 // were two thirds of a pass: about 1.7 cycles each per SM.)  A digit place that all keys share is left out,
 // as in the general sort.  Same order, same stability.
 //
-// Measured on B200, microseconds here / on the general route, at 1 k, 32 k and 128 k items: u32 + u32 18 / 63,
-// 28 / 68, 61 / 74; f32 keys 17 / 64, 24 / 66, 51 / 66; f64 + u64 31 / 95, 53 / 101.  A pair of 16 bytes stops at 64 k
-// (81 / 103): the staged copy and the cluster's would not fit in shared memory.
+// Measured on B200, microseconds here / on the general route, at 1 k, 32 k and 64 k items: u32 + u32 17 / 51, 27 / 53, 35 / 54;
+// f32 keys 16 / 53, 23 / 55, 33 / 57; u64 + u64 31 / 66, 54 / 83, 80 / 85.  csort_max_items says where it stops.
 #pragma once
 #include "bulk_copy.cuh"
 #include "common.cuh"
@@ -29,7 +28,6 @@ namespace tb200 {
 constexpr int CSORT_BLOCK = 512;
 constexpr int CSORT_MAX_CTAS = 16;
 constexpr int CSORT_MAX_IPT = 16;
-constexpr size_t CSORT_MAX_ITEMS = (size_t)CSORT_BLOCK * CSORT_MAX_IPT * CSORT_MAX_CTAS;   // 131072
 
 __device__ __forceinline__ unsigned cluster_rank() { unsigned r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ unsigned cluster_size() { unsigned r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
@@ -92,6 +90,16 @@ __device__ __forceinline__ unsigned csort_rank(unsigned* my_hist, unsigned d, un
     rank = now - __popc(peers & lanemask_ge);
   }
   return rank;
+}
+
+// Up to how many items the cluster is the faster route: rows per warp of the largest cluster.  Microseconds here / on the
+// general route on either side of each line: u32 keys 49 / 54 and f32 50 / 57 at 128 k (as many as fit); u32 + u32 53 / 54 at
+// 112 k, 59 / 54 at 128 k; u16 + u32 29 / 31 at 96 k, 33 / 32 at 112 k; u8 + u32 19 / 24 at 128 k; u64 keys 79 / 86 at 80 k, 88 / 86 at
+// 96 k.  Pairs of 16 bytes stop at 64 k, where the staged copy and the cluster's fill shared memory (u64 + u32 84 / 94,
+// u64 + u64 80 / 85, u32 + u64 45 / 52).
+template <class UK, class UV, bool HAS_V> constexpr size_t csort_max_items() {
+  constexpr size_t item = sizeof(typename csort_item<UK, UV, HAS_V>::type), row = (size_t)CSORT_BLOCK * CSORT_MAX_CTAS;
+  return row * (item > 8 ? 8 : item < 8 ? CSORT_MAX_IPT : !HAS_V ? 11 : sizeof(UK) == 1 ? CSORT_MAX_IPT : 14);
 }
 
 template <class Item, int IPT> constexpr size_t csort_smem_bytes() {
@@ -271,7 +279,7 @@ cudaError_t cluster_sort_launch(UK* keys, UV* vals, size_t n, key_coding coding,
 template <class UK, class UV, bool HAS_V>
 cudaError_t cluster_sort_async(UK* keys, UV* vals, size_t n, key_coding coding, int first_pass, int num_passes, ws_header* hdr, cudaStream_t stream, bool& launched) {
   launched = false;
-  if (n > CSORT_MAX_ITEMS) return cudaSuccess;
+  if (n > csort_max_items<UK, UV, HAS_V>()) return cudaSuccess;
   auto go = [&](auto is_float, auto ipt) {
     return cluster_sort_launch<UK, UV, HAS_V, decltype(is_float)::value, decltype(ipt)::value>(keys, vals, n, coding, first_pass, num_passes, hdr, stream, launched);
   };

@@ -233,3 +233,16 @@ def test_sort_by_key_host_buffers_match_the_oracle(tb, port, n):
         assert np.array_equal(hk.numpy().view(np.uint8), k.view(np.uint8))             # inputs untouched when outputs are given
         tb.sort_by_key_host(hk, hv, descending=desc)                                   # in place
         assert np.array_equal(hk.numpy().view(np.uint8), wk.view(np.uint8)) and np.array_equal(hv.numpy().view(np.uint8), wv.view(np.uint8))
+
+
+@pytest.mark.parametrize("n", [81920, 90111, 90112, 90113, 114687, 114688, 114689])
+def test_small_sorts_where_the_cluster_hands_over(tb, port, n):
+    """The last sizes of 8-byte items that one cluster sorts and the first that the general route does."""
+    for dt, vt in [(np.uint64, None), (np.float64, None), (np.uint32, np.uint32), (np.uint16, np.uint32), (np.int8, np.uint32), (np.float32, np.uint32)]:
+        for small in (False, True):
+            k = rand_of(dt, n, 58, small=small)
+            v = None if vt is None else np.arange(n, dtype=vt)
+            kd, vd = dev(k), None if v is None else dev(v)
+            tb.sort(kd) if v is None else tb.sort_by_key(kd, vd)
+            ok, ov = port.sort_by_key(k, v, False)
+            assert np.array_equal(host(kd), ok) and (v is None or np.array_equal(host(vd), ov)), (dt, vt, small)
