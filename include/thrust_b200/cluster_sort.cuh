@@ -5,7 +5,7 @@
 // At these sizes the general sort (radix_sort.cuh) is a chain of dependent launches -- clear, histogram, bucket
 // bases, one per digit place, copy back -- each far too small to fill the chip; its time is launch and
 // look-back latency, whatever n is.  Here a digit place costs two cluster barriers:
-//   rank      every warp ranks its rows on private counters in shared memory (as onesweep_kernel does), the
+//   rank      every warp ranks its rows on private counters in shared memory (warp_rank, as onesweep_kernel does), the
 //             CTA stacks its warps' counts, pushes the 256 sums into every CTA of the cluster and puts its items
 //             in digit order in its own shared memory;
 //   barrier
@@ -64,33 +64,6 @@ template <class UK, class UV, bool HAS_V> struct csort_item { using type = UK; }
 template <class UK, class UV> struct csort_item<UK, UV, true> {
   struct alignas(sizeof(UK) + sizeof(UV) <= 8 ? 8 : 16) type { UV v; UK k; };
 };
-
-// Rank of this lane's digit d among the warp's items so far; bumps the warp's counters.  See onesweep_tile.
-__device__ __forceinline__ unsigned csort_rank(unsigned* my_hist, unsigned d, unsigned lanemask_ge) {
-  const unsigned old = atomicAdd(&my_hist[d], 1u);
-  __syncwarp();
-  const unsigned now = *reinterpret_cast<volatile unsigned*>(&my_hist[d]);
-  unsigned pending = __ballot_sync(FULL_MASK, now - old > 1u);
-  unsigned rank = old;
-  if (__popc(pending) <= 6) {
-    while (pending) {
-      const unsigned dsrc = __shfl_sync(FULL_MASK, d, 31 - __clz(pending));
-      const unsigned peers = __ballot_sync(FULL_MASK, d == dsrc);
-      if (d == dsrc) rank = now - __popc(peers & lanemask_ge);
-      pending &= ~peers;
-    }
-  } else {
-    unsigned peers = FULL_MASK;
-#pragma unroll
-    for (int b = 0; b < RADIX_BITS; ++b) {
-      const bool bit = (d >> b) & 1;
-      const unsigned vote = __ballot_sync(FULL_MASK, bit);
-      peers &= bit ? vote : ~vote;
-    }
-    rank = now - __popc(peers & lanemask_ge);
-  }
-  return rank;
-}
 
 // Up to how many items the cluster is the faster route: rows per warp of the largest cluster.  Microseconds here / on the
 // general route on either side of each line: u32 keys 49 / 54 and f32 50 / 57 at 128 k (as many as fit); u32 + u32 53 / 54 at
@@ -153,7 +126,7 @@ cluster_sort_kernel(UK* keys, UV* vals, unsigned n, unsigned rows, key_coding co
       if ((unsigned)i < rows && warp * (32 * rows) + i * 32 < mine) {       // the row holds items
         // places past the end in the input's last row hold the highest digit and rank last
         const unsigned d = wofs + i * 32 < mine ? key_digit<IS_FLOAT>(key[i], shift, dmask) : (unsigned)(RADIX_BINS - 1);
-        pd[i] = csort_rank(my_hist, d, lanemask_ge) | (d << 16);
+        pd[i] = warp_rank<RADIX_BITS>(my_hist, d, lanemask_ge) | (d << 16);
       }
     }
     __syncthreads();

@@ -197,9 +197,6 @@ template <class UK, class UV> struct bucket_policy {
 #ifndef TB200_SWEEP_LB_BATCH
 #define TB200_SWEEP_LB_BATCH 4      // descriptors fetched per round trip of the look-back
 #endif
-#ifndef TB200_SWEEP_LOOP_MAX
-#define TB200_SWEEP_LOOP_MAX 6      // rows with more colliding lanes than this are ranked with ballots
-#endif
 
 // Staged item: a key and its value side by side, so that one shared-memory store / load moves both.
 template <class UK, class UV, bool HAS_V, bool PACKED> struct sweep_stage;
@@ -262,16 +259,6 @@ __device__ __forceinline__ void sweep_load_any(sweep_regs<UK, UV, HAS_V, IPT>& r
 // needs no registers for ranks.  Measured on B200 against ranking first, 2^26 u32 + u32 pairs 1.40 ms (1.59),
 // 2^26 f32 keys 1.12 (1.26), 20 M u64 + u32 0.86 (0.94), 4 M f64 + u64 0.356 (0.387); 256-thread CTAs, 20 items per
 // thread and eight descriptors per round trip of the look-back were all slower or the same.
-//
-// Ranking.  Every lane adds 1 to its warp's private counter of its digit and then reads the counter
-// back: `old` is some slot of the digit's group in this row, `now - old > 1` tells all members of a
-// group of two or more lanes, except the one that drew the last slot, that they collided.  Lanes
-// that did not collide are done (rank = old).  Groups are then put in lane order one at a time: the
-// highest colliding lane announces its digit, one ballot finds its group, each member takes
-// base + (members in lower lanes).  With 256 bins and 32 lanes a row has about two groups, which
-// costs half the instructions of finding every lane's peers with one ballot per digit bit; rows
-// with more than TB200_SWEEP_LOOP_MAX colliding lanes (skewed digits, the padded last tile) take
-// the ballots.  The result does not depend on the order in which the hardware serves the atomics.
 template <class UK, class UV, bool HAS_V, class Policy, class LB, int IPT, bool FULL>
 __device__ __forceinline__ void onesweep_tile(sweep_regs<UK, UV, HAS_V, IPT>& r, const UK* __restrict__ src, const UV* __restrict__ vsrc, unsigned n,
                                               unsigned tile, unsigned num_tiles, unsigned* next_ticket, unsigned& next, const Policy policy,
@@ -339,28 +326,7 @@ __device__ __forceinline__ void onesweep_tile(sweep_regs<UK, UV, HAS_V, IPT>& r,
     unsigned d;
     if constexpr (FEW) d = (unsigned)(kept[i / 16] >> (4 * (i % 16))) & 15u;
     else d = (FULL || wofs + i * 32 < tile_n) ? policy.digit(r.key[i]) : (unsigned)PAD_DIGIT;
-    const unsigned old = atomicAdd(&my_hist[d], 1u);
-    __syncwarp();   // every lane's increment precedes every lane's read
-    const unsigned now = *reinterpret_cast<volatile unsigned*>(&my_hist[d]);
-    unsigned pending = __ballot_sync(FULL_MASK, now - old > 1u);
-    unsigned place = old;
-    if (Policy::BITS > 4 && __popc(pending) <= TB200_SWEEP_LOOP_MAX) {
-      while (pending) {
-        const unsigned dsrc = __shfl_sync(FULL_MASK, d, 31 - __clz(pending));
-        const unsigned peers = __ballot_sync(FULL_MASK, d == dsrc);
-        if (d == dsrc) place = now - __popc(peers & lanemask_ge);   // base + members in lower lanes
-        pending &= ~peers;
-      }
-    } else if (pending) {
-      unsigned peers = FULL_MASK;
-#pragma unroll
-      for (int b = 0; b < Policy::BITS; ++b) {
-        const bool bit = (d >> b) & 1;
-        const unsigned vote = __ballot_sync(FULL_MASK, bit);
-        peers &= bit ? vote : ~vote;
-      }
-      place = now - __popc(peers & lanemask_ge);
-    }
+    const unsigned place = warp_rank<Policy::BITS>(my_hist, d, lanemask_ge);
     stage.put(place, r.key[i], r.val[HAS_V ? i : 0]);
   }
   next = *s_next;

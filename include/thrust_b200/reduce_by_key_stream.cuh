@@ -25,7 +25,7 @@ namespace tb200 {
 // This lane's VEC items of row `row` (32 lanes x VEC items); items past the end read as T().
 // FULL: the caller knows that the row lies wholly inside the input (no bounds checks at all).
 template <class T, int VEC, bool FULL = false>
-__device__ __forceinline__ void select_row_load(const T* in, size_t n, size_t row, int lane, T (&x)[VEC]) {
+__device__ __forceinline__ void rbk_row_load(const T* in, size_t n, size_t row, int lane, T (&x)[VEC]) {
   const size_t i0 = (row * 32 + lane) * VEC;
   if (FULL || (row + 1) * 32 * VEC <= n) {
     vec16 r = load_stream16(reinterpret_cast<const char*>(in) + i0 * sizeof(T));
@@ -38,39 +38,32 @@ __device__ __forceinline__ void select_row_load(const T* in, size_t n, size_t ro
   }
 }
 
-// Shared by both passes: this lane's keep bits for the items x of row `row`.  `prev_tail` carries
-// the last item of the previous row for SEL_UNIQUE-style predicates.
-template <bool UNIQUE, class T, class Pred, int VEC, bool FULL = false>
-__device__ __forceinline__ unsigned select_row_flags(size_t n, size_t row, int lane, Pred pred, const T (&x)[VEC], T& prev_tail, bool& have_prev) {
+// Shared by both passes: this lane's run heads among the keys x of row `row`, bit k for its k-th.  `prev_tail` carries
+// the last key of the previous row.
+template <class T, class Eq, int VEC, bool FULL = false>
+__device__ __forceinline__ unsigned rbk_row_heads(size_t n, size_t row, int lane, Eq eq, const T (&x)[VEC], T& prev_tail, bool& have_prev) {
   const size_t i0 = (row * 32 + lane) * VEC;
   const bool row_full = FULL || (row + 1) * 32 * VEC <= n;
   unsigned bits = 0;
-  if constexpr (UNIQUE) {
-    // predecessor of this lane's first item: the previous lane's last item, or the previous row's
-    T prev = shfl_up(x[VEC - 1], 1);
-    bool has = true;
-    if (lane == 0) { prev = prev_tail; has = have_prev; }
+  // predecessor of this lane's first key: the previous lane's last one, or the previous row's
+  T prev = shfl_up(x[VEC - 1], 1);
+  bool has = true;
+  if (lane == 0) { prev = prev_tail; has = have_prev; }
 #pragma unroll
-    for (int k = 0; k < VEC; ++k) {
-      const bool head = (k == 0 && !has) ? true : !pred(k == 0 ? prev : x[k - 1], x[k]);
-      if ((row_full || i0 + k < n) && head) bits |= 1u << k;
-    }
-    prev_tail = shfl_idx(x[VEC - 1], 31);
-    have_prev = true;
-  } else {
-#pragma unroll
-    for (int k = 0; k < VEC; ++k)
-      if ((row_full || i0 + k < n) && pred(x[k])) bits |= 1u << k;
+  for (int k = 0; k < VEC; ++k) {
+    const bool head = (k == 0 && !has) ? true : !eq(k == 0 ? prev : x[k - 1], x[k]);
+    if ((row_full || i0 + k < n) && head) bits |= 1u << k;
   }
+  prev_tail = shfl_idx(x[VEC - 1], 31);
+  have_prev = true;
   return bits;
 }
 
-// predecessor of a batch's first item, for SEL_UNIQUE-style predicates
-template <class T> __device__ __forceinline__ void select_batch_start(const T* in, size_t first_row, int vec, T& prev_tail, bool& have_prev) {
+// predecessor of a batch's first key
+template <class T> __device__ __forceinline__ void rbk_batch_start(const T* in, size_t first_row, int vec, T& prev_tail, bool& have_prev) {
   have_prev = first_row > 0;
   prev_tail = have_prev ? in[first_row * 32 * vec - 1] : T();
 }
-
 
 constexpr int RBK_STREAM_BLOCK = 256;
 // Measured on B200, 2^28 int32 keys + fp32 values, runs of mean length 4: 1.24 ms with two rows per batch
@@ -100,7 +93,7 @@ template <class V, class Op> struct rbk_stream_combine {
 template <class K, class V, class Eq, class Op, int VEC, bool FULL = false>
 __device__ __forceinline__ rbk_stream_pair<V> rbk_stream_row(const K* keys, const V* vals, size_t n, size_t row, int lane, Eq eq, Op op, const K (&k)[VEC],
                                                             const V (&v)[VEC], K& prev_tail, bool& have_prev, unsigned& bits, unsigned& valid) {
-  bits = select_row_flags<true, K, Eq, VEC, FULL>(n, row, lane, eq, k, prev_tail, have_prev);
+  bits = rbk_row_heads<K, Eq, VEC, FULL>(n, row, lane, eq, k, prev_tail, have_prev);
   const size_t i0 = (row * 32 + lane) * VEC;
   valid = FULL ? (1u << VEC) - 1 : 0u;
   if (!FULL) {
@@ -175,7 +168,7 @@ rbk_stream_count_kernel(const K* keys, const V* vals, size_t n, size_t rows, siz
   for (size_t batch = gwarp; batch < batches; batch += nwarps) {
     const size_t first = batch * RBK_STREAM_ROWS;
     K prev_tail = K(); bool have_prev = false;
-    select_batch_start(keys, first, VEC, prev_tail, have_prev);
+    rbk_batch_start(keys, first, VEC, prev_tail, have_prev);
     P acc; acc.count = 0; acc.value = V();
     bool have_acc = false;
     // all batches but the last lie wholly inside the input: no bounds checks for them
@@ -185,7 +178,7 @@ rbk_stream_count_kernel(const K* keys, const V* vals, size_t n, size_t rows, siz
       V v[RBK_STREAM_ROWS][VEC];
 #pragma unroll
       for (int u = 0; u < RBK_STREAM_ROWS; ++u)
-        if (FULL || first + u < rows) { select_row_load<K, VEC, FULL>(keys, n, first + u, lane, k[u]); select_row_load<V, VEC, FULL>(vals, n, first + u, lane, v[u]); }
+        if (FULL || first + u < rows) { rbk_row_load<K, VEC, FULL>(keys, n, first + u, lane, k[u]); rbk_row_load<V, VEC, FULL>(vals, n, first + u, lane, v[u]); }
 #pragma unroll
       for (int u = 0; u < RBK_STREAM_ROWS; ++u) {
         if (!FULL && first + u >= rows) break;
@@ -221,14 +214,14 @@ rbk_stream_emit_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, s
     P carry; carry.count = 0; carry.value = V();
     if (batch > 0) carry = batch_incl[batch - 1];
     K prev_tail = K(); bool have_prev = false;
-    select_batch_start(keys, first, VEC, prev_tail, have_prev);
+    rbk_batch_start(keys, first, VEC, prev_tail, have_prev);
     auto body = [&](auto full_tag) {
     constexpr bool FULL = decltype(full_tag)::value;
     K k[RBK_STREAM_ROWS][VEC];
     V v[RBK_STREAM_ROWS][VEC];
 #pragma unroll
     for (int u = 0; u < RBK_STREAM_ROWS; ++u)
-      if (FULL || first + u < rows) { select_row_load<K, VEC, FULL>(keys, n, first + u, lane, k[u]); select_row_load<V, VEC, FULL>(vals, n, first + u, lane, v[u]); }
+      if (FULL || first + u < rows) { rbk_row_load<K, VEC, FULL>(keys, n, first + u, lane, k[u]); rbk_row_load<V, VEC, FULL>(vals, n, first + u, lane, v[u]); }
 #pragma unroll
     for (int u = 0; u < RBK_STREAM_ROWS; ++u) {
       if (!FULL && first + u >= rows) break;
@@ -352,14 +345,14 @@ scan_by_key_stream_kernel(const K* keys, const V* vals, V* out, size_t n, size_t
     P carry; carry.count = 0; carry.value = V();
     if (batch > 0) carry = batch_incl[batch - 1];
     K prev_tail = K(); bool have_prev = false;
-    select_batch_start(keys, first, VEC, prev_tail, have_prev);
+    rbk_batch_start(keys, first, VEC, prev_tail, have_prev);
     auto body = [&](auto full_tag) {
     constexpr bool FULL = decltype(full_tag)::value;
     K k[RBK_STREAM_ROWS][VEC];
     V v[RBK_STREAM_ROWS][VEC];
 #pragma unroll
     for (int u = 0; u < RBK_STREAM_ROWS; ++u)
-      if (FULL || first + u < rows) { select_row_load<K, VEC, FULL>(keys, n, first + u, lane, k[u]); select_row_load<V, VEC, FULL>(vals, n, first + u, lane, v[u]); }
+      if (FULL || first + u < rows) { rbk_row_load<K, VEC, FULL>(keys, n, first + u, lane, k[u]); rbk_row_load<V, VEC, FULL>(vals, n, first + u, lane, v[u]); }
 #pragma unroll
     for (int u = 0; u < RBK_STREAM_ROWS; ++u) {
       if (!FULL && first + u >= rows) break;

@@ -178,9 +178,8 @@ template <class T> size_t select_workspace_bytes(size_t n) {
 constexpr size_t SELECT_PIPE_MIN_BYTES = (size_t)1 << 22;
 constexpr size_t SELECT_PIPE_MIN_BYTES_REJECTS = (size_t)1 << 20;
 
-// Whether the pipeline may serve a call: a large, 16-byte aligned input and outputs that do not overlap it
-// (out_rej: null if
-// there is no second one).  rejects: dropped items are written too.
+// Whether the pipeline may serve a call: a large, 16-byte aligned input and outputs that do not overlap it (out_rej: null
+// if there is no second one; the in-place partition passes its scratch as out_sel).  rejects: dropped items are written too.
 inline bool select_pipe_eligible(const void* in, const void* out_sel, const void* out_rej, size_t n, size_t item_bytes, bool rejects) {
   const char* ib = static_cast<const char*>(in);
   const char* ob = static_cast<const char*>(out_sel);

@@ -115,7 +115,7 @@ __device__ __forceinline__ double_pair add_to_pair(const double_pair& a, double 
   return r;
 }
 
-template <class Chain> __device__ typename Chain::C pipe_fold_round(const typename Chain::C (&v)[PIPE_SLOTS], int count);
+template <class Chain> __device__ __forceinline__ typename Chain::C pipe_fold_round(const typename Chain::C (&v)[PIPE_SLOTS], int count);
 
 template <class T, class Op> struct tile_chain {
   using C = T;
@@ -215,8 +215,8 @@ __device__ __forceinline__ unsigned pipe_tail_fill(T* dst, const T* src, size_t 
 }
 
 // The same for a tile whose warps' parts lie 16 bytes apart in shared memory, so that a warp can compact its part in
-// place at the distance from a 16-byte boundary that its output has: PIPE_PARTS parts of PART items, one per lane of
-// the loader.  bytes(left): what the copies of a tile with `left` items up to the input's end bring in all.
+// place at the distance from a 16-byte boundary that its output has: PIPE_WARPS parts of PART items, copied by one
+// lane of the loader each.  bytes(left): what the copies of a tile with `left` items up to the input's end bring in all.
 template <class T, int PART> struct pipe_parts {
   static constexpr unsigned STRIDE = PART * sizeof(T) + 16, BYTES = PIPE_WARPS * STRIDE;
   __device__ static unsigned part_bytes(size_t left, unsigned part) {
