@@ -52,7 +52,8 @@ int tb200_workspace_status(const void* d_ws, tb200_stream_t stream, unsigned* h_
 /* Synchronises `stream` and copies the first `bytes` (at most 256) of a workspace's header to h_dst, in one
  * transfer through pinned memory: bytes 0-3 the status word above, bytes 8-15 the count that the selecting and
  * counting entry points leave there.  Bytes 32-255 are free for a caller's own small results once a call has been
- * enqueued: tb200_reduce may be given d_ws + 32 as its d_out. */
+ * enqueued: tb200_reduce may be given d_ws + 32 as its d_out.  Threads that share a workspace must keep one call's launch
+ * and this read together (a lock, as the Python layer holds): the header is the last call's. */
 int tb200_workspace_read(const void* d_ws, size_t bytes, void* h_dst, tb200_stream_t stream);
 
 /* thrust::reduce(first, last, init, op) -- thrust/system/cuda/detail/reduce.h:1015-1067
