@@ -233,8 +233,21 @@ template <class T> __device__ __forceinline__ void slice_ends(T* dst, const T* s
   if (t + lane < n) dst[t + lane] = src[t + lane];   // fewer than 16 / sizeof(T) items
 }
 
-// First item of A in every tile, by a warp per tile: 32 probes of the diagonal per round trip, so that the
-// search over 2^k items takes k / 5 of them instead of k (a chain of cache misses that small inputs waited for).
+// Where diagonal `diag` of merge(a[0, alen), b[0, blen)) is split, by a warp with 32 probes per round trip, so that the search over
+// 2^k items takes k / 5 of them instead of k.  The same result in every lane.
+template <class K, class Comp>
+__device__ __forceinline__ size_t warp_merge_path(const K* a, size_t alen, const K* b, size_t blen, size_t diag, Comp comp) {
+  size_t lo = diag > blen ? diag - blen : 0, hi = diag < alen ? diag : alen;
+  while (lo < hi) {
+    const size_t step = (hi - lo + 31) / 32, mid = lo + lane_id() * step;
+    const unsigned below = __popc(__ballot_sync(FULL_MASK, mid < hi && !comp(b[diag - 1 - mid], a[mid])));   // a prefix of the lanes
+    if (below < 32 && lo + below * step < hi) hi = lo + below * step;
+    if (below) lo += (below - 1) * step + 1;
+  }
+  return lo;
+}
+
+// First item of A in every tile, by a warp per tile: few round trips, which is what a small input waits for.
 template <class K, class Comp, int TILE>
 __global__ void __launch_bounds__(256)
 merge_split_kernel(const K* ka, const K* kb, merge_geometry g, unsigned num_tiles, Comp comp, size_t* a_split) {
@@ -244,17 +257,68 @@ merge_split_kernel(const K* ka, const K* kb, merge_geometry g, unsigned num_tile
   if (t >= num_tiles) return;
   size_t a0, alen, b0, blen, pair_out, local;
   g.locate<TILE>(t, a0, alen, b0, blen, pair_out, local);
-  const size_t total = alen + blen, diag = local < total ? local : total;
+  const size_t total = alen + blen;
+  const size_t lo = warp_merge_path(ka + a0, alen, kb + b0, blen, local < total ? local : total, comp);
+  if (lane_id() == 0) a_split[t] = a0 + lo;
+}
+
+// The same for many tiles, a thread per tile.  What bounds it there is the number of scattered 32-byte reads: a warp per tile
+// makes 64 of them in each round trip that misses.  Here two warps find the splits of the CTA's first and last diagonal,
+// which bound all splits between; a thread starts from where the split would lie if A and B were evenly mixed
+// in between, widens its step until the split is passed, and halves.
+constexpr int SPLIT_GROUP = 256;   // tiles of a CTA
+template <class K, class Comp, int TILE>
+__global__ void __launch_bounds__(SPLIT_GROUP)
+merge_split_group_kernel(const K* ka, const K* kb, merge_geometry g, unsigned groups_per_pair, Comp comp, size_t* a_split) {
+  __shared__ size_t s_end[2];
+  grid_dependents_launch();
+  grid_dependency_wait();
+  const size_t pair = blockIdx.x / groups_per_pair, first = (size_t)(blockIdx.x % groups_per_pair) * SPLIT_GROUP;   // inside the pair
+  const size_t in_pair = first + threadIdx.x, t = pair * g.tiles_per_pair + in_pair;
+  size_t a0, alen, b0, blen, pair_out, local;
+  g.locate<TILE>(pair * g.tiles_per_pair, a0, alen, b0, blen, pair_out, local);
+  const size_t total = alen + blen;
   const K* a = ka + a0;
   const K* b = kb + b0;
-  size_t lo = diag > blen ? diag - blen : 0, hi = diag < alen ? diag : alen;
-  while (lo < hi) {
-    const size_t step = (hi - lo + 31) / 32, mid = lo + lane_id() * step;
-    const unsigned below = __popc(__ballot_sync(FULL_MASK, mid < hi && !comp(b[diag - 1 - mid], a[mid])));   // a prefix of the lanes
-    if (below < 32 && lo + below * step < hi) hi = lo + below * step;
-    if (below) lo += (below - 1) * step + 1;
+  auto diag_of = [&](size_t tile) { const size_t d = tile * TILE; return d < total ? d : total; };
+  const size_t d0 = diag_of(first), d1 = diag_of(first + SPLIT_GROUP);
+  const int warp = threadIdx.x >> 5;
+  if (warp < 2) {
+    const size_t s = warp_merge_path(a, alen, b, blen, warp ? d1 : d0, comp);
+    if (lane_id() == 0) s_end[warp] = s;
   }
-  if (lane_id() == 0) a_split[t] = a0 + lo;
+  __syncthreads();
+  if (in_pair >= g.tiles_per_pair) return;
+  const size_t diag = diag_of(in_pair), s0 = s_end[0], s1 = s_end[1];
+  size_t lo = diag > blen ? diag - blen : 0, hi = diag < alen ? diag : alen;
+  // a split lies between those of earlier and later diagonals (under a comparator that is no order it need not; then the
+  // diagonal's own bounds stand, as everywhere)
+  const size_t lo2 = lo > s0 ? lo : s0, hi2 = hi < s1 ? hi : s1;
+  if (lo2 <= hi2) { lo = lo2; hi = hi2; }
+  auto past = [&](size_t mid) { return !comp(b[diag - 1 - mid], a[mid]); };   // the split lies behind item `mid`
+  if (lo < hi) {
+    size_t mid = s1 > s0 && d1 > d0 ? s0 + (size_t)((double)(s1 - s0) * (double)(diag - d0) / (double)(d1 - d0)) : lo;
+    mid = mid < lo ? lo : mid >= hi ? hi - 1 : mid;
+    size_t width = 64;
+    if (past(mid)) {
+      lo = mid + 1;
+      while (lo < hi) {
+        mid = hi - lo > width ? lo + width : hi - 1;
+        if (past(mid)) { lo = mid + 1; width *= 4; } else { hi = mid; break; }
+      }
+    } else {
+      hi = mid;
+      while (lo < hi) {
+        mid = hi - lo > width ? hi - width : lo;
+        if (past(mid)) { lo = mid + 1; break; } else { hi = mid; width *= 4; }
+      }
+    }
+    while (lo < hi) {
+      mid = (lo + hi) >> 1;
+      if (past(mid)) lo = mid + 1; else hi = mid;
+    }
+  }
+  a_split[t] = a0 + lo;
 }
 
 template <class K, class V, bool HAS_V, class Comp>
@@ -391,6 +455,19 @@ template <class K, class V, bool HAS_V> size_t merge_workspace_bytes(size_t tota
   return sizeof(ws_header) + align_up((4 * tiles + 8) * sizeof(size_t), 256);
 }
 
+// The splits of a pass.  Beyond 4096 tiles a thread per tile is faster on every shape tried (2 x 2^26 u64, microseconds here /
+// a warp per tile: 39 / 201 uniform, 29 / 164 normal against uniform, 57 / 184 with 1000 distinct values, 12 / 164 disjoint;
+// 16384 tiles in sorted runs of 2^12 20 / 25, of 2^17 16 / 37); at 4096 tiles both take 18, at 1024 it is 16 / 10.
+constexpr unsigned SPLIT_WARP_TILES = 4096;
+template <class K, class Comp, int TILE>
+cudaError_t merge_split_async(const K* ka, const K* kb, const merge_geometry& g, unsigned tiles, Comp comp, size_t* a_split, bool overlap, cudaStream_t stream) {
+  if (tiles <= SPLIT_WARP_TILES) return launch_after(merge_split_kernel<K, Comp, TILE>, (tiles + 7) / 8, 256, 0, stream, ka, kb, g, tiles, comp, a_split);
+  const unsigned groups = (unsigned)((g.tiles_per_pair + SPLIT_GROUP - 1) / SPLIT_GROUP), grid = (unsigned)(tiles / g.tiles_per_pair) * groups;
+  if (overlap) return launch_after(merge_split_group_kernel<K, Comp, TILE>, grid, SPLIT_GROUP, 0, stream, ka, kb, g, groups, comp, a_split);
+  merge_split_group_kernel<K, Comp, TILE><<<grid, SPLIT_GROUP, 0, stream>>>(ka, kb, g, groups, comp, a_split);
+  return cudaGetLastError();
+}
+
 // One merge pass (single or pairwise geometry); no sync.
 template <class K, class V, bool HAS_V, class KeyItA, class KeyItB, class ValItA, class ValItB, class KeyOutIt, class ValOutIt, class Comp>
 cudaError_t merge_pass_async(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutIt ko, ValOutIt vo, merge_geometry g, Comp comp, void* ws,
@@ -405,16 +482,16 @@ cudaError_t merge_pass_async(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutI
     const unsigned tiles = (unsigned)g.num_tiles();
     // Up to 8192 tiles (16 M outputs) the pass's launches overlap the kernels before them (8 M pairs sorted in 0.47 ms
     // against 0.51); beyond, waiting CTAs only take slots from running ones (2^26 pairs 4.53 ms against 4.35).
-    if (tiles <= 8192) {
-      cudaError_t e = launch_after(merge_split_kernel<K, Comp, Tuning::TILE>, (tiles + 7) / 8, 256, 0, stream, ka, kb, g, tiles, comp, a_split);
-      if (e != cudaSuccess) return e;
+    const bool overlap = tiles <= 8192;
+    const cudaError_t e = merge_split_async<K, Comp, Tuning::TILE>(ka, kb, g, tiles, comp, a_split, overlap, stream);
+    if (e != cudaSuccess) return e;
+    if (overlap) {
       timed_launch tl(KID_MERGE, stream);
-      e = launch_after(merge_slices_kernel<K, V, HAS_V, Comp>, tiles, MERGE_BLOCK, 0, stream, ka, kb, va, vb, ko, vo, g, comp, (const size_t*)a_split,
-                       &static_cast<ws_header*>(ws)->error);
+      const cudaError_t le = launch_after(merge_slices_kernel<K, V, HAS_V, Comp>, tiles, MERGE_BLOCK, 0, stream, ka, kb, va, vb, ko, vo, g, comp,
+                                          (const size_t*)a_split, &static_cast<ws_header*>(ws)->error);
       log_launch("merge_slices_kernel", tiles, MERGE_BLOCK, 0, g.n, stream);
-      return e;
+      return le;
     }
-    merge_split_kernel<K, Comp, Tuning::TILE><<<(tiles + 7) / 8, 256, 0, stream>>>(ka, kb, g, tiles, comp, a_split);
     timed_launch tl(KID_MERGE, stream);
     merge_slices_kernel<K, V, HAS_V, Comp><<<tiles, MERGE_BLOCK, 0, stream>>>(ka, kb, va, vb, ko, vo, g, comp, a_split, &static_cast<ws_header*>(ws)->error);
     log_launch("merge_slices_kernel", tiles, MERGE_BLOCK, 0, g.n, stream);

@@ -127,3 +127,29 @@ def test_merge_of_keys_with_nans_ends(tb, port, dt):
         ko, vo = tb.merge_by_key(dev(a), dev(b), dev(va), dev(vb))
         rk, rv = port.merge_by_key(a, b, va, vb)
         assert np.array_equal(host(ko), rk) and np.array_equal(host(vo), rv)
+
+
+@pytest.mark.parametrize("n", [4096 * 2048 + 1, 256 * 17 * 2048, 256 * 18 * 2048 + 2047])
+def test_merge_splits_of_many_tiles(tb, port, n):
+    """More than 4096 tiles of 2048 outputs: a thread per tile between the splits of its group of 256.  Even and uneven mixes,
+    ties, ranges that do not overlap, one side empty or a single item; whole groups and a last group of one tile."""
+    rnd = lambda seed, m, bits: np.sort((dg.rand64(seed, m) >> np.uint64(64 - bits)).astype(np.uint32))  # noqa: E731
+    third, high = n // 3, np.uint32(1 << 31)
+    for a, b in [(rnd(1, n - third, 31), rnd(2, third, 31)), (rnd(3, n // 2, 2), rnd(4, n - n // 2, 3)), (rnd(5, third, 30) + high, rnd(6, n - third, 30)),
+                 (rnd(7, n - 1, 30), rnd(8, 1, 30)), (rnd(9, 0, 30), rnd(10, n, 30)),
+                 (np.sort(rnd(11, n // 2, 30) // np.uint32(1 << 20) * np.uint32(1 << 10)), rnd(12, n - n // 2, 20))]:
+        va, vb = np.arange(a.size, dtype=np.uint32), np.arange(b.size, dtype=np.uint32) + high
+        ko, vo = tb.merge_by_key(dev(a), dev(b), dev(va), dev(vb))
+        rk, rv = port.merge_by_key(a, b, va, vb)
+        assert np.array_equal(host(ko), rk) and np.array_equal(host(vo), rv), (a.size, b.size)
+
+
+def test_merge_sort_splits_of_many_tiles(tb, port):
+    """The same in the passes of a sort: pairs of fewer and of more tiles than a group, a short last pair."""
+    n = 4200 * 2048 + 777
+    for bits in (32, 3):
+        k, v = (dg.rand64(13, n) >> np.uint64(64 - bits)).astype(np.uint32), np.arange(n, dtype=np.uint32)
+        dk, dv = dev(k), dev(v)
+        tb.merge_sort_by_key(dk, dv)
+        rk, rv = port.sort_by_key(k, v)
+        assert np.array_equal(host(dk), rk) and np.array_equal(host(dv), rv)
