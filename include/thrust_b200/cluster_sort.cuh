@@ -244,6 +244,7 @@ cudaError_t cluster_sort_launch(UK* keys, UV* vals, size_t n, key_coding coding,
   timed_launch tl(KID_ONESWEEP, stream);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, keys, vals, (unsigned)n, rows, coding, first_pass, num_passes, hdr);
   if (launch_refused(e)) return cudaSuccess;
+  reported(report_of(hdr), hdr);   // nothing to report: no wait of this kernel runs out
   launched = true;
   log_launch("cluster_sort_kernel", ctas, CSORT_BLOCK, smem, n, stream);
   return e;

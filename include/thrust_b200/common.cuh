@@ -66,6 +66,20 @@ struct ws_header {
 };
 static_assert(sizeof(ws_header) == 256, "workspace header is 256 bytes");
 
+// Where a call's kernels leave its status and count for the host.  A caller that waits for its result anyway names the
+// workspace beforehand (tb200_workspace_watch, in the thread that makes the call), and the kernels then write status and count to a block of
+// pinned host memory instead of the header, so that the wait for the stream is all there is left to do: fetching 16 bytes
+// with a copy took 5 us of the 14.8 that clearing, a one-CTA kernel, that copy and the wait take together.
+struct host_report {
+  const void* ws = nullptr;      // the watched workspace
+  ws_header* block = nullptr;    // pinned, mapped, a header's layout
+  bool served = false;           // kernels that write to `block` were launched
+};
+inline host_report& thread_report() { static thread_local host_report r; return r; }
+// the header to which kernels launched on workspace `hdr` report, and the note that they were launched
+inline ws_header* report_of(ws_header* hdr) { const host_report& r = thread_report(); return r.ws == hdr && r.block ? r.block : hdr; }
+inline void reported(const ws_header* rep, const ws_header* hdr) { if (rep != hdr) thread_report().served = true; }
+
 #ifdef TB200_TEST_HOOKS
 // Test builds only: a process-wide switch.  Bits 0 and 1 are copied into the workspace header's flags (0: tile 0 of the
 // single-pass scan and of the pipelines does not publish; 1: a merge tile waits for bytes that nobody sends), bit 2 asks for
@@ -386,7 +400,11 @@ template <class T> __device__ __forceinline__ T load_cg_any(const T* p) {
   return v;
 }
 
-__device__ __forceinline__ void record_error(unsigned* err, unsigned code) { atomicCAS(err, ERR_NONE, code); }
+// (no atomic: `err` may lie in host memory; whichever of several codes stays is as good)
+__device__ __forceinline__ void record_error(unsigned* err, unsigned code) {
+  volatile unsigned* const e = err;
+  if (*e == ERR_NONE) *e = code;
+}
 
 __device__ __forceinline__ void backoff(unsigned iter) { if (iter > 8) __nanosleep(iter > 64 ? 200 : 40); }
 

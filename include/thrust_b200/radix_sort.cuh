@@ -431,7 +431,7 @@ __device__ __forceinline__ void sweep_tiles(const UK* __restrict__ src, const UV
 template <class UK, class UV, bool HAS_V, bool IS_FLOAT, class LB, int IPT>
 __global__ void __launch_bounds__(ONESWEEP_BLOCK, ONESWEEP_CTAS_PER_SM)
 onesweep_kernel(UK* buf_a, UK* buf_b, UV* val_a, UV* val_b, unsigned n, key_coding coding, int pass, int first_pass,
-                radix_ctrl* ctrl, LB* lookback, ws_header* hdr) {
+                radix_ctrl* ctrl, LB* lookback, ws_header* rep) {
   grid_dependents_launch();
   grid_dependency_wait();
   if (ctrl->skip[pass]) return;
@@ -446,7 +446,7 @@ onesweep_kernel(UK* buf_a, UK* buf_b, UV* val_a, UV* val_b, unsigned n, key_codi
   using Policy = radix_pass_policy<UK, UV, IS_FLOAT>;
   const Policy policy{dst, vdst, shift, digit_mask<UK>(coding, shift)};
   const unsigned my_bin_base = threadIdx.x < RADIX_BINS ? (unsigned)ctrl->hist[pass][threadIdx.x] : 0u;
-  sweep_tiles<UK, UV, HAS_V, Policy, LB, IPT>(src, vsrc, n, &ctrl->tickets[pass], policy, my_bin_base, lookback, &hdr->error, smem_raw);
+  sweep_tiles<UK, UV, HAS_V, Policy, LB, IPT>(src, vsrc, n, &ctrl->tickets[pass], policy, my_bin_base, lookback, &rep->error, smem_raw);
 }
 
 // ---------------------------------------------------------------- multi-GPU: bucket count and scatter
@@ -760,15 +760,17 @@ cudaError_t radix_sort_async(UK* keys_a, UK* keys_b, UV* vals_a, UV* vals_b, siz
   // persistent CTAs, two resident per SM; tiles are handed out by ticket
   const size_t tiles_all = sweep_tiles_of<KB, VB>(n);
   const unsigned grid = (unsigned)(tiles_all < (size_t)di.sm_count * ONESWEEP_CTAS_PER_SM ? tiles_all : (size_t)di.sm_count * ONESWEEP_CTAS_PER_SM);
+  ws_header* const rep = report_of(hdr);
+  reported(rep, hdr);
   for (int p = 0; p < num_passes; ++p) {
     char* lb = lb0 + lb_bytes * p;
     timed_launch tl(KID_ONESWEEP, stream);
     if (lb32)
       e = launch_after(k32, grid, ONESWEEP_BLOCK, smem, stream, keys_a, keys_b, vals_a, vals_b, (unsigned)n, coding, first_pass + p, first_pass, ctrl,
-                       reinterpret_cast<uint32_t*>(lb), hdr);
+                       reinterpret_cast<uint32_t*>(lb), rep);
     else
       e = launch_after(k64, grid, ONESWEEP_BLOCK, smem, stream, keys_a, keys_b, vals_a, vals_b, (unsigned)n, coding, first_pass + p, first_pass, ctrl,
-                       reinterpret_cast<unsigned long long*>(lb), hdr);
+                       reinterpret_cast<unsigned long long*>(lb), rep);
     if (e != cudaSuccess) return e;
     log_launch("onesweep_kernel", grid, ONESWEEP_BLOCK, smem, n, stream);
   }

@@ -36,7 +36,7 @@ __device__ __forceinline__ opt<AccT> block_reduce_opt(opt<AccT> x, Op op, opt<Ac
 template <class InIt, class AccT, class Op, int VEC>
 __global__ void __launch_bounds__(REDUCE_BLOCK)
 reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* partial_has,
-              unsigned* ticket, AccT* out) {
+              ws_header* hdr, AccT* out) {
   TB200_SHARED_ARRAY(opt<AccT>, smem, 32);
   __shared__ bool is_last;
   const size_t tid = (size_t)blockIdx.x * REDUCE_BLOCK + threadIdx.x;
@@ -87,12 +87,18 @@ reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* par
     for (; i < n; i += stride) acc.append((AccT)in[i], op);
   }
 
+  if (gridDim.x == 1) {   // nobody to wait for, and a header that nobody has cleared (`out` may lie behind its first fields)
+    if (threadIdx.x < sizeof(ws_header) / 4) reinterpret_cast<unsigned*>(hdr)[threadIdx.x] = 0;
+    const opt<AccT> all = block_reduce_opt(acc, op, smem);
+    if (threadIdx.x == 0) *out = all.has ? op(init, all.v) : init;
+    return;
+  }
   opt<AccT> blk = block_reduce_opt(acc, op, smem);
   if (threadIdx.x == 0) {
     if (blk.has) partials[blockIdx.x] = blk.v;
     partial_has[blockIdx.x] = blk.has;
     __threadfence();
-    unsigned t = atomicAdd(ticket, 1u);
+    unsigned t = atomicAdd(&hdr->ticket, 1u);
     is_last = (t == gridDim.x - 1);
   }
   __syncthreads();
@@ -106,12 +112,15 @@ reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* par
   f = block_reduce_opt(f, op, smem);
   if (threadIdx.x == 0) {
     *out = f.has ? op(init, f.v) : init;
-    *ticket = 0;
+    hdr->ticket = 0;
   }
 }
 
+// One CTA up to four loads per thread: without partials, ticket and the launch that clears them a call of 1000 int32 takes
+// (measured below) less, and a CTA has its four loads in flight together anyway.
 inline int reduce_grid(size_t work_items /* vectors or elements */) {
   const device_info& di = current_device_info();
+  if (work_items <= (size_t)REDUCE_BLOCK * REDUCE_UNROLL) return 1;
   size_t want = (work_items + REDUCE_BLOCK - 1) / REDUCE_BLOCK;
   size_t cap = (size_t)di.sm_count * REDUCE_CTAS_PER_SM;
   if (cap > REDUCE_MAX_GRID) cap = REDUCE_MAX_GRID;
@@ -132,8 +141,14 @@ cudaError_t reduce_async(InIt in, size_t n, AccT init, Op op, AccT* d_out, void*
   ws_header* hdr = reinterpret_cast<ws_header*>(base);
   AccT* partials = reinterpret_cast<AccT*>(base + sizeof(ws_header));
   unsigned* has = reinterpret_cast<unsigned*>(base + sizeof(ws_header) + align_up(REDUCE_MAX_GRID * sizeof(AccT), 256));
-  cudaError_t e = cudaMemsetAsync(hdr, 0, sizeof(ws_header), stream);
-  if (e != cudaSuccess) return e;
+  // a result inside the header is reported with it
+  ws_header* const rep = report_of(hdr);
+  char* const out_at = reinterpret_cast<char*>(d_out);
+  if (rep != hdr && out_at >= base && out_at < base + sizeof(ws_header)) {
+    d_out = reinterpret_cast<AccT*>(reinterpret_cast<char*>(rep) + (out_at - base));
+    reported(rep, hdr);
+  }
+  auto clear = [&](int grid) { return grid == 1 ? cudaSuccess : cudaMemsetAsync(hdr, 0, sizeof(ws_header), stream); };
   constexpr bool is_ptr = std::is_pointer<InIt>::value;
   if constexpr (is_ptr) {
     using In = typename std::remove_cv<typename std::remove_pointer<InIt>::type>::type;
@@ -142,16 +157,20 @@ cudaError_t reduce_async(InIt in, size_t n, AccT init, Op op, AccT* d_out, void*
       if (is_aligned16(in)) {
         constexpr int VEC = 16 / sizeof(In);
         int grid = reduce_grid(n / VEC);
+        const cudaError_t e = clear(grid);
+        if (e != cudaSuccess) return e;
         timed_launch tl(KID_REDUCE, stream);
-        reduce_kernel<InIt, AccT, Op, VEC><<<grid, REDUCE_BLOCK, 0, stream>>>(in, n, init, op, partials, has, &hdr->ticket, d_out);
+        reduce_kernel<InIt, AccT, Op, VEC><<<grid, REDUCE_BLOCK, 0, stream>>>(in, n, init, op, partials, has, hdr, d_out);
         log_launch("reduce_kernel (16-byte loads)", grid, REDUCE_BLOCK, 0, n, stream);
         return cudaGetLastError();
       }
     }
   }
   int grid = reduce_grid(n);
+  const cudaError_t e = clear(grid);
+  if (e != cudaSuccess) return e;
   timed_launch tl(KID_REDUCE, stream);
-  reduce_kernel<InIt, AccT, Op, 0><<<grid, REDUCE_BLOCK, 0, stream>>>(in, n, init, op, partials, has, &hdr->ticket, d_out);
+  reduce_kernel<InIt, AccT, Op, 0><<<grid, REDUCE_BLOCK, 0, stream>>>(in, n, init, op, partials, has, hdr, d_out);
   log_launch("reduce_kernel (generic iterator)", grid, REDUCE_BLOCK, 0, n, stream);
   return cudaGetLastError();
 }

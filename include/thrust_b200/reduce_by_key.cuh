@@ -45,7 +45,7 @@ template <class K, class V> struct rbk_tuning {
 template <class KeyIt, class ValIt, class KeyOutIt, class ValOutIt, class K, class V, class Eq, class Op, class Off, bool VEC_LOAD, int IPT>
 __global__ void __launch_bounds__(RBK_BLOCK)
 reduce_by_key_kernel(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOutIt vals_out, size_t n, Eq key_eq, Op op,
-                     tile_state<rbk_pair<Off, V>> ts, ws_header* hdr, unsigned long long* d_count) {
+                     tile_state<rbk_pair<Off, V>> ts, ws_header* hdr, ws_header* rep, unsigned long long* d_count) {
   using P = rbk_pair<Off, V>;
   using Comb = rbk_combine<Off, V, Op>;
   constexpr int NWARPS = RBK_BLOCK / 32;
@@ -116,7 +116,7 @@ reduce_by_key_kernel(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOutIt vals_ou
   P vec_total[1] = {summary};
   opt<P> pre[1];
   P none; none.count = 0; none.value = V();
-  tile_exclusive_prefix<P, Comb, 1, NWARPS>(vec_total, pre, tile, none, false, comb, ts, &hdr->error, sm);
+  tile_exclusive_prefix<P, Comb, 1, NWARPS>(vec_total, pre, tile, none, false, comb, ts, &rep->error, sm);
   const Off head_off = sm.has_prefix ? sm.prefix.count : (Off)0;   // run heads in all preceding tiles
   __syncthreads();                                                  // everyone has its items in registers: reuse the tile buffers
 
@@ -139,7 +139,7 @@ reduce_by_key_kernel(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOutIt vals_ou
         }
         if (g0 + j == n - 1) {
           vals_out[(size_t)run - 1] = acc;
-          hdr->count = (unsigned long long)run;
+          hdr->count = rep->count = (unsigned long long)run;
           if (d_count) *d_count = (unsigned long long)run;
         }
       }
@@ -229,8 +229,10 @@ cudaError_t reduce_by_key_async(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOu
     auto kern = reduce_by_key_kernel<KeyIt, ValIt, KeyOutIt, ValOutIt, K, V, Eq, Op, Off, VEC, IPT>;
     const size_t smem = (rbk_tile_items<K, V>() * sizeof(K) + 15) / 16 * 16 + rbk_tile_items<K, V>() * sizeof(V);
     if (smem > 48 * 1024 && (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return;
+    ws_header* const rep = report_of(hdr);
+    reported(rep, hdr);
     timed_launch tl(KID_REDUCE_BY_KEY, stream);
-    kern<<<(unsigned)tiles, RBK_BLOCK, smem, stream>>>(keys, vals, keys_out, vals_out, n, eq, op, ts, hdr, d_count);
+    kern<<<(unsigned)tiles, RBK_BLOCK, smem, stream>>>(keys, vals, keys_out, vals_out, n, eq, op, ts, hdr, rep, d_count);
   };
   constexpr bool ptrs = std::is_pointer<KeyIt>::value && std::is_pointer<ValIt>::value;
   bool use_vec = false;

@@ -97,7 +97,7 @@ template <class T, int N> __device__ __forceinline__ void lane_items(const T* p,
 template <class K, class V, class Eq, class Op>
 __global__ void __launch_bounds__(PIPE_BLOCK, 1)
 rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n, unsigned tiles, Eq eq, rbk_chain<V, Op> chain, ws_header* hdr,
-                unsigned long long* d_count) {
+                ws_header* rep, unsigned long long* d_count) {
   using Chain = rbk_chain<V, Op>;
   using C = typename Chain::C;
   using Shape = rbk_pipe_shape<K, V>;
@@ -121,7 +121,7 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
 
   if (warp == PIPE_LOADER) {
     const unsigned long long policy = l2_stream_policy();
-    pipe_loader(st, tiles, &hdr->error, [&](unsigned s, unsigned tile) {
+    pipe_loader(st, tiles, &rep->error, [&](unsigned s, unsigned tile) {
       unsigned char* const kstage = stages + s * Shape::STAGE_BYTES;
       unsigned char* const vstage = kstage + Shape::Keys::BYTES;
       const size_t base = (size_t)tile * ITEMS, left = n - base;
@@ -138,11 +138,11 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
       else if (lane < 2 * PIPE_WARPS) Shape::Vals::copy(vstage, vals + base, left, lane - PIPE_WARPS, &st.full[s], policy);
     });
   } else if (warp == PIPE_PUBLISHER) {
-    pipe_publisher<false>(st, chain, tiles, &hdr->error, [&](const rbk_part<V>& part) { return fold_parts(lane < PIPE_WARPS ? Chain::lift(part) : Chain::identity()); });
+    pipe_publisher<false>(st, chain, tiles, &rep->error, [&](const rbk_part<V>& part) { return fold_parts(lane < PIPE_WARPS ? Chain::lift(part) : Chain::identity()); });
   } else if (warp == PIPE_FOLDER) {
-    pipe_folder<false>(st, chain, tiles, Chain::identity(), &hdr->error, [&](const C& all) {
+    pipe_folder<false>(st, chain, tiles, Chain::identity(), &rep->error, [&](const C& all) {
       vals_out[all.heads - 1] = (V)all.value;   // the last run ends with the input
-      hdr->count = all.heads;
+      hdr->count = rep->count = all.heads;
       if (d_count) *d_count = all.heads;
     });
   } else {
@@ -191,7 +191,7 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
       for (int j = 1; j < VEC; ++j) t = (row_bits >> j) & 1 ? x[j] : op(t, x[j]);
       return t;
     };
-    pipe_compute<true>(st, tiles, &hdr->error,
+    pipe_compute<true>(st, tiles, &rep->error,
       [&](unsigned s, unsigned tile) {
         K k[ROWS][VEC]; V x[ROWS][VEC];
         // nobody compacts its part of this tile before every warp has been here
@@ -240,7 +240,7 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
         // same twice is reported and nothing is stored)
         const unsigned part_heads = __reduce_add_sync(FULL_MASK, (unsigned)__popc(bits));
         if (part_heads != st.part[s][mine].heads || run0 > (size_t)tile * ITEMS + (size_t)mine * PART) {
-          if (lane == 0) record_error(&hdr->error, ERR_INCONSISTENT);
+          if (lane == 0) record_error(&rep->error, ERR_INCONSISTENT);
           return;
         }
         const unsigned kshift = run_shift(keys_out + run0);
@@ -316,8 +316,10 @@ cudaError_t rbk_pipe_launch(const K* keys, const V* vals, K* keys_out, V* vals_o
   cudaError_t e = pipe_clear(base, sizeof(ws_header) + rbk_chain<V, Op>::bytes(tiles), stream);
   if (e != cudaSuccess) return e;
   timed_launch tl(KID_REDUCE_BY_KEY, stream);
-  e = pipe_launch(kern, grid, smem, stream, keys, vals, keys_out, vals_out, n, (unsigned)tiles, eq, chain, hdr, d_count);
+  ws_header* const rep = report_of(hdr);
+  e = pipe_launch(kern, grid, smem, stream, keys, vals, keys_out, vals_out, n, (unsigned)tiles, eq, chain, hdr, rep, d_count);
   if (launch_refused(e)) return cudaSuccess;
+  reported(rep, hdr);
   launched = true;
   log_launch("rbk_pipe_kernel", grid, PIPE_BLOCK, smem, n, stream);
   return e;

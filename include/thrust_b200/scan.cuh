@@ -30,7 +30,7 @@ template <class T> struct scan_tuning {
 
 template <class InIt, class OutIt, class T, class Op, bool INCLUSIVE, int VEC, int IPT>
 __global__ void __launch_bounds__(SCAN_BLOCK, 4)
-scan_kernel(InIt in, OutIt out, size_t n, T init, bool has_init, const T* init_ptr, Op op, tile_state<T> ts, ws_header* hdr) {
+scan_kernel(InIt in, OutIt out, size_t n, T init, bool has_init, const T* init_ptr, Op op, tile_state<T> ts, ws_header* hdr, ws_header* rep) {
   if (init_ptr) { init = *init_ptr; has_init = true; }   // an initial value that lives on the device (the carry of a sharded scan)
   constexpr int VPT = IPT / VEC;
   constexpr int NWARPS = SCAN_BLOCK / 32;
@@ -86,7 +86,7 @@ scan_kernel(InIt in, OutIt out, size_t n, T init, bool has_init, const T* init_p
     vec_total[v] = x[v][VEC - 1];
   }
   opt<T> pre[VPT];   // everything before vector v of this lane, across tiles, including init
-  tile_exclusive_prefix<T, Op, VPT, NWARPS>(vec_total, pre, tile, init, has_init, op, ts, &hdr->error, sm);
+  tile_exclusive_prefix<T, Op, VPT, NWARPS>(vec_total, pre, tile, init, has_init, op, ts, &rep->error, sm);
 
   // ---- apply and store
 #pragma unroll
@@ -450,6 +450,8 @@ cudaError_t scan_async(InIt in, OutIt out, size_t n, T init, bool has_init, Op o
 #ifdef TB200_TEST_HOOKS
   if (test_hook_flags() & 1u) { if ((e = cudaMemsetAsync(&hdr->flags, 1, 1, stream)) != cudaSuccess) return e; }
 #endif
+  ws_header* const rep = report_of(hdr);
+  reported(rep, hdr);
   timed_launch tl(KID_SCAN, stream);
   if constexpr (ptrs) {
     using In = typename std::remove_cv<typename std::remove_pointer<InIt>::type>::type;
@@ -459,13 +461,13 @@ cudaError_t scan_async(InIt in, OutIt out, size_t n, T init, bool has_init, Op o
     if constexpr (vec_ok) {
       if (vectors) {
         constexpr int VEC = 16 / sizeof(T);
-        scan_kernel<InIt, OutIt, T, Op, INCLUSIVE, VEC, IPT><<<(unsigned)tiles, SCAN_BLOCK, 0, stream>>>(in, out, n, init, has_init, d_init, op, ts, hdr);
+        scan_kernel<InIt, OutIt, T, Op, INCLUSIVE, VEC, IPT><<<(unsigned)tiles, SCAN_BLOCK, 0, stream>>>(in, out, n, init, has_init, d_init, op, ts, hdr, rep);
         log_launch("scan_kernel (16-byte loads)", tiles, SCAN_BLOCK, 0, n, stream);
         return cudaGetLastError();
       }
     }
   }
-  scan_kernel<InIt, OutIt, T, Op, INCLUSIVE, 1, IPT><<<(unsigned)tiles, SCAN_BLOCK, 0, stream>>>(in, out, n, init, has_init, d_init, op, ts, hdr);
+  scan_kernel<InIt, OutIt, T, Op, INCLUSIVE, 1, IPT><<<(unsigned)tiles, SCAN_BLOCK, 0, stream>>>(in, out, n, init, has_init, d_init, op, ts, hdr, rep);
   log_launch("scan_kernel (generic iterator)", tiles, SCAN_BLOCK, 0, n, stream);
   return cudaGetLastError();
 }

@@ -11,7 +11,7 @@ namespace tb200 {
 
 template <class T, class Op, bool INCLUSIVE>
 __global__ void __launch_bounds__(PIPE_BLOCK, 1)
-scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has_init, const T* init_ptr, tile_chain<T, Op> chain, ws_header* hdr) {
+scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has_init, const T* init_ptr, tile_chain<T, Op> chain, ws_header* rep) {
   using Chain = tile_chain<T, Op>;
   using C = typename Chain::C;
   constexpr int VEC = 16 / sizeof(T);
@@ -26,7 +26,7 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
 
   if (warp == PIPE_LOADER) {
     const unsigned long long policy = l2_stream_policy();
-    pipe_loader(st, tiles, &hdr->error, [&](unsigned s, unsigned tile) {
+    pipe_loader(st, tiles, &rep->error, [&](unsigned s, unsigned tile) {
       T* dst = reinterpret_cast<T*>(stages + (size_t)s * PIPE_TILE_BYTES);
       const size_t base = (size_t)tile * ITEMS;
       const unsigned bytes = pipe_tail_fill<T, ITEMS>(dst, in + base, n - base, ID);
@@ -36,7 +36,7 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
       }
     });
   } else if (warp == PIPE_PUBLISHER) {
-    pipe_publisher<false>(st, chain, tiles, &hdr->error, [&](const T& part) {
+    pipe_publisher<false>(st, chain, tiles, &rep->error, [&](const T& part) {
       C t = lane < PIPE_WARPS ? Chain::lift(part) : Chain::identity();
 #pragma unroll
       for (int d = 1; d < PIPE_WARPS; d <<= 1) t = Chain::join(t, shfl_down(t, d));   // lane 0: all parts, in order
@@ -45,7 +45,7 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
   } else if (warp == PIPE_FOLDER) {
     C first = Chain::identity();
     if (init_ptr) first = Chain::lift(no_nan<Op>(*init_ptr)); else if (has_init) first = Chain::lift(no_nan<Op>(init));
-    pipe_folder<false>(st, chain, tiles, first, &hdr->error, [](const C&) {});
+    pipe_folder<false>(st, chain, tiles, first, &rep->error, [](const C&) {});
   } else {
     const int mine = warp % PIPE_WARPS;
     // what a loop would start from: if that is a NaN, so is every result (in place in[0] is stored unchanged)
@@ -53,7 +53,7 @@ scan_pipe_kernel(const T* in, T* out, size_t n, unsigned tiles, T init, bool has
     if constexpr (drops_nans<Op, T>::value) first = init_ptr ? *init_ptr : has_init ? init : in[0];
     const bool stuck = first != first;
     auto rows_of = [&](unsigned s) { return reinterpret_cast<const vec16*>(stages + (size_t)s * PIPE_TILE_BYTES) + mine * (PIPE_ROWS * 32) + lane; };
-    pipe_compute<false>(st, tiles, &hdr->error,
+    pipe_compute<false>(st, tiles, &rep->error,
       [&](unsigned s, unsigned) {
         const vec16* src = rows_of(s);
         T acc[PIPE_ROWS];
@@ -165,8 +165,10 @@ cudaError_t scan_pipe_launch(const T* in, T* out, size_t n, T init, bool has_ini
   cudaError_t e = pipe_clear(base, sizeof(ws_header) + tile_chain<T, Op>::bytes(tiles), stream);
   if (e != cudaSuccess) return e;
   timed_launch tl(KID_SCAN, stream);
-  e = pipe_launch(kern, grid, smem, stream, in, out, n, (unsigned)tiles, init, has_init, d_init, chain, hdr);
+  ws_header* const rep = report_of(hdr);
+  e = pipe_launch(kern, grid, smem, stream, in, out, n, (unsigned)tiles, init, has_init, d_init, chain, rep);
   if (launch_refused(e)) return cudaSuccess;
+  reported(rep, hdr);
   launched = true;
   log_launch("scan_pipe_kernel", grid, PIPE_BLOCK, smem, n, stream);
   return e;

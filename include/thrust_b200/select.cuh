@@ -40,7 +40,7 @@ template <class T> struct select_tuning {
 template <int MODE, bool KEEP_REJECTS, class InIt, class StIt, class SelIt, class RejIt, class T, class Pred, class Off, int VEC, int IPT>
 __global__ void __launch_bounds__(SELECT_BLOCK, 4)
 select_kernel(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, size_t n, Pred pred, tile_state<Off> ts, ws_header* hdr,
-              unsigned long long* d_count, bool mirrored) {
+              ws_header* rep, unsigned long long* d_count, bool mirrored) {
   constexpr int VPT = IPT / VEC;
   constexpr int NWARPS = SELECT_BLOCK / 32;
   constexpr int WCHUNK = 32 * IPT;
@@ -120,7 +120,7 @@ select_kernel(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, size_t n, Pre
 
   // ---- number of kept items before each vector, across tiles
   opt<Off> pre[VPT];
-  tile_exclusive_prefix<Off, plus_op, VPT, NWARPS>(vec_total, pre, tile, (Off)0, true, plus_op(), ts, &hdr->error, sm);
+  tile_exclusive_prefix<Off, plus_op, VPT, NWARPS>(vec_total, pre, tile, (Off)0, true, plus_op(), ts, &rep->error, sm);
   const Off sel_off = sm.prefix;                       // kept items in all preceding tiles
   const unsigned tile_nsel = (unsigned)(sm.inclusive - sm.prefix);
 
@@ -147,7 +147,7 @@ select_kernel(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, size_t n, Pre
     }
   }
   if (threadIdx.x == 0 && tile_base + TILE >= n) {
-    hdr->count = (unsigned long long)sm.inclusive;
+    hdr->count = rep->count = (unsigned long long)sm.inclusive;
     if (d_count) *d_count = (unsigned long long)sm.inclusive;
   }
 }
@@ -229,9 +229,11 @@ cudaError_t select_async(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, si
     constexpr int VEC = decltype(vec_tag)::value;
     tile_state<Off> ts;
     ts.bind(base + sizeof(ws_header), tiles + 1);
+    ws_header* const rep = report_of(hdr);
+    reported(rep, hdr);
     timed_launch tl(KID_SELECT, stream);
     select_kernel<MODE, KEEP_REJECTS, InIt, StIt, SelIt, RejIt, T, Pred, Off, VEC, IPT>
-        <<<(unsigned)tiles, SELECT_BLOCK, 0, stream>>>(in, stencil, out_sel, out_rej, n, pred, ts, hdr, d_count, mirrored);
+        <<<(unsigned)tiles, SELECT_BLOCK, 0, stream>>>(in, stencil, out_sel, out_rej, n, pred, ts, hdr, rep, d_count, mirrored);
   };
   constexpr bool vec_ok = std::is_pointer<InIt>::value && std::is_arithmetic<T>::value && (sizeof(T) == 4 || sizeof(T) == 8) && MODE != SEL_STENCIL;
   bool use_vec = false;

@@ -31,7 +31,7 @@ template <class T> using select_parts = pipe_parts<T, PIPE_ROWS * 512 / (int)siz
 template <bool UNIQUE, int REJ, bool IN_PLACE, class T, class Pred>
 __global__ void __launch_bounds__(PIPE_BLOCK, 1)
 select_pipe_kernel(const T* in, T* out_sel, T* out_rej, size_t n, unsigned tiles, Pred pred, tile_chain<unsigned long long, plus_op> chain, ws_header* hdr,
-                   unsigned long long* d_count) {
+                   ws_header* rep, unsigned long long* d_count) {
   using C = unsigned long long;
   constexpr int VEC = 16 / sizeof(T);
   constexpr int ITEMS = PIPE_TILE_BYTES / sizeof(T);
@@ -47,7 +47,7 @@ select_pipe_kernel(const T* in, T* out_sel, T* out_rej, size_t n, unsigned tiles
 
   if (warp == PIPE_LOADER) {
     const unsigned long long policy = l2_stream_policy();
-    pipe_loader(st, tiles, &hdr->error, [&](unsigned s, unsigned tile) {
+    pipe_loader(st, tiles, &rep->error, [&](unsigned s, unsigned tile) {
       unsigned char* const stage = stages + (size_t)s * Parts::BYTES;
       const size_t base = (size_t)tile * ITEMS;
       Parts::ragged(stage, in + base, n - base);
@@ -61,9 +61,9 @@ select_pipe_kernel(const T* in, T* out_sel, T* out_rej, size_t n, unsigned tiles
       if (lane < PIPE_WARPS) Parts::copy(stage, in + base, n - base, lane, &st.full[s], policy);
     });
   } else if (warp == PIPE_PUBLISHER) {
-    pipe_publisher<IN_PLACE>(st, chain, tiles, &hdr->error, [&](unsigned part) { return (C)__reduce_add_sync(FULL_MASK, lane < PIPE_WARPS ? part : 0u); });
+    pipe_publisher<IN_PLACE>(st, chain, tiles, &rep->error, [&](unsigned part) { return (C)__reduce_add_sync(FULL_MASK, lane < PIPE_WARPS ? part : 0u); });
   } else if (warp == PIPE_FOLDER) {
-    pipe_folder<IN_PLACE>(st, chain, tiles, (C)0, &hdr->error, [&](C total) { hdr->count = total; if (d_count) *d_count = total; });
+    pipe_folder<IN_PLACE>(st, chain, tiles, (C)0, &rep->error, [&](C total) { hdr->count = rep->count = total; if (d_count) *d_count = total; });
   } else {
     const int mine = warp % PIPE_WARPS;
     // UNIQUE: the item in front of the stage's tile, for its first warp.  Nothing lies in front of the input: its first item is
@@ -110,7 +110,7 @@ select_pipe_kernel(const T* in, T* out_sel, T* out_rej, size_t n, unsigned tiles
       if (UNIQUE && first == 0 && lane == 0) bits |= 1u;   // the input's first item is kept
       return bits;
     };
-    pipe_compute<true>(st, tiles, &hdr->error,
+    pipe_compute<true>(st, tiles, &rep->error,
       [&](unsigned s, unsigned tile) {
         T x[PIPE_ROWS][VEC];
         T edge = T();
@@ -151,7 +151,7 @@ select_pipe_kernel(const T* in, T* out_sel, T* out_rej, size_t n, unsigned tiles
         // what is stored now is what was counted then, and lies inside the output: a predicate that does not answer the same
         // twice (or a broken carry) is reported and nothing is stored
         if (row_off != st.part[s][mine] || kept0 > first || row_off > part_n) {
-          if (lane == 0) record_error(&hdr->error, ERR_INCONSISTENT);
+          if (lane == 0) record_error(&rep->error, ERR_INCONSISTENT);
           return;
         }
         T* const dst = out_sel + kept0;
@@ -252,8 +252,10 @@ cudaError_t select_pipe_launch(const T* in, T* out_sel, T* out_rej, size_t n, Pr
   cudaError_t e = pipe_clear(base, sizeof(ws_header) + tile_chain<unsigned long long, plus_op>::bytes(tiles), stream);
   if (e != cudaSuccess) return e;
   timed_launch tl(KID_SELECT, stream);
-  e = pipe_launch(kern, grid, smem, stream, in, out_sel, out_rej, n, (unsigned)tiles, pred, chain, hdr, d_count);
+  ws_header* const rep = report_of(hdr);
+  e = pipe_launch(kern, grid, smem, stream, in, out_sel, out_rej, n, (unsigned)tiles, pred, chain, hdr, rep, d_count);
   if (launch_refused(e)) return cudaSuccess;
+  reported(rep, hdr);
   launched = true;
   log_launch("select_pipe_kernel", grid, PIPE_BLOCK, smem, n, stream);
   return e;

@@ -18,6 +18,7 @@ PROTOTYPES = {
     "tb200_sm_arch": [],
     "tb200_workspace_status": [_vp, _vp, C.POINTER(C.c_uint)],
     "tb200_workspace_read": [_vp, _sz, _vp, _vp],
+    "tb200_workspace_watch": [_vp],
     "tb200_reduce": [_vp, _sz, _i, _i, _i, _vp, _vp, _vp, _szp, _vp],
     "tb200_inclusive_scan": [_vp, _vp, _sz, _i, _i, _vp, _vp, _szp, _vp],
     "tb200_exclusive_scan": [_vp, _vp, _sz, _i, _i, _vp, _vp, _szp, _vp],

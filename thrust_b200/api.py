@@ -57,18 +57,26 @@ def _require_cuda(*tensors):
             raise ValueError("thrust_b200 operates on contiguous CUDA tensors")
 
 
+# the workspace header (ws_header in common.cuh): status, ticket, count, ..., and from byte 32 on room that a result may use
+_HEADER = struct.Struct("<IIQ")
+_HEADER_RESULT, _HEADER_BYTES = 32, 256
+
+
 class _Kept:
-    """One kept buffer: the tensor, its address and size as the C ABI takes them, and its lock (re-entrant)."""
-    __slots__ = ("lock", "buf", "ptr", "size")
+    """One kept buffer: the tensor, its address and size as the C ABI takes them, its lock (re-entrant), and where its
+    header is read to."""
+    __slots__ = ("lock", "buf", "ptr", "size", "size_ref", "head")
 
     def __init__(self):
         self.lock = threading.RLock()
+        self.head = C.create_string_buffer(_HEADER_BYTES)
         self.keep(None)
 
     def keep(self, buf):
         self.buf = buf
         self.ptr = None if buf is None else buf.data_ptr()
         self.size = C.c_size_t(0 if buf is None else buf.numel())
+        self.size_ref = C.byref(self.size)
 
 
 class _Workspaces:
@@ -118,7 +126,7 @@ def _enqueue(key, kept, fn, args, result=None):
     rc = None
     if kept.ptr is not None:
         out = () if result is None else (kept.ptr + result,)
-        rc = lib_fn(*args, *out, kept.ptr, C.byref(kept.size), stream)
+        rc = lib_fn(*args, *out, kept.ptr, kept.size_ref, stream)
         if rc != _TOO_SMALL:
             return _check(rc, fn)
     need = C.c_size_t(0)
@@ -128,7 +136,36 @@ def _enqueue(key, kept, fn, args, result=None):
         _check(rc, fn)
     workspaces.get(key[2], need.value, key)
     out = () if result is None else (kept.ptr + result,)
-    _check(lib_fn(*args, *out, kept.ptr, C.byref(kept.size), stream), fn)
+    _check(lib_fn(*args, *out, kept.ptr, kept.size_ref, stream), fn)
+
+
+def _enqueue_and_read(key, kept, what, fn, args, nbytes=_HEADER.size, result=None):
+    """_enqueue, then the first `nbytes` of the header to kept.head once the stream has got there; returns the count.  The
+    read is announced, so that the kernels can leave there what it fetches."""
+    lib = _lib.load()
+    watch = getattr(lib, "tb200_workspace_watch", None)
+    if watch is None or kept.ptr is None:      # the first call makes the workspace
+        _enqueue(key, kept, fn, args, result)
+    else:
+        watch(kept.ptr)
+        try:
+            _enqueue(key, kept, fn, args, result)
+        except BaseException:
+            watch(None)
+            raise
+    return _read_header(lib, kept.ptr, what, key[1], kept.head, nbytes)
+
+
+def _read_header(lib, ptr, what, stream, head, nbytes):
+    """Waits for the stream and reads the first `nbytes` of the workspace's header to `head`; returns the count and raises if
+    the kernels reported a wait that ran out or looks at a tile that disagree."""
+    rc = lib.tb200_workspace_read(ptr, nbytes, head, stream)
+    if rc != 0:
+        _check(rc, what + " (result)")
+    status, _, count = _HEADER.unpack_from(head)
+    if status != 0:
+        raise Tb200Error("%s: device reported status %d (%s)" % (what, status, "an inter-CTA wait ran out" if status == 1 else "two looks at a tile disagree"))
+    return count
 
 
 def _call_with_ws(tag, fn, *args):
@@ -146,28 +183,11 @@ def _call_and_wait(tag, what, fn, *args, sync=True, key=None):
     key = key or workspaces.key(tag)
     kept = workspaces.at(key)
     with kept.lock:
-        _enqueue(key, kept, fn, args)
-        return _HEADER.unpack_from(_read_header(kept.ptr, what, key[1]))[2] if sync else None
-
-
-# the workspace header (ws_header in common.cuh): status, ticket, count, ..., and room that a result may use
-_HEADER = struct.Struct("<IIQ")
-_HEADER_RESULT = 32
-
-
-def _read_header(ptr, what, stream, nbytes=_HEADER.size):
-    """Waits for the stream, then the first `nbytes` of the workspace's header in one copy; raises if the
-    kernels reported a wait that ran out or looks at a tile that disagree."""
-    head = C.create_string_buffer(nbytes)
-    _check(_lib.load().tb200_workspace_read(ptr, nbytes, head, stream), what + " (result)")
-    status = _HEADER.unpack_from(head)[0]
-    if status != 0:
-        raise Tb200Error("%s: device reported status %d (%s)" % (what, status, "an inter-CTA wait ran out" if status == 1 else "two looks at a tile disagree"))
-    return head
+        return _enqueue_and_read(key, kept, what, fn, args) if sync else _enqueue(key, kept, fn, args)
 
 
 def _sync_and_check(ws, what):
-    _read_header(ws.data_ptr(), what, _stream())
+    _read_header(_lib.load(), ws.data_ptr(), what, _stream(), C.create_string_buffer(_HEADER.size), _HEADER.size)
 
 
 # ------------------------------------------------------------------------------------- reduce
@@ -180,12 +200,11 @@ def reduce(x, init=None, op="plus", acc_dtype=None):
     h_init = np.asarray(0 if init is None else init, dtype=NP_OF[acc_dtype])
     # the result lands in the workspace's header and comes back together with the status
     key = workspaces.key("reduce")
-    args = (_ptr(x), x.numel(), DTYPE_CODE[x.dtype], DTYPE_CODE[acc_dtype], OPS[op], h_init.ctypes.data)
+    args = (_ptr(x), x.numel(), DTYPE_CODE[x.dtype], DTYPE_CODE[acc_dtype], OPS[op], h_init.tobytes())
     kept = workspaces.at(key)
     with kept.lock:
-        _enqueue(key, kept, "tb200_reduce", args, _HEADER_RESULT)
-        head = _read_header(kept.ptr, "reduce", key[1], _HEADER_RESULT + 8)
-    return np.frombuffer(head.raw, dtype=NP_OF[acc_dtype], count=1, offset=_HEADER_RESULT)[0]
+        _enqueue_and_read(key, kept, "reduce", "tb200_reduce", args, _HEADER_RESULT + 8, _HEADER_RESULT)
+        return np.frombuffer(kept.head, dtype=h_init.dtype, count=1, offset=_HEADER_RESULT)[0]
 
 
 def reduce_to_device(x, init, op="plus", acc_dtype=None, out=None):
@@ -196,7 +215,7 @@ def reduce_to_device(x, init, op="plus", acc_dtype=None, out=None):
     h_init = np.asarray(init, dtype=NP_OF[acc_dtype])
     out = torch.empty(1, dtype=acc_dtype, device=x.device) if out is None else out
     _call_with_ws("reduce", "tb200_reduce", _ptr(x), x.numel(), DTYPE_CODE[x.dtype], DTYPE_CODE[acc_dtype], OPS[op],
-                  h_init.ctypes.data, _ptr(out))
+                  h_init.tobytes(), _ptr(out))
     return out
 
 
@@ -213,7 +232,7 @@ def inclusive_scan(x, out=None, op="plus", init=None, sync=True):
     else:
         h_init = None if init is None else np.asarray(init, dtype=NP_OF[x.dtype])
         _call_and_wait("scan", "inclusive_scan", "tb200_inclusive_scan", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], OPS[op],
-                       None if h_init is None else h_init.ctypes.data, sync=sync)
+                       None if h_init is None else h_init.tobytes(), sync=sync)
     return out
 
 
@@ -227,7 +246,7 @@ def exclusive_scan(x, init=0, out=None, op="plus", sync=True):
     else:
         h_init = np.asarray(init, dtype=NP_OF[x.dtype])
         _call_and_wait("scan", "exclusive_scan", "tb200_exclusive_scan", _ptr(x), _ptr(out), x.numel(), DTYPE_CODE[x.dtype], OPS[op],
-                       h_init.ctypes.data, sync=sync)
+                       h_init.tobytes(), sync=sync)
     return out
 
 
@@ -385,7 +404,7 @@ def exclusive_scan_by_key(keys, vals, init=0, out=None, op="plus"):
     out = torch.empty_like(vals) if out is None else out
     h_init = np.asarray(init, dtype=NP_OF[vals.dtype])
     _call_and_wait("rbk", "exclusive_scan_by_key", "tb200_scan_by_key", _ptr(keys), _ptr(vals), _ptr(out), keys.numel(), DTYPE_CODE[keys.dtype],
-                   DTYPE_CODE[vals.dtype], OPS[op], 1, h_init.ctypes.data)
+                   DTYPE_CODE[vals.dtype], OPS[op], 1, h_init.tobytes())
     return out
 
 

@@ -1,6 +1,7 @@
-// C ABI: tb200_reduce, tb200_version, tb200_sm_arch, tb200_workspace_status, tb200_workspace_read.
+// C ABI: tb200_reduce, tb200_version, tb200_sm_arch, tb200_workspace_status, tb200_workspace_watch, tb200_workspace_read.
 #include "abi_common.cuh"
 #include "thrust_b200/reduce.cuh"
+#include <vector>
 
 using namespace tb200_abi;
 
@@ -16,22 +17,53 @@ TB200_API int tb200_workspace_status(const void* d_ws, tb200_stream_t stream, un
 
 namespace {
 
-// One pinned header's worth per host thread: a read-back into pageable memory is staged by the driver first.
+// One pinned header's worth per host thread, which kernels can write to (host_report) and copies can land in: a read-back into
+// pageable memory is staged by the driver first.  give_up(): the block of a call that failed half-way may still be written to by what it
+// did launch; it is not used again and freed with the thread.
 struct pinned_header {
-  void* p = nullptr;
-  void* get() { if (!p && cudaHostAlloc(&p, sizeof(tb200::ws_header), cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); p = nullptr; } return p; }
-  ~pinned_header() { if (p) cudaFreeHost(p); }
+  tb200::ws_header* p = nullptr;
+  std::vector<void*> old;
+  tb200::ws_header* get() {
+    void* q = nullptr;
+    if (!p && cudaHostAlloc(&q, sizeof(tb200::ws_header), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) p = static_cast<tb200::ws_header*>(q);
+    else if (!p) cudaGetLastError();
+    return p;
+  }
+  void give_up() { old.push_back(p); p = nullptr; }
+  ~pinned_header() { if (p) cudaFreeHost(p); for (void* q : old) cudaFreeHost(q); }
 };
+thread_local pinned_header pinned;
 
 }  // namespace
 
+TB200_API int tb200_workspace_watch(const void* d_ws) {
+  tb200::host_report& r = tb200::thread_report();
+  if (r.served) pinned.give_up();            // watched and launched, but never read
+  r = tb200::host_report();
+  if (!d_ws) return 0;
+  tb200::ws_header* const block = pinned.get();
+  void* mapped = nullptr;
+  // (where the device sees the block at another address than the host, calls report through their workspaces)
+  if (!block || cudaHostGetDevicePointer(&mapped, block, 0) != cudaSuccess || mapped != block) { cudaGetLastError(); return 0; }
+  memset(block, 0, sizeof(*block));
+#ifdef TB200_TEST_HOOKS
+  block->flags = tb200::test_hook_flags() & 3u;
+#endif
+  r.ws = d_ws;
+  r.block = block;
+  return 0;
+}
+
 TB200_API int tb200_workspace_read(const void* d_ws, size_t bytes, void* h_dst, tb200_stream_t stream) {
   if (!d_ws || !h_dst || bytes > sizeof(tb200::ws_header)) return ERR_INVALID;
-  static thread_local pinned_header pinned;
+  tb200::host_report& r = tb200::thread_report();
+  const bool there = r.served && r.ws == d_ws;   // the watched call's kernels write what is asked for to the block
   void* const via = pinned.get();
-  cudaError_t e = cudaMemcpyAsync(via ? via : h_dst, d_ws, bytes, cudaMemcpyDeviceToHost, stream);
+  cudaError_t e = there ? cudaSuccess : cudaMemcpyAsync(via ? via : h_dst, d_ws, bytes, cudaMemcpyDeviceToHost, stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
   if (e == cudaSuccess && via) memcpy(h_dst, via, bytes);
+  if (e != cudaSuccess && r.served) pinned.give_up();
+  r = tb200::host_report();
   return (int)e;
 }
 
