@@ -6,7 +6,6 @@ namespace tb200 {
 
 constexpr unsigned MBAR_SPIN_LIMIT = SPIN_LIMIT >> 3;   // polls of an mbarrier; each may suspend for about a microsecond
 
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
 }

@@ -19,45 +19,15 @@
 // Measured on B200, microseconds here / on the general route, at 1 k, 32 k and 64 k items: u32 + u32 17 / 51, 27 / 53, 35 / 54;
 // f32 keys 16 / 53, 23 / 55, 33 / 57; u64 + u64 31 / 66, 54 / 83, 80 / 85.  csort_max_items says where it stops.
 #pragma once
-#include "bulk_copy.cuh"
+#include "cluster.cuh"
 #include "common.cuh"
 #include "radix_keys.cuh"
 
 namespace tb200 {
 
 constexpr int CSORT_BLOCK = 512;
-constexpr int CSORT_MAX_CTAS = 16;
+constexpr int CSORT_MAX_CTAS = CLUSTER_MAX_CTAS;
 constexpr int CSORT_MAX_IPT = 16;
-
-__device__ __forceinline__ unsigned cluster_rank() { unsigned r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ unsigned cluster_size() { unsigned r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ unsigned cluster_addr(unsigned local, unsigned cta) {
-  unsigned a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(cta));
-  return a;
-}
-template <class T> __device__ __forceinline__ void cluster_store(unsigned addr, const T& v) {
-  if constexpr (sizeof(T) == 16) {
-    unsigned long long w[2];
-    memcpy(w, &v, 16);
-    asm volatile("st.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(addr), "l"(w[0]), "l"(w[1]) : "memory");
-  } else if constexpr (sizeof(T) == 8) {
-    unsigned long long w;
-    memcpy(&w, &v, 8);
-    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(w) : "memory");
-  } else if constexpr (sizeof(T) == 4) {
-    unsigned w;
-    memcpy(&w, &v, 4);
-    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(w) : "memory");
-  } else if constexpr (sizeof(T) == 2) {
-    asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(addr), "h"((unsigned short)v) : "memory");
-  } else {
-    asm volatile("st.shared::cluster.u8 [%0], %1;" ::"r"(addr), "r"((unsigned)v) : "memory");
-  }
-}
 
 // What moves between the CTAs: a key alone, or a key and its value in one 8- or 16-byte word.
 template <class UK, class UV, bool HAS_V> struct csort_item { using type = UK; };
@@ -209,43 +179,11 @@ cudaError_t cluster_sort_launch(UK* keys, UV* vals, size_t n, key_coding coding,
   while (ctas * (size_t)CSORT_BLOCK * IPT < n) ctas <<= 1;
   if (ctas > (unsigned)CSORT_MAX_CTAS) return cudaSuccess;
   const unsigned rows = (unsigned)((n + (size_t)ctas * CSORT_BLOCK - 1) / ((size_t)ctas * CSORT_BLOCK));   // the items spread evenly
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(CSORT_BLOCK);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = ctas; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  // largest cluster that fits, looked up once per thread, device and kernel (0: not yet)
   static thread_local unsigned largest[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || smem > (size_t)current_device_info().max_smem_optin) return cudaSuccess;
-  if (largest[dev] == 0) {
-    unsigned most = 1;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) { cudaGetLastError(); return cudaSuccess; }
-    for (unsigned c = CSORT_MAX_CTAS; c > 1; c >>= 1) {
-      cudaLaunchConfig_t probe = cfg;
-      cudaLaunchAttribute pa[1];
-      pa[0].id = cudaLaunchAttributeClusterDimension;
-      pa[0].val.clusterDim.x = c; pa[0].val.clusterDim.y = 1; pa[0].val.clusterDim.z = 1;
-      probe.gridDim = dim3(c);
-      probe.attrs = pa;
-      int clusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&clusters, kern, &probe) == cudaSuccess && clusters > 0) { most = c; break; }
-      cudaGetLastError();
-    }
-    largest[dev] = most;
-  }
-  if (ctas > largest[dev]) return cudaSuccess;
   timed_launch tl(KID_ONESWEEP, stream);
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, keys, vals, (unsigned)n, rows, coding, first_pass, num_passes, hdr);
-  if (launch_refused(e)) return cudaSuccess;
+  const cudaError_t e = cluster_launch(kern, ctas, CSORT_BLOCK, smem, stream, largest, launched, keys, vals, (unsigned)n, rows, coding, first_pass, num_passes, hdr);
+  if (!launched) return e;
   reported(report_of(hdr), hdr);   // nothing to report: no wait of this kernel runs out
-  launched = true;
   log_launch("cluster_sort_kernel", ctas, CSORT_BLOCK, smem, n, stream);
   return e;
 }

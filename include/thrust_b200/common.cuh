@@ -85,6 +85,10 @@ inline void reported(const ws_header* rep, const ws_header* hdr) { if (rep != hd
 // single-pass scan and of the pipelines does not publish; 1: a merge tile waits for bytes that nobody sends), bit 2 asks for
 // more CTAs than the pipelines' cooperative launch can place.
 inline unsigned& test_hook_flags() { static unsigned f = 0; return f; }
+// with bit 0 a tile's total is withheld in global memory: inputs of a few tiles then take the kernels that look there, not a cluster
+inline bool tiles_stay_apart() { return (test_hook_flags() & 1u) != 0; }
+#else
+inline bool tiles_stay_apart() { return false; }
 #endif
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -278,6 +282,47 @@ template <class T> struct opt {
   template <class Op> __device__ __forceinline__ void prepend(const opt<T>& left, Op op) {  // this = left (+) this
     if (left.has) { v = has ? op(left.v, v) : left.v; has = true; }
   }
+};
+
+// ---------------------------------------------------------------- thread-block clusters (launched by cluster.cuh)
+constexpr int CLUSTER_MAX_CTAS = 16;
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned cluster_rank() { unsigned r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ unsigned cluster_size() { unsigned r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned cluster_addr(unsigned local, unsigned cta) {
+  unsigned a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(cta));
+  return a;
+}
+template <class T> __device__ __forceinline__ void cluster_store(unsigned addr, const T& v) {
+  if constexpr (sizeof(T) == 16) {
+    unsigned long long w[2];
+    memcpy(w, &v, 16);
+    asm volatile("st.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(addr), "l"(w[0]), "l"(w[1]) : "memory");
+  } else if constexpr (sizeof(T) == 8) {
+    unsigned long long w;
+    memcpy(&w, &v, 8);
+    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(w) : "memory");
+  } else if constexpr (sizeof(T) == 4) {
+    unsigned w;
+    memcpy(&w, &v, 4);
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(w) : "memory");
+  } else if constexpr (sizeof(T) == 2) {
+    asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(addr), "h"((unsigned short)v) : "memory");
+  } else {
+    asm volatile("st.shared::cluster.u8 [%0], %1;" ::"r"(addr), "r"((unsigned)v) : "memory");
+  }
+}
+// A CTA may store into another one's shared memory once that has started: every thread arrives at the kernel's start and
+// waits before the first such store.
+__device__ __forceinline__ void cluster_arrive_started() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_started() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+// what may travel that way in one store
+template <class T> struct cluster_storable {
+  static constexpr bool value = std::is_trivially_copyable<T>::value && (sizeof(T) == 4 || sizeof(T) == 8 || sizeof(T) == 16);
 };
 
 // ---------------------------------------------------------------- shuffles of any small POD
@@ -557,12 +602,13 @@ template <class T, int NWARPS> struct tile_prefix_smem {
   T prefix;          // combination of all preceding tiles (and init)
   T inclusive;       // prefix (+) this tile's aggregate
   bool has_prefix;
+  alignas(16) unsigned char cluster_total[cluster_storable<T>::value ? CLUSTER_MAX_CTAS * sizeof(T) : 1];   // the tiles' totals, where the grid is one cluster
 };
 
 template <class T, class Op, int VPT, int NWARPS, class State>
 __device__ __forceinline__ void tile_exclusive_prefix(const T (&vec_total)[VPT], opt<T> (&pre)[VPT], size_t tile, const T& init,
                                                       bool has_init, Op op, const State& ts, unsigned* err,
-                                                      tile_prefix_smem<T, NWARPS>& sm) {
+                                                      tile_prefix_smem<T, NWARPS>& sm, bool one_cluster = false) {
   const int lane = lane_id(), warp = threadIdx.x >> 5;
   T rowacc = vec_total[0];
 #pragma unroll
@@ -579,7 +625,25 @@ __device__ __forceinline__ void tile_exclusive_prefix(const T (&vec_total)[VPT],
   __syncthreads();
   opt<T> wp; wp.has = false;
   for (int w = 0; w < warp; ++w) wp.append(sm.warp_total[w], op);
-  if (warp == 0) {
+  if constexpr (cluster_storable<T>::value) {
+    if (one_cluster) {   // the grid is one cluster (or one CTA), a tile per CTA: totals by stores into every later CTA's shared memory
+      T* const totals = reinterpret_cast<T*>(sm.cluster_total);
+      T agg = sm.warp_total[0];
+#pragma unroll
+      for (int w = 1; w < NWARPS; ++w) agg = op(agg, sm.warp_total[w]);
+      if (gridDim.x > 1) {
+        cluster_wait_started();
+        if (warp == 0 && lane > (int)tile && lane < (int)gridDim.x) cluster_store(cluster_addr(smem_addr(totals + tile), lane), agg);
+        cluster_barrier();
+      }
+      if (threadIdx.x == 0) {
+        opt<T> p; p.v = init; p.has = has_init;
+        for (unsigned q = 0; q < (unsigned)tile; ++q) p.append(totals[q], op);
+        sm.prefix = p.v; sm.has_prefix = p.has; sm.inclusive = p.has ? op(p.v, agg) : agg;
+      }
+    }
+  }
+  if (warp == 0 && !one_cluster) {
     T agg = sm.warp_total[0];
 #pragma unroll
     for (int w = 1; w < NWARPS; ++w) agg = op(agg, sm.warp_total[w]);

@@ -1,11 +1,15 @@
 // Single-pass device-wide reduction for sm_100a.
 //
+// Up to 512 KB: one launch of one cluster, whose CTAs store their totals into the first one's shared memory; nothing to clear.  A call
+// and the wait for it: 1000 int32 9.8 us against 12.5 with partials, ticket and clearing launch, 65 k 11.5 against 13.0, 131 k
+// 11.8 against 13.4.  Larger inputs:
 // One launch: a grid sized to the SM count streams the input with 16-byte evict-first loads
 // (four in flight per thread), folds it with warp shuffles, and the last CTA to finish (found
 // with an atomic ticket) folds the per-CTA partials and `init` into the result.  Replaces the
 // two-kernel cub::DispatchReduce call of thrust/system/cuda/detail/reduce.h:946-983.
 // Like that path it needs an associative and commutative operator.
 #pragma once
+#include "cluster.cuh"
 #include "common.cuh"
 
 namespace tb200 {
@@ -36,7 +40,8 @@ __device__ __forceinline__ opt<AccT> block_reduce_opt(opt<AccT> x, Op op, opt<Ac
 template <class InIt, class AccT, class Op, int VEC>
 __global__ void __launch_bounds__(REDUCE_BLOCK)
 reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* partial_has,
-              ws_header* hdr, AccT* out) {
+              ws_header* hdr, AccT* out, bool one_cluster) {
+  if (one_cluster && gridDim.x > 1) cluster_arrive_started();
   TB200_SHARED_ARRAY(opt<AccT>, smem, 32);
   __shared__ bool is_last;
   const size_t tid = (size_t)blockIdx.x * REDUCE_BLOCK + threadIdx.x;
@@ -87,11 +92,27 @@ reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* par
     for (; i < n; i += stride) acc.append((AccT)in[i], op);
   }
 
-  if (gridDim.x == 1) {   // nobody to wait for, and a header that nobody has cleared (`out` may lie behind its first fields)
-    if (threadIdx.x < sizeof(ws_header) / 4) reinterpret_cast<unsigned*>(hdr)[threadIdx.x] = 0;
-    const opt<AccT> all = block_reduce_opt(acc, op, smem);
-    if (threadIdx.x == 0) *out = all.has ? op(init, all.v) : init;
-    return;
+  if constexpr (cluster_storable<AccT>::value) {
+    if (one_cluster) {   // a header that nobody has cleared (`out` may lie behind its first fields); the CTAs' totals travel to the first one
+      __shared__ __align__(16) unsigned char totals_raw[CLUSTER_MAX_CTAS * sizeof(AccT)];
+      __shared__ unsigned has_total[CLUSTER_MAX_CTAS];
+      AccT* const totals = reinterpret_cast<AccT*>(totals_raw);
+      if (blockIdx.x == 0 && threadIdx.x < sizeof(ws_header) / 4) reinterpret_cast<unsigned*>(hdr)[threadIdx.x] = 0;
+      opt<AccT> all = block_reduce_opt(acc, op, smem);
+      if (gridDim.x > 1) {
+        cluster_wait_started();
+        if (threadIdx.x == 0) {
+          if (all.has) cluster_store(cluster_addr(smem_addr(totals + blockIdx.x), 0), all.v);
+          cluster_store(cluster_addr(smem_addr(has_total + blockIdx.x), 0), (unsigned)all.has);
+        }
+        cluster_barrier();
+        all.has = false;
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+          for (unsigned q = 0; q < gridDim.x; ++q) if (has_total[q]) all.append(totals[q], op);
+      }
+      if (blockIdx.x == 0 && threadIdx.x == 0) *out = all.has ? op(init, all.v) : init;
+      return;
+    }
   }
   opt<AccT> blk = block_reduce_opt(acc, op, smem);
   if (threadIdx.x == 0) {
@@ -116,11 +137,11 @@ reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* par
   }
 }
 
-// One CTA up to four loads per thread: without partials, ticket and the launch that clears them a call of 1000 int32 takes
-// (measured below) less, and a CTA has its four loads in flight together anyway.
+// Up to which input one cluster of up to 16 CTAs does it, without partials, ticket and the launch that clears them.
+constexpr size_t REDUCE_CLUSTER_BYTES = (size_t)1 << 19;
+
 inline int reduce_grid(size_t work_items /* vectors or elements */) {
   const device_info& di = current_device_info();
-  if (work_items <= (size_t)REDUCE_BLOCK * REDUCE_UNROLL) return 1;
   size_t want = (work_items + REDUCE_BLOCK - 1) / REDUCE_BLOCK;
   size_t cap = (size_t)di.sm_count * REDUCE_CTAS_PER_SM;
   if (cap > REDUCE_MAX_GRID) cap = REDUCE_MAX_GRID;
@@ -148,31 +169,35 @@ cudaError_t reduce_async(InIt in, size_t n, AccT init, Op op, AccT* d_out, void*
     d_out = reinterpret_cast<AccT*>(reinterpret_cast<char*>(rep) + (out_at - base));
     reported(rep, hdr);
   }
-  auto clear = [&](int grid) { return grid == 1 ? cudaSuccess : cudaMemsetAsync(hdr, 0, sizeof(ws_header), stream); };
-  constexpr bool is_ptr = std::is_pointer<InIt>::value;
-  if constexpr (is_ptr) {
+  auto launch = [&](auto vec_tag) -> cudaError_t {
+    constexpr int VEC = decltype(vec_tag)::value;
+    auto kern = reduce_kernel<InIt, AccT, Op, VEC>;
+    const char* const name = VEC > 0 ? "reduce_kernel (16-byte loads)" : "reduce_kernel (generic iterator)";
+    const size_t work_items = VEC > 0 ? n / (VEC > 0 ? VEC : 1) : n, per_cta = (size_t)REDUCE_BLOCK * (VEC > 0 ? REDUCE_UNROLL : REDUCE_UNROLL_GENERIC);
+    timed_launch tl(KID_REDUCE, stream);
+    if (cluster_storable<AccT>::value && work_items * (VEC > 0 ? 16 : sizeof(AccT)) <= REDUCE_CLUSTER_BYTES) {
+      static thread_local unsigned largest[64] = {0};
+      bool launched = false;
+      unsigned ctas = cluster_ctas((work_items + per_cta - 1) / per_cta);
+      if (ctas == 0) ctas = CLUSTER_MAX_CTAS;
+      const cudaError_t e = cluster_launch(kern, ctas, REDUCE_BLOCK, 0, stream, largest, launched, in, n, init, op, partials, has, hdr, d_out, true);
+      if (launched) log_launch(name, ctas, REDUCE_BLOCK, 0, n, stream);
+      if (launched || e != cudaSuccess) return e;
+    }
+    const cudaError_t e = cudaMemsetAsync(hdr, 0, sizeof(ws_header), stream);
+    if (e != cudaSuccess) return e;
+    const int grid = reduce_grid(work_items);
+    kern<<<grid, REDUCE_BLOCK, 0, stream>>>(in, n, init, op, partials, has, hdr, d_out, false);
+    log_launch(name, grid, REDUCE_BLOCK, 0, n, stream);
+    return cudaGetLastError();
+  };
+  if constexpr (std::is_pointer<InIt>::value) {
     using In = typename std::remove_cv<typename std::remove_pointer<InIt>::type>::type;
-    constexpr bool vec_ok = std::is_arithmetic<In>::value && (16 % sizeof(In) == 0);
-    if constexpr (vec_ok) {
-      if (is_aligned16(in)) {
-        constexpr int VEC = 16 / sizeof(In);
-        int grid = reduce_grid(n / VEC);
-        const cudaError_t e = clear(grid);
-        if (e != cudaSuccess) return e;
-        timed_launch tl(KID_REDUCE, stream);
-        reduce_kernel<InIt, AccT, Op, VEC><<<grid, REDUCE_BLOCK, 0, stream>>>(in, n, init, op, partials, has, hdr, d_out);
-        log_launch("reduce_kernel (16-byte loads)", grid, REDUCE_BLOCK, 0, n, stream);
-        return cudaGetLastError();
-      }
+    if constexpr (std::is_arithmetic<In>::value && 16 % sizeof(In) == 0) {
+      if (is_aligned16(in)) return launch(std::integral_constant<int, 16 / (int)sizeof(In)>());
     }
   }
-  int grid = reduce_grid(n);
-  const cudaError_t e = clear(grid);
-  if (e != cudaSuccess) return e;
-  timed_launch tl(KID_REDUCE, stream);
-  reduce_kernel<InIt, AccT, Op, 0><<<grid, REDUCE_BLOCK, 0, stream>>>(in, n, init, op, partials, has, hdr, d_out);
-  log_launch("reduce_kernel (generic iterator)", grid, REDUCE_BLOCK, 0, n, stream);
-  return cudaGetLastError();
+  return launch(std::integral_constant<int, 0>());
 }
 
 }  // namespace tb200

@@ -11,10 +11,12 @@
 // item.  A second walk over the registers then emits, at every head, the key of the new run and
 // the finished total of the run before it; heads are compacted through shared memory so that
 // keys_out / values_out are written with consecutive threads on consecutive addresses.  Values
-// inside a run are combined left to right.  Replaces InitAgent + ReduceByKeyAgent of
+// inside a run are combined left to right.  Up to 16 tiles are one cluster's, a tile per CTA: nothing to clear, no ticket, no look-back.
+// Replaces InitAgent + ReduceByKeyAgent of
 // thrust/system/cuda/detail/reduce_by_key.h:197-860.
 #pragma once
 #include "common.cuh"
+#include "cluster.cuh"
 #include "reduce_by_key_pipe.cuh"
 #include "reduce_by_key_stream.cuh"
 
@@ -45,7 +47,8 @@ template <class K, class V> struct rbk_tuning {
 template <class KeyIt, class ValIt, class KeyOutIt, class ValOutIt, class K, class V, class Eq, class Op, class Off, bool VEC_LOAD, int IPT>
 __global__ void __launch_bounds__(RBK_BLOCK)
 reduce_by_key_kernel(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOutIt vals_out, size_t n, Eq key_eq, Op op,
-                     tile_state<rbk_pair<Off, V>> ts, ws_header* hdr, ws_header* rep, unsigned long long* d_count) {
+                     tile_state<rbk_pair<Off, V>> ts, ws_header* hdr, ws_header* rep, unsigned long long* d_count,
+                     bool one_cluster) {
   using P = rbk_pair<Off, V>;
   using Comb = rbk_combine<Off, V, Op>;
   constexpr int NWARPS = RBK_BLOCK / 32;
@@ -59,12 +62,16 @@ reduce_by_key_kernel(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOutIt vals_ou
   V* s_val = reinterpret_cast<V*>(rbk_smem + (TILE * sizeof(K) + 15) / 16 * 16);
   TB200_SHARED_OBJECT(K, s_prev);
 
-  if (threadIdx.x == 0) s_tile = atomicAdd(&hdr->ticket, 1u);
+  if (one_cluster) {
+    if (gridDim.x > 1) cluster_arrive_started();
+    if (threadIdx.x == 0) s_tile = blockIdx.x;
+    if (blockIdx.x == 0 && threadIdx.x < sizeof(ws_header) / 4) reinterpret_cast<unsigned*>(hdr)[threadIdx.x] = 0;   // nobody has cleared it
+  } else if (threadIdx.x == 0) s_tile = atomicAdd(&hdr->ticket, 1u);
   __syncthreads();
   const size_t tile = s_tile;
   const size_t tile_base = tile * (size_t)TILE;
   const bool full = tile_base + TILE <= n;
-  const unsigned tile_n = full ? (unsigned)TILE : (unsigned)(n - tile_base);
+  const unsigned tile_n = full ? (unsigned)TILE : tile_base < n ? (unsigned)(n - tile_base) : 0u;   // none in a CTA that only fills the cluster
   Comb comb; comb.op = op;
 
   // ---- coalesced load of the tile into shared memory
@@ -85,7 +92,7 @@ reduce_by_key_kernel(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOutIt vals_ou
       if (c < tile_n) { stash(&s_key[c], (K)keys[tile_base + c]); stash(&s_val[c], (V)vals[tile_base + c]); }
     }
   }
-  if (threadIdx.x == 0 && tile_base > 0) s_prev = keys[tile_base - 1];
+  if (threadIdx.x == 0 && tile_base > 0 && tile_n > 0) s_prev = keys[tile_base - 1];
   __syncthreads();
 
   // ---- my ITEMS consecutive items; walk 1: head flags and summary
@@ -116,7 +123,7 @@ reduce_by_key_kernel(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOutIt vals_ou
   P vec_total[1] = {summary};
   opt<P> pre[1];
   P none; none.count = 0; none.value = V();
-  tile_exclusive_prefix<P, Comb, 1, NWARPS>(vec_total, pre, tile, none, false, comb, ts, &rep->error, sm);
+  tile_exclusive_prefix<P, Comb, 1, NWARPS>(vec_total, pre, tile, none, false, comb, ts, &rep->error, sm, one_cluster);
   const Off head_off = sm.has_prefix ? sm.prefix.count : (Off)0;   // run heads in all preceding tiles
   __syncthreads();                                                  // everyone has its items in registers: reuse the tile buffers
 
@@ -159,9 +166,9 @@ reduce_by_key_kernel(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOutIt vals_ou
   }
 }
 
-// Where the pipeline starts: 2^19 items of 4 + 4 bytes 15.6 us against 19.7 single-pass, 2^18 14.4 against 17.0, 50 k 14.6
-// against 15.4.
-constexpr size_t RBK_PIPE_MIN_BYTES = (size_t)1 << 20;
+// Where the pipeline starts (a call and the wait for it, items of 4 + 4 bytes): 131 k 15.6 us against 18.8 single-pass, 100 k 15.9 against
+// 16.1; 65 k, which one cluster does, 15.3 against 14.6 and 50 k 15.4 against 14.3 (16.0 single-pass).
+constexpr size_t RBK_PIPE_MIN_BYTES = (size_t)5 << 17;
 
 template <class K, class V> constexpr size_t rbk_tile_items() { return (size_t)RBK_BLOCK * rbk_tuning<K, V>::IPT; }
 template <class K, class V> size_t rbk_workspace_bytes(size_t n) {
@@ -216,8 +223,10 @@ cudaError_t reduce_by_key_async(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOu
         return reduce_by_key_stream_async<K, V, Eq, Op>(keys, vals, keys_out, vals_out, n, eq, op, d_count, ws, stream);
     }
   }
-  cudaError_t e = cudaMemsetAsync(base, 0, sizeof(ws_header) + tile_state<rbk_pair<unsigned long long, V>>::bytes(tiles + 1), stream);
-  if (e != cudaSuccess) return e;
+  const unsigned ctas = tiles_stay_apart() || n == 0 || !cluster_storable<rbk_pair<unsigned, V>>::value ? 0u : cluster_ctas(tiles);
+  cudaError_t e = cudaSuccess;
+  auto clear = [&] { return cudaMemsetAsync(base, 0, sizeof(ws_header) + tile_state<rbk_pair<unsigned long long, V>>::bytes(tiles + 1), stream); };
+  if (n == 0 && (e = clear()) != cudaSuccess) return e;
   if (n == 0) { if (d_count) return cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), stream); return cudaSuccess; }
   const bool small = n < (1ull << 31);
   if (!ALLOW_BIG && !small) return cudaErrorInvalidValue;
@@ -230,9 +239,18 @@ cudaError_t reduce_by_key_async(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOu
     const size_t smem = (rbk_tile_items<K, V>() * sizeof(K) + 15) / 16 * 16 + rbk_tile_items<K, V>() * sizeof(V);
     if (smem > 48 * 1024 && (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return;
     ws_header* const rep = report_of(hdr);
-    reported(rep, hdr);
     timed_launch tl(KID_REDUCE_BY_KEY, stream);
-    kern<<<(unsigned)tiles, RBK_BLOCK, smem, stream>>>(keys, vals, keys_out, vals_out, n, eq, op, ts, hdr, rep, d_count);
+    if (ctas) {
+      static thread_local unsigned largest[64] = {0};
+      bool launched = false;
+      e = cluster_launch(kern, ctas, RBK_BLOCK, smem, stream, largest, launched, keys, vals, keys_out, vals_out, n, eq, op, ts, hdr, rep, d_count, true);
+      if (launched && e == cudaSuccess) reported(rep, hdr);
+      if (launched || e != cudaSuccess) return;
+    }
+    if ((e = clear()) != cudaSuccess) return;
+    reported(rep, hdr);
+    kern<<<(unsigned)tiles, RBK_BLOCK, smem, stream>>>(keys, vals, keys_out, vals_out, n, eq, op, ts, hdr, rep, d_count, false);
+    e = cudaGetLastError();
   };
   constexpr bool ptrs = std::is_pointer<KeyIt>::value && std::is_pointer<ValIt>::value;
   bool use_vec = false;
@@ -243,12 +261,12 @@ cudaError_t reduce_by_key_async(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOu
       use_vec = is_aligned16((const void*)keys) && is_aligned16((const void*)vals);
       if (use_vec) {
         if (small) launch((unsigned)0, std::true_type()); else if constexpr (ALLOW_BIG) launch((unsigned long long)0, std::true_type());
-        return e != cudaSuccess ? e : cudaGetLastError();
+        return e;
       }
     }
   }
   if (small) launch((unsigned)0, std::false_type()); else if constexpr (ALLOW_BIG) launch((unsigned long long)0, std::false_type());
-  return e != cudaSuccess ? e : cudaGetLastError();
+  return e;
 }
 
 }  // namespace tb200

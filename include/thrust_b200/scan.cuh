@@ -10,9 +10,12 @@
 // vector totals with shuffles, and warp 0 resolves the tile's prefix by looking back over the
 // preceding tiles' published aggregates.  The output is written with the same 16-byte pattern,
 // so every element is read once and written once: 2 * sizeof(T) bytes of HBM traffic per element.
+// An input of up to 16 tiles is one cluster's, a tile per CTA: nothing to clear, no ticket, no look-back (a call and the wait for it: 50 k
+// int32 11.4 us against 13.4, 131 k 11.5 against 14.0, 65 k doubles 12.2 against 14.9).
 // Replaces the cub::DispatchScan call of thrust/system/cuda/detail/scan.h:61-114 and :139-192.
 #pragma once
 #include "common.cuh"
+#include "cluster.cuh"
 #include "reduce.cuh"
 #include "scan_pipe.cuh"
 
@@ -30,7 +33,9 @@ template <class T> struct scan_tuning {
 
 template <class InIt, class OutIt, class T, class Op, bool INCLUSIVE, int VEC, int IPT>
 __global__ void __launch_bounds__(SCAN_BLOCK, 4)
-scan_kernel(InIt in, OutIt out, size_t n, T init, bool has_init, const T* init_ptr, Op op, tile_state<T> ts, ws_header* hdr, ws_header* rep) {
+scan_kernel(InIt in, OutIt out, size_t n, T init, bool has_init, const T* init_ptr, Op op, tile_state<T> ts, ws_header* hdr, ws_header* rep,
+            bool one_cluster) {
+  if (one_cluster && gridDim.x > 1) cluster_arrive_started();
   if (init_ptr) { init = *init_ptr; has_init = true; }   // an initial value that lives on the device (the carry of a sharded scan)
   constexpr int VPT = IPT / VEC;
   constexpr int NWARPS = SCAN_BLOCK / 32;
@@ -42,7 +47,10 @@ scan_kernel(InIt in, OutIt out, size_t n, T init, bool has_init, const T* init_p
   using prefix_smem_t = tile_prefix_smem<T, NWARPS>;
   TB200_SHARED_OBJECT(prefix_smem_t, sm);
 
-  if (threadIdx.x == 0) s_tile = atomicAdd(&hdr->ticket, 1u);
+  if (one_cluster) {
+    if (threadIdx.x == 0) s_tile = blockIdx.x;
+    if (blockIdx.x == 0 && threadIdx.x < sizeof(ws_header) / 4) reinterpret_cast<unsigned*>(hdr)[threadIdx.x] = 0;   // nobody has cleared it
+  } else if (threadIdx.x == 0) s_tile = atomicAdd(&hdr->ticket, 1u);
   __syncthreads();
   const size_t tile = s_tile;
   const int lane = lane_id(), warp = threadIdx.x >> 5;
@@ -86,7 +94,7 @@ scan_kernel(InIt in, OutIt out, size_t n, T init, bool has_init, const T* init_p
     vec_total[v] = x[v][VEC - 1];
   }
   opt<T> pre[VPT];   // everything before vector v of this lane, across tiles, including init
-  tile_exclusive_prefix<T, Op, VPT, NWARPS>(vec_total, pre, tile, init, has_init, op, ts, &rep->error, sm);
+  tile_exclusive_prefix<T, Op, VPT, NWARPS>(vec_total, pre, tile, init, has_init, op, ts, &rep->error, sm, one_cluster);
 
   // ---- apply and store
 #pragma unroll
@@ -347,8 +355,9 @@ template <class Kernel> int resident_ctas(Kernel kernel, int block, size_t smem)
   return per_sm * current_device_info().sm_count;
 }
 
-// Where the pipeline starts: 2^20 int32 12.4 us against 15.4 single-pass, 2^18 12.0 against 12.4.
-constexpr size_t SCAN_PIPE_MIN_BYTES = (size_t)1 << 22;
+// Where the pipeline starts (a call and the wait for it): 1 M int32 14.2 us against 16.2 single-pass, 2^19 13.7 against 13.9, 400 k
+// 13.9 against 13.6.
+constexpr size_t SCAN_PIPE_MIN_BYTES = (size_t)1 << 21;
 // inputs of two tiles and more for every CTA of the windowed kernel: where that one starts
 template <class T> bool scan_fills_windows(size_t n) {
   const size_t tile = (size_t)SCAN_BLOCK * scanw_tuning<T>::IPT, ctas = (size_t)current_device_info().sm_count * SCANW_CTAS_PER_SM;
@@ -445,31 +454,40 @@ cudaError_t scan_async(InIt in, OutIt out, size_t n, T init, bool has_init, Op o
   }
   tile_state<T> ts;
   ts.bind(base + sizeof(ws_header), tiles + 1);
-  cudaError_t e = cudaMemsetAsync(base, 0, scan_workspace_bytes<T>(n), stream);
-  if (e != cudaSuccess) return e;
-#ifdef TB200_TEST_HOOKS
-  if (test_hook_flags() & 1u) { if ((e = cudaMemsetAsync(&hdr->flags, 1, 1, stream)) != cudaSuccess) return e; }
-#endif
   ws_header* const rep = report_of(hdr);
-  reported(rep, hdr);
-  timed_launch tl(KID_SCAN, stream);
+  auto launch = [&](auto vec_tag) -> cudaError_t {
+    constexpr int VEC = decltype(vec_tag)::value;
+    auto kern = scan_kernel<InIt, OutIt, T, Op, INCLUSIVE, VEC, IPT>;
+    const char* const name = VEC > 1 ? "scan_kernel (16-byte loads)" : "scan_kernel (generic iterator)";
+    timed_launch tl(KID_SCAN, stream);
+    const unsigned ctas = cluster_ctas(tiles);
+    if (cluster_storable<T>::value && ctas != 0 && !tiles_stay_apart()) {
+      static thread_local unsigned largest[64] = {0};
+      bool launched = false;
+      const cudaError_t e = cluster_launch(kern, ctas, SCAN_BLOCK, 0, stream, largest, launched, in, out, n, init, has_init, d_init, op, ts, hdr, rep, true);
+      if (launched) { reported(rep, hdr); log_launch(name, ctas, SCAN_BLOCK, 0, n, stream); }
+      if (launched || e != cudaSuccess) return e;
+    }
+    cudaError_t e = cudaMemsetAsync(base, 0, sizeof(ws_header) + tile_state<T>::bytes(tiles + 1), stream);
+    if (e != cudaSuccess) return e;
+#ifdef TB200_TEST_HOOKS
+    if (test_hook_flags() & 1u) { if ((e = cudaMemsetAsync(&hdr->flags, 1, 1, stream)) != cudaSuccess) return e; }
+#endif
+    reported(rep, hdr);
+    kern<<<(unsigned)tiles, SCAN_BLOCK, 0, stream>>>(in, out, n, init, has_init, d_init, op, ts, hdr, rep, false);
+    log_launch(name, tiles, SCAN_BLOCK, 0, n, stream);
+    return cudaGetLastError();
+  };
   if constexpr (ptrs) {
     using In = typename std::remove_cv<typename std::remove_pointer<InIt>::type>::type;
     using Out = typename std::remove_pointer<OutIt>::type;
     constexpr bool vec_ok = std::is_same<In, T>::value && std::is_same<Out, T>::value && std::is_arithmetic<T>::value &&
                             (sizeof(T) == 4 || sizeof(T) == 8);
     if constexpr (vec_ok) {
-      if (vectors) {
-        constexpr int VEC = 16 / sizeof(T);
-        scan_kernel<InIt, OutIt, T, Op, INCLUSIVE, VEC, IPT><<<(unsigned)tiles, SCAN_BLOCK, 0, stream>>>(in, out, n, init, has_init, d_init, op, ts, hdr, rep);
-        log_launch("scan_kernel (16-byte loads)", tiles, SCAN_BLOCK, 0, n, stream);
-        return cudaGetLastError();
-      }
+      if (vectors) return launch(std::integral_constant<int, 16 / sizeof(T)>());
     }
   }
-  scan_kernel<InIt, OutIt, T, Op, INCLUSIVE, 1, IPT><<<(unsigned)tiles, SCAN_BLOCK, 0, stream>>>(in, out, n, init, has_init, d_init, op, ts, hdr, rep);
-  log_launch("scan_kernel (generic iterator)", tiles, SCAN_BLOCK, 0, n, stream);
-  return cudaGetLastError();
+  return launch(std::integral_constant<int, 1>());
 }
 
 }  // namespace tb200

@@ -13,12 +13,16 @@
 // UniqueAgent pairs of thrust/system/cuda/detail/copy_if.h:160-593, partition.h:134-602 and
 // unique.h:183-541.
 //
+// An input of up to 16 tiles is one cluster's, a tile per CTA: nothing to clear, no ticket, no look-back (a call and the wait for it: 50 k
+// int32 selected 13.1 us against 13.8, made unique 12.1 against 13.1, 131 k 13.5 against 14.2 and 12.5 against 13.5).
+//
 // Order guarantees: kept items keep their input order (stable).  Dropped items are written in
 // input order too, either to a second output (partition_copy) or -- for the in-place partition --
 // mirrored from the end of a scratch copy that partition_finish_kernel reads back reversed, which
 // restores input order; so partition here is always the stable one.
 #pragma once
 #include "common.cuh"
+#include "cluster.cuh"
 #include "select_pipe.cuh"
 
 namespace tb200 {
@@ -40,7 +44,7 @@ template <class T> struct select_tuning {
 template <int MODE, bool KEEP_REJECTS, class InIt, class StIt, class SelIt, class RejIt, class T, class Pred, class Off, int VEC, int IPT>
 __global__ void __launch_bounds__(SELECT_BLOCK, 4)
 select_kernel(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, size_t n, Pred pred, tile_state<Off> ts, ws_header* hdr,
-              ws_header* rep, unsigned long long* d_count, bool mirrored) {
+              ws_header* rep, unsigned long long* d_count, bool mirrored, bool one_cluster) {
   constexpr int VPT = IPT / VEC;
   constexpr int NWARPS = SELECT_BLOCK / 32;
   constexpr int WCHUNK = 32 * IPT;
@@ -49,14 +53,18 @@ select_kernel(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, size_t n, Pre
   __shared__ tile_prefix_smem<Off, NWARPS> sm;
   TB200_SHARED_ARRAY(T, stage, TILE);
 
-  if (threadIdx.x == 0) s_tile = atomicAdd(&hdr->ticket, 1u);
+  if (one_cluster) {
+    if (gridDim.x > 1) cluster_arrive_started();
+    if (threadIdx.x == 0) s_tile = blockIdx.x;
+    if (blockIdx.x == 0 && threadIdx.x < sizeof(ws_header) / 4) reinterpret_cast<unsigned*>(hdr)[threadIdx.x] = 0;   // nobody has cleared it
+  } else if (threadIdx.x == 0) s_tile = atomicAdd(&hdr->ticket, 1u);
   __syncthreads();
   const size_t tile = s_tile;
   const int lane = lane_id(), warp = threadIdx.x >> 5;
   const size_t tile_base = tile * (size_t)TILE;
   const size_t wbase = tile_base + (size_t)warp * WCHUNK;
   const bool full = tile_base + TILE <= n;
-  const unsigned tile_n = full ? (unsigned)TILE : (unsigned)(n - tile_base);
+  const unsigned tile_n = full ? (unsigned)TILE : tile_base < n ? (unsigned)(n - tile_base) : 0u;   // none in a CTA that only fills the cluster
 
   // ---- load
   T x[VPT][VEC];
@@ -120,7 +128,7 @@ select_kernel(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, size_t n, Pre
 
   // ---- number of kept items before each vector, across tiles
   opt<Off> pre[VPT];
-  tile_exclusive_prefix<Off, plus_op, VPT, NWARPS>(vec_total, pre, tile, (Off)0, true, plus_op(), ts, &rep->error, sm);
+  tile_exclusive_prefix<Off, plus_op, VPT, NWARPS>(vec_total, pre, tile, (Off)0, true, plus_op(), ts, &rep->error, sm, one_cluster);
   const Off sel_off = sm.prefix;                       // kept items in all preceding tiles
   const unsigned tile_nsel = (unsigned)(sm.inclusive - sm.prefix);
 
@@ -146,7 +154,7 @@ select_kernel(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, size_t n, Pre
       if (mirrored) out_sel[n - 1 - r] = stage[j]; else out_rej[r] = stage[j];
     }
   }
-  if (threadIdx.x == 0 && tile_base + TILE >= n) {
+  if (threadIdx.x == 0 && tile_base < n && tile_base + TILE >= n) {
     hdr->count = rep->count = (unsigned long long)sm.inclusive;
     if (d_count) *d_count = (unsigned long long)sm.inclusive;
   }
@@ -173,9 +181,10 @@ template <class T> size_t select_workspace_bytes(size_t n) {
   return single;
 }
 
-// Where the pipeline starts.  2^20 int32 selected 13.3 us against 14.3 single-pass, 2^18 12.0 against 11.4; with the
-// dropped items written too 2^20 14.9 against 17.6, 2^18 12.3 against 15.1.
-constexpr size_t SELECT_PIPE_MIN_BYTES = (size_t)1 << 22;
+// Where the pipeline starts (a call and the wait for it): 1 M int32 made unique 15.6 us against 16.7 single-pass, selected 18.1 against
+// 18.1, 700 k 15.4 against 15.3 and 17.7 against 16.6; with the dropped items written too (kernels) 2^20 14.9 against 17.6,
+// 2^18 12.3 against 15.1.
+constexpr size_t SELECT_PIPE_MIN_BYTES = (size_t)3 << 20;
 constexpr size_t SELECT_PIPE_MIN_BYTES_REJECTS = (size_t)1 << 20;
 
 // Whether the pipeline may serve a call: a large, 16-byte aligned input and outputs that do not overlap it (out_rej: null
@@ -221,8 +230,10 @@ cudaError_t select_async(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, si
       }
     }
   }
-  cudaError_t e = cudaMemsetAsync(base, 0, sizeof(ws_header) + tile_state<unsigned long long>::bytes(tiles + 1), stream);
-  if (e != cudaSuccess) return e;
+  const unsigned ctas = tiles_stay_apart() || n == 0 ? 0u : cluster_ctas(tiles);
+  cudaError_t e = cudaSuccess;
+  auto clear = [&] { return cudaMemsetAsync(base, 0, sizeof(ws_header) + tile_state<unsigned long long>::bytes(tiles + 1), stream); };
+  if (n == 0 && (e = clear()) != cudaSuccess) return e;
   if (n == 0) { if (d_count) return cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), stream); return cudaSuccess; }
   auto launch = [&](auto off_tag, auto vec_tag) {
     using Off = decltype(off_tag);
@@ -230,10 +241,19 @@ cudaError_t select_async(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, si
     tile_state<Off> ts;
     ts.bind(base + sizeof(ws_header), tiles + 1);
     ws_header* const rep = report_of(hdr);
-    reported(rep, hdr);
+    auto kern = select_kernel<MODE, KEEP_REJECTS, InIt, StIt, SelIt, RejIt, T, Pred, Off, VEC, IPT>;
     timed_launch tl(KID_SELECT, stream);
-    select_kernel<MODE, KEEP_REJECTS, InIt, StIt, SelIt, RejIt, T, Pred, Off, VEC, IPT>
-        <<<(unsigned)tiles, SELECT_BLOCK, 0, stream>>>(in, stencil, out_sel, out_rej, n, pred, ts, hdr, rep, d_count, mirrored);
+    if (ctas) {
+      static thread_local unsigned largest[64] = {0};
+      bool launched = false;
+      e = cluster_launch(kern, ctas, SELECT_BLOCK, 0, stream, largest, launched, in, stencil, out_sel, out_rej, n, pred, ts, hdr, rep, d_count, mirrored, true);
+      if (launched && e == cudaSuccess) reported(rep, hdr);
+      if (launched || e != cudaSuccess) return;
+    }
+    if ((e = clear()) != cudaSuccess) return;
+    reported(rep, hdr);
+    kern<<<(unsigned)tiles, SELECT_BLOCK, 0, stream>>>(in, stencil, out_sel, out_rej, n, pred, ts, hdr, rep, d_count, mirrored, false);
+    e = cudaGetLastError();
   };
   constexpr bool vec_ok = std::is_pointer<InIt>::value && std::is_arithmetic<T>::value && (sizeof(T) == 4 || sizeof(T) == 8) && MODE != SEL_STENCIL;
   bool use_vec = false;
@@ -243,11 +263,11 @@ cudaError_t select_async(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, si
     constexpr int V = 16 / sizeof(T);
     if (use_vec) {
       if (small) launch((unsigned)0, std::integral_constant<int, V>()); else launch((unsigned long long)0, std::integral_constant<int, V>());
-      return cudaGetLastError();
+      return e;
     }
   }
   if (small) launch((unsigned)0, std::integral_constant<int, 1>()); else launch((unsigned long long)0, std::integral_constant<int, 1>());
-  return cudaGetLastError();
+  return e;
 }
 
 template <class T>

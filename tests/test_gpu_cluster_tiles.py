@@ -1,0 +1,62 @@
+"""Inputs of a few tiles, which one thread-block cluster does (scan, reduce, compaction, reduce_by_key): both sides of one tile, of
+cluster sizes that are no power of two, of the largest cluster; aligned and not."""
+import numpy as np
+import pytest
+
+from thrust_b200 import datagen as dg
+from gpu_util import dev, host, misaligned, rand_of
+
+pytestmark = pytest.mark.gpu
+SCAN_TILE, RBK_TILE = {4: 8192, 8: 4096}, {4: 4352, 8: 2304}     # items; 16 of them at most
+
+
+def edges(tile):
+    return [1, 31, tile - 1, tile, tile + 1, 3 * tile, 5 * tile - 3, 9 * tile + 5, 16 * tile - 1, 16 * tile, 16 * tile + 1]
+
+
+@pytest.mark.parametrize("place", [dev, lambda x: misaligned(x, 1)], ids=["aligned", "misaligned"])
+@pytest.mark.parametrize("dt", [np.int32, np.int64])
+def test_scan_and_reduce(tb, port, dt, place):
+    for n in edges(SCAN_TILE[np.dtype(dt).itemsize]):
+        x = rand_of(dt, n, 21, small=True)
+        d = place(x)
+        for op in ("plus", "min", "max"):
+            assert np.array_equal(host(tb.inclusive_scan(d, op=op)), port.inclusive_scan(x, op)), (n, op)
+            assert np.array_equal(host(tb.exclusive_scan(d, 7, op=op)), port.exclusive_scan(x, 7, op)), (n, op)
+            assert tb.reduce(d, dt(3), op=op) == port.reduce(x, dt(3), op), (n, op)
+        y = place(x)
+        assert np.array_equal(host(tb.inclusive_scan(y, out=y)), port.inclusive_scan(x)), n       # in place
+        assert np.array_equal(host(tb.inclusive_scan(d, init=5)), port.inclusive_scan(x) + dt(5)), n
+
+
+@pytest.mark.parametrize("place", [dev, lambda x: misaligned(x, 1)], ids=["aligned", "misaligned"])
+@pytest.mark.parametrize("dt", [np.int32, np.int64])
+def test_compaction(tb, port, dt, place):
+    for n in edges(SCAN_TILE[np.dtype(dt).itemsize]):
+        x = (dg.rand64(31, n) >> np.uint64(40)).astype(dt)
+        assert np.array_equal(host(tb.copy_if(place(x), "mod_eq", 3, 1)), port.copy_if(x, "mod_eq", 3, 1)), n
+        s = (dg.rand64(32, n) & np.uint64(1)).astype(np.uint8)
+        assert np.array_equal(host(tb.copy_if(place(x), "ne", 0, 0, stencil=dev(s))), x[s != 0]), n
+        kept, dropped = tb.partition_copy(place(x), "lt", 1 << 23)
+        assert np.array_equal(host(kept), x[x < 1 << 23]) and np.array_equal(host(dropped), x[x >= 1 << 23]), n
+        d = place(x)
+        want, split = port.stable_partition(x, "mod_eq", 2, 0)
+        assert tb.partition(d, "mod_eq", 2, 0) == split and np.array_equal(host(d), want), n
+        r = np.cumsum((dg.rand64(33, n) >> np.uint64(62)) == 0).astype(dt)
+        assert np.array_equal(host(tb.unique_copy(place(r))), port.unique_copy(r)), n
+        d = place(r)
+        assert np.array_equal(host(tb.unique(d)), port.unique_copy(r)), n                          # in place
+
+
+@pytest.mark.parametrize("place", [dev, lambda x: misaligned(x, 1)], ids=["aligned", "misaligned"])
+@pytest.mark.parametrize("kt,vt", [(np.int32, np.int32), (np.int64, np.int64), (np.int32, np.int64)])
+def test_reduce_by_key(tb, port, kt, vt, place):
+    tile = RBK_TILE[max(np.dtype(kt).itemsize, np.dtype(vt).itemsize)]
+    for n in edges(tile):
+        for shift in (62, 51):                                       # runs of 4; runs that cross several tiles
+            k = np.cumsum((dg.rand64(41, n) >> np.uint64(shift)) == 0).astype(kt)
+            v = rand_of(vt, n, 42, small=True)
+            for op in ("plus", "max"):
+                gk, gv = tb.reduce_by_key(place(k), place(v), op=op)
+                wk, wv = port.reduce_by_key(k, v, op)
+                assert np.array_equal(host(gk), wk) and np.array_equal(host(gv), wv), (n, op)
