@@ -330,6 +330,7 @@ merge_slices_kernel(const K* ka, const K* kb, const V* va, const V* vb, K* ko, V
   __shared__ __align__(16) unsigned char s_vals[HAS_V ? Tuning::VAL_BYTES : 16];
   __shared__ __align__(16) unsigned short s_src[TILE];
   __shared__ unsigned long long bars[2];               // the keys' slices have arrived, the payloads'
+  __shared__ size_t s_split[2];
   grid_dependents_launch();
   grid_dependency_wait();
   const unsigned t = blockIdx.x;
@@ -338,7 +339,17 @@ merge_slices_kernel(const K* ka, const K* kb, const V* va, const V* vb, K* ko, V
   const size_t pair_total = alen + blen;
   if (local >= pair_total) return;                     // a short last pair leaves its later tiles empty
   const unsigned tile_n = pair_total - local < TILE ? (unsigned)(pair_total - local) : (unsigned)TILE;
-  const merge_slices slices(a_split[t], local + TILE < pair_total ? a_split[t + 1] : a0p + alen, a0p, b0p, local, tile_n);
+  const int warp = threadIdx.x >> 5;
+  if (!a_split) {   // no pass before this one has found the splits: two warps do
+    if (warp < 2) {
+      const size_t s = a0p + warp_merge_path(ka + a0p, alen, kb + b0p, blen, warp ? local + tile_n : local, comp);
+      if (lane_id() == 0) s_split[warp] = s;
+    }
+    __syncthreads();
+  }
+  const size_t split_begin = a_split ? a_split[t] : s_split[0];
+  const size_t split_end = !a_split ? s_split[1] : local + TILE < pair_total ? a_split[t + 1] : a0p + alen;
+  const merge_slices slices(split_begin, split_end, a0p, b0p, local, tile_n);
   if (!slices.consistent) { if (threadIdx.x == 0) record_error(err, ERR_INCONSISTENT); return; }   // before any copy is sized by them
   const size_t a_begin = slices.a_begin, b_begin = slices.b_begin;
   const unsigned na = slices.na, nb = slices.nb;
@@ -373,7 +384,6 @@ merge_slices_kernel(const K* ka, const K* kb, const V* va, const V* vb, K* ko, V
       slice_issue(sv_b, vb + b_begin, nb, &bars[1], policy);
     }
   }
-  const int warp = threadIdx.x >> 5;
   if (warp == 1) slice_ends(sk_a, ka + a_begin, na);
   if (warp == 2) slice_ends(sk_b, kb + b_begin, nb);
   if constexpr (HAS_V) {
@@ -485,7 +495,11 @@ cudaError_t merge_pass_async(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutI
     // Up to 8192 tiles (16 M outputs) the pass's launches overlap the kernels before them (8 M pairs sorted in 0.47 ms
     // against 0.51); beyond, waiting CTAs only take slots from running ones (2^26 pairs 4.53 ms against 4.35).
     const bool overlap = tiles <= 8192;
-    const cudaError_t e = merge_split_async<K, Comp, Tuning::TILE>(ka, kb, g, tiles, comp, a_split, overlap, stream);
+    // Up to 2048 tiles (4 M outputs) of a sort's pass the tiles find their splits themselves, with a launch less (1 M pairs sorted in 120 us
+    // against 145, 3 M 207 against 222; 8 M 500 against 484: many CTAs per SM then wait for their searches).
+    const bool own_splits = g.run != 0 && tiles <= 2048;
+    if (own_splits) a_split = nullptr;
+    const cudaError_t e = own_splits ? cudaSuccess : merge_split_async<K, Comp, Tuning::TILE>(ka, kb, g, tiles, comp, a_split, overlap, stream);
     if (e != cudaSuccess) return e;
     if (overlap) {
       timed_launch tl(KID_MERGE, stream);
@@ -525,130 +539,143 @@ cudaError_t merge_async(KeyItA ka, size_t na, KeyItB kb, size_t nb, ValItA va, V
 // ---------------------------------------------------------------- merge sort
 template <int KB, int VB> struct block_sort_tuning {
   // power-of-two friendly tile of 256 * IPT items whose keys (+ a 2-byte index each) fit 44 KB of shared memory
-  static constexpr int FIT = MERGE_SMEM_BUDGET / (MERGE_BLOCK * (KB + 2));
+  static constexpr int BLOCK = MERGE_BLOCK;
+  static constexpr int FIT = MERGE_SMEM_BUDGET / (BLOCK * (KB + 2));
   static constexpr int IPT = (KB + VB) <= 8 ? TB200_BSORT_IPT8 : (FIT >= 8 ? 8 : FIT >= 4 ? 4 : FIT >= 2 ? 2 : 1);
   // one slot of padding per thread, where static shared memory has room for it (20-byte keys at 8 items: it has not)
-  static constexpr int TILE = MERGE_BLOCK * IPT, SMEM = 48 * 1024;
-  static constexpr bool PADDED = IPT >= 8 && (TILE + MERGE_BLOCK + 1) * (KB + 2) + 16 <= SMEM;
-  static constexpr int SLOTS = TILE + (PADDED ? MERGE_BLOCK : 0) + 1;
-  static_assert(SLOTS * (KB + 2) <= SMEM, "key too large for the block sort tile (more than 170 bytes)");
+  static constexpr int TILE = BLOCK * IPT, SMEM = 48 * 1024;
+  static constexpr int OVER = IPT + 2;   // slots that may be read past the tile's end
+  static constexpr int IDX_SLOTS = TILE + OVER;
+  static constexpr bool PADDED = IPT >= 8 && (TILE + BLOCK + OVER) * KB + IDX_SLOTS * 2 + 32 <= SMEM;
+  static constexpr int SLOTS = TILE + (PADDED ? BLOCK : 0) + OVER;
+  static_assert(SLOTS * KB + IDX_SLOTS * 2 <= SMEM, "key too large for the block sort tile (more than 170 bytes)");
 };
 
-// What bounds it is shared memory: a thread's IPT consecutive items are written and read back in every round,
-// and unpadded that is a stride of IPT words, IPT / 2 lanes to a bank.  One slot of padding per IPT items makes the
-// stride odd.  Rounds whose pairs of runs lie inside one warp's items need no barrier of the CTA, and whole
-// tiles are compared without the bookkeeping for the items past the end.  With the merge passes above the sort
-// of 2^26 (u32, u32) pairs takes 4.35 ms (6.89 before), of 8 M pairs 0.51 ms (1.00).
+// What bounds it is shared memory (the pipe is busy 91 % of a large sort's tiles: 122 wavefronts per 32 items before the
+// indexes left in 16-byte stores, 110 since): a thread's IPT consecutive items are written and read back in every round, and
+// unpadded that is a stride of IPT words, IPT / 2 lanes to a bank.  One slot of padding per IPT items makes the
+// stride odd.  Rounds whose pairs of runs lie inside one warp's items need no barrier of the CTA.  The merge takes its next
+// item without a branch: two candidates in registers, one load of the side that was taken.  With a branch for either side a
+// warp ran both, and a tile took 46 us instead of 20: 1000 (u32, u32) pairs sorted in 24 us (54 before), 100 k in 50 (85), 8 M in
+// 431 (484), of them 127 for the tiles (178).  512 threads of 8 items each: 100 k pairs 47 us, 8 M 447.  Payloads kept in shared
+// memory instead of fetched by their index: the same.
 template <class KeyIt, class ValIt, class KeyOutIt, class ValOutIt, class K, class V, bool HAS_V, class Comp, int IPT>
-__global__ void __launch_bounds__(MERGE_BLOCK, sizeof(K) <= 4 ? TB200_BSORT_CTAS8 : 1)
+__global__ void __launch_bounds__((block_sort_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>::BLOCK), sizeof(K) <= 4 ? TB200_BSORT_CTAS8 : 1)
 block_sort_kernel(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOutIt vals_out, size_t n, Comp comp) {
-  constexpr int TILE = MERGE_BLOCK * IPT;
   using Tuning = block_sort_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>;
+  constexpr int BLOCK = Tuning::BLOCK, TILE = Tuning::TILE;
   constexpr bool PADDED = Tuning::PADDED;
   constexpr int SLOTS = Tuning::SLOTS;
   static_assert(IPT == Tuning::IPT, "the tile is the tuning's");
   TB200_SHARED_ARRAY(K, s_key, SLOTS);
-  __shared__ unsigned short s_idx[SLOTS];
+  __shared__ __align__(16) unsigned short s_idx[Tuning::IDX_SLOTS];
   auto slot = [](unsigned j) { return PADDED ? j + j / IPT : j; };
   grid_dependents_launch();
   const size_t base = (size_t)blockIdx.x * TILE;
   const unsigned tile_n = n - base < TILE ? (unsigned)(n - base) : (unsigned)TILE;
 
-  auto sort_tile = [&](auto full_tag) {
-    constexpr bool FULL = decltype(full_tag)::value;
-    // ---- coalesced load, then each thread takes IPT consecutive items
+  // ---- coalesced load, then each thread takes IPT consecutive items (the last of a partial tile fewer)
 #pragma unroll
-    for (int i = 0; i < IPT; ++i) { unsigned c = threadIdx.x + i * MERGE_BLOCK; if (FULL || c < tile_n) stash(&s_key[slot(c)], (K)keys[base + c]); }
-    __syncthreads();
-    K k[IPT]; unsigned short idx[IPT];
-    const unsigned first = threadIdx.x * IPT, first_slot = slot(first);
-    // items past the end are "infinite": they carry the flag in idx and never move ahead of a real item
-    const unsigned mine = FULL ? (unsigned)IPT : first >= tile_n ? 0u : (tile_n - first < (unsigned)IPT ? tile_n - first : (unsigned)IPT);
+  for (int i = 0; i < IPT; ++i) { const unsigned c = threadIdx.x + i * BLOCK; if (c < tile_n) stash(&s_key[slot(c)], (K)keys[base + c]); }
+  __syncthreads();
+  K k[IPT]; unsigned short idx[IPT];
+  const unsigned first = threadIdx.x * IPT, first_slot = slot(first);
+  const unsigned mine = first >= tile_n ? 0u : tile_n - first < (unsigned)IPT ? tile_n - first : (unsigned)IPT;
 #pragma unroll
-    for (int i = 0; i < IPT; ++i) { idx[i] = (unsigned short)(first + i); if (FULL || (unsigned)i < mine) k[i] = s_key[first_slot + i]; else k[i] = K(); }
-    auto before = [&](const K& x, unsigned short xi, const K& y, unsigned short yi) {
-      // strict "x must come before y" honouring padding: real < pad; pad never before anything
-      if (!FULL) {
-        const bool xp = xi >= tile_n, yp = yi >= tile_n;
-        if (xp) return false;
-        if (yp) return true;
-      }
-      return (bool)comp(x, y);
-    };
-    // ---- odd-even transposition sort of the thread's items (stable: only swaps when strictly out of order)
+  for (int i = 0; i < IPT; ++i) { idx[i] = (unsigned short)(first + i); if ((unsigned)i < mine) k[i] = s_key[first_slot + i]; else k[i] = K(); }
+  // ---- odd-even transposition sort of the thread's items (stable: only swaps when strictly out of order)
 #pragma unroll
-    for (int r = 0; r < IPT; ++r) {
+  for (int r = 0; r < IPT; ++r) {
 #pragma unroll
-      for (int i = r & 1; i + 1 < IPT; i += 2) {
-        if (before(k[i + 1], idx[i + 1], k[i], idx[i])) {
-          K tk = k[i]; k[i] = k[i + 1]; k[i + 1] = tk;
-          unsigned short ti = idx[i]; idx[i] = idx[i + 1]; idx[i + 1] = ti;
-        }
-      }
+    for (int i = r & 1; i + 1 < IPT; i += 2) {
+      const bool swap = (unsigned)(i + 1) < mine && comp(k[i + 1], k[i]);
+      const K lo = swap ? k[i + 1] : k[i];
+      k[i + 1] = swap ? k[i] : k[i + 1];
+      k[i] = lo;
+      const unsigned short li = swap ? idx[i + 1] : idx[i];
+      idx[i + 1] = swap ? idx[i] : idx[i + 1];
+      idx[i] = li;
     }
-    // ---- log2(BLOCK) rounds: runs of `len` items merge pairwise in shared memory
-    for (unsigned len = IPT; len < (unsigned)TILE; len <<= 1) {
-      const bool in_warp = 2 * len <= 32u * IPT;     // both runs are this warp's own items, in this round and the ones before
-      if (in_warp && len > (unsigned)IPT) __syncwarp(); else __syncthreads();
+  }
+  // the thread's source indexes, in 16-byte stores where they fill one
+  auto put_idx = [&] {
+    if constexpr (IPT % 8 == 0) {
 #pragma unroll
-      for (int i = 0; i < IPT; ++i) { stash(&s_key[first_slot + i], k[i]); s_idx[first_slot + i] = idx[i]; }
-      if (in_warp) __syncwarp(); else __syncthreads();
-      const unsigned pair0 = first / (2 * len) * (2 * len);
-      const unsigned a0 = pair0, b0 = pair0 + len;
-      const unsigned d = first - pair0;
-      // merge path over the two runs (padding compares as +infinity, ties take from the left run)
-      unsigned lo = d > len ? d - len : 0, hi = d < len ? d : len;
-      while (lo < hi) {
-        const unsigned mid = (lo + hi) >> 1, at_b = slot(b0 + d - 1 - mid), at_a = slot(a0 + mid);
-        if (!before(s_key[at_b], FULL ? 0 : s_idx[at_b], s_key[at_a], FULL ? 0 : s_idx[at_a])) lo = mid + 1; else hi = mid;
+      for (int q = 0; q < IPT / 8; ++q) {
+        uint4 w;
+        w.x = idx[8 * q] | (unsigned)idx[8 * q + 1] << 16;
+        w.y = idx[8 * q + 2] | (unsigned)idx[8 * q + 3] << 16;
+        w.z = idx[8 * q + 4] | (unsigned)idx[8 * q + 5] << 16;
+        w.w = idx[8 * q + 6] | (unsigned)idx[8 * q + 7] << 16;
+        reinterpret_cast<uint4*>(s_idx + first)[q] = w;
       }
-      unsigned ai = lo, bi = d - lo;
-      // the two candidates stay in registers; only the side that was taken is read again
-      K cand_a = K(), cand_b = K();
-      unsigned short cand_ai = 0, cand_bi = 0;
-      if (ai < len) { const unsigned at = slot(a0 + ai); cand_a = s_key[at]; cand_ai = s_idx[at]; }
-      if (bi < len) { const unsigned at = slot(b0 + bi); cand_b = s_key[at]; cand_bi = s_idx[at]; }
+    } else {
 #pragma unroll
-      for (int i = 0; i < IPT; ++i) {
-        bool take_b;
-        if (bi >= len) take_b = false;
-        else if (ai >= len) take_b = true;
-        else take_b = before(cand_b, cand_bi, cand_a, cand_ai);
-        if (take_b) {
-          k[i] = cand_b; idx[i] = cand_bi;
-          ++bi;
-          if (bi < len) { const unsigned at = slot(b0 + bi); cand_b = s_key[at]; cand_bi = s_idx[at]; }
-        } else {
-          k[i] = cand_a; idx[i] = cand_ai;
-          ++ai;
-          if (ai < len) { const unsigned at = slot(a0 + ai); cand_a = s_key[at]; cand_ai = s_idx[at]; }
-        }
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < IPT; ++i) { stash(&s_key[first_slot + i], k[i]); s_idx[first_slot + i] = idx[i]; }
-    __syncthreads();
-    // gather the payloads by source index before anything is written: the output may be the input
-    [[maybe_unused]] V v_out[HAS_V ? IPT : 1];
-    if constexpr (HAS_V) {
-#pragma unroll
-      for (int i = 0; i < IPT; ++i) { unsigned c = threadIdx.x + i * MERGE_BLOCK; if (FULL || c < tile_n) v_out[i] = vals[base + s_idx[slot(c)]]; }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < IPT; ++i) {
-      unsigned c = threadIdx.x + i * MERGE_BLOCK;
-      if (FULL || c < tile_n) {
-        keys_out[base + c] = s_key[slot(c)];
-        if constexpr (HAS_V) vals_out[base + c] = v_out[i];
-      }
+      for (int i = 0; i < IPT; ++i) s_idx[first + i] = idx[i];
     }
   };
-  if (tile_n == (unsigned)TILE) sort_tile(std::true_type()); else sort_tile(std::false_type());
+  // ---- rounds of pairwise merges in shared memory
+  for (unsigned len = IPT; len < (unsigned)TILE; len <<= 1) {
+    const bool in_warp = 2 * len <= 32u * IPT;     // both runs are this warp's own items, in this round and the ones before
+    if (in_warp && len > (unsigned)IPT) __syncwarp(); else __syncthreads();
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) stash(&s_key[first_slot + i], k[i]);
+    put_idx();
+    if (in_warp) __syncwarp(); else __syncthreads();
+    const unsigned a0 = first & ~(2 * len - 1), b0 = a0 + len;
+    const unsigned an = a0 >= tile_n ? 0u : tile_n - a0 < len ? tile_n - a0 : len, bn = b0 >= tile_n ? 0u : tile_n - b0 < len ? tile_n - b0 : len;
+    unsigned d = first - a0;
+    if (d > an + bn) d = an + bn;
+    // merge path over the two runs (ties take from the left one)
+    unsigned lo = d > bn ? d - bn : 0, hi = d < an ? d : an;
+    while (lo < hi) {
+      const unsigned mid = (lo + hi) >> 1;
+      if (!comp(s_key[slot(b0 + d - 1 - mid)], s_key[slot(a0 + mid)])) lo = mid + 1; else hi = mid;
+    }
+    unsigned ai = a0 + lo, bi = b0 + (d - lo);
+    const unsigned a_end = a0 + an, b_end = b0 + bn;
+    // the two candidates stay in registers; only the side that was taken is read again, always: past a run's end that is some
+    // slot of the tile which nothing looks at
+    K key_a = K(), key_b = K();
+    if (std::is_trivially_copyable<K>::value || ai < a_end) key_a = s_key[slot(ai)];
+    if (std::is_trivially_copyable<K>::value || bi < b_end) key_b = s_key[slot(bi)];
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) {
+      const bool take_b = bi < b_end && (ai >= a_end || comp(key_b, key_a));
+      idx[i] = s_idx[take_b ? bi : ai];
+      k[i] = take_b ? key_b : key_a;
+      ai += take_b ? 0u : 1u;
+      bi += take_b ? 1u : 0u;
+      if (std::is_trivially_copyable<K>::value || (take_b ? bi < b_end : ai < a_end)) {
+        const K next = s_key[slot(take_b ? bi : ai)];
+        key_b = take_b ? next : key_b;
+        key_a = take_b ? key_a : next;
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) stash(&s_key[first_slot + i], k[i]);
+  put_idx();
+  __syncthreads();
+  // gather the payloads by source index before anything is written: the output may be the input
+  [[maybe_unused]] V v_out[HAS_V ? IPT : 1];
+  if constexpr (HAS_V) {
+#pragma unroll
+    for (int i = 0; i < IPT; ++i) { const unsigned c = threadIdx.x + i * BLOCK; if (c < tile_n) v_out[i] = vals[base + s_idx[c]]; }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < IPT; ++i) {
+    const unsigned c = threadIdx.x + i * BLOCK;
+    if (c < tile_n) {
+      keys_out[base + c] = s_key[slot(c)];
+      if constexpr (HAS_V) vals_out[base + c] = v_out[i];
+    }
+  }
 }
 
-template <class K, class V, bool HAS_V> constexpr int block_sort_tile_items() { return MERGE_BLOCK * block_sort_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>::IPT; }
+template <class K, class V, bool HAS_V> constexpr int block_sort_tile_items() { return block_sort_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>::TILE; }
 
 template <class K, class V, bool HAS_V> size_t merge_sort_workspace_bytes(size_t n) { return merge_workspace_bytes<K, V, HAS_V>(n); }
 
@@ -656,7 +683,8 @@ template <class K, class V, bool HAS_V> size_t merge_sort_workspace_bytes(size_t
 template <class K, class V, bool HAS_V, class Comp>
 cudaError_t merge_sort_async(K* keys, K* keys_alt, V* vals, V* vals_alt, size_t n, Comp comp, void* ws, cudaStream_t stream) {
   constexpr int BS_IPT = block_sort_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>::IPT;
-  constexpr size_t BS_TILE = (size_t)MERGE_BLOCK * BS_IPT;
+  using Tuning = block_sort_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>;
+  constexpr size_t BS_TILE = (size_t)Tuning::TILE;
   cudaError_t e = cudaMemsetAsync(ws, 0, sizeof(ws_header), stream);
   if (e != cudaSuccess || n <= 1) return e;
   const size_t tiles = (n + BS_TILE - 1) / BS_TILE;
@@ -668,8 +696,8 @@ cudaError_t merge_sort_async(K* keys, K* keys_alt, V* vals, V* vals_alt, size_t 
   K* oth_k = (passes & 1) ? keys : keys_alt;
   V* oth_v = (passes & 1) ? vals : vals_alt;
   { timed_launch tl(KID_BLOCK_SORT, stream);
-  block_sort_kernel<const K*, const V*, K*, V*, K, V, HAS_V, Comp, BS_IPT><<<(unsigned)tiles, MERGE_BLOCK, 0, stream>>>(keys, vals, cur_k, cur_v, n, comp); }
-  log_launch("block_sort_kernel", tiles, MERGE_BLOCK, 0, n, stream);
+  block_sort_kernel<const K*, const V*, K*, V*, K, V, HAS_V, Comp, BS_IPT><<<(unsigned)tiles, Tuning::BLOCK, 0, stream>>>(keys, vals, cur_k, cur_v, n, comp); }
+  log_launch("block_sort_kernel", tiles, Tuning::BLOCK, 0, n, stream);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   for (size_t run = BS_TILE; run < n; run <<= 1) {
     e = merge_pass_async<K, V, HAS_V>((const K*)cur_k, (const K*)cur_k, (const V*)cur_v, (const V*)cur_v, oth_k, oth_v,
