@@ -16,8 +16,8 @@
 // were two thirds of a pass: about 1.7 cycles each per SM.)  A digit place that all keys share is left out,
 // as in the general sort.  Same order, same stability.
 //
-// Measured on B200, microseconds here / on the general route, at 1 k, 32 k and 64 k items: u32 + u32 17 / 51, 27 / 53, 35 / 54;
-// f32 keys 16 / 53, 23 / 55, 33 / 57; u64 + u64 31 / 66, 54 / 83, 80 / 85.  csort_max_items says where it stops.
+// Measured on B200, microseconds: f32 keys 22 at 1 k, 26 at 10 k, 30 at 32 k; u32 + u32 23, 30, 36; u64 + u64 35, 44, 58.  CSORT_MAX_ITEMS says
+// where it stops.
 #pragma once
 #include "cluster.cuh"
 #include "common.cuh"
@@ -27,7 +27,7 @@ namespace tb200 {
 
 constexpr int CSORT_BLOCK = 512;
 constexpr int CSORT_MAX_CTAS = CLUSTER_MAX_CTAS;
-constexpr int CSORT_MAX_IPT = 16;
+constexpr int CSORT_MAX_IPT = 4;
 
 // What moves between the CTAs: a key alone, or a key and its value in one 8- or 16-byte word.
 template <class UK, class UV, bool HAS_V> struct csort_item { using type = UK; };
@@ -35,15 +35,9 @@ template <class UK, class UV> struct csort_item<UK, UV, true> {
   struct alignas(sizeof(UK) + sizeof(UV) <= 8 ? 8 : 16) type { UV v; UK k; };
 };
 
-// Up to how many items the cluster is the faster route: rows per warp of the largest cluster.  Microseconds here / on the
-// general route on either side of each line: u32 keys 49 / 54 and f32 50 / 57 at 128 k (as many as fit); u32 + u32 53 / 54 at
-// 112 k, 59 / 54 at 128 k; u16 + u32 29 / 31 at 96 k, 33 / 32 at 112 k; u8 + u32 19 / 24 at 128 k; u64 keys 79 / 86 at 80 k, 88 / 86 at
-// 96 k.  Pairs of 16 bytes stop at 64 k, where the staged copy and the cluster's fill shared memory (u64 + u32 84 / 94,
-// u64 + u64 80 / 85, u32 + u64 45 / 52).
-template <class UK, class UV, bool HAS_V> constexpr size_t csort_max_items() {
-  constexpr size_t item = sizeof(typename csort_item<UK, UV, HAS_V>::type), row = (size_t)CSORT_BLOCK * CSORT_MAX_CTAS;
-  return row * (item > 8 ? 8 : item < 8 ? CSORT_MAX_IPT : !HAS_V ? 11 : sizeof(UK) == 1 ? CSORT_MAX_IPT : 14);
-}
+// Up to how many items the cluster is the faster route: four rows per warp of the largest one.  Microseconds here / in the grid sort at 20 k,
+// 32 k and 50 k: f32 keys 29 / 36, 30 / 35, 36 / 37; u32 + u32 32 / 36, 36 / 33, 43 / 37; u64 + u32 50 / 61, 56 / 57, 73 / 65.
+constexpr size_t CSORT_MAX_ITEMS = (size_t)CSORT_BLOCK * CSORT_MAX_CTAS * CSORT_MAX_IPT;
 
 template <class Item, int IPT> constexpr size_t csort_smem_bytes() {
   return 2 * (size_t)CSORT_BLOCK * IPT * sizeof(Item) + (CSORT_BLOCK / 32) * RADIX_BINS * 4 + 2 * CSORT_MAX_CTAS * RADIX_BINS * 4;
@@ -102,23 +96,10 @@ cluster_sort_kernel(UK* keys, UV* vals, unsigned n, unsigned rows, key_coding co
     __syncthreads();
     if (!started) { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); started = true; }
     unsigned* const table = counts + parity * (CSORT_MAX_CTAS * RADIX_BINS);
-    unsigned run = 0, local = 0;
-    if (t < RADIX_BINS) {
-#pragma unroll
-      for (int w = 0; w < NWARPS; ++w) { const unsigned c = warp_hist[w * RADIX_BINS + t]; warp_hist[w * RADIX_BINS + t] = run; run += c; }
+    const unsigned local = stack_digits<NWARPS>(warp_hist, s_scan[0], [&](unsigned count) {
       const unsigned at = smem_addr(table + me * RADIX_BINS + t);
-      for (unsigned q = 0; q < ctas; ++q) cluster_store(cluster_addr(at, q), run);
-      local = warp_inclusive_scan(run, plus_op());
-      if (lane == 31) s_scan[0][warp] = local;
-      local -= run;
-    }
-    __syncthreads();
-    if (t < RADIX_BINS) {
-      for (int w = 0; w < warp; ++w) local += s_scan[0][w];
-#pragma unroll
-      for (int w = 0; w < NWARPS; ++w) warp_hist[w * RADIX_BINS + t] += local;
-    }
-    __syncthreads();
+      for (unsigned q = 0; q < ctas; ++q) cluster_store(cluster_addr(at, q), count);
+    });
 #pragma unroll
     for (int i = 0; i < IPT; ++i) {
       if ((unsigned)i < rows && wofs + i * 32 < mine) {
@@ -130,6 +111,7 @@ cluster_sort_kernel(UK* keys, UV* vals, unsigned n, unsigned rows, key_coding co
     cluster_barrier();     // the tables are complete, and every CTA holds its items in registers and s_stage
     unsigned total = 0, before = 0, incl = 0;
     if (t < RADIX_BINS) {
+#pragma unroll 4
       for (unsigned q = 0; q < ctas; ++q) { const unsigned c = table[q * RADIX_BINS + t]; if (q < me) before += c; total += c; }
       incl = warp_inclusive_scan(total, plus_op());
       if (lane == 31) s_scan[1][warp] = incl;
@@ -138,7 +120,8 @@ cluster_sort_kernel(UK* keys, UV* vals, unsigned n, unsigned rows, key_coding co
     if (__syncthreads_or(shared_digit)) continue;   // every key has this digit: nothing moves
     if (t < RADIX_BINS) {
       unsigned off = incl - total + before - local;   // from this CTA's staged order to the cluster's
-      for (int w = 0; w < warp; ++w) off += s_scan[1][w];
+#pragma unroll
+      for (int w = 0; w < RADIX_BINS / 32; ++w) { const unsigned x = s_scan[1][w]; off += w < warp ? x : 0u; }
       s_goff[t] = off;
     }
     __syncthreads();
@@ -191,19 +174,11 @@ cudaError_t cluster_sort_launch(UK* keys, UV* vals, size_t n, key_coding coding,
 template <class UK, class UV, bool HAS_V>
 cudaError_t cluster_sort_async(UK* keys, UV* vals, size_t n, key_coding coding, int first_pass, int num_passes, ws_header* hdr, cudaStream_t stream, bool& launched) {
   launched = false;
-  if (n > csort_max_items<UK, UV, HAS_V>()) return cudaSuccess;
-  auto go = [&](auto is_float, auto ipt) {
-    return cluster_sort_launch<UK, UV, HAS_V, decltype(is_float)::value, decltype(ipt)::value>(keys, vals, n, coding, first_pass, num_passes, hdr, stream, launched);
-  };
-  auto by_size = [&](auto is_float) {
-    if (n <= (size_t)CSORT_BLOCK * CSORT_MAX_CTAS * 4) return go(is_float, std::integral_constant<int, 4>());
-    if (n <= (size_t)CSORT_BLOCK * CSORT_MAX_CTAS * 8) return go(is_float, std::integral_constant<int, 8>());
-    // a pair in 16 bytes: the staged copy and the cluster's would not fit
-    if constexpr (sizeof(typename csort_item<UK, UV, HAS_V>::type) <= 8) return go(is_float, std::integral_constant<int, 16>());
-    return cudaSuccess;
-  };
-  if constexpr (sizeof(UK) >= 4) { if (coding.kind == KEY_FLOAT) return by_size(std::true_type()); }
-  return by_size(std::false_type());
+  if (n > CSORT_MAX_ITEMS) return cudaSuccess;
+  if constexpr (sizeof(UK) >= 4) {
+    if (coding.kind == KEY_FLOAT) return cluster_sort_launch<UK, UV, HAS_V, true, CSORT_MAX_IPT>(keys, vals, n, coding, first_pass, num_passes, hdr, stream, launched);
+  }
+  return cluster_sort_launch<UK, UV, HAS_V, false, CSORT_MAX_IPT>(keys, vals, n, coding, first_pass, num_passes, hdr, stream, launched);
 }
 
 }  // namespace tb200

@@ -28,12 +28,13 @@ template <class UK> __host__ __device__ __forceinline__ unsigned digit_mask(key_
   if (c.kind != KEY_UNSIGNED) m ^= (UK)1 << (B - 1);
   return (unsigned)(m >> shift) & 0xffu;
 }
-template <bool IS_FLOAT, class UK> __device__ __forceinline__ unsigned key_digit(UK k, int shift, unsigned dmask) {
+template <class UK> __device__ __forceinline__ UK float_digits(UK k) {   // negative: flip the non-sign bits too
   constexpr int B = 8 * sizeof(UK);
-  if (IS_FLOAT) {
-    using SK = typename std::make_signed<UK>::type;
-    k ^= (UK)((SK)k >> (B - 1)) & (UK)~((UK)1 << (B - 1));   // negative: flip the non-sign bits too
-  }
+  using SK = typename std::make_signed<UK>::type;
+  return k ^ ((UK)((SK)k >> (B - 1)) & (UK)~((UK)1 << (B - 1)));
+}
+template <bool IS_FLOAT, class UK> __device__ __forceinline__ unsigned key_digit(UK k, int shift, unsigned dmask) {
+  if (IS_FLOAT) k = float_digits(k);
   return ((unsigned)(k >> shift) & 0xffu) ^ dmask;
 }
 
@@ -74,6 +75,35 @@ template <int BITS> __device__ __forceinline__ unsigned warp_rank(unsigned* coun
     rank = now - __popc(peers & lanemask_ge);
   }
   return rank;
+}
+
+// Turns per-warp digit counts into places, by the first 256 threads of a CTA (thread t: digit t); two barriers of the CTA lie inside, so
+// every thread calls it.  hist: [WARPS][256], on return each warp's first place of each digit inside the CTA.  publish(count) is called
+// with the CTA's count of the digit as soon as that is known; returns the digit's first place.  All loads of a step are
+// issued before the first result is used: one after the other they are much of a small sort's digit place.
+template <int WARPS, class Publish>
+__device__ __forceinline__ unsigned stack_digits(unsigned* hist, unsigned (&s_scan)[RADIX_BINS / 32], Publish publish) {
+  const int t = threadIdx.x, warp = t >> 5;
+  unsigned first[WARPS], run = 0, place = 0;
+  if (t < RADIX_BINS) {
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) first[w] = hist[w * RADIX_BINS + t];
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) { const unsigned c = first[w]; first[w] = run; run += c; }
+    publish(run);
+    place = warp_inclusive_scan(run, plus_op());
+    if (lane_id() == 31) s_scan[warp] = place;
+    place -= run;
+  }
+  __syncthreads();
+  if (t < RADIX_BINS) {
+#pragma unroll
+    for (int w = 0; w < RADIX_BINS / 32; ++w) { const unsigned c = s_scan[w]; place += w < warp ? c : 0u; }
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) hist[w * RADIX_BINS + t] = first[w] + place;
+  }
+  __syncthreads();
+  return place;
 }
 
 }  // namespace tb200

@@ -22,10 +22,12 @@
 //   4. radix_copy_back_kernel only if an odd number of places ran: moves the result from the
 //                             alternate buffer to the caller's.
 // A pass therefore reads and writes each key (and value) exactly once.  The sort is stable.
-// Inputs of up to 128 k items take one launch of one thread-block cluster instead (cluster_sort.cuh).
+// Inputs of up to 32 k items take one launch of one thread-block cluster instead (cluster_sort.cuh), up to 448 k one cooperative launch
+// (grid_sort.cuh).
 #pragma once
 #include "cluster_sort.cuh"
 #include "common.cuh"
+#include "grid_sort.cuh"
 #include "radix_keys.cuh"
 
 namespace tb200 {
@@ -707,7 +709,9 @@ template <int KB, int VB> size_t onesweep_smem_bytes() {
 template <int KB, int VB> size_t sweep_tiles_of(size_t n) { return (n + onesweep_tile_items<KB, VB>() - 1) / onesweep_tile_items<KB, VB>(); }
 template <int KB, int VB> size_t radix_workspace_bytes(size_t n) {
   size_t lb_word = n < (1ull << 30) ? 4 : 8;
-  return sizeof(ws_header) + sizeof(radix_ctrl) + align_up(sweep_tiles_of<KB, VB>(n) * RADIX_BINS * lb_word, 256) * KB;
+  const size_t sweeps = sizeof(radix_ctrl) + align_up(sweep_tiles_of<KB, VB>(n) * RADIX_BINS * lb_word, 256) * KB;
+  const size_t resident = gsort_workspace_bytes<KB, VB>(n);
+  return sizeof(ws_header) + (sweeps > resident ? sweeps : resident);
 }
 
 // Sorts keys (and values) held in keys_a / vals_a, in place from the caller's point of view:
@@ -727,11 +731,13 @@ cudaError_t radix_sort_async(UK* keys_a, UK* keys_b, UV* vals_a, UV* vals_b, siz
   const size_t lb_bytes = align_up(sweep_tiles_of<KB, VB>(n) * RADIX_BINS * (lb32 ? 4 : 8), 256);
   char* base = static_cast<char*>(ws);
   ws_header* hdr = reinterpret_cast<ws_header*>(base);
-  // small inputs: one launch of one cluster
+  // small inputs: one launch of one cluster or of a resident grid
   {
     bool launched = false;
     const cudaError_t ce = cluster_sort_async<UK, UV, HAS_V>(keys_a, vals_a, n, coding, first_pass, num_passes, hdr, stream, launched);
     if (launched || ce != cudaSuccess) return ce;
+    const cudaError_t ge = grid_sort_async<UK, UV, HAS_V>(keys_a, vals_a, n, coding, first_pass, num_passes, hdr, stream, launched);
+    if (launched || ge != cudaSuccess) return ge;
   }
   radix_ctrl* ctrl = reinterpret_cast<radix_ctrl*>(base + sizeof(ws_header));
   char* lb0 = base + sizeof(ws_header) + sizeof(radix_ctrl);

@@ -429,19 +429,8 @@ inline cudaError_t pipe_clear(void* ws, size_t bytes, cudaStream_t stream) {
   return e;
 }
 
-// Cooperative, so that the CTAs of a round are all resident whatever else runs on the device.
 template <class... Params, class... Args> cudaError_t pipe_launch(void (*kernel)(Params...), size_t grid, size_t smem, cudaStream_t stream, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(PIPE_BLOCK);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+  return cooperative_launch(kernel, grid, PIPE_BLOCK, smem, stream, args...);
 }
 
 }  // namespace tb200
