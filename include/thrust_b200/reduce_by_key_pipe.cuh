@@ -111,7 +111,6 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
   pipe_init(st);
   const int lane = lane_id(), warp = threadIdx.x >> 5;
 
-  __shared__ K s_last[PIPE_STAGES][PIPE_WARPS];         // the last key of each warp's part
   // the fold of the parts held by lanes 0 ... PIPE_WARPS - 1, in order; result in lane 0
   auto fold_parts = [&](C t) {
 #pragma unroll
@@ -152,9 +151,10 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
     auto tile_front = [&](unsigned s, unsigned tile) {
       return tile > 0 ? reinterpret_cast<const K*>(&s_edge[s])[16 / sizeof(K) - 1] : Shape::Keys::part(stages + s * Shape::STAGE_BYTES, 0)[0];
     };
-    // this lane's items and their head flags, bit v * VEC + k; items past the end are no heads and hold the identity;
-    // `edge`: the key in front of the warp's part
-    auto load_heads = [&](unsigned s, unsigned tile, const K& edge, K (&k)[ROWS][VEC], V (&x)[ROWS][VEC]) {
+    // this lane's items, and their head flags (bit v * VEC + k, held from a tile's summary to its end: 2^27 u32 + f32 352 us, 368 with the
+    // flags found twice); items past the end are no heads and hold the identity; `edge`: the key in front of the warp's part
+    open_words head_words;
+    auto load_items = [&](unsigned s, K (&k)[ROWS][VEC], V (&x)[ROWS][VEC]) {
       const K* kp = Shape::Keys::part(stages + s * Shape::STAGE_BYTES, mine);
       const V* vp = Shape::Vals::part(stages + s * Shape::STAGE_BYTES + Shape::Keys::BYTES, mine);
 #pragma unroll
@@ -162,6 +162,18 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
         lane_items<K, VEC>(kp + (v * 32 + lane) * VEC, k[v]);
         lane_items<V, VEC>(vp + (v * 32 + lane) * VEC, x[v]);
       }
+    };
+    // items past the end hold the identity
+    auto blank_past_end = [&](unsigned tile, V (&x)[ROWS][VEC]) {
+      const size_t first = (size_t)tile * ITEMS + (size_t)mine * PART;
+      if (first + PART <= n) return;
+#pragma unroll
+      for (int v = 0; v < ROWS; ++v) {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) if (first + (size_t)(v * 32 + lane) * VEC + j >= n) x[v][j] = ID;
+      }
+    };
+    auto heads_of = [&](unsigned tile, const K& edge, const K (&k)[ROWS][VEC]) {
       const size_t first = (size_t)tile * ITEMS + (size_t)mine * PART;
       unsigned bits = 0;
       auto scan_heads = [&](auto whole_tag) {
@@ -175,7 +187,6 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
           for (int j = 0; j < VEC; ++j) {
             const bool in = WHOLE || first + (size_t)(v * 32 + lane) * VEC + j < n;
             if (in && !eq(j == 0 ? prev : k[v][j > 0 ? j - 1 : 0], k[v][j])) bits |= 1u << (v * VEC + j);
-            if (!in) x[v][j] = ID;
           }
         }
       };
@@ -197,8 +208,10 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
         // nobody compacts its part of this tile before every warp has been here
         unsigned char* const kstage = stages + s * Shape::STAGE_BYTES;
         const K edge = mine > 0 ? Shape::Keys::part(kstage, mine > 0 ? mine - 1 : 0)[PART - 1] : tile_front(s, tile);
-        if (lane == 0) s_last[s][mine] = Shape::Keys::part(kstage, mine)[PART - 1];
-        const unsigned bits = load_heads(s, tile, edge, k, x);
+        load_items(s, k, x);
+        blank_past_end(tile, x);
+        const unsigned bits = heads_of(tile, edge, k);
+        head_words.put(bits);
         // only what lies behind the part's last head counts: later rows entirely, the head's row from the head's lane on
         V open = ID;
         bool live = true;   // no head behind the current row
@@ -219,8 +232,9 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
       },
       [&](unsigned s, unsigned tile) {
         K k[ROWS][VEC]; V x[ROWS][VEC];
-        const K edge = mine > 0 ? s_last[s][mine > 0 ? mine - 1 : 0] : tile_front(s, tile);
-        const unsigned bits = load_heads(s, tile, edge, k, x);
+        load_items(s, k, x);
+        blank_past_end(tile, x);
+        const unsigned bits = head_words.take();
         K* const kbuf = Shape::Keys::part(stages + s * Shape::STAGE_BYTES, mine);
         V* const vbuf = Shape::Vals::part(stages + s * Shape::STAGE_BYTES + Shape::Keys::BYTES, mine);
         __syncwarp();   // every lane has its items: the parts may be overwritten
@@ -236,8 +250,7 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
         const unsigned incl = warp_inclusive_scan(packed, plus_op());
         const unsigned totals = __shfl_sync(FULL_MASK, incl, 31);
         const unsigned excl = incl - packed;
-        // what is stored now is what was counted then, and lies inside the outputs (an equality that does not answer the
-        // same twice is reported and nothing is stored)
+        // what is stored lies inside the outputs (a broken carry is reported and nothing is stored)
         const unsigned part_heads = __reduce_add_sync(FULL_MASK, (unsigned)__popc(bits));
         if (part_heads != st.part[s][mine].heads || run0 > (size_t)tile * ITEMS + (size_t)mine * PART) {
           if (lane == 0) record_error(&rep->error, ERR_INCONSISTENT);

@@ -376,6 +376,15 @@ __device__ __forceinline__ void pipe_compute(S& st, unsigned tiles, unsigned* er
   }
 }
 
+// A word per lane for each of a warp's open tiles, kept from a tile's summary to its end: tiles are finished in the order in which
+// they were summarised, at most PIPE_LOOKAHEAD + 1 are open.
+struct open_words {
+  static_assert(PIPE_LOOKAHEAD == 1, "two tiles are open at most");
+  unsigned even = 0, odd = 0, put_at = 0, taken = 0;
+  __device__ __forceinline__ void put(unsigned w) { if (put_at & 1) odd = w; else even = w; ++put_at; }
+  __device__ __forceinline__ unsigned take() { return taken++ & 1 ? odd : even; }
+};
+
 // Compacted output, by one warp: a run of items staged at the same distance from a 16-byte boundary as its
 // place in the output leaves in 16-byte stores.  run_shift(dst): that distance in items.
 template <class T> __device__ __forceinline__ unsigned run_shift(const T* dst) { return (unsigned)(reinterpret_cast<uintptr_t>(dst) & 15) / sizeof(T); }
