@@ -246,3 +246,31 @@ def test_small_sorts_where_the_cluster_hands_over(tb, port, n):
             tb.sort(kd) if v is None else tb.sort_by_key(kd, vd)
             ok, ov = port.sort_by_key(k, v, False)
             assert np.array_equal(host(kd), ok) and (v is None or np.array_equal(host(vd), ov)), (dt, vt, small)
+
+
+@pytest.mark.parametrize("n", [(1 << 26) - 1, 1 << 26, (1 << 26) + 9215, 9216 * 7300 + 1])
+def test_pairs_around_the_size_of_larger_tiles(tb, n):
+    """4-byte pairs from 2^26 on are sorted in tiles of 9216 items; whole tiles, a tile less one, one more."""
+    keys = torch.randint(-(1 << 31), (1 << 31) - 1, (n,), device="cuda", dtype=torch.int32)
+    k, v = keys.clone().view(torch.uint32), torch.arange(n, device="cuda", dtype=torch.int32).view(torch.uint32)
+    tb.sort_by_key(k, v)
+    k, v = k.view(torch.int32), v.view(torch.int32)
+    assert torch.equal(keys[v.long()], k)
+    u = k ^ torch.tensor(-(1 << 31), dtype=torch.int32, device="cuda")         # unsigned order as signed order
+    assert bool(((u[1:] > u[:-1]) | ((u[1:] == u[:-1]) & (v[1:] > v[:-1]))).all())
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+def test_an_odd_number_of_places_comes_back_from_any_address(tb, port, shift):
+    """Three digit places move, so the result is copied back: 16 bytes at a time where both sides allow it.  The high places of 8-byte
+    keys are shared by all keys, or by all but one."""
+    n = 700001
+    k64 = dg.rand64(81, n) >> np.uint64(40)
+    odd_one = k64.copy()
+    odd_one[n // 2] = np.uint64(1) << np.uint64(63)
+    for k, vt in [(k64, np.uint32), (odd_one, np.uint64), (k64.astype(np.uint32), np.uint32), (k64.astype(np.float32), np.uint32), ((k64 | np.uint64(1 << 60)).view(np.int64), np.uint64)]:
+        v = np.arange(n, dtype=vt)
+        dk, dv = misaligned(k, shift), misaligned(v, shift)
+        tb.sort_by_key(dk, dv)
+        wk, wv = port.sort_by_key(k, v)
+        assert np.array_equal(host(dk), wk) and np.array_equal(host(dv), wv), (k.dtype, vt)
