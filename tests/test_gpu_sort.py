@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from thrust_b200 import datagen as dg
-from gpu_util import EDGE_SIZES, dev, host, rand_of
+from gpu_util import EDGE_SIZES, dev, host, misaligned, rand_of
 
 pytestmark = pytest.mark.gpu
 KEY_TYPES = [np.int8, np.uint8, np.int16, np.uint16, np.int32, np.uint32, np.float32, np.int64, np.uint64, np.float64]
