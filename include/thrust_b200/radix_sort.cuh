@@ -97,8 +97,9 @@ radix_hist_kernel(const UK* keys, size_t n, key_coding coding, int first_pass, i
 #pragma unroll
       for (int k = 0; k < VEC; ++k) { x[u * VEC + k] = digits_of(e[k]); differ |= (UK)(x[u * VEC + k] ^ x[0]); }
     }
-    // Of 8-byte keys a digit place that the thread's keys share (the high bytes of packed ids, say) is one increment (20 M
-    // u64 + u32 pairs of 40 random bits 845 -> 807 us together with the copy back's wider pieces).  For 4-byte keys the look costs more than it saves (2^28 random pairs sorted in 5.37 ms against 5.34).
+    // Of 8-byte keys a digit place that the thread's keys share (the high bytes of packed ids, say) is one increment (20 M u64 + u32 pairs
+    // of 40 random bits 845 -> 807 us together with the copy back's wider pieces).  For 4-byte keys the look costs more than it
+    // saves (2^28 random pairs sorted in 5.37 ms against 5.34).
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       if (sizeof(UK) == 8 && ((unsigned)(differ >> (p * RADIX_BITS)) & 0xffu) == 0) {
