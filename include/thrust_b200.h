@@ -56,11 +56,13 @@ int tb200_workspace_status(const void* d_ws, tb200_stream_t stream, unsigned* h_
  * and this read together (a lock, as the Python layer holds): the header is the last call's. */
 int tb200_workspace_read(const void* d_ws, size_t bytes, void* h_dst, tb200_stream_t stream);
 
-/* Announces tb200_workspace_read(d_ws, ...) by this thread behind the one call that it makes next with workspace d_ws.  Status, count and a
- * result that tb200_reduce was told to leave in the header may then go to pinned host memory instead of the header while
- * the kernels run, and the read is a wait for the stream without a copy; other calls' status and count go to their
- * headers as ever, and so do an announced call's where its kernels cannot do it.  NULL withdraws the announcement (the call failed).  Not for a
- * call that is captured into a graph. */
+/* Announces tb200_workspace_read(d_ws, ...) by this thread behind the one call that it makes next with workspace d_ws.  That call's status,
+ * count and a result that tb200_reduce was told to leave at d_ws + 32 may then go to pinned host memory while the kernels
+ * run, and the read is a wait for the stream without a copy.  Count and result are in the header as well; the status is found by
+ * tb200_workspace_read and tb200_workspace_status in this thread.  The announcement ends with that read, with the next call on
+ * d_ws (which reports to the header, as calls on other workspaces do all along), or with the next announcement; NULL withdraws it (the call
+ * failed).  The status of an announced call that ends unread is lost.  A call that is captured into a graph reports to its
+ * header, announced or not. */
 int tb200_workspace_watch(const void* d_ws);
 
 /* thrust::reduce(first, last, init, op) -- thrust/system/cuda/detail/reduce.h:1015-1067

@@ -166,7 +166,7 @@ cudaError_t cluster_sort_launch(UK* keys, UV* vals, size_t n, key_coding coding,
   timed_launch tl(KID_ONESWEEP, stream);
   const cudaError_t e = cluster_launch(kern, ctas, CSORT_BLOCK, smem, stream, largest, launched, keys, vals, (unsigned)n, rows, coding, first_pass, num_passes, hdr);
   if (!launched) return e;
-  reported(report_of(hdr), hdr);   // nothing to report: no wait of this kernel runs out
+  reported(e, report_of(hdr, stream), hdr);   // nothing to report: no wait of this kernel runs out
   log_launch("cluster_sort_kernel", ctas, CSORT_BLOCK, smem, n, stream);
   return e;
 }

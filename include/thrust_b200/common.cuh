@@ -70,15 +70,26 @@ static_assert(sizeof(ws_header) == 256, "workspace header is 256 bytes");
 // workspace beforehand (tb200_workspace_watch, in the thread that makes the call), and the kernels then write status and count to a block of
 // pinned host memory instead of the header, so that the wait for the stream is all there is left to do: fetching 16 bytes
 // with a copy took 5 us of the 14.8 that clearing, a one-CTA kernel, that copy and the wait take together.
+// Counts and results go to the header as well; the status of an announced call is only in the block.
 struct host_report {
   const void* ws = nullptr;      // the watched workspace
   ws_header* block = nullptr;    // pinned, mapped, a header's layout
-  bool served = false;           // kernels that write to `block` were launched
+  bool begun = false;            // the call that was announced has begun; the next one on `ws` is not announced
+  size_t bytes = 0;              // how much of a header's front the launched kernels leave in `block` (0: none was launched)
 };
 inline host_report& thread_report() { static thread_local host_report r; return r; }
-// the header to which kernels launched on workspace `hdr` report, and the note that they were launched
-inline ws_header* report_of(ws_header* hdr) { const host_report& r = thread_report(); return r.ws == hdr && r.block ? r.block : hdr; }
-inline void reported(const ws_header* rep, const ws_header* hdr) { if (rep != hdr) thread_report().served = true; }
+// The header to which kernels launched on workspace `hdr` report: a captured launch may run again at any time, so it reports to the
+// workspace.  reported(): they were launched with result `e` and leave the first `bytes` bytes of a header there.
+inline ws_header* report_of(ws_header* hdr, cudaStream_t stream) {
+  const host_report& r = thread_report();
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (r.ws != hdr || !r.block || cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return hdr;
+  return r.block;
+}
+inline cudaError_t reported(cudaError_t e, const ws_header* rep, const ws_header* hdr, size_t bytes = offsetof(ws_header, ticket2)) {
+  if (e == cudaSuccess && rep != hdr && thread_report().bytes < bytes) thread_report().bytes = bytes;
+  return e;
+}
 
 #ifdef TB200_TEST_HOOKS
 // Test builds only: a process-wide switch.  Bits 0 and 1 are copied into the workspace header's flags (0: tile 0 of the

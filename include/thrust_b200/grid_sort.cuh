@@ -193,12 +193,12 @@ cudaError_t grid_sort_launch(UK* keys, UV* vals, size_t n, unsigned ctas, unsign
   if (e == cudaSuccess) e = cudaMemsetAsync(&hdr->flags, (int)(test_hook_flags() & 1u), 1, stream);
 #endif
   if (e != cudaSuccess) return e;
-  ws_header* const rep = report_of(hdr);
+  ws_header* const rep = report_of(hdr, stream);
   timed_launch tl(KID_ONESWEEP, stream);
   e = cooperative_launch(kern, ctas, GSORT_BLOCK, smem, stream, keys, vals, (unsigned)n, rows, coding, first_pass, num_passes,
                          reinterpret_cast<unsigned short*>(hdr + 1), hdr, rep);
   if (launch_refused(e)) return cudaSuccess;
-  reported(rep, hdr);
+  reported(e, rep, hdr);
   launched = true;
   log_launch("grid_sort_kernel", ctas, GSORT_BLOCK, smem, n, stream);
   return e;

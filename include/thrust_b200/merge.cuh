@@ -486,8 +486,8 @@ cudaError_t merge_pass_async(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutI
   constexpr int TILE = MERGE_BLOCK * IPT;
   if (g.n == 0) return cudaSuccess;
   size_t* a_split = reinterpret_cast<size_t*>(static_cast<char*>(ws) + sizeof(ws_header));
-  ws_header* const rep = report_of(static_cast<ws_header*>(ws));
-  reported(rep, static_cast<ws_header*>(ws));
+  ws_header* const hdr = static_cast<ws_header*>(ws);
+  ws_header* const rep = report_of(hdr, stream);
   if constexpr (merge_slices_ok<K, V, HAS_V, KeyItA, KeyItB, ValItA, ValItB, KeyOutIt, ValOutIt>::value) {
     using Tuning = merge_slices_tuning<sizeof(K), HAS_V ? sizeof(V) : 0>;
     g.cut(Tuning::TILE);
@@ -506,12 +506,12 @@ cudaError_t merge_pass_async(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutI
       const cudaError_t le = launch_after(merge_slices_kernel<K, V, HAS_V, Comp>, tiles, MERGE_BLOCK, 0, stream, ka, kb, va, vb, ko, vo, g, comp,
                                           (const size_t*)a_split, &rep->error);
       log_launch("merge_slices_kernel", tiles, MERGE_BLOCK, 0, g.n, stream);
-      return le;
+      return reported(le, rep, hdr);
     }
     timed_launch tl(KID_MERGE, stream);
     merge_slices_kernel<K, V, HAS_V, Comp><<<tiles, MERGE_BLOCK, 0, stream>>>(ka, kb, va, vb, ko, vo, g, comp, a_split, &rep->error);
     log_launch("merge_slices_kernel", tiles, MERGE_BLOCK, 0, g.n, stream);
-    return cudaGetLastError();
+    return reported(cudaGetLastError(), rep, hdr);
   } else {
   g.cut(TILE);
   const size_t tiles = g.num_tiles();
@@ -520,7 +520,7 @@ cudaError_t merge_pass_async(KeyItA ka, KeyItB kb, ValItA va, ValItB vb, KeyOutI
   merge_kernel<KeyItA, KeyItB, ValItA, ValItB, KeyOutIt, ValOutIt, K, V, HAS_V, Comp, IPT>
       <<<(unsigned)tiles, MERGE_BLOCK, 0, stream>>>(ka, kb, va, vb, ko, vo, g, comp, a_split, &rep->error);
   log_launch("merge_kernel", tiles, MERGE_BLOCK, 0, g.n, stream);
-  return cudaGetLastError();
+  return reported(cudaGetLastError(), rep, hdr);
   }
 }
 

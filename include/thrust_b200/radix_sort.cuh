@@ -803,8 +803,7 @@ cudaError_t radix_sort_async(UK* keys_a, UK* keys_b, UV* vals_a, UV* vals_b, siz
     // persistent CTAs, two resident per SM; tiles are handed out by ticket
     const size_t tiles_all = (n + ONESWEEP_BLOCK * IPT - 1) / (ONESWEEP_BLOCK * IPT);
     const unsigned grid = (unsigned)(tiles_all < (size_t)di.sm_count * ONESWEEP_CTAS_PER_SM ? tiles_all : (size_t)di.sm_count * ONESWEEP_CTAS_PER_SM);
-    ws_header* const rep = report_of(hdr);
-    reported(rep, hdr);
+    ws_header* const rep = report_of(hdr, stream);
     for (int p = 0; p < num_passes; ++p) {
       char* lb = lb0 + lb_bytes * p;
       timed_launch tl(KID_ONESWEEP, stream);
@@ -814,7 +813,7 @@ cudaError_t radix_sort_async(UK* keys_a, UK* keys_b, UV* vals_a, UV* vals_b, siz
       else
         e = launch_after(k64, grid, ONESWEEP_BLOCK, smem, stream, keys_a, keys_b, vals_a, vals_b, (unsigned)n, coding, first_pass + p, first_pass, ctrl,
                          reinterpret_cast<unsigned long long*>(lb), rep);
-      if (e != cudaSuccess) return e;
+      if (reported(e, rep, hdr) != cudaSuccess) return e;
       log_launch("onesweep_kernel", grid, ONESWEEP_BLOCK, smem, n, stream);
     }
     return cudaSuccess;

@@ -40,7 +40,7 @@ __device__ __forceinline__ opt<AccT> block_reduce_opt(opt<AccT> x, Op op, opt<Ac
 template <class InIt, class AccT, class Op, int VEC>
 __global__ void __launch_bounds__(REDUCE_BLOCK)
 reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* partial_has,
-              ws_header* hdr, AccT* out, bool one_cluster) {
+              ws_header* hdr, AccT* out, AccT* rep_out, bool one_cluster) {
   if (one_cluster && gridDim.x > 1) cluster_arrive_started();
   TB200_SHARED_ARRAY(opt<AccT>, smem, 32);
   __shared__ bool is_last;
@@ -110,7 +110,10 @@ reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* par
         if (blockIdx.x == 0 && threadIdx.x == 0)
           for (unsigned q = 0; q < gridDim.x; ++q) if (has_total[q]) all.append(totals[q], op);
       }
-      if (blockIdx.x == 0 && threadIdx.x == 0) *out = all.has ? op(init, all.v) : init;
+      if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *out = all.has ? op(init, all.v) : init;
+        if (rep_out) *rep_out = *out;
+      }
       return;
     }
   }
@@ -133,6 +136,7 @@ reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* par
   f = block_reduce_opt(f, op, smem);
   if (threadIdx.x == 0) {
     *out = f.has ? op(init, f.v) : init;
+    if (rep_out) *rep_out = *out;
     hdr->ticket = 0;
   }
 }
@@ -162,13 +166,11 @@ cudaError_t reduce_async(InIt in, size_t n, AccT init, Op op, AccT* d_out, void*
   ws_header* hdr = reinterpret_cast<ws_header*>(base);
   AccT* partials = reinterpret_cast<AccT*>(base + sizeof(ws_header));
   unsigned* has = reinterpret_cast<unsigned*>(base + sizeof(ws_header) + align_up(REDUCE_MAX_GRID * sizeof(AccT), 256));
-  // a result inside the header is reported with it
-  ws_header* const rep = report_of(hdr);
-  char* const out_at = reinterpret_cast<char*>(d_out);
-  if (rep != hdr && out_at >= base && out_at < base + sizeof(ws_header)) {
-    d_out = reinterpret_cast<AccT*>(reinterpret_cast<char*>(rep) + (out_at - base));
-    reported(rep, hdr);
-  }
+  // a result behind the header's own fields is reported too (of 8 bytes at most; its room in the report is 8 bytes whatever its size)
+  constexpr size_t RESULT = offsetof(ws_header, aux) + sizeof(unsigned long long);
+  ws_header* const rep = sizeof(AccT) <= 8 && reinterpret_cast<char*>(d_out) == base + RESULT ? report_of(hdr, stream) : hdr;
+  AccT* const rep_out = rep != hdr ? reinterpret_cast<AccT*>(reinterpret_cast<char*>(rep) + RESULT) : nullptr;
+  auto with_result = [&](cudaError_t e) { return reported(e, rep, hdr, RESULT + 8); };
   auto launch = [&](auto vec_tag) -> cudaError_t {
     constexpr int VEC = decltype(vec_tag)::value;
     auto kern = reduce_kernel<InIt, AccT, Op, VEC>;
@@ -180,16 +182,16 @@ cudaError_t reduce_async(InIt in, size_t n, AccT init, Op op, AccT* d_out, void*
       bool launched = false;
       unsigned ctas = cluster_ctas((work_items + per_cta - 1) / per_cta);
       if (ctas == 0) ctas = CLUSTER_MAX_CTAS;
-      const cudaError_t e = cluster_launch(kern, ctas, REDUCE_BLOCK, 0, stream, largest, launched, in, n, init, op, partials, has, hdr, d_out, true);
-      if (launched) log_launch(name, ctas, REDUCE_BLOCK, 0, n, stream);
+      const cudaError_t e = cluster_launch(kern, ctas, REDUCE_BLOCK, 0, stream, largest, launched, in, n, init, op, partials, has, hdr, d_out, rep_out, true);
+      if (launched) { with_result(e); log_launch(name, ctas, REDUCE_BLOCK, 0, n, stream); }
       if (launched || e != cudaSuccess) return e;
     }
     const cudaError_t e = cudaMemsetAsync(hdr, 0, sizeof(ws_header), stream);
     if (e != cudaSuccess) return e;
     const int grid = reduce_grid(work_items);
-    kern<<<grid, REDUCE_BLOCK, 0, stream>>>(in, n, init, op, partials, has, hdr, d_out, false);
+    kern<<<grid, REDUCE_BLOCK, 0, stream>>>(in, n, init, op, partials, has, hdr, d_out, rep_out, false);
     log_launch(name, grid, REDUCE_BLOCK, 0, n, stream);
-    return cudaGetLastError();
+    return with_result(cudaGetLastError());
   };
   if constexpr (std::is_pointer<InIt>::value) {
     using In = typename std::remove_cv<typename std::remove_pointer<InIt>::type>::type;

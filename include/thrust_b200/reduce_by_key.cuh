@@ -238,19 +238,18 @@ cudaError_t reduce_by_key_async(KeyIt keys, ValIt vals, KeyOutIt keys_out, ValOu
     auto kern = reduce_by_key_kernel<KeyIt, ValIt, KeyOutIt, ValOutIt, K, V, Eq, Op, Off, VEC, IPT>;
     const size_t smem = (rbk_tile_items<K, V>() * sizeof(K) + 15) / 16 * 16 + rbk_tile_items<K, V>() * sizeof(V);
     if (smem > 48 * 1024 && (e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return;
-    ws_header* const rep = report_of(hdr);
+    ws_header* const rep = report_of(hdr, stream);
     timed_launch tl(KID_REDUCE_BY_KEY, stream);
     if (ctas) {
       static thread_local unsigned largest[64] = {0};
       bool launched = false;
       e = cluster_launch(kern, ctas, RBK_BLOCK, smem, stream, largest, launched, keys, vals, keys_out, vals_out, n, eq, op, ts, hdr, rep, d_count, true);
-      if (launched && e == cudaSuccess) reported(rep, hdr);
+      if (launched) reported(e, rep, hdr);
       if (launched || e != cudaSuccess) return;
     }
     if ((e = clear()) != cudaSuccess) return;
-    reported(rep, hdr);
     kern<<<(unsigned)tiles, RBK_BLOCK, smem, stream>>>(keys, vals, keys_out, vals_out, n, eq, op, ts, hdr, rep, d_count, false);
-    e = cudaGetLastError();
+    e = reported(cudaGetLastError(), rep, hdr);
   };
   constexpr bool ptrs = std::is_pointer<KeyIt>::value && std::is_pointer<ValIt>::value;
   bool use_vec = false;

@@ -329,10 +329,10 @@ cudaError_t rbk_pipe_launch(const K* keys, const V* vals, K* keys_out, V* vals_o
   cudaError_t e = pipe_clear(base, sizeof(ws_header) + rbk_chain<V, Op>::bytes(tiles), stream);
   if (e != cudaSuccess) return e;
   timed_launch tl(KID_REDUCE_BY_KEY, stream);
-  ws_header* const rep = report_of(hdr);
+  ws_header* const rep = report_of(hdr, stream);
   e = pipe_launch(kern, grid, smem, stream, keys, vals, keys_out, vals_out, n, (unsigned)tiles, eq, chain, hdr, rep, d_count);
   if (launch_refused(e)) return cudaSuccess;
-  reported(rep, hdr);
+  reported(e, rep, hdr);
   launched = true;
   log_launch("rbk_pipe_kernel", grid, PIPE_BLOCK, smem, n, stream);
   return e;

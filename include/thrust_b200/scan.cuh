@@ -454,7 +454,7 @@ cudaError_t scan_async(InIt in, OutIt out, size_t n, T init, bool has_init, Op o
   }
   tile_state<T> ts;
   ts.bind(base + sizeof(ws_header), tiles + 1);
-  ws_header* const rep = report_of(hdr);
+  ws_header* const rep = report_of(hdr, stream);
   auto launch = [&](auto vec_tag) -> cudaError_t {
     constexpr int VEC = decltype(vec_tag)::value;
     auto kern = scan_kernel<InIt, OutIt, T, Op, INCLUSIVE, VEC, IPT>;
@@ -465,7 +465,7 @@ cudaError_t scan_async(InIt in, OutIt out, size_t n, T init, bool has_init, Op o
       static thread_local unsigned largest[64] = {0};
       bool launched = false;
       const cudaError_t e = cluster_launch(kern, ctas, SCAN_BLOCK, 0, stream, largest, launched, in, out, n, init, has_init, d_init, op, ts, hdr, rep, true);
-      if (launched) { reported(rep, hdr); log_launch(name, ctas, SCAN_BLOCK, 0, n, stream); }
+      if (launched) { reported(e, rep, hdr); log_launch(name, ctas, SCAN_BLOCK, 0, n, stream); }
       if (launched || e != cudaSuccess) return e;
     }
     cudaError_t e = cudaMemsetAsync(base, 0, sizeof(ws_header) + tile_state<T>::bytes(tiles + 1), stream);
@@ -473,10 +473,9 @@ cudaError_t scan_async(InIt in, OutIt out, size_t n, T init, bool has_init, Op o
 #ifdef TB200_TEST_HOOKS
     if (test_hook_flags() & 1u) { if ((e = cudaMemsetAsync(&hdr->flags, 1, 1, stream)) != cudaSuccess) return e; }
 #endif
-    reported(rep, hdr);
     kern<<<(unsigned)tiles, SCAN_BLOCK, 0, stream>>>(in, out, n, init, has_init, d_init, op, ts, hdr, rep, false);
     log_launch(name, tiles, SCAN_BLOCK, 0, n, stream);
-    return cudaGetLastError();
+    return reported(cudaGetLastError(), rep, hdr);
   };
   if constexpr (ptrs) {
     using In = typename std::remove_cv<typename std::remove_pointer<InIt>::type>::type;

@@ -165,10 +165,10 @@ cudaError_t scan_pipe_launch(const T* in, T* out, size_t n, T init, bool has_ini
   cudaError_t e = pipe_clear(base, sizeof(ws_header) + tile_chain<T, Op>::bytes(tiles), stream);
   if (e != cudaSuccess) return e;
   timed_launch tl(KID_SCAN, stream);
-  ws_header* const rep = report_of(hdr);
+  ws_header* const rep = report_of(hdr, stream);
   e = pipe_launch(kern, grid, smem, stream, in, out, n, (unsigned)tiles, init, has_init, d_init, chain, rep);
   if (launch_refused(e)) return cudaSuccess;
-  reported(rep, hdr);
+  reported(e, rep, hdr);
   launched = true;
   log_launch("scan_pipe_kernel", grid, PIPE_BLOCK, smem, n, stream);
   return e;

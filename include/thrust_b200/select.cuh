@@ -240,20 +240,19 @@ cudaError_t select_async(InIt in, StIt stencil, SelIt out_sel, RejIt out_rej, si
     constexpr int VEC = decltype(vec_tag)::value;
     tile_state<Off> ts;
     ts.bind(base + sizeof(ws_header), tiles + 1);
-    ws_header* const rep = report_of(hdr);
+    ws_header* const rep = report_of(hdr, stream);
     auto kern = select_kernel<MODE, KEEP_REJECTS, InIt, StIt, SelIt, RejIt, T, Pred, Off, VEC, IPT>;
     timed_launch tl(KID_SELECT, stream);
     if (ctas) {
       static thread_local unsigned largest[64] = {0};
       bool launched = false;
       e = cluster_launch(kern, ctas, SELECT_BLOCK, 0, stream, largest, launched, in, stencil, out_sel, out_rej, n, pred, ts, hdr, rep, d_count, mirrored, true);
-      if (launched && e == cudaSuccess) reported(rep, hdr);
+      if (launched) reported(e, rep, hdr);
       if (launched || e != cudaSuccess) return;
     }
     if ((e = clear()) != cudaSuccess) return;
-    reported(rep, hdr);
     kern<<<(unsigned)tiles, SELECT_BLOCK, 0, stream>>>(in, stencil, out_sel, out_rej, n, pred, ts, hdr, rep, d_count, mirrored, false);
-    e = cudaGetLastError();
+    e = reported(cudaGetLastError(), rep, hdr);
   };
   constexpr bool vec_ok = std::is_pointer<InIt>::value && std::is_arithmetic<T>::value && (sizeof(T) == 4 || sizeof(T) == 8) && MODE != SEL_STENCIL;
   bool use_vec = false;

@@ -255,10 +255,10 @@ cudaError_t select_pipe_launch(const T* in, T* out_sel, T* out_rej, size_t n, Pr
   cudaError_t e = pipe_clear(base, sizeof(ws_header) + tile_chain<unsigned long long, plus_op>::bytes(tiles), stream);
   if (e != cudaSuccess) return e;
   timed_launch tl(KID_SELECT, stream);
-  ws_header* const rep = report_of(hdr);
+  ws_header* const rep = report_of(hdr, stream);
   e = pipe_launch(kern, grid, smem, stream, in, out_sel, out_rej, n, (unsigned)tiles, pred, chain, hdr, rep, d_count);
   if (launch_refused(e)) return cudaSuccess;
-  reported(rep, hdr);
+  reported(e, rep, hdr);
   launched = true;
   log_launch("select_pipe_kernel", grid, PIPE_BLOCK, smem, n, stream);
   return e;

@@ -24,12 +24,17 @@ inline size_t dtype_size(int t) {
   return 0;
 }
 
+// A call on workspace d_ws begins in this thread: if it is the one that tb200_workspace_watch announced, its kernels may report to the
+// thread's pinned block; if that one has already been made, the announcement is over (abi_reduce.cu).
+void call_begins(const void* d_ws);
+
 // Size query / size check shared by every entry point.  Returns true when the caller only asked
 // for the size (or passed too little) and `rc` holds the value to return.
 inline bool workspace_gate(void* d_ws, size_t* ws_bytes, size_t need, int& rc) {
   if (!ws_bytes) { rc = ERR_INVALID; return true; }
   if (!d_ws) { *ws_bytes = need; rc = 0; return true; }
   if (*ws_bytes < need) { rc = ERR_INVALID; return true; }
+  if (tb200::thread_report().ws == d_ws) call_begins(d_ws);
   return false;
 }
 

@@ -8,40 +8,74 @@ using namespace tb200_abi;
 TB200_API int tb200_version(void) { return 100; }
 TB200_API int tb200_sm_arch(void) { return 100; }
 
-TB200_API int tb200_workspace_status(const void* d_ws, tb200_stream_t stream, unsigned* h_status) {
-  if (!d_ws || !h_status) return ERR_INVALID;
-  cudaError_t e = cudaMemcpyAsync(h_status, d_ws, sizeof(unsigned), cudaMemcpyDeviceToHost, stream);
-  if (e != cudaSuccess) return (int)e;
-  return (int)cudaStreamSynchronize(stream);
-}
-
 namespace {
 
-// One pinned header's worth per host thread, which kernels can write to (host_report) and copies can land in: a read-back into
-// pageable memory is staged by the driver first.  give_up(): the block of a call that failed half-way may still be written to by what it
-// did launch; it is not used again and freed with the thread.
-struct pinned_header {
-  tb200::ws_header* p = nullptr;
-  std::vector<void*> old;
-  tb200::ws_header* get() {
+// Pinned memory of a host thread: the block that an announced call's kernels write to (host_report), and room for copies of headers (a
+// read-back into pageable memory is staged by the driver first).  A block whose call was never read may still be written to: it is
+// retired, not used again, and freed with the thread once the device is idle.  When RETIRED_MAX blocks have gone that way the
+// thread's calls are no longer announced.
+struct pinned_headers {
+  static constexpr size_t RETIRED_MAX = 16;
+  struct retired_block { tb200::ws_header* p; int device; };
+  tb200::ws_header* report = nullptr;
+  tb200::ws_header* staging = nullptr;
+  int device = 0;                    // on which the announced call's kernels run
+  std::vector<retired_block> retired;
+
+  static tb200::ws_header* get(tb200::ws_header*& p) {
     void* q = nullptr;
     if (!p && cudaHostAlloc(&q, sizeof(tb200::ws_header), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) p = static_cast<tb200::ws_header*>(q);
     else if (!p) cudaGetLastError();
     return p;
   }
-  void give_up() { old.push_back(p); p = nullptr; }
-  ~pinned_header() { if (p) cudaFreeHost(p); for (void* q : old) cudaFreeHost(q); }
+  void retire() { retired.push_back({report, device}); report = nullptr; }
+  ~pinned_headers() {
+    if (tb200::thread_report().bytes) retire();
+    if (staging) cudaFreeHost(staging);
+    if (report) cudaFreeHost(report);
+    int current = 0;
+    if (retired.empty() || cudaGetDevice(&current) != cudaSuccess) return;
+    for (const retired_block& b : retired)
+      if (cudaSetDevice(b.device) == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess) cudaFreeHost(b.p);
+    cudaSetDevice(current);
+  }
 };
-thread_local pinned_header pinned;
+thread_local pinned_headers pinned;
+
+// The announcement ends; a block that kernels may still write to is put aside.
+void end_announcement() {
+  tb200::host_report& r = tb200::thread_report();
+  if (r.bytes) pinned.retire();
+  r = tb200::host_report();
+}
+
+// What the announced call has left in the block, once the stream is idle, as part of the header that was read to h_dst
+void overlay_report(void* h_dst, size_t bytes) {
+  const tb200::host_report& r = tb200::thread_report();
+  if (bytes >= sizeof(unsigned) && r.block->error != tb200::ERR_NONE) memcpy(h_dst, &r.block->error, sizeof(unsigned));
+}
 
 }  // namespace
 
-TB200_API int tb200_workspace_watch(const void* d_ws) {
+void tb200_abi::call_begins(const void*) {
   tb200::host_report& r = tb200::thread_report();
-  if (r.served) pinned.give_up();            // watched and launched, but never read
-  r = tb200::host_report();
-  if (!d_ws) return 0;
-  tb200::ws_header* const block = pinned.get();
+  if (r.begun) end_announcement();
+  else r.begun = true;
+}
+
+TB200_API int tb200_workspace_status(const void* d_ws, tb200_stream_t stream, unsigned* h_status) {
+  if (!d_ws || !h_status) return ERR_INVALID;
+  cudaError_t e = cudaMemcpyAsync(h_status, d_ws, sizeof(unsigned), cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  const tb200::host_report& r = tb200::thread_report();
+  if (e == cudaSuccess && r.bytes && r.ws == d_ws) overlay_report(h_status, sizeof(unsigned));
+  return (int)e;
+}
+
+TB200_API int tb200_workspace_watch(const void* d_ws) {
+  end_announcement();
+  if (!d_ws || pinned.retired.size() >= pinned_headers::RETIRED_MAX || cudaGetDevice(&pinned.device) != cudaSuccess) return 0;
+  tb200::ws_header* const block = pinned_headers::get(pinned.report);
   void* mapped = nullptr;
   // (where the device sees the block at another address than the host, calls report through their workspaces)
   if (!block || cudaHostGetDevicePointer(&mapped, block, 0) != cudaSuccess || mapped != block) { cudaGetLastError(); return 0; }
@@ -49,6 +83,7 @@ TB200_API int tb200_workspace_watch(const void* d_ws) {
 #ifdef TB200_TEST_HOOKS
   block->flags = tb200::test_hook_flags() & 3u;
 #endif
+  tb200::host_report& r = tb200::thread_report();
   r.ws = d_ws;
   r.block = block;
   return 0;
@@ -57,12 +92,23 @@ TB200_API int tb200_workspace_watch(const void* d_ws) {
 TB200_API int tb200_workspace_read(const void* d_ws, size_t bytes, void* h_dst, tb200_stream_t stream) {
   if (!d_ws || !h_dst || bytes > sizeof(tb200::ws_header)) return ERR_INVALID;
   tb200::host_report& r = tb200::thread_report();
-  const bool there = r.served && r.ws == d_ws;   // the watched call's kernels write what is asked for to the block
-  void* const via = pinned.get();
-  cudaError_t e = there ? cudaSuccess : cudaMemcpyAsync(via ? via : h_dst, d_ws, bytes, cudaMemcpyDeviceToHost, stream);
+  const bool announced = r.bytes && r.ws == d_ws;
+  const void* from = announced ? r.block : nullptr;
+  cudaError_t e = cudaSuccess;
+  if (!announced || bytes > r.bytes) {           // more than the announced call's kernels leave in the block
+    from = pinned_headers::get(pinned.staging);
+    e = cudaMemcpyAsync(from ? pinned.staging : h_dst, d_ws, bytes, cudaMemcpyDeviceToHost, stream);
+  }
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-  if (e == cudaSuccess && via) memcpy(h_dst, via, bytes);
-  if (e != cudaSuccess && r.served) pinned.give_up();
+  if (e == cudaSuccess && from) memcpy(h_dst, from, bytes);
+  if (r.ws != d_ws) return (int)e;               // another workspace's announcement stands
+  if (e != cudaSuccess) { end_announcement(); return (int)e; }
+  if (announced) {
+    overlay_report(h_dst, bytes);
+    // a later look at the workspace finds an error there too
+    if (r.block->error != tb200::ERR_NONE && cudaMemcpyAsync(const_cast<void*>(d_ws), r.block, sizeof(unsigned), cudaMemcpyHostToDevice, stream) == cudaSuccess)
+      e = cudaStreamSynchronize(stream);
+  }
   r = tb200::host_report();
   return (int)e;
 }
