@@ -39,7 +39,7 @@ template <class T> __device__ __forceinline__ void stash(T* slot, const T& v) {
 }
 
 // Error codes a kernel may leave in the workspace status word (see ws_header).
-enum : unsigned { ERR_NONE = 0, ERR_LOOKBACK_TIMEOUT = 1, ERR_INCONSISTENT = 2 };   // 2: two evaluations of a tile disagree
+enum : unsigned { ERR_NONE = 0, ERR_LOOKBACK_TIMEOUT = 1, ERR_INCONSISTENT = 2 };   // 2: two looks at a tile disagree
 inline const char* error_text(unsigned code) {
   return code == ERR_LOOKBACK_TIMEOUT ? "thrust_b200: an inter-CTA wait ran out"
        : code == ERR_INCONSISTENT ? "thrust_b200: two looks at a tile disagree (a functor that does not answer the same twice, or is no order on the data)"

@@ -1,8 +1,8 @@
 // Stream compaction of large contiguous inputs on sm_100a on the tile pipeline (tile_pipe.cuh): copy_if,
 // partition_copy, the in-place partition and unique_copy, for 4- and 8-byte arithmetic types.
 //
-// The compute warps count what their part of a tile keeps some tiles ahead and hold its flags in a register; once the number of items
-// kept before the tile is known they compact their part in place --
+// The compute warps count what their part of a tile keeps some tiles ahead and hold its flags in a register (the in-place partition
+// finds them again); once the number of items kept before the tile is known they compact their part in place --
 // kept items first, dropped ones in a second round --, shifted so that 16-byte pieces in shared memory are
 // 16-byte pieces of the output, and store it with one 16-byte store per lane.  The input is read from HBM once.
 //
@@ -123,13 +123,15 @@ select_pipe_kernel(const T* in, T* out_sel, T* out_rej, size_t n, unsigned tiles
         }
         load_items(s, x);
         const unsigned bits = flags_of(tile, edge, x);
-        flags.put(bits);
+        if constexpr (!IN_PLACE) flags.put(bits);
         return __reduce_add_sync(FULL_MASK, (unsigned)__popc(bits));
       },
       [&](unsigned s, unsigned tile) {
         T x[PIPE_ROWS][VEC];
         load_items(s, x);
-        const unsigned bits = flags.take();
+        // In place, where a store may hit what another tile is read from, the flags are those of the items as they are now, and
+        // what they keep is checked against the count below (2^27 int32: kernel 267 to 269 us, 264 to 265 with held flags and no such check).
+        const unsigned bits = IN_PLACE ? flags_of(tile, T(), x) : flags.take();
         T* const buf = Parts::part(stages + (size_t)s * Parts::BYTES, mine);
         __syncwarp();   // every lane has its items: the part may be overwritten
         // kept items before this lane in each row: a scan over the lanes carries four rows' counts, a byte each
@@ -152,7 +154,8 @@ select_pipe_kernel(const T* in, T* out_sel, T* out_rej, size_t n, unsigned tiles
         unsigned row_off = 0;
 #pragma unroll
         for (int q = 0; q < PIPE_ROWS / 4; ++q) row_off += (totals[q] & 255) + ((totals[q] >> 8) & 255) + ((totals[q] >> 16) & 255) + (totals[q] >> 24);
-        // what is stored lies inside the output: a broken carry is reported and nothing is stored
+        // What is stored lies inside the output and is what was counted, else it is reported and nothing is stored: the flags held are
+        // those of this stage and the carry leaves room.
         if (row_off != st.part[s][mine] || kept0 > first || row_off > part_n) {
           if (lane == 0) record_error(&rep->error, ERR_INCONSISTENT);
           return;

@@ -72,3 +72,19 @@ def test_waits_of_the_pipelines_and_the_merge_run_out(tb, tmp_path):
     assert r.returncode == 0, r.stdout + r.stderr
     r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "all checks passed" in r.stdout, r.stdout + r.stderr
+
+
+def test_a_second_look_that_disagrees_is_reported(tb, tmp_path):
+    """tests/cpp/predicate_twice_test.cu: the in-place partition looks at its items again before it stores over its input."""
+    import shutil
+    import subprocess
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.isfile(nvcc):
+        pytest.skip("nvcc is not available on this machine")
+    exe = str(tmp_path / "predicate_twice_test")
+    r = subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O2", "-I" + os.path.join(root, "include"),
+                        os.path.join(root, "tests", "cpp", "predicate_twice_test.cu"), "-o", exe], capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stdout + r.stderr
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "all checks passed" in r.stdout, r.stdout + r.stderr
