@@ -171,8 +171,13 @@ inline unsigned gsort_ctas(size_t n) {
 // 400 k, f32 keys 37 / 53, 41 / 61, 49 / 62 (a million: 67 / 73); u64 of 40 bits + u32 66 / 77 at 100 k, 75 / 80 at 262 k,
 // 92 / 84 at 400 k; i64 + i64 70 / 91, 84 / 101, 105 / 111.
 template <int KB, int VB> constexpr size_t gsort_max_items() { return (KB <= 4 ? (size_t)448 : (size_t)288) << 10; }
-// scratch behind the header
-template <int KB, int VB> size_t gsort_workspace_bytes(size_t n) { return n <= gsort_max_items<KB, VB>() ? gsort_table_bytes(gsort_ctas(n)) : 0; }
+// Scratch behind the header: the table of as many CTAs as any input of up to n items has here, so that what was asked for a large input
+// is enough for every smaller one.
+template <int KB, int VB> size_t gsort_workspace_bytes(size_t n) {
+  const size_t most = gsort_max_items<KB, VB>(), sms = (size_t)current_device_info().sm_count;
+  const size_t of_two_rows = ((n < most ? n : most) + 2 * GSORT_BLOCK - 1) / (2 * GSORT_BLOCK);
+  return gsort_table_bytes(of_two_rows < sms ? of_two_rows : sms);
+}
 
 // Launches the sort if the input is small enough and the device can hold its CTAs (launched = true).
 template <class UK, class UV, bool HAS_V, bool IS_FLOAT, int IPT>

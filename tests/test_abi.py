@@ -46,6 +46,21 @@ def test_size_queries_need_no_gpu():
     assert lib.tb200_reduce(None, 8, 4, 6, 0, None, None, None, None, None) == 1                      # no size pointer
 
 
+@pytest.mark.parametrize("key_t", range(10))
+@pytest.mark.parametrize("val_bytes", [0, 4, 8])
+def test_scratch_for_a_large_sort_serves_every_smaller_one(key_t, val_bytes):
+    """A caller that sizes its scratch once, for its largest input: sizes around the limits of the sort's routes and in steps between them."""
+    from thrust_b200 import _lib
+    lib = _lib.load()
+    limits = [148 * 1024, 148 * 2048, 32 << 10, 56 << 10, 256 << 10, 288 << 10, 448 << 10, 1 << 26, 1 << 30]
+    sizes = sorted({max(1, x + d) for x in limits for d in (-1, 0, 1)} | {int(1.02 ** i) for i in range(1, 1080)})
+    need, before = ctypes.c_size_t(0), 0
+    for n in sizes:
+        assert lib.tb200_sort_by_key(None, None, None, None, n, key_t, val_bytes, 0, 0, 8, None, ctypes.byref(need), None) == 0
+        assert need.value >= before, n
+        before = need.value
+
+
 def test_missing_library_fails_loudly(monkeypatch):
     from thrust_b200 import _lib
     monkeypatch.setattr(_lib, "_lib", None)
