@@ -1,8 +1,8 @@
 // Single-pass device-wide reduction for sm_100a.
 //
-// Up to 512 KB: one launch of one cluster, whose CTAs store their totals into the first one's shared memory; nothing to clear.  A call
+// Small inputs: one launch of one cluster, whose CTAs store their totals into the first one's shared memory; nothing to clear.  A call
 // and the wait for it: 1000 int32 9.8 us against 12.5 with partials, ticket and clearing launch, 65 k 11.5 against 13.0, 131 k
-// 11.8 against 13.4.  Larger inputs:
+// 11.8 against 13.4.  reduce_cluster says where it ends.  Larger inputs:
 // One launch: a grid sized to the SM count streams the input with 16-byte evict-first loads
 // (four in flight per thread), folds it with warp shuffles, and the last CTA to finish (found
 // with an atomic ticket) folds the per-CTA partials and `init` into the result.  Replaces the
@@ -141,8 +141,17 @@ reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* par
   }
 }
 
-// Up to which input one cluster of up to 16 CTAs does it, without partials, ticket and the launch that clears them.
-constexpr size_t REDUCE_CLUSTER_BYTES = (size_t)1 << 19;
+// Up to how many vectors (or items behind an iterator) one cluster of up to 16 CTAs does it, without partials, ticket and the launch that
+// clears them, and how many of them a thread takes: one where a step may cost something (an iterator that computes or gathers, a caller's
+// operator), which is what the grid gives it too; as many as are read at a time where it is an addition or a comparison, up to 512 KB.
+// A transform of 2000 dependent multiply-adds, a call and the wait for it, here / when 16 items a thread and 512 KB went for all: 4000 items
+// 15 us / 77, 65 k 18 / 78, 131 k 23 / 145; item & 7 behind an iterator 65 k 13.6 / 11.5 (the grid then clears its header first).
+template <class AccT, class Op, int VEC> struct reduce_cluster {
+  static constexpr bool SHORT_STEP = VEC > 0 && std::is_arithmetic<AccT>::value &&
+                                     (std::is_same<Op, plus_op>::value || std::is_same<Op, min_op>::value || std::is_same<Op, max_op>::value);
+  static constexpr size_t MOST = SHORT_STEP ? ((size_t)1 << 19) / sizeof(vec16) : (size_t)CLUSTER_MAX_CTAS * REDUCE_BLOCK;
+  static constexpr size_t PER_CTA = (size_t)REDUCE_BLOCK * (SHORT_STEP ? REDUCE_UNROLL : 1);
+};
 
 inline int reduce_grid(size_t work_items /* vectors or elements */) {
   const device_info& di = current_device_info();
@@ -175,12 +184,13 @@ cudaError_t reduce_async(InIt in, size_t n, AccT init, Op op, AccT* d_out, void*
     constexpr int VEC = decltype(vec_tag)::value;
     auto kern = reduce_kernel<InIt, AccT, Op, VEC>;
     const char* const name = VEC > 0 ? "reduce_kernel (16-byte loads)" : "reduce_kernel (generic iterator)";
-    const size_t work_items = VEC > 0 ? n / (VEC > 0 ? VEC : 1) : n, per_cta = (size_t)REDUCE_BLOCK * (VEC > 0 ? REDUCE_UNROLL : REDUCE_UNROLL_GENERIC);
+    using Cluster = reduce_cluster<AccT, Op, VEC>;
+    const size_t work_items = VEC > 0 ? n / (VEC > 0 ? VEC : 1) : n;
     timed_launch tl(KID_REDUCE, stream);
-    if (cluster_storable<AccT>::value && work_items * (VEC > 0 ? 16 : sizeof(AccT)) <= REDUCE_CLUSTER_BYTES) {
+    if (cluster_storable<AccT>::value && work_items <= Cluster::MOST) {
       static thread_local unsigned largest[64] = {0};
       bool launched = false;
-      unsigned ctas = cluster_ctas((work_items + per_cta - 1) / per_cta);
+      unsigned ctas = cluster_ctas((work_items + Cluster::PER_CTA - 1) / Cluster::PER_CTA);
       if (ctas == 0) ctas = CLUSTER_MAX_CTAS;
       const cudaError_t e = cluster_launch(kern, ctas, REDUCE_BLOCK, 0, stream, largest, launched, in, n, init, op, partials, has, hdr, d_out, rep_out, true);
       if (launched) { with_result(e); log_launch(name, ctas, REDUCE_BLOCK, 0, n, stream); }

@@ -1,5 +1,9 @@
 """Inputs of a few tiles, which one thread-block cluster does (scan, reduce, compaction, reduce_by_key): both sides of one tile, of
 cluster sizes that are no power of two, of the largest cluster; aligned and not."""
+import os
+import shutil
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -60,3 +64,17 @@ def test_reduce_by_key(tb, port, kt, vt, place):
                 gk, gv = tb.reduce_by_key(place(k), place(v), op=op)
                 wk, wv = port.reduce_by_key(k, v, op)
                 assert np.array_equal(host(gk), wk) and np.array_equal(host(gv), wv), (n, op)
+
+
+def test_small_reductions_are_spread_over_threads(tmp_path):
+    """tests/cpp/reduce_spread_test.cu: items behind an iterator that computes, and a caller's operator, up to and past a cluster's size."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.isfile(nvcc):
+        pytest.skip("nvcc is not available on this machine")
+    exe = str(tmp_path / "reduce_spread_test")
+    r = subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O2", "-I" + os.path.join(root, "include"),
+                        os.path.join(root, "tests", "cpp", "reduce_spread_test.cu"), "-o", exe], capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stdout + r.stderr
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "all checks passed" in r.stdout, r.stdout + r.stderr
