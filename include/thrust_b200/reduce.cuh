@@ -34,6 +34,20 @@ __device__ __forceinline__ opt<AccT> block_reduce_opt(opt<AccT> x, Op op, opt<Ac
   return r;  // valid in thread 0
 }
 
+// Up to how many vectors (or items behind an iterator) one cluster of up to 16 CTAs does it, without partials, ticket and the launch that
+// clears them, and how many of them a thread takes: one where a step may cost something (an iterator that computes or gathers, a caller's
+// operator), which is what the grid gives it too; as many as are read at a time where it is an addition or a comparison, up to 512 KB.
+// A transform of 2000 dependent multiply-adds, a call and the wait for it, here / when 16 items a thread and 512 KB went for all: 4000 items
+// 15 us / 77, 65 k 18 / 78, 131 k 23 / 145; item & 7 behind an iterator 65 k 13.6 / 11.5 (the grid then clears its header first).
+template <class AccT, class Op, int VEC> struct reduce_cluster {
+  static constexpr bool SHORT_STEP = VEC > 0 && std::is_arithmetic<AccT>::value &&
+                                     (std::is_same<Op, plus_op>::value || std::is_same<Op, min_op>::value || std::is_same<Op, max_op>::value);
+  static constexpr size_t MOST = SHORT_STEP ? ((size_t)1 << 19) / sizeof(vec16) : (size_t)CLUSTER_MAX_CTAS * REDUCE_BLOCK;
+  static constexpr int ROWS = SHORT_STEP ? (int)(MOST / (CLUSTER_MAX_CTAS * REDUCE_BLOCK)) : 1;   // what a thread takes at most
+  static_assert((size_t)ROWS * CLUSTER_MAX_CTAS * REDUCE_BLOCK == MOST, "whole rows");
+  static constexpr size_t PER_CTA = (size_t)REDUCE_BLOCK * (SHORT_STEP ? REDUCE_UNROLL : 1);
+};
+
 // In = element type read from memory (or an iterator's value), AccT = accumulator.
 // VEC = elements per 16-byte load when `in` is a 16-byte-aligned pointer to a 1/2/4/8-byte type,
 // 0 for the generic path (any random-access iterator, one element per load).
@@ -41,6 +55,7 @@ template <class InIt, class AccT, class Op, int VEC>
 __global__ void __launch_bounds__(REDUCE_BLOCK)
 reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* partial_has,
               ws_header* hdr, AccT* out, AccT* rep_out, bool one_cluster) {
+  using Cluster = reduce_cluster<AccT, Op, VEC>;
   if (one_cluster && gridDim.x > 1) cluster_arrive_started();
   TB200_SHARED_ARRAY(opt<AccT>, smem, 32);
   __shared__ bool is_last;
@@ -53,6 +68,36 @@ reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* par
     const size_t nvec = n / VEC;
     const vec16* vin = reinterpret_cast<const vec16*>(in);
     size_t v = tid;
+    if constexpr (Cluster::ROWS > 1) {
+      // Every vector a thread takes is in flight, and their sums are added up as a tree, which is what the grid's CTAs make of them.  Root mean
+      // square of the relative error of uniform 4-byte floats, here / one after the other: 19 k 4.1e-8 / 5.7e-8, 60 k 3.2e-8 / 5.7e-8, 131 k
+      // 4.3e-8 / 5.9e-8; a call and the wait 11.6 us / 11.9 at 131 k.
+      if (one_cluster) {
+        vec16 r[Cluster::ROWS];
+        opt<AccT> row[Cluster::ROWS];
+#pragma unroll
+        for (int u = 0; u < Cluster::ROWS; ++u) {
+          row[u].has = v + u * stride < nvec;
+          if (row[u].has) r[u] = load_stream16(vin + v + u * stride);
+        }
+#pragma unroll
+        for (int u = 0; u < Cluster::ROWS; ++u) {
+          if (!row[u].has) continue;
+          const In* e = reinterpret_cast<const In*>(&r[u]);
+          AccT t = (AccT)e[0];
+#pragma unroll
+          for (int k = 1; k < VEC; ++k) t = op(t, (AccT)e[k]);
+          row[u].v = t;
+        }
+#pragma unroll
+        for (int d = 1; d < Cluster::ROWS; d <<= 1) {
+#pragma unroll
+          for (int u = 0; u + d < Cluster::ROWS; u += 2 * d) row[u].append_opt(row[u + d], op);
+        }
+        acc = row[0];
+        v = nvec;
+      }
+    }
     for (; v + (REDUCE_UNROLL - 1) * stride < nvec; v += REDUCE_UNROLL * stride) {
       vec16 r[REDUCE_UNROLL];
 #pragma unroll
@@ -107,8 +152,10 @@ reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* par
         }
         cluster_barrier();
         all.has = false;
-        if (blockIdx.x == 0 && threadIdx.x == 0)
-          for (unsigned q = 0; q < gridDim.x; ++q) if (has_total[q]) all.append(totals[q], op);
+        if (blockIdx.x == 0 && threadIdx.x < 32) {
+          if (threadIdx.x < gridDim.x && has_total[threadIdx.x]) { all.v = totals[threadIdx.x]; all.has = true; }
+          all = warp_reduce_opt(all, op);
+        }
       }
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         *out = all.has ? op(init, all.v) : init;
@@ -140,18 +187,6 @@ reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* par
     hdr->ticket = 0;
   }
 }
-
-// Up to how many vectors (or items behind an iterator) one cluster of up to 16 CTAs does it, without partials, ticket and the launch that
-// clears them, and how many of them a thread takes: one where a step may cost something (an iterator that computes or gathers, a caller's
-// operator), which is what the grid gives it too; as many as are read at a time where it is an addition or a comparison, up to 512 KB.
-// A transform of 2000 dependent multiply-adds, a call and the wait for it, here / when 16 items a thread and 512 KB went for all: 4000 items
-// 15 us / 77, 65 k 18 / 78, 131 k 23 / 145; item & 7 behind an iterator 65 k 13.6 / 11.5 (the grid then clears its header first).
-template <class AccT, class Op, int VEC> struct reduce_cluster {
-  static constexpr bool SHORT_STEP = VEC > 0 && std::is_arithmetic<AccT>::value &&
-                                     (std::is_same<Op, plus_op>::value || std::is_same<Op, min_op>::value || std::is_same<Op, max_op>::value);
-  static constexpr size_t MOST = SHORT_STEP ? ((size_t)1 << 19) / sizeof(vec16) : (size_t)CLUSTER_MAX_CTAS * REDUCE_BLOCK;
-  static constexpr size_t PER_CTA = (size_t)REDUCE_BLOCK * (SHORT_STEP ? REDUCE_UNROLL : 1);
-};
 
 inline int reduce_grid(size_t work_items /* vectors or elements */) {
   const device_info& di = current_device_info();
