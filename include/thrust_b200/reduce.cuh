@@ -158,8 +158,9 @@ reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* par
         }
       }
       if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *out = all.has ? op(init, all.v) : init;
-        if (rep_out) *rep_out = *out;
+        const AccT result = all.has ? op(init, all.v) : init;
+        *out = result;
+        if (rep_out) *rep_out = result;
       }
       return;
     }
@@ -182,8 +183,9 @@ reduce_kernel(InIt in, size_t n, AccT init, Op op, AccT* partials, unsigned* par
   __syncthreads();
   f = block_reduce_opt(f, op, smem);
   if (threadIdx.x == 0) {
-    *out = f.has ? op(init, f.v) : init;
-    if (rep_out) *rep_out = *out;
+    const AccT result = f.has ? op(init, f.v) : init;
+    *out = result;
+    if (rep_out) *rep_out = result;
     hdr->ticket = 0;
   }
 }

@@ -28,6 +28,13 @@ struct pinned_headers {
     else if (!p) cudaGetLastError();
     return p;
   }
+  // The block for reports: kernels reach it under its host address (one address space of host and devices; without that there is no block).
+  tb200::ws_header* report_block() {
+    if (report || !get(report)) return report;
+    void* mapped = nullptr;
+    if (cudaHostGetDevicePointer(&mapped, report, 0) != cudaSuccess || mapped != report) { cudaGetLastError(); cudaFreeHost(report); report = nullptr; }
+    return report;
+  }
   void retire() { retired.push_back({report, device}); report = nullptr; }
   ~pinned_headers() {
     if (tb200::thread_report().bytes) retire();
@@ -75,10 +82,8 @@ TB200_API int tb200_workspace_status(const void* d_ws, tb200_stream_t stream, un
 TB200_API int tb200_workspace_watch(const void* d_ws) {
   end_announcement();
   if (!d_ws || pinned.retired.size() >= pinned_headers::RETIRED_MAX || cudaGetDevice(&pinned.device) != cudaSuccess) return 0;
-  tb200::ws_header* const block = pinned_headers::get(pinned.report);
-  void* mapped = nullptr;
-  // (where the device sees the block at another address than the host, calls report through their workspaces)
-  if (!block || cudaHostGetDevicePointer(&mapped, block, 0) != cudaSuccess || mapped != block) { cudaGetLastError(); return 0; }
+  tb200::ws_header* const block = pinned.report_block();
+  if (!block) return 0;
   memset(block, 0, sizeof(*block));
 #ifdef TB200_TEST_HOOKS
   block->flags = tb200::test_hook_flags() & 3u;
