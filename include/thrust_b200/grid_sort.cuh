@@ -20,7 +20,8 @@ namespace tb200 {
 constexpr int GSORT_BLOCK = 512;
 constexpr int GSORT_PARTS = GSORT_BLOCK / (RADIX_BINS / 2);   // in which the CTAs' counts are added up
 // Counts that a thread has in flight, the last ones of the table too: one after the other those past a multiple of 32 CTAs cost up to 1 us a
-// digit place (microseconds, 8 at a time / only whole batches so: u64 of 40 bits at 224 k 71 / 76, 70 on the general route; u64 + u32 84 / 88).
+// digit place (microseconds, now / so: u64 50 k 61 / 67, 114 k 69 / 74, 300 k 80 / 87; f32 37 / 40, 41 / 43, 44 / 47; with every batch checked
+// for the table's end up to 1 us more again).
 constexpr int GSORT_BATCH = 8;
 
 template <class Item, int IPT> constexpr size_t gsort_smem_bytes() {
@@ -123,17 +124,23 @@ grid_sort_kernel(UK* keys, UV* vals, unsigned n, unsigned rows, key_coding codin
       const unsigned part = t / (RADIX_BINS / 2), pair = t % (RADIX_BINS / 2);
       unsigned before0 = 0, before1 = 0, all0 = 0, all1 = 0;
       const unsigned* const words = reinterpret_cast<const unsigned*>(counts) + pair;
-      for (unsigned first = part; first < ctas; first += GSORT_BATCH * GSORT_PARTS) {
+      auto add_batch = [&](unsigned first, auto whole_tag) {
         unsigned w[GSORT_BATCH];
 #pragma unroll
-        for (int b = 0; b < GSORT_BATCH; ++b) { const unsigned q = first + b * GSORT_PARTS; w[b] = q < ctas ? __ldcg(words + q * (RADIX_BINS / 2)) : 0u; }
+        for (int b = 0; b < GSORT_BATCH; ++b) {
+          const unsigned q = first + b * GSORT_PARTS;
+          w[b] = decltype(whole_tag)::value || q < ctas ? __ldcg(words + q * (RADIX_BINS / 2)) : 0u;
+        }
 #pragma unroll
         for (int b = 0; b < GSORT_BATCH; ++b) {
           const unsigned c0 = w[b] & 0xffffu, c1 = w[b] >> 16;
           if (first + b * GSORT_PARTS < me) { before0 += c0; before1 += c1; }
           all0 += c0; all1 += c1;
         }
-      }
+      };
+      unsigned first = part;
+      for (; first + (GSORT_BATCH - 1) * GSORT_PARTS < ctas; first += GSORT_BATCH * GSORT_PARTS) add_batch(first, std::true_type());
+      if (first < ctas) add_batch(first, std::false_type());
       s_before[part * RADIX_BINS + 2 * pair] = before0; s_before[part * RADIX_BINS + 2 * pair + 1] = before1;
       s_total[part * RADIX_BINS + 2 * pair] = all0; s_total[part * RADIX_BINS + 2 * pair + 1] = all1;
     }
