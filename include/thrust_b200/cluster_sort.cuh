@@ -16,7 +16,7 @@
 // were two thirds of a pass: about 1.7 cycles each per SM.)  A digit place that all keys share is left out,
 // as in the general sort.  Same order, same stability.
 //
-// Measured on B200, microseconds: f32 keys 22 at 1 k, 26 at 10 k, 30 at 32 k; u32 + u32 23, 30, 36; u64 + u64 35, 44, 58.  CSORT_MAX_ITEMS says
+// Measured on B200, microseconds: f32 keys 22 at 1 k, 26 at 10 k, 30 at 32 k; u32 + u32 23, 30, 36; u64 + u64 35, 44, 58.  csort_max_items says
 // where it stops.
 #pragma once
 #include "cluster.cuh"
@@ -27,7 +27,6 @@ namespace tb200 {
 
 constexpr int CSORT_BLOCK = 512;
 constexpr int CSORT_MAX_CTAS = CLUSTER_MAX_CTAS;
-constexpr int CSORT_MAX_IPT = 4;
 
 // What moves between the CTAs: a key alone, or a key and its value in one 8- or 16-byte word.
 template <class UK, class UV, bool HAS_V> struct csort_item { using type = UK; };
@@ -35,9 +34,13 @@ template <class UK, class UV> struct csort_item<UK, UV, true> {
   struct alignas(sizeof(UK) + sizeof(UV) <= 8 ? 8 : 16) type { UV v; UK k; };
 };
 
-// Up to how many items the cluster is the faster route: four rows per warp of the largest one.  Microseconds here / in the grid sort at 20 k,
-// 32 k and 50 k: f32 keys 29 / 36, 30 / 35, 36 / 37; u32 + u32 32 / 36, 36 / 33, 43 / 37; u64 + u32 50 / 61, 56 / 57, 73 / 65.
-constexpr size_t CSORT_MAX_ITEMS = (size_t)CSORT_BLOCK * CSORT_MAX_CTAS * CSORT_MAX_IPT;
+// Up to how many items the cluster is the faster route.  Microseconds here / in the grid sort on either side of the lines: keys alone at 32 k,
+// 44 k and 56 k: f32 29 / 33, 33 / 35, 37 / 35; u64 53 / 57, 62 / 62, 69 / 61; u16 19 / 21, 22 / 22, 23 / 23; u8 14 / 15, 16 / 15, 16 / 15; u32 + u32 32 / 34,
+// 36 / 36, 40 / 36; at 28 k, 32 k and 36 k: u32 + u64 34 / 35, 36 / 35, 39 / 36; u64 + u32 59 / 61, 61 / 61, 68 / 64; u16 + u32 21 / 22, 21 / 22,
+// 23 / 23; u64 of which 40 bits vary: alone 55 / 56 at 44 k, with u32 52 / 54 at 32 k.
+template <class UK, class UV, bool HAS_V> constexpr size_t csort_max_items() {
+  return (size_t)(!HAS_V || (sizeof(UK) == 4 && sizeof(UV) == 4) ? 44 : 32) << 10;
+}
 
 template <class Item, int IPT> constexpr size_t csort_smem_bytes() {
   return 2 * (size_t)CSORT_BLOCK * IPT * sizeof(Item) + (CSORT_BLOCK / 32) * RADIX_BINS * 4 + 2 * CSORT_MAX_CTAS * RADIX_BINS * 4;
@@ -174,11 +177,18 @@ cudaError_t cluster_sort_launch(UK* keys, UV* vals, size_t n, key_coding coding,
 template <class UK, class UV, bool HAS_V>
 cudaError_t cluster_sort_async(UK* keys, UV* vals, size_t n, key_coding coding, int first_pass, int num_passes, ws_header* hdr, cudaStream_t stream, bool& launched) {
   launched = false;
-  if (n > CSORT_MAX_ITEMS) return cudaSuccess;
-  if constexpr (sizeof(UK) >= 4) {
-    if (coding.kind == KEY_FLOAT) return cluster_sort_launch<UK, UV, HAS_V, true, CSORT_MAX_IPT>(keys, vals, n, coding, first_pass, num_passes, hdr, stream, launched);
-  }
-  return cluster_sort_launch<UK, UV, HAS_V, false, CSORT_MAX_IPT>(keys, vals, n, coding, first_pass, num_passes, hdr, stream, launched);
+  constexpr size_t MOST = csort_max_items<UK, UV, HAS_V>(), ROW = (size_t)CSORT_BLOCK * CSORT_MAX_CTAS;
+  if (n > MOST) return cudaSuccess;
+  auto go = [&](auto is_float, auto ipt) {
+    return cluster_sort_launch<UK, UV, HAS_V, decltype(is_float)::value, decltype(ipt)::value>(keys, vals, n, coding, first_pass, num_passes, hdr, stream, launched);
+  };
+  auto by_rows = [&](auto is_float) {
+    if constexpr (MOST > 4 * ROW) { if (n > 4 * ROW) return go(is_float, std::integral_constant<int, 6>()); }
+    return go(is_float, std::integral_constant<int, 4>());
+  };
+  static_assert(MOST <= 6 * ROW, "rows of the largest cluster");
+  if constexpr (sizeof(UK) >= 4) { if (coding.kind == KEY_FLOAT) return by_rows(std::true_type()); }
+  return by_rows(std::false_type());
 }
 
 }  // namespace tb200
