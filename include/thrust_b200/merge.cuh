@@ -544,11 +544,13 @@ template <int KB, int VB> struct block_sort_tuning {
   static constexpr int IPT = (KB + VB) <= 8 ? TB200_BSORT_IPT8 : (FIT >= 8 ? 8 : FIT >= 4 ? 4 : FIT >= 2 ? 2 : 1);
   // one slot of padding per thread, where static shared memory has room for it (20-byte keys at 8 items: it has not)
   static constexpr int TILE = BLOCK * IPT, SMEM = 48 * 1024;
-  static constexpr int OVER = IPT + 2;   // slots that may be read past the tile's end
+  // A merge reads one slot past the tile's end at most: the first run of a pair ends a run's length or more in front of it, and a thread goes
+  // no more than its own items, which is the shortest run, past that.
+  static constexpr int OVER = 1;
   static constexpr int IDX_SLOTS = TILE + OVER;
   static constexpr bool PADDED = IPT >= 8 && (TILE + BLOCK + OVER) * KB + IDX_SLOTS * 2 + 32 <= SMEM;
   static constexpr int SLOTS = TILE + (PADDED ? BLOCK : 0) + OVER;
-  static_assert(SLOTS * KB + IDX_SLOTS * 2 <= SMEM, "key too large for the block sort tile (more than 170 bytes)");
+  static_assert(SLOTS * KB + IDX_SLOTS * 2 <= SMEM, "key too large for the block sort tile (more than 189 bytes)");
 };
 
 // What bounds it is shared memory (the pipe is busy 91 % of a large sort's tiles: 122 wavefronts per 32 items before the
