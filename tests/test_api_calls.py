@@ -20,6 +20,7 @@ class FakeLibrary:
         self.between = lambda: None       # what happens between a call's launch and its read-back
         self.launches = []
         self.result = 0                   # what the next calls return once they are past the size check
+        self.watched = []                 # what was announced, in order
 
     def _gate(self, d_ws, size):
         if d_ws is None:
@@ -50,6 +51,10 @@ class FakeLibrary:
         C.memmove(out, kept.ctypes.data, kept.nbytes)
         C.memmove(d_ws, struct.pack("<IIQ", 0, 0, kept.size), 16)
         return self._launched("copy_if")
+
+    def tb200_workspace_watch(self, d_ws):
+        self.watched.append(d_ws)
+        return 0
 
     def tb200_workspace_read(self, d_ws, nbytes, dst, stream):
         C.memmove(dst, d_ws, nbytes)
@@ -112,3 +117,17 @@ def test_a_refused_call_is_made_again_only_for_its_size(fake, name):
     api.workspaces.at(key).keep(torch.empty(NEED - 1, dtype=torch.uint8))
     call()
     assert fake.launches == [name] * 3 and api.workspaces.at(key).buf.numel() == NEED
+
+
+@pytest.mark.parametrize("name", ["reduce", "copy_if"])
+def test_a_failed_call_is_no_longer_announced(fake, name):
+    x = torch.arange(10, dtype=torch.int64)
+    call = (lambda: api.reduce(x)) if name == "reduce" else (lambda: api.copy_if(x, "ne", 3))
+    call()
+    call()
+    kept = api.workspaces.at(api.workspaces.key("reduce" if name == "reduce" else "select"))
+    assert fake.watched == [kept.ptr]              # the first call has made its workspace
+    fake.result = 700
+    with pytest.raises(api.Tb200Error):
+        call()
+    assert fake.watched == [kept.ptr, kept.ptr, None]

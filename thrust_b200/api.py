@@ -143,15 +143,14 @@ def _enqueue_and_read(key, kept, what, fn, args, nbytes=_HEADER.size, result=Non
     """_enqueue, then the first `nbytes` of the header to kept.head once the stream has got there; returns the count.  The
     read is announced, so that the kernels can leave there what it fetches."""
     lib = _lib.load()
-    watch = getattr(lib, "tb200_workspace_watch", None)
-    if watch is None or kept.ptr is None:      # the first call makes the workspace
+    if kept.ptr is None:      # the first call makes the workspace
         _enqueue(key, kept, fn, args, result)
     else:
-        watch(kept.ptr)
+        lib.tb200_workspace_watch(kept.ptr)
         try:
             _enqueue(key, kept, fn, args, result)
         except BaseException:
-            watch(None)
+            lib.tb200_workspace_watch(None)
             raise
     return _read_header(lib, kept.ptr, what, key[1], kept.head, nbytes)
 
