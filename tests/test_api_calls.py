@@ -131,3 +131,14 @@ def test_a_failed_call_is_no_longer_announced(fake, name):
     with pytest.raises(api.Tb200Error):
         call()
     assert fake.watched == [kept.ptr, kept.ptr, None]
+
+
+def test_a_workspace_that_was_replaced_is_no_longer_announced(fake):
+    """Its memory may become another call's."""
+    x = torch.arange(10, dtype=torch.int64)
+    api.reduce(x)
+    kept = api.workspaces.at(api.workspaces.key("reduce"))
+    kept.keep(torch.empty(NEED - 1, dtype=torch.uint8))
+    small = kept.ptr
+    assert int(api.reduce(x)) == 45
+    assert fake.watched == [small, None]

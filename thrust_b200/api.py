@@ -146,12 +146,15 @@ def _enqueue_and_read(key, kept, what, fn, args, nbytes=_HEADER.size, result=Non
     if kept.ptr is None:      # the first call makes the workspace
         _enqueue(key, kept, fn, args, result)
     else:
-        lib.tb200_workspace_watch(kept.ptr)
+        announced = kept.ptr
+        lib.tb200_workspace_watch(announced)
         try:
             _enqueue(key, kept, fn, args, result)
         except BaseException:
             lib.tb200_workspace_watch(None)
             raise
+        if kept.ptr != announced:      # refused there, and made in a larger one
+            lib.tb200_workspace_watch(None)
     return _read_header(lib, kept.ptr, what, key[1], kept.head, nbytes)
 
 
