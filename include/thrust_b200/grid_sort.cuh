@@ -1,4 +1,4 @@
-// Radix sort of inputs that fit the registers of the chip's CTAs (up to half a million items), in one cooperative launch.
+// Radix sort of inputs that fit the registers of the chip's CTAs (up to 448 k items, 288 k with 8-byte keys), in one cooperative launch.
 //
 // Between the cluster sort (cluster_sort.cuh: up to 16 SMs) and the general one (radix_sort.cuh: a chain of launches with look-backs between
 // tiles) lies a range where a digit place is latency, not work.  Here every CTA keeps its share of the items in registers;
@@ -182,9 +182,10 @@ inline unsigned gsort_ctas(size_t n) {
   const size_t rows = n <= sms * row * 2 ? 2 : n <= sms * row * 4 ? 4 : (n + sms * row - 1) / (sms * row);
   return (unsigned)((n + row * rows - 1) / (row * rows));
 }
-// Up to which input it is the faster route, microseconds here / on the general one: u32 + u32 39 / 61 at 100 k, 43 / 66 at 262 k, 51 / 68 at
-// 400 k, f32 keys 37 / 53, 41 / 61, 49 / 62 (a million: 67 / 73); u64 of 40 bits + u32 66 / 77 at 100 k, 75 / 80 at 262 k,
-// 92 / 84 at 400 k; i64 + i64 70 / 91, 84 / 101, 105 / 111.
+// Up to which input it is the faster route.  A call and the wait for it, microseconds here / on the general route at 160 k, 256 k, 288 k and
+// 448 k: u32 + u32 44 / 60, 44 / 62, 46 / 62, 51 / 63; u32 + u64 44 / 58, 46 / 60, 49 / 59, 56 / 62; f32 keys 40 / 61, 42 / 63, 44 / 63, 49 / 64;
+// u64 of 64 random bits + u32 80 / 102, 84 / 106, 88 / 106, 98 / 119, of 40 bits 72 / 75, 74 / 77, 80 / 78, 89 / 85.  How many bits vary is
+// not known beforehand, so the line of the 8-byte keys lies where the one loses 5 us at most (40 bits, keys alone: 76 / 71) and the other gains 16.
 template <int KB, int VB> constexpr size_t gsort_max_items() { return (KB <= 4 ? (size_t)448 : (size_t)288) << 10; }
 // Scratch behind the header: the table of as many CTAs as any input of up to n items has here, so that what was asked for a large input
 // is enough for every smaller one.

@@ -554,7 +554,7 @@ template <int KB, int VB> struct block_sort_tuning {
 };
 
 // What bounds it is shared memory (the pipe is busy 91 % of a large sort's tiles: 122 wavefronts per 32 items before the
-// indexes left in 16-byte stores, 110 since): a thread's IPT consecutive items are written and read back in every round, and
+// indexes left in 16-byte stores, 113 since): a thread's IPT consecutive items are written and read back in every round, and
 // unpadded that is a stride of IPT words, IPT / 2 lanes to a bank.  One slot of padding per IPT items makes the
 // stride odd.  Rounds whose pairs of runs lie inside one warp's items need no barrier of the CTA.  The merge takes its next
 // item without a branch: two candidates in registers, one load of the side that was taken.  With a branch for either side a

@@ -22,8 +22,8 @@
 //   4. radix_copy_back_kernel only if an odd number of places ran: moves the result from the
 //                             alternate buffer to the caller's.
 // A pass therefore reads and writes each key (and value) exactly once.  The sort is stable.
-// Inputs of up to 32 k items take one launch of one thread-block cluster instead (cluster_sort.cuh), up to 448 k one cooperative launch
-// (grid_sort.cuh).
+// Inputs of up to 32 k items (44 k: keys alone, pairs of 4-byte items) take one launch of one thread-block cluster instead (cluster_sort.cuh),
+// up to 448 k (288 k with 8-byte keys) one cooperative launch (grid_sort.cuh).
 #pragma once
 #include "cluster_sort.cuh"
 #include "common.cuh"
@@ -818,9 +818,9 @@ cudaError_t radix_sort_async(UK* keys_a, UK* keys_b, UV* vals_a, UV* vals_b, siz
     }
     return cudaSuccess;
   };
-  // Larger tiles for large inputs of 4-byte pairs: longer runs in the output, fewer descriptors (18 items per thread against 16: 2^26 pairs
-  // 1376 us against 1389, 2^27 2669 against 2720, 2^28 5246 against 5357; 2^24, where the last wave shows, 392 against 384).  The
-  // workspace is sized for the smaller tiles.
+  // Larger tiles for large inputs of 4-byte pairs: longer runs in the output, fewer descriptors (18 items per thread against 16: 2^24, where
+  // the last wave shows, 393 us against 388, 2^25 722 both, 2^25.5 994 against 1001, 2^26 1366 against 1385, 2^27 2654 against 2703, 2^28 5246
+  // against 5357).  Other widths were not tried.  The workspace is sized for the smaller tiles.
   constexpr int LARGE_IPT = KB == 4 && VB == 4 ? 18 : IPT;
   e = LARGE_IPT != IPT && n >= ONESWEEP_LARGE_MIN ? sweeps(std::integral_constant<int, LARGE_IPT>()) : sweeps(std::integral_constant<int, IPT>());
   if (e != cudaSuccess) return e;
