@@ -235,8 +235,21 @@ def test_sort_by_key_host_buffers_match_the_oracle(tb, port, n):
         assert np.array_equal(hk.numpy().view(np.uint8), wk.view(np.uint8)) and np.array_equal(hv.numpy().view(np.uint8), wv.view(np.uint8))
 
 
-@pytest.mark.parametrize("n", [32767, 32768, 32769, 40961, 45055, 45056, 45057, 81920, 114689, 288 << 10, (288 << 10) + 1, 448 << 10, (448 << 10) + 1])
+@pytest.mark.parametrize("n", [81920, 90111, 90112, 90113, 114687, 114688, 114689])
 def test_small_sorts_where_the_cluster_hands_over(tb, port, n):
+    """The last sizes of 8-byte items that one cluster sorts and the first that the general route does."""
+    for dt, vt in [(np.uint64, None), (np.float64, None), (np.uint32, np.uint32), (np.uint16, np.uint32), (np.int8, np.uint32), (np.float32, np.uint32)]:
+        for small in (False, True):
+            k = rand_of(dt, n, 58, small=small)
+            v = None if vt is None else np.arange(n, dtype=vt)
+            kd, vd = dev(k), None if v is None else dev(v)
+            tb.sort(kd) if v is None else tb.sort_by_key(kd, vd)
+            ok, ov = port.sort_by_key(k, v, False)
+            assert np.array_equal(host(kd), ok) and (v is None or np.array_equal(host(vd), ov)), (dt, vt, small)
+
+
+@pytest.mark.parametrize("n", [32767, 32768, 32769, 40961, 45055, 45056, 45057, 288 << 10, (288 << 10) + 1, 448 << 10, (448 << 10) + 1])
+def test_small_sorts_around_their_routes_limits(tb, port, n):
     """The last sizes that one cluster sorts (32 k, 44 k for keys alone and pairs of 4-byte items) and that the resident grid does (288 k with
     8-byte keys, 448 k), and the first that the next route takes."""
     for dt, vt in [(np.uint64, None), (np.float64, None), (np.uint32, np.uint32), (np.uint16, np.uint32), (np.int8, np.uint32), (np.float32, np.uint32),
