@@ -250,7 +250,8 @@ rbk_pipe_kernel(const K* keys, const V* vals, K* keys_out, V* vals_out, size_t n
         const unsigned incl = warp_inclusive_scan(packed, plus_op());
         const unsigned totals = __shfl_sync(FULL_MASK, incl, 31);
         const unsigned excl = incl - packed;
-        // what is stored lies inside the outputs (a broken carry is reported and nothing is stored)
+        // What is stored lies inside the outputs, else it is reported and nothing is stored: the heads held are those of this stage and
+        // the carry leaves room.  (A store cannot hit the input: rbk_pipe_eligible.)
         const unsigned part_heads = __reduce_add_sync(FULL_MASK, (unsigned)__popc(bits));
         if (part_heads != st.part[s][mine].heads || run0 > (size_t)tile * ITEMS + (size_t)mine * PART) {
           if (lane == 0) record_error(&rep->error, ERR_INCONSISTENT);
